@@ -23,6 +23,14 @@ __device__ __forceinline__ void nanosleep(uint32_t ns) {
   asm volatile("nanosleep.u32 %0;" ::"r"(ns));
 }
 
+// ---- overlapping launches -----------------------------------------------------
+// A kernel launched with programmatic stream serialisation may start while the kernel before it in the stream is
+// still running: nothing that kernel touches may be read or written before prior_work_done(), which waits for
+// its completion and makes its writes visible to the calling thread.  next_may_start() lets the kernel behind
+// this one be placed on SMs as they become free; it too waits before it touches memory.
+__device__ __forceinline__ void prior_work_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- mbarrier --------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");

@@ -22,6 +22,7 @@ TILE_N = 128     # weight rows per CTA
 TILE_M = 256     # activation rows per CTA
 TILE_K = 64
 
+_WORKSPACE_BYTES = 256     # what mk_gemm_bf16_workspace_bytes answers
 _workspaces: Dict[Tuple[int, int], torch.Tensor] = {}
 
 
@@ -34,7 +35,7 @@ def _check(rc: int, what: str) -> None:
 
 def gemm_workspace(M: int, N_out: int, K: int, device) -> torch.Tensor:
     """A zeroed workspace for ``gemm_sm100`` (cached per device and size; the kernel leaves it zero)."""
-    need = int(N.lib().mk_gemm_bf16_workspace_bytes(M, N_out, K))
+    need = int(N.lib().mk_gemm_bf16_workspace_bytes(M, N_out, K))    # the status block: the same for every size
     dev = torch.device(device)
     key = (dev.index if dev.index is not None else torch.cuda.current_device(), need)
     ws = _workspaces.get(key)
@@ -78,44 +79,70 @@ def gemm_sm100(a: torch.Tensor, b, c: torch.Tensor, *, activation=None, split_k:
     (``a.view(-1, K)`` must be a view).  ``check_status`` synchronises and raises if a device-side
     wait ran out.
     """
-    if not (a.is_cuda and c.is_cuda):
-        raise RuntimeError("gemm_sm100 runs on a CUDA device only; there is no CPU path")
-    if activation not in ACTIVATIONS:
-        raise ValueError(f"Unknown activation: {activation}")
     packed = isinstance(b, PackedWeight)
     bt = b.data if packed else b
-    if not bt.is_cuda:
+    if not (a.is_cuda and c.is_cuda and bt.is_cuda):
         raise RuntimeError("gemm_sm100 runs on a CUDA device only; there is no CPU path")
-    if a.dtype != torch.bfloat16 or bt.dtype != torch.bfloat16 or c.dtype != torch.bfloat16:
+    act = ACTIVATIONS.get(activation)
+    if act is None:
+        raise ValueError(f"Unknown activation: {activation}")
+    bf16 = torch.bfloat16
+    if a.dtype != bf16 or bt.dtype != bf16 or c.dtype != bf16:
         raise ValueError("gemm_sm100: a, b and c must be bfloat16")
-    K, n_out = int(a.shape[-1]), int(b.shape[0])
-    if (not packed and b.dim() != 2) or int(b.shape[1]) != K or int(c.shape[-1]) != n_out or a.shape[:-1] != c.shape[:-1]:
-        raise ValueError(f"gemm_sm100: shapes a{tuple(a.shape)} b{tuple(b.shape)} c{tuple(c.shape)} do not match"
+    sa, sb, sc = a.shape, b.shape, c.shape
+    K, n_out = sa[-1], sb[0]
+    if (not packed and len(sb) != 2) or sb[1] != K or sc[-1] != n_out or sa[:-1] != sc[:-1]:
+        raise ValueError(f"gemm_sm100: shapes a{tuple(sa)} b{tuple(sb)} c{tuple(sc)} do not match"
                          + (" (a packed weight pads K to a multiple of 64: pad the activations too)" if packed else ""))
     if a.stride(-1) != 1 or (not packed and b.stride(-1) != 1) or c.stride(-1) != 1:
         raise ValueError("gemm_sm100: K (a, b) and N (c) must be contiguous")
-    a2, c2 = a.view(-1, K), c.view(-1, n_out)          # raises if the rows are not equally spaced
-    M = int(a2.shape[0])
-    ws = workspace if workspace is not None else gemm_workspace(M, n_out, K, a.device)
-    base = (ws.data_ptr() + 255) // 256 * 256
-    stream = torch.cuda.current_stream(a.device).cuda_stream
-    with torch.cuda.device(a.device):
-        if packed:
-            _check(N.lib().mk_gemm_bf16_packed(a2.data_ptr(), bt.data_ptr(), c2.data_ptr(), M, n_out, K, a2.stride(0),
-                                               c2.stride(0), base, ws.numel() - (base - ws.data_ptr()), int(split_k),
-                                               ACTIVATIONS[activation], int(timeout_ms), C.c_void_p(stream)),
-                   "mk_gemm_bf16_packed")
-        else:
-            _check(N.lib().mk_gemm_bf16(a2.data_ptr(), b.data_ptr(), c2.data_ptr(), M, n_out, K, a2.stride(0), b.stride(0),
-                                        c2.stride(0), base, ws.numel() - (base - ws.data_ptr()), int(split_k),
-                                        ACTIVATIONS[activation], int(timeout_ms), C.c_void_p(stream)), "mk_gemm_bf16")
-        if check_status:
-            st = (C.c_int32 * 4)()
-            _check(N.lib().mk_gemm_bf16_status(C.c_void_p(base), st), "mk_gemm_bf16_status")
-            if st[0] != 0:
-                torch.cuda.synchronize(a.device)
-                ws.zero_()
-                raise RuntimeError(f"gemm_sm100 aborted: wait {st[0]} ran out (cta={st[1]}, role={st[2]}, step={st[3]})")
+    M, lda = _rows(a, K)
+    _, ldc = _rows(c, n_out)
+    idx = a.device.index
+    ws = workspace if workspace is not None else _workspaces.get((idx, _WORKSPACE_BYTES))
+    if ws is None:
+        ws = gemm_workspace(M, n_out, K, a.device)
+    ptr = ws.data_ptr()
+    base = (ptr + 255) // 256 * 256
+    # the host side of a call is longer than a small product takes on the device: the device guard is entered
+    # only when another device is current, and the stream handle is read without building a Stream object
+    if idx == torch._C._cuda_getDevice():
+        return _call(a, bt, c, packed, M, n_out, K, lda, ldc, base, ws, ptr, split_k, act, timeout_ms, idx, check_status)
+    with torch.cuda.device(idx):
+        return _call(a, bt, c, packed, M, n_out, K, lda, ldc, base, ws, ptr, split_k, act, timeout_ms, idx, check_status)
+
+
+def _rows(t: torch.Tensor, width: int):
+    """(rows, row stride) of a tensor whose last dimension is ``width`` and contiguous."""
+    if t.dim() == 2:
+        return t.shape[0], t.stride(0)
+    if t.is_contiguous():
+        return t.numel() // width if width else 0, width
+    v = t.view(-1, width)                              # raises if the rows are not equally spaced
+    return v.shape[0], v.stride(0)
+
+
+def _call(a, bt, c, packed, M, n_out, K, lda, ldc, base, ws, ptr, split_k, act, timeout_ms, idx, check_status):
+    lib = N.lib()
+    stream = torch._C._cuda_getCurrentRawStream(idx)
+    room = ws.numel() - (base - ptr)
+    if packed:
+        rc = lib.mk_gemm_bf16_packed(a.data_ptr(), bt.data_ptr(), c.data_ptr(), M, n_out, K, lda, ldc, base, room,
+                                     int(split_k), act, int(timeout_ms), stream)
+        if rc:
+            _check(rc, "mk_gemm_bf16_packed")
+    else:
+        rc = lib.mk_gemm_bf16(a.data_ptr(), bt.data_ptr(), c.data_ptr(), M, n_out, K, lda, bt.stride(0), ldc, base, room,
+                              int(split_k), act, int(timeout_ms), stream)
+        if rc:
+            _check(rc, "mk_gemm_bf16")
+    if check_status:
+        st = (C.c_int32 * 4)()
+        _check(lib.mk_gemm_bf16_status(C.c_void_p(base), st), "mk_gemm_bf16_status")
+        if st[0] != 0:
+            torch.cuda.synchronize(idx)
+            ws.zero_()
+            raise RuntimeError(f"gemm_sm100 aborted: wait {st[0]} ran out (cta={st[1]}, role={st[2]}, step={st[3]})")
     return c
 
 

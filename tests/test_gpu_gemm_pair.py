@@ -1,0 +1,56 @@
+"""Both tcgen05 GEMM kernels at the sizes where their cuts go wrong: one row, the edges of the 16-row granularity and
+of a full tile, ragged columns and K, few tiles (K is split over a cluster) and many (persistent pairs that walk
+several tiles each), odd column counts (no two-column stores), and every activation.
+
+The bar of test_gpu_gemm_sm100.py: one bf16 rounding plus K * 2^-24 relative fp32 accumulation noise; silu adds a
+relative 2^-9 for the exponential and the division."""
+
+import pytest
+import torch
+
+from machete_b200.kernels.gemm import gemm_pack_weight, gemm_sm100
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+
+SHAPES = [(1, 256, 64), (15, 1000, 1000), (129, 257, 72), (160, 4096, 4096), (255, 512, 2048), (257, 300, 8192),
+          (512, 4096, 512), (777, 1025, 1032), (1031, 5000, 328), (2049, 2304, 264), (96, 19000, 136)]
+
+
+@pytest.mark.parametrize("M,N_out,K", SHAPES)
+@pytest.mark.parametrize("activation", [None, "relu", "silu"])
+def test_every_cut_against_fp64(M, N_out, K, activation):
+    g = torch.Generator(device="cuda").manual_seed(M + N_out)
+    a = torch.randn(M, K, generator=g, device="cuda").to(BF)
+    b = (torch.randn(N_out, K, generator=g, device="cuda") * K ** -0.5).to(BF)
+    want = a.double() @ b.double().t()
+    noise = (a.double().abs() @ b.double().abs().t()) * K * 2.0 ** -24
+    rounding = 2.0 ** -8
+    if activation == "relu":
+        want = want.clamp_min(0)
+    elif activation == "silu":
+        want, rounding = torch.nn.functional.silu(want), 2.0 ** -8 + 2.0 ** -9
+        noise = noise * 1.1                                   # the slope of silu is below 1.1
+    for weight in (b, gemm_pack_weight(b)) if K % 64 == 0 else (b,):
+        c = torch.full((M, N_out), float("nan"), dtype=BF, device="cuda")
+        gemm_sm100(a, weight, c, activation=activation, check_status=True)
+        bad = ~((c.double() - want).abs() <= want.abs() * rounding + noise + 1e-30)
+        assert not bool(bad.any()), f"{int(bad.sum())} of {bad.numel()} entries outside the bar"
+
+
+def test_results_do_not_depend_on_the_launch_before():
+    """Launches overlap their set-up with the kernel before them: a product that reads the one before it sees all of it."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    w = [(torch.randn(512, 512, generator=g, device="cuda") * 512 ** -0.5).to(BF) for _ in range(6)]
+    x0 = torch.randn(320, 512, generator=g, device="cuda").to(BF)
+    bufs = [torch.zeros(320, 512, dtype=BF, device="cuda") for _ in range(6)]
+    steps = []
+    for rep in range(3):
+        x = x0
+        for i in range(6):
+            x = gemm_sm100(x, w[i], bufs[i])
+            if rep == 0:
+                torch.cuda.synchronize()                      # the first time every step waits for the one before
+        torch.cuda.synchronize()
+        steps.append(bufs[5].clone())
+    assert torch.equal(steps[0], steps[1]) and torch.equal(steps[0], steps[2])
