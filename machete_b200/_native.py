@@ -199,8 +199,8 @@ def _declare(h: C.CDLL) -> None:
     h.mk_gemm_bf16_status.argtypes = [vp, C.POINTER(i32)]
     h.mk_gemm_bf16_status.restype = C.c_int
     h.mk_gemm_last_error.restype = C.c_char_p
-    p64 = C.POINTER(C.c_int64)
-    h.mk_flash_prefill_bf16.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, p64, p64, p64, p64, f32, i32,
+    # the four stride arguments point into one array of the caller
+    h.mk_flash_prefill_bf16.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp, vp, vp, f32, i32,
                                         vp, u64, i32, vp]
     h.mk_flash_prefill_bf16.restype = C.c_int
     h.mk_flash_prefill_status.argtypes = [vp, C.POINTER(i32)]

@@ -36,6 +36,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
+#include <mutex>
 #include <string>
 #include <type_traits>
 
@@ -83,22 +85,30 @@ __device__ __forceinline__ void tmem_alloc(uint32_t slot, uint32_t cols) {
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// The issuing warp runs these as a whole and `elected` (one lane of it) predicates the instruction itself: with
+// one lane in the loop, or a branch around the instruction, the descriptors leave the uniform registers and an
+// MMA costs 115 clocks of issue, more than the tensor pipe takes for it (128 x 64 x 16: 48 clocks).
+__device__ __forceinline__ void tc_commit(uint32_t bar, uint32_t elected) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(elected)
       : "memory");
 }
-__device__ __forceinline__ void tc_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate,
+                                       uint32_t elected) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %4, 0;\n\tsetp.ne.u32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(elected)
+      : "memory");
+}
+__device__ __forceinline__ void tc_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate,
+                                          uint32_t elected) {
   // the M x K operand comes from tensor memory (lane = row, one 32-bit column = two bf16 along K)
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %4, 0;\n\tsetp.ne.u32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(elected)
       : "memory");
 }
 __device__ __forceinline__ float max3(float a, float b, float c) {
@@ -245,6 +255,17 @@ __device__ __forceinline__ bool wait_bar(const Params& p, Shared* sh, uint32_t b
   }
 }
 
+// The same wait for a whole warp: every lane polls, the outcome is the same for all.
+__device__ __forceinline__ bool wait_bar_warp(const Params& p, Shared* sh, uint32_t bar, uint32_t parity, int code, int aux) {
+  if (__all_sync(0xffffffffu, mk::mbar_try_wait(bar, parity))) return true;
+  return __all_sync(0xffffffffu, wait_bar(p, sh, bar, parity, code, aux));
+}
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 template <int D>
 __global__ void __launch_bounds__(kThreads, 2)
 prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -295,6 +316,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&sh->tmem_base);
+  mk::prior_work_done();
+  mk::next_may_start();
 
   // Tile j uses slot j & 1 of every double-buffered resource; its barrier phase is (j >> 1) & 1.
   if (warp == 0) {
@@ -328,21 +351,21 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t id_s = idesc_bf16(kBN, false), id_o = idesc_bf16(D, true);
-      bool ok = wait_bar(p, sh, mk::smem_u32(&sh->q_full), 0, PF_ST_TIMEOUT_FULL, -1);
+    {
+      const uint32_t id_s = idesc_bf16(kBN, false), id_o = idesc_bf16(D, true), elected = elect_one() ? 1u : 0u;
+      bool ok = wait_bar_warp(p, sh, mk::smem_u32(&sh->q_full), 0, PF_ST_TIMEOUT_FULL, -1);
       auto issue_s = [&](int j) -> bool {
         const int s = j & 1;
-        if (!wait_bar(p, sh, mk::smem_u32(&sh->k_full[s]), (uint32_t)(j >> 1) & 1u, PF_ST_TIMEOUT_FULL, j)) return false;
+        if (!wait_bar_warp(p, sh, mk::smem_u32(&sh->k_full[s]), (uint32_t)(j >> 1) & 1u, PF_ST_TIMEOUT_FULL, j)) return false;
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
           const uint32_t in_box = (uint32_t)(k & 3) * 32u;
           tc_mma(tmem + (uint32_t)s * kBN, desc_kmajor(q_s + (uint32_t)(k >> 2) * kBox + in_box),
-                 desc_kmajor(k_s + s * kKVTile + (uint32_t)(k >> 2) * kKVBox + in_box), id_s, k > 0 ? 1u : 0u);
+                 desc_kmajor(k_s + s * kKVTile + (uint32_t)(k >> 2) * kKVBox + in_box), id_s, k > 0 ? 1u : 0u, elected);
         }
-        tc_commit(mk::smem_u32(&sh->s_ready[s]));
-        tc_commit(mk::smem_u32(&sh->k_empty[s]));
+        tc_commit(mk::smem_u32(&sh->s_ready[s]), elected);
+        tc_commit(mk::smem_u32(&sh->k_empty[s]), elected);
         return true;
       };
       // Issue order S(0), S(1), P V(0), S(2), P V(1), S(3), ...  The tensor cores run the products in this
@@ -355,18 +378,18 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         const int s = j & 1;
         const uint32_t ph = (uint32_t)(j >> 1) & 1u;
         // O += P V once the row threads have written P (and rescaled O)
-        ok = wait_bar(p, sh, mk::smem_u32(&sh->p_ready[s]), ph, PF_ST_TIMEOUT_P, j) &&
-             wait_bar(p, sh, mk::smem_u32(&sh->v_full[s]), ph, PF_ST_TIMEOUT_FULL, j);
+        ok = wait_bar_warp(p, sh, mk::smem_u32(&sh->p_ready[s]), ph, PF_ST_TIMEOUT_P, j) &&
+             wait_bar_warp(p, sh, mk::smem_u32(&sh->v_full[s]), ph, PF_ST_TIMEOUT_FULL, j);
         if (!ok) break;
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < kBN / 16; ++k) {
           // P: 16 tokens = 8 tensor-memory columns of bf16 pairs; V: MN-major, 16 tokens = 16 rows of 128 bytes
           const uint64_t dv = desc_mnmajor(v_s + (uint32_t)s * kKVTile + (uint32_t)k * 2048u, kKVBox);
-          tc_mma_ts(tmem + kOCol, tmem + (uint32_t)s * kBN + (uint32_t)k * 8u, dv, id_o, (j > 0 || k > 0) ? 1u : 0u);
+          tc_mma_ts(tmem + kOCol, tmem + (uint32_t)s * kBN + (uint32_t)k * 8u, dv, id_o, (j > 0 || k > 0) ? 1u : 0u, elected);
         }
-        tc_commit(mk::smem_u32(&sh->pv_done[s]));
-        tc_commit(mk::smem_u32(&sh->v_empty[s]));
+        tc_commit(mk::smem_u32(&sh->pv_done[s]), elected);
+        tc_commit(mk::smem_u32(&sh->v_empty[s]), elected);
       }
     }
   } else {
@@ -553,6 +576,35 @@ static int encode_rows_map(CUtensorMap* out, const void* base, int D, int rows, 
   return 0;
 }
 
+// What a launch needs to know of its device, read once per device (the kernels' shared-memory limits are raised
+// at the same time).  Entries are written under the lock and never change afterwards.
+struct Device {
+  int smem_optin = 0, cc = 0;
+};
+static const Device* device_facts(int dev) {
+  constexpr int kMax = 64;
+  static Device facts[kMax];
+  static std::atomic<bool> known[kMax];
+  static std::mutex lock;
+  if (dev < 0 || dev >= kMax) return nullptr;
+  if (!known[dev].load(std::memory_order_acquire)) {
+    std::lock_guard<std::mutex> g(lock);
+    if (!known[dev].load(std::memory_order_relaxed)) {
+      Device d;
+      if (cudaDeviceGetAttribute(&d.smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+          cudaDeviceGetAttribute(&d.cc, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess)
+        return nullptr;
+      if (d.cc == 10 &&
+          (cudaFuncSetAttribute(prefill_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem_optin) != cudaSuccess ||
+           cudaFuncSetAttribute(prefill_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem_optin) != cudaSuccess))
+        return nullptr;
+      facts[dev] = d;
+      known[dev].store(true, std::memory_order_release);
+    }
+  }
+  return &facts[dev];
+}
+
 }  // namespace mkp
 
 extern "C" {
@@ -574,11 +626,12 @@ int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, 
   if (workspace_bytes < 256 || ((uint64_t)workspace & 255)) return fail(-2, "mk_flash_prefill_bf16: workspace of 256 aligned bytes");
   if (((uint64_t)o & 15) || o_strides[2] % 8 || o_strides[1] % 8 || o_strides[0] % 8)
     return fail(-2, "mk_flash_prefill_bf16: o must be 16-byte aligned with strides that are multiples of 8 elements");
-  int dev = 0, smem_optin = 0, cc = 0;
+  int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return fail(-1001, "cudaGetDevice failed");
-  cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  cudaDeviceGetAttribute(&cc, cudaDevAttrComputeCapabilityMajor, dev);
-  if (cc != 10) return fail(-6, "mk_flash_prefill_bf16 needs an sm_100 device (compute capability %d.x found)", cc);
+  const Device* d = device_facts(dev);
+  if (!d) return fail(-1001, "mk_flash_prefill_bf16: cannot read the attributes of device %d", dev);
+  if (d->cc != 10) return fail(-6, "mk_flash_prefill_bf16 needs an sm_100 device (compute capability %d.x found)", d->cc);
+  const int smem_optin = d->smem_optin;
   const int bn = kBN;                              // tokens per KV tile
   CUtensorMap mq, mkk, mv;
   int rc = encode_rows_map(&mq, q, D, M, H, B, q_strides[2], q_strides[1], q_strides[0], kBM, "q");
@@ -600,21 +653,19 @@ int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, 
   p.scale_log2 = scale * 1.4426950408889634f;
   p.timeout_ns = (uint64_t)(timeout_ms > 0 ? timeout_ms : 1000) * 1000000ull;
   const dim3 grid(H, B, (M + kBM - 1) / kBM);
-  static bool attr64[64] = {}, attr128[64] = {};
-  cudaError_t e = cudaSuccess;
-  if (D == 64) {
-    if (dev < 64 && !attr64[dev]) {
-      e = cudaFuncSetAttribute(prefill_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin);
-      attr64[dev] = e == cudaSuccess;
-    }
-    if (e == cudaSuccess) prefill_kernel<64><<<grid, kThreads, smem, reinterpret_cast<cudaStream_t>(cuda_stream)>>>(mq, mkk, mv, p);
-  } else {
-    if (dev < 64 && !attr128[dev]) {
-      e = cudaFuncSetAttribute(prefill_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin);
-      attr128[dev] = e == cudaSuccess;
-    }
-    if (e == cudaSuccess) prefill_kernel<128><<<grid, kThreads, smem, reinterpret_cast<cudaStream_t>(cuda_stream)>>>(mq, mkk, mv, p);
-  }
+  // the kernel may be placed while the one before it in the stream drains (it waits before it touches memory)
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = reinterpret_cast<cudaStream_t>(cuda_stream);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = D == 64 ? cudaLaunchKernelEx(&cfg, prefill_kernel<64>, mq, mkk, mv, p)
+                          : cudaLaunchKernelEx(&cfg, prefill_kernel<128>, mq, mkk, mv, p);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return fail(-(int)e - 1000, "mk_flash_prefill_bf16 launch: %s", cudaGetErrorString(e));
   return 0;

@@ -431,6 +431,8 @@ __global__ void __launch_bounds__(kThreads, 1) mk_persistent_kernel(const __grid
     c.ctrl->bulk_done[0] = c.ctrl->bulk_done[1] = 0;
     fence_mbar_init();
   }
+  prior_work_done();
+  next_may_start();
   __syncthreads();
   if (threadIdx.x < 32) {
     // one position per batch row (or one for all): a warp reads them side by side

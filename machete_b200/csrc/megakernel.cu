@@ -733,9 +733,19 @@ int mk_create(const mk_program_t* prog, mk_handle_t* out) { return create_progra
 int mk_run(mk_handle_t h, void* cuda_stream) {
   using namespace mk;
   if (!h) return fail(-1, "null handle");
-  void* args[] = {&h->pv};
-  CUDA_TRY(cudaLaunchKernel(reinterpret_cast<const void*>(h->kernel), dim3(h->n_ctas), dim3(kThreads), args,
-                            (size_t)h->smem_bytes, reinterpret_cast<cudaStream_t>(cuda_stream)));
+  // The launch may be placed while the kernel before it in the stream drains: its CTAs set up their shared
+  // memory and wait (prior_work_done) before they touch global memory.
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)h->n_ctas);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = (size_t)h->smem_bytes;
+  cfg.stream = reinterpret_cast<cudaStream_t>(cuda_stream);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  CUDA_TRY(cudaLaunchKernelEx(&cfg, h->kernel, h->pv));
   return 0;
 }
 

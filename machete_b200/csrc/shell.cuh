@@ -224,6 +224,7 @@ __device__ __forceinline__ void trace_init(Ctx& c) {
   c.trace_base = nullptr;   // stays null in a kernel built without tracing: every trace point folds away
   TraceRec* base = TRACED ? c.pv->trace : nullptr;
   if (TRACED && base != nullptr && c.lane == 0) {
+    prior_work_done();   // the launch before this one may still be writing its records
     c.trace_cap = c.pv->trace_cap - 2;   // room for the closing pair
     c.trace_base = base + ((size_t)blockIdx.x * (kConsumerWarps + 1) + c.warp) * c.pv->trace_cap;
     trace_sync_pair(c);

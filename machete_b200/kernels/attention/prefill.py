@@ -31,11 +31,7 @@ def _check(rc: int, what: str) -> None:
     raise ValueError(msg) if rc in (-2, -3) else RuntimeError(msg)
 
 
-def _strides(t: torch.Tensor, layout: str):
-    """(batch, head, row) element strides of a 4-D tensor in ``bhmd`` or ``bmhd`` order."""
-    if layout == "bhmd":
-        return (C.c_int64 * 3)(t.stride(0), t.stride(1), t.stride(2))
-    return (C.c_int64 * 3)(t.stride(0), t.stride(2), t.stride(1))
+_Strides = C.c_int64 * 12      # (batch, head, row) element strides of q, k, v and o
 
 
 def flash_prefill(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Tensor, *, causal: bool = False,
@@ -50,38 +46,59 @@ def flash_prefill(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Te
     """
     if layout not in ("bhmd", "bmhd"):
         raise ValueError(f"layout must be 'bhmd' or 'bmhd', got {layout!r}")
+    bf16 = torch.bfloat16
     for name, t in (("q", q), ("k", k), ("v", v), ("o", o)):
         if not t.is_cuda:
             raise RuntimeError("flash_prefill runs on a CUDA device only; there is no CPU path")
-        if t.dtype != torch.bfloat16 or t.dim() != 4 or t.stride(-1) != 1:
+        if t.dtype != bf16 or t.dim() != 4 or t.stride(3) != 1:
             raise ValueError(f"flash_prefill: {name} must be a 4-D bfloat16 tensor with a contiguous head dimension")
     hd, md = (1, 2) if layout == "bhmd" else (2, 1)
-    B, H, M, D = int(q.shape[0]), int(q.shape[hd]), int(q.shape[md]), int(q.shape[3])
-    Hkv, Nk = int(k.shape[hd]), int(k.shape[md])
-    if k.shape != v.shape or k.shape[0] != B or k.shape[3] != D or o.shape != q.shape:
+    qs, ks = q.shape, k.shape
+    B, H, M, D = qs[0], qs[hd], qs[md], qs[3]
+    Hkv, Nk = ks[hd], ks[md]
+    if ks != v.shape or ks[0] != B or ks[3] != D or o.shape != qs:
         raise ValueError(f"flash_prefill: shapes q{tuple(q.shape)} k{tuple(k.shape)} v{tuple(v.shape)} o{tuple(o.shape)} do not match")
     if lse is not None and (lse.dtype != torch.float32 or tuple(lse.shape) != (B, H, M) or not lse.is_contiguous()):
         raise ValueError("flash_prefill: lse must be a contiguous float32 (B, H, M) tensor")
-    dev = q.device.index if q.device.index is not None else torch.cuda.current_device()
+    dev = q.device.index
     ws = _status_blocks.get(dev)
     if ws is None:
         ws = torch.zeros(512, dtype=torch.uint8, device=q.device)
         _status_blocks[dev] = ws
     base = (ws.data_ptr() + 255) // 256 * 256
-    stream = torch.cuda.current_stream(q.device).cuda_stream
-    with torch.cuda.device(q.device):
-        _check(N.lib().mk_flash_prefill_bf16(
-            q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr() if lse is not None else None,
-            B, H, Hkv, M, Nk, D, _strides(q, layout), _strides(k, layout), _strides(v, layout), _strides(o, layout),
-            float(scale if scale is not None else 1.0 / math.sqrt(D)), int(bool(causal)), C.c_void_p(base), 256,
-            int(timeout_ms), C.c_void_p(stream)), "mk_flash_prefill_bf16")
+    # the device guard is entered only when another device is current: the host side of a call is longer than a
+    # short prompt's attention takes on the device
+    args = (q, k, v, o, lse, B, H, Hkv, M, Nk, D, hd, md, scale, causal, base, timeout_ms, dev)
+    if dev == torch._C._cuda_getDevice():
+        _call(*args)
         if check_status:
-            st = (C.c_int32 * 4)()
-            _check(N.lib().mk_flash_prefill_status(C.c_void_p(base), st), "mk_flash_prefill_status")
-            if st[0] != 0:
-                ws.zero_()
-                raise RuntimeError(f"flash_prefill aborted: wait {st[0]} ran out (cta={st[1]}, warp={st[2]}, tile={st[3]})")
+            _raise_on_timeout(base, ws)
+    else:
+        with torch.cuda.device(dev):
+            _call(*args)
+            if check_status:
+                _raise_on_timeout(base, ws)
     return o
+
+
+def _call(q, k, v, o, lse, B, H, Hkv, M, Nk, D, hd, md, scale, causal, base, timeout_ms, dev):
+    sq, sk, sv, so = q.stride(), k.stride(), v.stride(), o.stride()
+    st = _Strides(sq[0], sq[hd], sq[md], sk[0], sk[hd], sk[md], sv[0], sv[hd], sv[md], so[0], so[hd], so[md])
+    at = C.addressof(st)
+    rc = N.lib().mk_flash_prefill_bf16(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr() if lse is not None else None,
+        B, H, Hkv, M, Nk, D, at, at + 24, at + 48, at + 72, float(scale) if scale is not None else 1.0 / math.sqrt(D),
+        1 if causal else 0, base, 256, int(timeout_ms), torch._C._cuda_getCurrentRawStream(dev))
+    if rc:
+        _check(rc, "mk_flash_prefill_bf16")
+
+
+def _raise_on_timeout(base, ws):
+    st = (C.c_int32 * 4)()
+    _check(N.lib().mk_flash_prefill_status(C.c_void_p(base), st), "mk_flash_prefill_status")
+    if st[0] != 0:
+        ws.zero_()
+        raise RuntimeError(f"flash_prefill aborted: wait {st[0]} ran out (cta={st[1]}, warp={st[2]}, tile={st[3]})")
 
 
 class FlashAttentionSm100Op(Op):
