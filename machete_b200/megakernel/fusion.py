@@ -92,7 +92,8 @@ def lower_program(ops: List[ScheduledOp], ctx: LowerCtx) -> List[NativeOp]:
                 out.append(fused_attn)
                 i += 2
                 continue
-        if ctx.fuse and i + 1 < len(ops):
+        if ctx.fuse and out and i + 1 < len(ops):
+            # (a program of these two ops alone has no decode step beside it and keeps them as they are)
             head = _fuse_final_add(sop, ops[i + 1], ctx)
             if head is not None:
                 out.append(head)
