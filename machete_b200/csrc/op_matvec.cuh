@@ -96,10 +96,20 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8], int ty) {
     w[i] = (ty == MK_T_BF16) ? pack_bf16(f[2 * i], f[2 * i + 1]) : pack_f16(f[2 * i], f[2 * i + 1]);
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
-// Round every element to the storage type `ty` (what a store + reload does).
-__device__ __forceinline__ void round8(float (&f)[8], int ty) {
-  uint4 v = pack8(f, ty);
-  unpack8(v, ty, f);
+// Sum / product of eight bf16 or f16 values, each rounded once to its own type.  The same bits as going through
+// fp32 and rounding there (24 significant bits are at least 2 p + 2 for p = 8 and p = 11, so the second rounding
+// changes no normal result) in 4 instructions instead of 36.
+__device__ __forceinline__ uint4 add8(const uint4& a, const uint4& b, int ty) {
+  uint4 d;
+  if (ty == MK_T_BF16) {
+    d.x = add_bf16x2(a.x, b.x), d.y = add_bf16x2(a.y, b.y), d.z = add_bf16x2(a.z, b.z), d.w = add_bf16x2(a.w, b.w);
+  } else {
+    d.x = add_f16x2(a.x, b.x), d.y = add_f16x2(a.y, b.y), d.z = add_f16x2(a.z, b.z), d.w = add_f16x2(a.w, b.w);
+  }
+  return d;
+}
+__device__ __forceinline__ uint4 mul8_bf16(const uint4& a, const uint4& b) {
+  return make_uint4(mul_bf16x2(a.x, b.x), mul_bf16x2(a.y, b.y), mul_bf16x2(a.z, b.z), mul_bf16x2(a.w, b.w));
 }
 
 __device__ __forceinline__ int mv_act_type(const mk_op_t* op) {
@@ -126,8 +136,10 @@ __device__ __forceinline__ bool mv_rstd_in_epilogue(const mk_op_t* op) {
 // The code is kept small on purpose (loops are not unrolled beyond what the
 // memory latency asks for): it runs once per op on every CTA, always from a
 // cold instruction cache.
-//   * no prologue, same type: the rows are copied global -> shared with
-//     16-byte asynchronous copies, all in flight at once;
+//   * no prologue: the rows are copied global -> shared with 16-byte asynchronous
+//     copies, all in flight at once, and converted in place where the mma's type is
+//     another.  (Through registers, a row at a time or several, a conversion took 7 us
+//     for 8 x 4096 values against 3.6: NVFP4 projection 16 x 2048 -> 4096 20.8 -> 17.4 us);
 //   * RMSNorm prologue: R rows x H chunks per thread are requested together
 //     (one trip to L2), then reduced; R x H = 1 x 4 for the bf16 kernel of up to 8
 //     rows, 2 x 4 for its NVFP4 counterpart (K = 4096 in one trip), 4 x 2 otherwise.
@@ -173,45 +185,61 @@ __device__ __forceinline__ void mv_stage(Ctx& c, const mk_op_t* op, bool stage, 
     return b * op->s[sb] + s2 * op->s[ss];
   };
 
-  if (pro == MK_PRO_NONE && xt == at) {
-    // plain copy
+  // f(row, chunk, value, address) for every staged chunk that this thread wrote itself, rows fastest.  Four chunks
+  // are loaded before the first is worked on: one at a time waits out every latency of the chain.
+  auto for_own_chunks = [&](auto f) {
+    int m = 0, ch = tid;
 #pragma unroll 1
-    for (int m = 0; m < M; ++m) {
+    while (ch < chunks) {
+      uint4 v[4];
+      uint32_t a[4];
+      int ms[4], cs[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        ms[j] = m;
+        cs[j] = ch;
+        a[j] = c.act_u32 + (uint32_t)m * xs + (uint32_t)ch * 16u;
+        if (ch < chunks) v[j] = lds128(a[j]);
+        if (++m == M) {
+          m = 0;
+          ch += T;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (cs[j] >= chunks) break;
+        f(ms[j], cs[j], v[j], a[j]);
+      }
+    }
+  };
+  if (pro == MK_PRO_NONE) {
+    // every CTA reads the same rows at the same time: the NVFP4 kernels start at different ones
+    // (4 layers of the 8B shape at 8 rows 615 -> 603 us; nothing at the bf16 kernels' shorter rows)
+    int m = WFC != 0 && M > 1 ? (int)(blockIdx.x % (unsigned)M) : 0;
+#pragma unroll 1
+    for (int it = 0; it < M; ++it, m = m + 1 < M ? m + 1 : 0) {
       const uint16_t* xr = x + row_off(m, MK_MV_S_X_B, MK_MV_S_X_S);
       const uint32_t dst = c.act_u32 + (uint32_t)m * xs;
 #pragma unroll 1
       for (int ch = tid; ch < chunks; ch += T) cp_async16(dst + (uint32_t)ch * 16u, xr + ch * 8);
     }
     cp_async_wait_all();
+    if (WFC == 0 || xt == at) return;
+    // the mma's type differs from the input's: every thread converts the chunks it copied, four side by side
+    for_own_chunks([&](int, int, const uint4& v, uint32_t a) {
+      float f[8];
+      unpack8(v, xt, f);
+      sts128(a, pack8(f, at));
+    });
     return;
   }
 
   const uint4 z = make_uint4(0, 0, 0, 0);
-  if (WFC != 0 && pro == MK_PRO_NONE) {
-    // no prologue, the mma's type differs from the input's: a converting copy, eight chunks per
-    // thread in flight (K = 12288 in one trip per row)
+  // every CTA reads the same rows at the same time: the NVFP4 kernels start at different ones, as above
+  const int groups = (M + R - 1) / R;
+  int m0 = WFC != 0 && groups > 1 ? (int)(blockIdx.x % (unsigned)groups) * R : 0;
 #pragma unroll 1
-    for (int m = 0; m < M; ++m) {
-      const uint16_t* xr = x + row_off(m, MK_MV_S_X_B, MK_MV_S_X_S);
-      const uint32_t dst = c.act_u32 + (uint32_t)m * xs;
-#pragma unroll 1
-      for (int ch0 = tid; ch0 < chunks; ch0 += 8 * T) {
-        uint4 v[8];
-#pragma unroll
-        for (int h = 0; h < 8; ++h) v[h] = (ch0 + h * T < chunks) ? *reinterpret_cast<const uint4*>(xr + (ch0 + h * T) * 8) : z;
-#pragma unroll
-        for (int h = 0; h < 8; ++h) {
-          if (ch0 + h * T >= chunks) break;
-          float f[8];
-          unpack8(v[h], xt, f);
-          sts128(dst + (uint32_t)(ch0 + h * T) * 16u, pack8(f, at));
-        }
-      }
-    }
-    return;
-  }
-#pragma unroll 1
-  for (int m0 = 0; m0 < M; m0 += R) {
+  for (int it = 0; it < groups; ++it, m0 = m0 + R < M ? m0 + R : 0) {
     const uint16_t *xr[R], *rr[R];
     uint16_t* wr[R];
     float sum[R];
@@ -232,7 +260,7 @@ __device__ __forceinline__ void mv_stage(Ctx& c, const mk_op_t* op, bool stage, 
         const bool ok = ch < chunks;
         wv[h] = (ok && fused) ? *reinterpret_cast<const uint4*>(nw + ch * 8) : z;
         // two-pass form: the second pass reads this thread's norm weights; have them in L1 by then
-        if (WFC != 0 && ok && !fused && pro != MK_PRO_NONE) asm volatile("prefetch.global.L1 [%0];" ::"l"(nw + ch * 8));
+        if (WFC != 0 && ok && !fused) asm volatile("prefetch.global.L1 [%0];" ::"l"(nw + ch * 8));
 #pragma unroll
         for (int j = 0; j < R; ++j) {
           const bool rok = ok && (R == 1 || m0 + j < M);   // rows past M are not fetched a second time
@@ -244,38 +272,27 @@ __device__ __forceinline__ void mv_stage(Ctx& c, const mk_op_t* op, bool stage, 
       for (int h = 0; h < H; ++h) {
         const int ch = ch0 + h * T;
         if (ch >= chunks) break;
-        float w[8];
-        unpack8(wv[h], xt, w);
 #pragma unroll
         for (int j = 0; j < R; ++j) {
           if (m0 + j >= M) break;
-          float f[8];
-          unpack8(v[j][h], xt, f);
           uint4 o = v[j][h];
           if (add) {
-            float q[8];
-            unpack8(r[j][h], xt, q);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] += q[i];
-            round8(f, xt);
-            o = pack8(f, xt);
+            o = add8(o, r[j][h], xt);
             if (wr[j]) *reinterpret_cast<uint4*>(wr[j] + ch * 8) = o;
           }
           if (stage) {
+            float f[8];
+            unpack8(o, xt, f);
 #pragma unroll
             for (int i = 0; i < 8; ++i) sum[j] += f[i] * f[i];
-            if (fused) {
-#pragma unroll
-              for (int i = 0; i < 8; ++i) f[i] *= w[i];
-              o = pack8(f, xt);
-            }
+            if (fused) o = mul8_bf16(o, wv[h]);         // the scale is taken out for bf16 rows only
             // not fused: keep the (rounded) input in its own type for now; pass 2 rescales
             sts128(c.act_u32 + (uint32_t)(m0 + j) * xs + (uint32_t)ch * 16u, o);
           }
         }
       }
     }
-    if (stage && pro != MK_PRO_NONE) {
+    if (stage) {
 #pragma unroll
       for (int j = 0; j < R; ++j) {
         const float t = warp_sum(sum[j]);
@@ -294,21 +311,15 @@ __device__ __forceinline__ void mv_stage(Ctx& c, const mk_op_t* op, bool stage, 
     c.ctrl->rstd[tid] = rsqrtf(tot / (float)K + op->f[MK_MV_F_EPS]);
   }
   named_bar_sync(kConsumerBarrier, T);
-#pragma unroll 1
-  for (int ch = tid; ch < chunks; ch += T) {
-    float w[8];
+  for_own_chunks([&](int m, int ch, const uint4& v, uint32_t a) {
+    float f[8], w[8];
+    unpack8(v, xt, f);
     unpack8(*reinterpret_cast<const uint4*>(nw + ch * 8), xt, w);
-#pragma unroll 1
-    for (int m = 0; m < M; ++m) {
-      const uint32_t a = c.act_u32 + (uint32_t)m * xs + (uint32_t)ch * 16u;
-      float f[8];
-      unpack8(lds128(a), xt, f);
-      const float rstd = c.ctrl->rstd[m];
+    const float rstd = c.ctrl->rstd[m];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) f[i] = f[i] * rstd * w[i];
-      sts128(a, pack8(f, at));
-    }
-  }
+    for (int i = 0; i < 8; ++i) f[i] = f[i] * rstd * w[i];
+    sts128(a, pack8(f, at));
+  });
 }
 
 // ---- epilogue ----------------------------------------------------------------------
