@@ -60,7 +60,7 @@ def schedule_decode_layer_nvfp4_sm100(*, layer_idx, batch, seq_len, cache_pos, w
     ``dynamic_position`` (not in the reference): the step follows the program's device-resident cache
     position instead of ``cache_pos`` (see ``schedule_decode_layer_sm100``); a q/k-norm layer then needs
     the fused form."""
-    from ..attention.flash_decoding import flash_decoding_schedule
+    from ..attention.flash_decoding import flash_decoding_schedule, layer_num_splits
 
     pfx = f"layer.{layer_idx}"
     if dynamic_position:
@@ -123,7 +123,8 @@ def schedule_decode_layer_nvfp4_sm100(*, layer_idx, batch, seq_len, cache_pos, w
         ops += proj(RmsVMatvecCacheNvfp4Sm120Op, "W_v", dst_cache=v_window, cache_pos=cache_pos)
     fa_ops, fa_config = flash_decoding_schedule(q=q_4d, k=k_window, v=v_window, o=o_4d,
                                                 kv_group_size=num_q_heads // num_kv_heads, page_size=page_size,
-                                                num_splits=fa_num_splits, qk_norm=qk_norm,
+                                                num_splits=fa_num_splits if fa_num_splits > 0
+                                                else layer_num_splits(q_4d, k_window), qk_norm=qk_norm,
                                                 dynamic_len=dynamic_position)
     ops += fa_ops
     wo = _w(weights, f"{pfx}.W_o")

@@ -359,7 +359,7 @@ def schedule_decode_layer_sm100(
     K-split projections write fp32 partials that an in-kernel all-reduce adds
     across ranks (plus the residual for the O-projection).
     """
-    from ..attention.flash_decoding import flash_decoding_schedule
+    from ..attention.flash_decoding import flash_decoding_schedule, layer_num_splits
 
     pfx = f"layer.{layer_idx}"
     if dynamic_position:
@@ -393,7 +393,8 @@ def schedule_decode_layer_sm100(
                                            cache_pos=cache_pos, **common)
     fa_ops, fa_config = flash_decoding_schedule(
         q=q_4d, k=k_window, v=v_window, o=o_4d, kv_group_size=kv_group_size, page_size=page_size,
-        num_splits=fa_num_splits, dynamic_len=dynamic_position,
+        num_splits=fa_num_splits if fa_num_splits > 0 else layer_num_splits(q_4d, k_window),
+        dynamic_len=dynamic_position,
     )
     ops += fa_ops
     tp_keep = []
