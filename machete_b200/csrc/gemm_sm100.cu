@@ -468,39 +468,56 @@ static EncodeTiledFn encode_fn() {
   fn = reinterpret_cast<EncodeTiledFn>(sym);
   return fn;
 }
-// Encoding a map costs about 2 us of host time, as much as the launch; a map is a function of the address and the
-// sizes alone.  Each thread keeps the last maps it encoded, direct-mapped by a hash of the arguments.
+// Encoding a map costs about 2 us of host time, as much as the launch.  Each thread keeps the last maps it encoded
+// by their sizes alone, direct-mapped by a hash; the address is put in on every call.
+typedef CUresult (*ReplaceAddressFn)(CUtensorMap*, void*);
+static ReplaceAddressFn replace_fn() {
+  static ReplaceAddressFn fn = nullptr;
+  if (fn) return fn;
+  void* sym = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPoint("cuTensorMapReplaceAddress", &sym, cudaEnableDefault, &q) != cudaSuccess ||
+      q != cudaDriverEntryPointSuccess)
+    return nullptr;
+  fn = reinterpret_cast<ReplaceAddressFn>(sym);
+  return fn;
+}
 struct MapKey {
-  uint64_t base;
   int64_t ld;
   int32_t rows, cols, box, kind;
   bool operator==(const MapKey& o) const {
-    return base == o.base && ld == o.ld && rows == o.rows && cols == o.cols && box == o.box && kind == o.kind;
+    return ld == o.ld && rows == o.rows && cols == o.cols && box == o.box && kind == o.kind;
   }
 };
 template <class F>
-static int cached_map(CUtensorMap* out, const MapKey& key, F encode) {
+static int cached_map(CUtensorMap* out, const void* base, const MapKey& key, F encode) {
   constexpr int kSlots = 64;
   struct Slot {
     MapKey key = {};
     CUtensorMap map;
   };
   static thread_local Slot slots[kSlots];
-  uint64_t h = key.base * 0x9E3779B97F4A7C15ull ^ (uint64_t)key.ld * 0xC2B2AE3D27D4EB4Full ^ ((uint64_t)(uint32_t)key.rows << 32) ^
+  uint64_t h = (uint64_t)key.ld * 0xC2B2AE3D27D4EB4Full ^ ((uint64_t)(uint32_t)key.rows << 32) ^
                (uint64_t)(uint32_t)(key.cols * 31 + key.box * 7 + key.kind);
   h ^= h >> 29;
   Slot& s = slots[(h * 0xBF58476D1CE4E5B9ull) >> 58];
-  if (key.base == 0 || !(s.key == key)) {
+  if (!(s.key == key)) {        // an unused slot has no columns
     const int rc = encode(&s.map);
     s.key = rc ? MapKey{} : key;
     if (rc) return rc;
+    *out = s.map;
+    return 0;
   }
   *out = s.map;
+  ReplaceAddressFn fn = replace_fn();
+  if (!fn) return fail(-5, "cuTensorMapReplaceAddress is not available from this driver");
+  const CUresult r = fn(out, const_cast<void*>(base));
+  if (r != CUDA_SUCCESS) return fail(-5, "cuTensorMapReplaceAddress failed with CUresult %d", (int)r);
   return 0;
 }
 // A row-major bf16 matrix [rows, K] with row stride `ld` elements; one box = 64 K values x box_rows rows.
 static int encode_bf16_map(CUtensorMap* map, const void* base, int rows, int K, int64_t ld, int box_rows) {
-  return cached_map(map, MapKey{(uint64_t)base, ld, rows, K, box_rows, 1}, [&](CUtensorMap* out) -> int {
+  return cached_map(map, base, MapKey{ld, rows, K, box_rows, 1}, [&](CUtensorMap* out) -> int {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return fail(-5, "cuTensorMapEncodeTiled is not available from this driver");
     cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
@@ -518,7 +535,7 @@ static int encode_bf16_map(CUtensorMap* map, const void* base, int rows, int K, 
 // The same matrix stored K-tile-major, [K/64][N][64]: dims (64, N, K/64), one box = 128 rows of one K tile,
 // which is one contiguous 16 KB piece of memory.
 static int encode_packed_map(CUtensorMap* map, const void* base, int N, int k_tiles) {
-  return cached_map(map, MapKey{(uint64_t)base, 0, N, k_tiles, kTileN, 2}, [&](CUtensorMap* out) -> int {
+  return cached_map(map, base, MapKey{0, N, k_tiles, kTileN, 2}, [&](CUtensorMap* out) -> int {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return fail(-5, "cuTensorMapEncodeTiled is not available from this driver");
     cuuint64_t dims[3] = {(cuuint64_t)kTileK, (cuuint64_t)N, (cuuint64_t)k_tiles};
@@ -710,7 +727,8 @@ static int pair_launch(const void* a, const void* b, void* c, int M, int N, int 
   p.wide_store = (N % 2 == 0 && ldc % 2 == 0 && ((uint64_t)c & 3) == 0) ? 1 : 0;
   p.timeout_ns = (uint64_t)(timeout_ms > 0 ? timeout_ms : 1000) * 1000000ull;
   const int clusters = plan.split > 1 ? p.tiles : std::min(p.tiles, d.pair_clusters[1]);
-  const size_t smem = 1024 + (size_t)p.ring_bytes + sizeof(PairShared);
+  // a pair holds all 512 columns of both its SMs: no CTA of the other kernel (38 KB or more) may share one with it
+  const size_t smem = std::max(1024 + (size_t)p.ring_bytes + sizeof(PairShared), (size_t)d.smem_optin - 32768);
   return launch(gemm_pair_kernel, dim3((unsigned)(2 * plan.split * clusters)), dim3((unsigned)(2 * plan.split)), kPairThreads, smem,
                 stream, map_a, map_b, p);
 }
@@ -759,7 +777,14 @@ static int gemm_launch(const void* a, const void* b, void* c, int M, int N, int 
   if (stages > per) stages = per < 2 ? 2 : per;
   uint32_t ring_bytes = (uint32_t)stages * stage_bytes;
   if (split_k > 1) ring_bytes = std::max(ring_bytes, (uint32_t)m_box * kTileN * 4u);
-  const size_t smem = 1024 + (size_t)ring_bytes + sizeof(Shared);
+  size_t smem = 1024 + (size_t)ring_bytes + sizeof(Shared);
+  if (split_k > 1) {
+    // CTAs of a cluster wait for one another while they hold tensor memory: no more of them (of this launch or of
+    // one in another stream) may share an SM than its 512 columns serve, or they could wait in a circle.
+    int cols = 32;
+    while (cols < m_box) cols <<= 1;
+    smem = std::max(smem, std::min((size_t)smem_optin, (size_t)smem_optin * cols / 512 + 1024));
+  }
   Params p;
   uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
   p.c = reinterpret_cast<__nv_bfloat16*>(c);
