@@ -351,12 +351,20 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    {
-      const uint32_t id_s = idesc_bf16(kBN, false), id_o = idesc_bf16(D, true), elected = elect_one() ? 1u : 0u;
-      bool ok = wait_bar_warp(p, sh, mk::smem_u32(&sh->q_full), 0, PF_ST_TIMEOUT_FULL, -1);
+    // Head dim 64 issues as a whole warp (see tc_mma).  At 128 the tensor pipe is the bound either way and one lane
+    // that waits and issues is the lighter neighbour: 4096 x 4096 causal, power-capped, 152.5 us against 154.8.
+    constexpr bool kOneLane = D == 128;
+    if (!kOneLane || lane == 0) {
+      auto wait_mma = [&](uint32_t bar, uint32_t parity, int code, int aux) -> bool {
+        if constexpr (kOneLane) return wait_bar(p, sh, bar, parity, code, aux);
+        else return wait_bar_warp(p, sh, bar, parity, code, aux);
+      };
+      const uint32_t id_s = idesc_bf16(kBN, false), id_o = idesc_bf16(D, true);
+      const uint32_t elected = kOneLane || elect_one() ? 1u : 0u;
+      bool ok = wait_mma(mk::smem_u32(&sh->q_full), 0, PF_ST_TIMEOUT_FULL, -1);
       auto issue_s = [&](int j) -> bool {
         const int s = j & 1;
-        if (!wait_bar_warp(p, sh, mk::smem_u32(&sh->k_full[s]), (uint32_t)(j >> 1) & 1u, PF_ST_TIMEOUT_FULL, j)) return false;
+        if (!wait_mma(mk::smem_u32(&sh->k_full[s]), (uint32_t)(j >> 1) & 1u, PF_ST_TIMEOUT_FULL, j)) return false;
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
@@ -378,8 +386,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         const int s = j & 1;
         const uint32_t ph = (uint32_t)(j >> 1) & 1u;
         // O += P V once the row threads have written P (and rescaled O)
-        ok = wait_bar_warp(p, sh, mk::smem_u32(&sh->p_ready[s]), ph, PF_ST_TIMEOUT_P, j) &&
-             wait_bar_warp(p, sh, mk::smem_u32(&sh->v_full[s]), ph, PF_ST_TIMEOUT_FULL, j);
+        ok = wait_mma(mk::smem_u32(&sh->p_ready[s]), ph, PF_ST_TIMEOUT_P, j) &&
+             wait_mma(mk::smem_u32(&sh->v_full[s]), ph, PF_ST_TIMEOUT_FULL, j);
         if (!ok) break;
         tc_fence_after();
 #pragma unroll
