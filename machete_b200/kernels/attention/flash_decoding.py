@@ -67,12 +67,22 @@ def splits_by_cost(B: int, H_kv: int, m_tiles: int, N_kv: int, num_sms: int, min
                key=lambda s: (math.ceil(base * s / num_sms) * (_UNIT_COST_TOKENS + -(-N_kv // s)), s))
 
 
+def _one_trip_splits(M: int, group: int, head_dim: int) -> int:
+    """The most splits whose lse values the fused combine of one query token fetches in one trip: 128 values for the
+    rows that it takes together (4 at head dim 64, 2 at 128).  More fill the last few SMs and cost more than that:
+    1 x 12729 tokens, 4 KV heads of 8 query heads at head dim 64, 19.5 us with 32 splits, 22.0 with 36, 23.4 with 37;
+    2 KV heads of 16: 28.4 with 32, 51.9 with 64."""
+    return 128 // max(1, min(group, 256 // head_dim)) if M == 1 else 64
+
+
 def layer_num_splits(q, k) -> int:
     """The decode layers' splits: they keep ``default_num_splits``, so that a model's tokens do not move with this
     rule (the sums of a split are rounded once, and some sixteen layers amplify a rounding to 1e-2 of the logits)."""
-    B, M, H, _ = (int(v) for v in q.shape)
+    B, M, H, D = (int(v) for v in q.shape)
     N_kv, H_kv = int(k.shape[1]), int(k.shape[2])
-    return default_num_splits(B, H_kv, -(-(M * (H // H_kv)) // 16), N_kv, _num_sms(q.device))
+    group = H // H_kv
+    return min(default_num_splits(B, H_kv, -(-(M * group) // 16), N_kv, _num_sms(q.device)),
+               _one_trip_splits(M, group, D))
 
 
 class FlashDecodingSplitBSHDOp(Op):
@@ -119,7 +129,7 @@ class FlashDecodingSplitBSHDOp(Op):
         m_tiles = -(-(M * group) // 16)
         if num_splits <= 0:
             rule = splits_by_cost if D == 64 and not dynamic_len else default_num_splits
-            num_splits = rule(B, H_kv, m_tiles, N_kv, _num_sms(q.device))
+            num_splits = min(rule(B, H_kv, m_tiles, N_kv, _num_sms(q.device)), _one_trip_splits(M, group, D))
         num_splits = max(1, min(int(num_splits), max(1, N_kv // 16)))
         o_partial = torch.empty(B, H, num_splits, M, D, dtype=torch.float32, device=q.device)
         lse_partial = torch.empty(B, H, num_splits, M, dtype=torch.float32, device=q.device)

@@ -139,3 +139,35 @@ def test_fused_qk_norm(B, H, Hkv, D, Nkv, splits):
     mk.run()
     assert torch.equal(first, o)
     assert (mk.read_counters() == 0).all()
+
+
+@pytest.mark.parametrize("M,H,Hkv,D,Nkv,splits", [
+    (1, 32, 4, 64, 3889, 0),      # one sequence, four KV heads: the default, which took 37 splits
+    (1, 32, 4, 64, 3889, 37),
+    (1, 32, 4, 64, 1600, 32),     # 4 rows of 32 splits: 128 lse values, one trip
+    (1, 32, 4, 64, 1600, 33),
+    (1, 6, 2, 64, 1600, 43),      # 3 rows of 43: 129
+    (1, 8, 8, 64, 2100, 128),     # one row
+    (1, 32, 4, 64, 2100, 128),    # the most that is combined in the op
+    (1, 32, 4, 128, 1600, 64),    # 2 rows of 64
+    (1, 32, 4, 128, 1600, 65),
+    (1, 24, 8, 128, 2100, 128),
+    (2, 16, 4, 64, 1600, 40),     # two query tokens
+])
+def test_many_splits(M, H, Hkv, D, Nkv, splits):
+    """The fused combine reads every lse value of its rows, however many splits there are.  Entry by entry: the
+    probabilities are rounded to bf16 (2^-9 each, as many as are summed) and so is the result."""
+    q, k, v = qkv(1, M, H, Hkv, D, Nkv, seed=splits)
+    o = torch.full((1, M, H, D), float("nan"), dtype=BF, device="cuda")
+    ops, _ = flash_decoding_schedule(q.cuda(), k.cuda(), v.cuda(), o, num_splits=splits, kv_group_size=H // Hkv)
+    mk = Megakernel(ops)
+    assert len(mk.native_ops) == 1                            # the combine is part of the op
+    heads = torch.arange(H) // (H // Hkv)
+    kh, vh = k[0].double()[:, heads], v[0].double()[:, heads]                       # (N, H, D)
+    p = torch.softmax(torch.einsum("mhd,nhd->mhn", q[0].double(), kh) / math.sqrt(D), dim=-1)
+    want = torch.einsum("mhn,nhd->mhd", p, vh)
+    bar = 2.0 ** -8 * (torch.einsum("mhn,nhd->mhd", p, vh.abs()) + want.abs()) + 1e-6
+    for _ in range(2):
+        mk.run()
+        assert bool(((o[0].cpu().double() - want).abs() <= bar).all())
+        o.fill_(float("nan"))
