@@ -352,7 +352,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&sh->tmem_base);
   mk::prior_work_done();
-  mk::next_may_start();
 
   if (warp == 0) {
     int issued = ahead, s = ahead == p.stages ? 0 : ahead;
@@ -366,6 +365,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         ph ^= 1u;
       }
     }
+    mk::next_may_start();
     if (lane == 0 && *reinterpret_cast<volatile int32_t*>(&sh->abort_flag)) {
       // shared memory must outlive the copies still in flight: wait (bounded) for the stages that
       // were issued but perhaps never consumed
