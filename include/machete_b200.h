@@ -478,6 +478,11 @@ int mk_gemm_bf16_packed(const void* a, const void* b_packed, void* c, int M, int
                         void* workspace, uint64_t workspace_bytes, int split_k, int activation, int timeout_ms,
                         void* cuda_stream);
 int mk_gemm_bf16_status(const void* workspace, int32_t out[4]);
+/* How mk_gemm_bf16 cuts a product of these sizes on the current device (ldb: the
+ * weight's row stride, 0 for a packed weight): out[0] 1 = CTA pairs on 256 weight
+ * rows, 0 = one CTA on 128; [1] CTAs or pairs that share a tile's K range;
+ * [2] activation rows per tile; [3] output tiles. */
+int mk_gemm_bf16_plan(int M, int N, int K, int64_t ldb, int32_t out[4]);
 const char* mk_gemm_last_error(void);
 
 /* ---- prefill attention on tcgen05 tensor cores -----------------------------------

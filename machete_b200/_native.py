@@ -116,7 +116,8 @@ EXPORTS = [
     "mk_update_op", "mk_read_counters", "mk_destroy",
     "mk_standalone_workspace_bytes", "mk_matvec_bf16", "mk_matvec_nvfp4", "mk_flash_decode",
     "mk_flash_decode_noalloc", "mk_flash_decode_noalloc_status",
-    "mk_gemm_bf16_workspace_bytes", "mk_gemm_bf16", "mk_gemm_bf16_packed", "mk_gemm_bf16_status", "mk_gemm_last_error",
+    "mk_gemm_bf16_workspace_bytes", "mk_gemm_bf16", "mk_gemm_bf16_packed", "mk_gemm_bf16_status", "mk_gemm_bf16_plan",
+    "mk_gemm_last_error",
     "mk_flash_prefill_bf16", "mk_flash_prefill_status", "mk_flash_prefill_last_error",
 ]
 
@@ -198,6 +199,8 @@ def _declare(h: C.CDLL) -> None:
     h.mk_gemm_bf16_packed.restype = C.c_int
     h.mk_gemm_bf16_status.argtypes = [vp, C.POINTER(i32)]
     h.mk_gemm_bf16_status.restype = C.c_int
+    h.mk_gemm_bf16_plan.argtypes = [i32, i32, i32, i64, C.POINTER(i32)]
+    h.mk_gemm_bf16_plan.restype = C.c_int
     h.mk_gemm_last_error.restype = C.c_char_p
     # the four stride arguments point into one array of the caller
     h.mk_flash_prefill_bf16.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp, vp, vp, f32, i32,

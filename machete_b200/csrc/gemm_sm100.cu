@@ -37,6 +37,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <mutex>
 #include <string>
 #include <type_traits>
@@ -631,34 +632,48 @@ static const Device* device_facts(int dev) {
   return &facts[dev];
 }
 
-// Which kernel, and how the work is cut.  The model's terms were fitted to timings of both kernels with the weight
-// in HBM (M 40..2048, N 1024..14336, K 1024..14336; within about 10 %): a fixed part (launch, barriers, first load,
-// tear-down), the K steps a CTA walks one after another or the weight's bytes through HBM, whichever is longer, the
-// store of `cols` accumulator columns, and the exchange of a split.  A K step takes what its MMAs take (at least
-// 0.18 us with the waits around them) or what its bytes take at the 13.4 TB/s that all SMs together draw from L2.
-// Clusters that do not all run at once cost a second pass, so a split is taken only where they do.
+// Which kernel, and how the work is cut.  The model's terms were fitted to 5700 timings of every cut of 330 shapes
+// (M 33..2048, N and K 1024..14336, the weight in HBM and in L2; half of them within 3 %, nine tenths within 8 %): a
+// fixed part (launch, barriers, first load, tear-down), the K steps that a CTA walks one after another, the store of
+// `cols` accumulator columns, and the exchange of a split.  A K step takes the longest of 0.197 us, its MMAs, its
+// bytes at what one SM draws (0.16 MB/us), and all CTAs' bytes at what L2 gives (21.5 TB/s); a 128-byte piece of a
+// row that does not begin on a 128-byte line costs more of both.  Where the weight comes from HBM its bytes set a floor under the
+// steps, and near that floor both count.  The library cannot know where the weight lies, so a plan is judged by the
+// mean of the two.  (By the longer of steps and bytes alone, every cut of a call near the floor costs the same and
+// the fewest CTAs win: 66 x 5576 -> 8616 28.9 us unsplit on 68 CTAs, 23.9 split in two on 136; 59 x 10760 -> 5392
+// 31.1 and 24.9, with pairs 24.2.)  Clusters that do not all run at once cost a second pass, so a split is taken
+// only where they do; clusters that take every place there is wait for the very last of the kernel before them
+// (3 to 20 % over the model, 42 x 1040 -> 5680 in three 7.6 us against 5.8 unsplit) and are charged 8 %.
 struct Plan {
   bool pair = false;
   int split = 1, rows = 0;       // rows: activation rows per tile (pair kernel)
   float us = 1e30f;
 };
-static float modelled_us(float fixed, int steps, int bytes_per_step, int ctas, double weight_bytes, int cols, int split) {
-  const float step = std::max(std::max(0.18f, 0.03f + 0.27f * (float)cols / kMaxM), (float)bytes_per_step * (float)ctas / 13.4e6f);
-  return fixed + std::max(steps * step, (float)(weight_bytes / 6.3e6)) + cols * 0.006f + (split > 1 ? 1.2f + cols * 0.012f : 0.f);
+static float line_cost(const void* base, int64_t row_elems) {
+  const uint64_t bits = (uint64_t)base | (uint64_t)row_elems * 2;
+  return bits % 128 == 0 ? 1.f : bits % 64 == 0 ? 1.08f : bits % 32 == 0 ? 1.24f : 1.85f;
 }
-static Plan plan_single(int M, int N, int K, const Device& d, int split) {
+static float modelled_us(float fixed, int steps, float bytes_per_step, int ctas, double weight_bytes, int cols, int split) {
+  const float bytes = std::max(bytes_per_step / 0.16e6f, bytes_per_step * (float)ctas / 21.5e6f);
+  const float walk = (float)steps * std::max(std::max(0.197f, 0.045f + 0.256f * (float)cols / kMaxM), bytes);
+  const float hbm = (float)(weight_bytes / 6.5e6), w2 = walk * walk, h2 = hbm * hbm;
+  const float cold = std::sqrt(std::sqrt(w2 * w2 + h2 * h2));
+  return fixed + 0.5f * (walk + cold) + cols * 0.009f + (split > 1 ? 1.0f + cols * 0.0095f : 0.f);
+}
+static Plan plan_single(int M, int N, int K, const Device& d, int split, float line) {
   Plan best;
   const int k_tiles = ceil_div(K, kTileK), mt = ceil_div(M, kMaxM), mpad = round_up(std::min(M, kMaxM), 16);
   const int tiles = ceil_div(N, kTileN) * mt;
   for (int s = split > 0 ? split : 1; s <= (split > 0 ? split : kMaxSplit); ++s) {
     if (split == 0 && s > 1 && (s > k_tiles / 2 || d.clusters[s] < tiles)) break;
     const int steps = ceil_div(tiles, std::max(1, d.clusters[s])) * ceil_div(k_tiles, s);
-    const float us = modelled_us(4.3f, steps, (int)kWBytes + mpad * kTileK * 2, std::min(tiles * s, d.sms), 2.0 * N * K, mpad, s);
+    const float us = modelled_us(2.2f, steps, line * (float)((int)kWBytes + mpad * kTileK * 2), std::min(tiles * s, d.sms),
+                                 2.0 * N * K, mpad, s) * (s > 1 && d.clusters[s] == tiles ? 1.08f : 1.f);
     if (us < best.us) best.split = s, best.us = us;
   }
   return best;
 }
-static Plan plan_pair(int M, int N, int K, const Device& d) {
+static Plan plan_pair(int M, int N, int K, const Device& d, float line) {
   Plan best;
   best.pair = true;
   const int k_tiles = ceil_div(K, kTileK), nt = ceil_div(N, kPairRows), mt0 = ceil_div(M, kMaxM);
@@ -668,11 +683,18 @@ static Plan plan_pair(int M, int N, int K, const Device& d) {
       const int room = d.pair_clusters[s];
       if (room < 1 || (s > 1 && (s > k_tiles / 2 || tiles > room))) break;
       const int steps = ceil_div(tiles, room) * ceil_div(k_tiles, s);
-      const float us = modelled_us(5.0f, steps, (int)kWBytes + bn * kTileK, std::min(2 * tiles * s, d.sms), 2.0 * N * K, bn, s);
+      const float us = modelled_us(3.35f, steps, line * (float)((int)kWBytes + bn * kTileK), std::min(2 * tiles * s, d.sms),
+                                   2.0 * N * K, bn, s);
       if (us < best.us) best.split = s, best.rows = bn, best.us = us;
     }
   }
   return best;
+}
+static Plan plan_for(int M, int N, int K, const Device& d, int split_k, float line) {
+  const Plan single = plan_single(M, N, K, d, std::max(0, split_k), line);
+  if (split_k > 0) return single;
+  const Plan pair = plan_pair(M, N, K, d, line);
+  return pair.us < single.us ? pair : single;
 }
 
 template <class F, class P>
@@ -755,11 +777,7 @@ static int gemm_launch(const void* a, const void* b, void* c, int M, int N, int 
   const int k_tiles = (K + kTileK - 1) / kTileK;
   if (split_k > k_tiles) split_k = k_tiles;
   if (split_k > kMaxSplit) return fail(-2, "mk_gemm_bf16: split_k is at most 8 (one portable thread-block cluster)");
-  Plan plan = plan_single(M, N, K, *d, std::max(0, split_k));
-  if (split_k <= 0) {
-    const Plan other = plan_pair(M, N, K, *d);
-    if (other.us < plan.us) plan = other;
-  }
+  const Plan plan = plan_for(M, N, K, *d, split_k, b_packed ? 1.f : line_cost(b, ldb));
   if (plan.pair)
     return pair_launch(a, b, c, M, N, K, lda, ldb, ldc, workspace, plan, timeout_ms, cuda_stream, b_packed, activation, *d);
   split_k = plan.split;
@@ -816,6 +834,23 @@ int mk_gemm_bf16_packed(const void* a, const void* b_packed, void* c, int M, int
   if (K % 64) return mkg::fail(-2, "mk_gemm_bf16_packed: K must be a multiple of 64 (the packer pads with zeros)");
   return mkg::gemm_launch(a, b_packed, c, M, N, K, lda, K, ldc, workspace, workspace_bytes, split_k, timeout_ms,
                           cuda_stream, true, activation);
+}
+
+int mk_gemm_bf16_plan(int M, int N, int K, int64_t ldb, int32_t out[4]) {
+  using namespace mkg;
+  if (!out || M < 1 || N < 1 || K < 1) return fail(-2, "mk_gemm_bf16_plan: M, N, K must be positive and out given");
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return fail(-1001, "cudaGetDevice failed");
+  const Device* d = device_facts(dev);
+  if (!d) return fail(-1001, "mk_gemm_bf16_plan: cannot read the attributes of device %d", dev);
+  if (d->cc != 10) return fail(-6, "mk_gemm_bf16_plan needs an sm_100 device (compute capability %d.x found)", d->cc);
+  const Plan plan = plan_for(M, N, K, *d, 0, ldb > 0 ? line_cost(nullptr, ldb) : 1.f);
+  const int rows = plan.pair ? plan.rows : std::min(M, kMaxM), tiles = ceil_div(M, rows) * ceil_div(N, plan.pair ? kPairRows : kTileN);
+  out[0] = plan.pair ? 1 : 0;
+  out[1] = plan.split;
+  out[2] = rows;
+  out[3] = tiles;
+  return 0;
 }
 
 int mk_gemm_bf16_status(const void* workspace, int32_t out[4]) {

@@ -5,9 +5,12 @@ several tiles each), odd column counts (no two-column stores), and every activat
 The bar of test_gpu_gemm_sm100.py: one bf16 rounding plus K * 2^-24 relative fp32 accumulation noise; silu adds a
 relative 2^-9 for the exponential and the division."""
 
+import ctypes
+
 import pytest
 import torch
 
+from machete_b200 import _native as native
 from machete_b200.kernels.gemm import gemm_pack_weight, gemm_sm100
 
 pytestmark = pytest.mark.gpu
@@ -54,3 +57,18 @@ def test_results_do_not_depend_on_the_launch_before():
         torch.cuda.synchronize()
         steps.append(bufs[5].clone())
     assert torch.equal(steps[0], steps[1]) and torch.equal(steps[0], steps[2])
+
+
+def _plan(M, N_out, K):
+    out = (ctypes.c_int32 * 4)()
+    assert native.lib().mk_gemm_bf16_plan(M, N_out, K, K, out) == 0
+    return tuple(out)                                         # pair kernel, split, rows per tile, tiles
+
+
+@pytest.mark.parametrize("M,N_out,K", [(66, 8616, 5576), (48, 8160, 5352), (53, 8608, 9360), (76, 9240, 3256),
+                                       (59, 5392, 10760), (91, 5128, 1544)])
+def test_few_rows_use_the_device(M, N_out, K):
+    """Where the weight's bytes are the bound, or nearly, a product must not settle for the fewest CTAs."""
+    pair, split, _, tiles = _plan(M, N_out, K)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert (2 if pair else 1) * split * tiles >= 0.6 * sms
