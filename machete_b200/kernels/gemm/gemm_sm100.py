@@ -113,9 +113,10 @@ def gemm_sm100(a: torch.Tensor, b, c: torch.Tensor, *, activation=None, split_k:
 
 
 def _rows(t: torch.Tensor, width: int):
-    """(rows, row stride) of a tensor whose last dimension is ``width`` and contiguous."""
+    """(rows, row stride) of a tensor whose last dimension is ``width`` and contiguous (one row has no stride)."""
     if t.dim() == 2:
-        return t.shape[0], t.stride(0)
+        rows = t.shape[0]
+        return rows, t.stride(0) if rows > 1 else width
     if t.is_contiguous():
         return t.numel() // width if width else 0, width
     v = t.view(-1, width)                              # raises if the rows are not equally spaced

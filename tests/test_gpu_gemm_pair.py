@@ -72,3 +72,18 @@ def test_few_rows_use_the_device(M, N_out, K):
     pair, split, _, tiles = _plan(M, N_out, K)
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     assert (2 if pair else 1) * split * tiles >= 0.6 * sms
+
+
+@pytest.mark.parametrize("K,N_out", [(256, 264), (2048, 512)])
+def test_one_row_of_any_stride(K, N_out):
+    g = torch.Generator(device="cuda").manual_seed(K)
+    b = (torch.randn(N_out, K, generator=g, device="cuda") * K ** -0.5).to(BF)
+    x = torch.randn(K, generator=g, device="cuda").to(BF)
+    odd = torch.zeros(5, K + 3, dtype=BF, device="cuda")
+    odd[0, :K] = x
+    want = x.double()[None] @ b.double().t()
+    bar = want.abs() * 2.0 ** -8 + (x.double().abs()[None] @ b.double().abs().t()) * K * 2.0 ** -24
+    for a in (x.view(K, 1).t(), x.as_strided((1, K), (0, 1)), odd[0:1, :K]):
+        for c in (torch.zeros(1, N_out, dtype=BF, device="cuda"), torch.zeros(N_out, 1, dtype=BF, device="cuda").t()):
+            gemm_sm100(a, b, c, check_status=True)
+            assert bool(((c.double() - want).abs() <= bar).all())
