@@ -129,10 +129,12 @@ def _fuse_final_add(add_sop: ScheduledOp, head_sop: ScheduledOp, ctx: LowerCtx):
     # the matvec's staging reads and writes 16 bytes at a time; the separate op has no such needs
     if any(t.stride(-1) != 1 or t.data_ptr() % 16 or t.stride(0) % 8 or t.stride(1) % 8 for t in (x, res, total)):
         return None
-    # every CTA re-reads the addends while one of them writes the sum
-    if any(tensor_meta_overlaps(meta_of(total), meta_of(t)) for t in (x, res)):
-        return None
     out = th["logits"]
+    # every CTA reads the addends and the weights while one of them writes the sum, and still reads the addends
+    # while others store logits; the separate ops had a dependency between the two
+    written = ((total, (x, res, th["norm_weight"], th["weight"])), (out, (x, res)))
+    if any(tensor_meta_overlaps(meta_of(w), meta_of(t)) for w, read in written for t in read):
+        return None
     return lower_matvec("FinalAddRmsLmHead", ctx, w0=dense_weight(th["weight"]), x=x, out=out,
                         out_strides=flat_out_strides(out), pro=N.PRO_ADD_RMS, norm_weight=th["norm_weight"],
                         residual_in=res, residual_out=total, eps=float(head_sop.static_dims.get("eps", 1e-5)),
