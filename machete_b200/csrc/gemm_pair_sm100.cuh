@@ -44,9 +44,10 @@ struct PairParams {
 };
 
 struct PairShared {
-  uint64_t full[kPairStages], empty[kPairStages], acc_full[2], acc_empty[2];   // initialised side by side, one lane each
+  uint64_t full[kPairStages], empty[kPairStages], acc_full[2], drained, acc_empty[2];   // initialised side by side, one lane each
   uint32_t tmem_base;
   int32_t abort_flag;
+  int32_t other_issued;            // leader: the K steps that the other CTA's producer has issued, once it is through
 };
 
 // TMA loads of a CTA pair: the data goes to this CTA's shared memory, the completion to `bar`, which may
@@ -86,6 +87,9 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar, uint16_t ranks, uin
       "h"(ranks), "r"(elected)
       : "memory");
 }
+__device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t v) {
+  asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -110,9 +114,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 
   const uint32_t full0 = mk::smem_u32(&sh->full[0]), empty0 = mk::smem_u32(&sh->empty[0]);
   if (warp == 0) {
-    constexpr int kOnes = 2 * kPairStages + 2;
+    constexpr int kOnes = 2 * kPairStages + 3;
     if (lane < kOnes + 2) mk::mbar_init(full0 + 8u * lane, lane < kOnes ? 1 : 2 * kPairEpiWarps);
-    if (lane == 0) sh->abort_flag = 0;
+    if (lane == 0) sh->abort_flag = 0, sh->other_issued = -1;
     mk::fence_mbar_init();
   }
   if (warp == 1) tmem_alloc_pair(mk::smem_u32(&sh->tmem_base), 512);
@@ -153,10 +157,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         }
       }
     }
-    if (lane == 0 && *reinterpret_cast<volatile int32_t*>(&sh->abort_flag)) {
-      // shared memory must outlive the copies in flight (their barrier is the leader's): a bounded wait
+    if (lane == 0 && rank == 1) st_cluster_u32(peer_smem(mk::smem_u32(&sh->other_issued), lead), (uint32_t)it);
+    if (lane == 0 && rank == 0 && *reinterpret_cast<volatile int32_t*>(&sh->abort_flag)) {
+      // Shared memory must outlive the copies in flight.  Both CTAs' copies are counted on the leader's barriers and
+      // neither CTA leaves before the leader is at the cluster barrier, so the leader waits (bounded) for each
+      // slot's last use: once the other producer's count is known, a step that only the other CTA issued is armed
+      // for that half alone.
       const uint64_t t0 = mk::globaltimer_ns();
-      while (mk::globaltimer_ns() - t0 < 50000ull) {
+      const volatile int32_t* other = &sh->other_issued;
+      while (*other < 0 && mk::globaltimer_ns() - t0 < 2 * p.timeout_ns) {
+      }
+      const int last = max(it, (int)*other);
+      for (int i = max(0, last - p.stages); i < last; ++i) {
+        const uint32_t bar = full0 + 8u * (i % p.stages);
+        if (i >= it) mk::mbar_arrive_expect_tx(bar, stage_bytes);
+        while (!mk::mbar_try_wait(bar, (uint32_t)(i / p.stages) & 1u) && mk::globaltimer_ns() - t0 < 3 * p.timeout_ns) {
+        }
       }
     }
   } else if (warp == 1) {
@@ -189,6 +205,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         }
         if (ok && kt1 > kt0) tc_commit_pair(mk::smem_u32(&sh->acc_full[buf]), both, elected);
       }
+      // Whoever has given up: the products in flight still read both CTAs' shared memory and write their tensor memory.
+      tc_commit_pair(mk::smem_u32(&sh->drained), both, elected);
+      wait_drained(p, mk::smem_u32(&sh->drained));
     }
   } else {
     const int q = warp & 3;                               // warp w may touch tensor-memory lanes 32 * (w % 4) ..

@@ -53,7 +53,7 @@ constexpr int kTileK = 64;         // one 128-byte swizzle atom of bf16
 constexpr int kMaxM = 256;         // activation rows per CTA (the MMA's N)
 constexpr int kMaxStages = 8;
 constexpr int kMaxSplit = 8;       // CTAs of one output tile (a portable cluster)
-constexpr int kBars = 2 * kMaxStages + 1;
+constexpr int kBars = 2 * kMaxStages + 2;
 constexpr uint32_t kWBytes = kTileN * kTileK * 2;
 
 struct Params {
@@ -77,6 +77,7 @@ struct Shared {
   uint64_t full[kMaxStages];      // the barriers are initialised side by side, one lane each
   uint64_t empty[kMaxStages];
   uint64_t acc_ready;
+  uint64_t drained;
   uint32_t tmem_base;
   int32_t abort_flag;
 };
@@ -208,6 +209,16 @@ template <class P, class S>
 __device__ __forceinline__ bool wait_bar_warp(const P& p, S* sh, uint32_t bar, uint32_t parity, int code, int role, int aux) {
   if (__all_sync(0xffffffffu, mk::mbar_try_wait(bar, parity))) return true;
   return __all_sync(0xffffffffu, wait_bar(p, sh, bar, parity, code, role, aux));
+}
+
+// The MMA warp waits, for a limited time, until the products that it issued are done: whether all is well (the
+// epilogue waits for the same) or somebody has given up.
+template <class P>
+__device__ __forceinline__ void wait_drained(const P& p, uint32_t bar) {
+  if (__all_sync(0xffffffffu, mk::mbar_try_wait(bar, 0))) return;
+  const uint64_t t0 = mk::globaltimer_ns();
+  while (!__all_sync(0xffffffffu, mk::mbar_try_wait(bar, 0)) && __all_sync(0xffffffffu, mk::globaltimer_ns() - t0 < p.timeout_ns)) {
+  }
 }
 
 template <int ACT>
@@ -398,6 +409,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       }
     }
     if (ok && n_steps > 0) tc_commit(mk::smem_u32(&sh->acc_ready), elected);
+    // Whoever has given up: the products in flight still read shared memory and write tensor memory.
+    tc_commit(mk::smem_u32(&sh->drained), elected);
+    wait_drained(p, mk::smem_u32(&sh->drained));
   }
   // Epilogue on all eight warps: warp w may touch TMEM lanes 32 * (w % 4) .. and takes every second block of
   // 32 activation rows.

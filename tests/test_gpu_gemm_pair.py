@@ -87,3 +87,25 @@ def test_one_row_of_any_stride(K, N_out):
         for c in (torch.zeros(1, N_out, dtype=BF, device="cuda"), torch.zeros(N_out, 1, dtype=BF, device="cuda").t()):
             gemm_sm100(a, b, c, check_status=True)
             assert bool(((c.double() - want).abs() <= bar).all())
+
+
+@pytest.mark.parametrize("split_k", [0, 1, 2])
+def test_a_wait_that_runs_out(split_k):
+    """K is so long that its products take more than the millisecond a wait is given: the kernel gives up in the
+    middle of its stream, with copies and products in flight, reports it, and the next call is right."""
+    M, N_out, K = 300, 3840, 1 << 20
+    if split_k == 0:
+        pair, split, _, _ = _plan(M, N_out, K)
+        assert pair and split > 1                             # 0 takes the pair kernel, the others the single one
+    a = torch.zeros(M, K, dtype=BF, device="cuda")
+    b = torch.zeros(N_out, K, dtype=BF, device="cuda")
+    c = torch.zeros(M, N_out, dtype=BF, device="cuda")
+    with pytest.raises(RuntimeError, match="aborted: wait"):
+        gemm_sm100(a, b, c, split_k=split_k, timeout_ms=1, check_status=True)
+    g = torch.Generator(device="cuda").manual_seed(split_k)
+    a = torch.randn(M, 2048, generator=g, device="cuda").to(BF)
+    b = (torch.randn(N_out, 2048, generator=g, device="cuda") * 2048 ** -0.5).to(BF)
+    gemm_sm100(a, b, c, split_k=split_k, check_status=True)
+    want = a.double() @ b.double().t()
+    bar = want.abs() * 2.0 ** -8 + (a.double().abs() @ b.double().abs().t()) * 2048 * 2.0 ** -24
+    assert bool(((c.double() - want).abs() <= bar).all())
