@@ -17,7 +17,8 @@ pytestmark = pytest.mark.gpu
 BF = torch.bfloat16
 
 SHAPES = [(1, 256, 64), (15, 1000, 1000), (129, 257, 72), (160, 4096, 4096), (255, 512, 2048), (257, 300, 8192),
-          (512, 4096, 512), (777, 1025, 1032), (1031, 5000, 328), (2049, 2304, 264), (96, 19000, 136)]
+          (512, 4096, 512), (777, 1025, 1032), (1031, 5000, 328), (2049, 2304, 264), (96, 19000, 136),
+          (1031, 14001, 328), (2049, 7000, 264)]
 
 
 @pytest.mark.parametrize("M,N_out,K", SHAPES)
@@ -42,27 +43,70 @@ def test_every_cut_against_fp64(M, N_out, K, activation):
 
 
 def test_results_do_not_depend_on_the_launch_before():
-    """Launches overlap their set-up with the kernel before them: a product that reads the one before it sees all of it."""
+    """Launches overlap their set-up with the kernel before them: a product that reads the one before it sees all of
+    it.  Every chain starts from another x0 and from buffers of NaN, so that nothing an earlier chain left is right;
+    long and short products alternate, so that a launch really is placed early."""
     g = torch.Generator(device="cuda").manual_seed(3)
-    w = [(torch.randn(512, 512, generator=g, device="cuda") * 512 ** -0.5).to(BF) for _ in range(6)]
-    x0 = torch.randn(320, 512, generator=g, device="cuda").to(BF)
-    bufs = [torch.zeros(320, 512, dtype=BF, device="cuda") for _ in range(6)]
-    steps = []
-    for rep in range(3):
-        x = x0
-        for i in range(6):
-            x = gemm_sm100(x, w[i], bufs[i])
-            if rep == 0:
-                torch.cuda.synchronize()                      # the first time every step waits for the one before
+    sizes = [512, 512, 4096, 512, 256, 8192, 512]
+    w = [(torch.randn(n, k, generator=g, device="cuda") * k ** -0.5).to(BF) for k, n in zip(sizes, sizes[1:])]
+    x0 = [torch.randn(320, 512, generator=g, device="cuda").to(BF) for _ in range(4)]
+    bufs = [torch.empty(320, n, dtype=BF, device="cuda") for n in sizes[1:]]
+
+    def chain(x, wait):
+        for t in bufs:
+            t.fill_(float("nan"))
         torch.cuda.synchronize()
-        steps.append(bufs[5].clone())
-    assert torch.equal(steps[0], steps[1]) and torch.equal(steps[0], steps[2])
+        for i in range(len(w)):
+            x = gemm_sm100(x, w[i], bufs[i])
+            if wait:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return x.clone()
+
+    want = [chain(x, True) for x in x0]
+    assert all(bool(torch.isfinite(t).all()) for t in want) and not torch.equal(want[0], want[1])
+    for _ in range(3):
+        for x, y in zip(x0, want):
+            assert torch.equal(chain(x, False), y)
 
 
-def _plan(M, N_out, K):
+def _plan(M, N_out, K, ldb=None):
     out = (ctypes.c_int32 * 4)()
-    assert native.lib().mk_gemm_bf16_plan(M, N_out, K, K, out) == 0
+    assert native.lib().mk_gemm_bf16_plan(M, N_out, K, ldb or K, out) == 0
     return tuple(out)                                         # pair kernel, split, rows per tile, tiles
+
+
+def test_the_shapes_above_take_every_cut():
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    cuts = [_plan(*shape) for shape in SHAPES]
+    assert {0, 1} <= {split > 1 for pair, split, _, _ in cuts if pair} and any(split > 1 for pair, split, _, _ in cuts if not pair)
+    assert any(split == 1 for pair, split, _, _ in cuts if not pair)
+    # a pair's two accumulators are waited for, and change their parity, from its third tile on
+    assert sum(tiles > 3 * pairs for pair, split, _, tiles in cuts if pair and split == 1) >= 2
+
+
+@pytest.mark.parametrize("M,N_out,K,split", [(320, 1000, 4096, True), (1031, 9001, 328, False)])
+@pytest.mark.parametrize("pad", [1, 2, 4, 32])
+def test_pair_kernel_on_strided_operands(M, N_out, K, split, pad):
+    """Rows of C that allow four, two or no columns at once (an even, an odd and a 4-byte-aligned row stride), A and B
+    cut from wider buffers; nothing beside C's columns is written."""
+    pair, parts, _, _ = _plan(M, N_out, K, K + 8)
+    assert pair and (parts > 1) == split
+    g = torch.Generator(device="cuda").manual_seed(pad)
+    a = torch.randn(M, K + 16, generator=g, device="cuda").to(BF)[:, :K]
+    b = (torch.randn(N_out, K + 8, generator=g, device="cuda") * K ** -0.5).to(BF)[:, :K]
+    whole = torch.full((M, N_out + pad), 7.0, dtype=BF, device="cuda")
+    c = whole[:, :N_out]
+    gemm_sm100(a, b, c, check_status=True)
+    want = a.double() @ b.double().t()
+    bar = want.abs() * 2.0 ** -8 + (a.double().abs() @ b.double().abs().t()) * K * 2.0 ** -24
+    assert bool(((c.double() - want).abs() <= bar).all())
+    assert bool((whole[:, N_out:] == 7.0).all())
+    if pad == 32:                                             # leading dimensions over equally spaced rows
+        lead = a[:M // 2 * 2].reshape(2, M // 2, K)
+        out = torch.empty(2, M // 2, N_out, dtype=BF, device="cuda")
+        gemm_sm100(lead, b, out, check_status=True)
+        assert bool(((out.view(-1, N_out).double() - want[:M // 2 * 2]).abs() <= bar[:M // 2 * 2]).all())
 
 
 @pytest.mark.parametrize("M,N_out,K", [(66, 8616, 5576), (48, 8160, 5352), (53, 8608, 9360), (76, 9240, 3256),
