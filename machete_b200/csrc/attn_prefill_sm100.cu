@@ -354,7 +354,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     }
   } else if (warp == 1) {
     // Head dim 64 issues as a whole warp (see tc_mma).  At 128 the tensor pipe is the bound either way and one lane
-    // that waits and issues is the lighter neighbour: 4096 x 4096 causal, power-capped, 152.5 us against 154.8.
+    // that waits and issues is the lighter neighbour: 0.9 % faster on average over fifteen prompts that fill the
+    // device, 2.3 % over three that do not (2190 x 2190 causal 52.5 us against 54.5, 1637 x 1637 61.9 against 61.3).
     constexpr bool kOneLane = D == 128;
     if (!kOneLane || lane == 0) {
       auto wait_mma = [&](uint32_t bar, uint32_t parity, int code, int aux) -> bool {

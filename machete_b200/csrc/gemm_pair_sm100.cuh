@@ -16,7 +16,10 @@
 // A problem with few tiles splits K as well: the pairs of one tile form one cluster, each takes a range of the
 // K steps, and their fp32 partial tiles are summed through distributed shared memory (reduce_slice).
 //
-// What bounds it: L2 -> SM bandwidth and, on large problems, the power cap.
+// What bounds it: the tensor pipe and, in a stream of large products, the power cap.  2048 x 4096 -> 14336: 160.6 us
+// alone (the tensor pipe active in 93 % of the SMs' active cycles, 12.8 TB/s from L2, DRAM 14 %; the clock at
+// 1.55 GHz), 178.6 us one after another: 1347 TFLOP/s of the 1383 that cuBLAS sustains under the cap.  The single
+// kernel, which draws 48 KB a K step into an SM instead of 32, takes 229.
 #pragma once
 
 namespace mkg {

@@ -1,25 +1,27 @@
-// Small-M bf16 GEMM on the 5th-generation tensor cores: C[M,N] = A[M,K] · B[N,K]^T.
+// bf16 GEMM on the 5th-generation tensor cores: C[M,N] = A[M,K] · B[N,K]^T.
 //
-// The decode path's own matvec ops cover M <= 32 with mma.sync; from M = 64 up the
-// work is worth a tcgen05 tile.  The problem is still weight-streaming bound
-// (M <= 256 rows against an N x K weight), so the tile is laid out around the
-// weight stream: the WEIGHT rows are the 128-row "M" operand of tcgen05.mma and the
-// activation rows are its "N" operand (16..256 columns), i.e. the kernel computes
-// C^T tile by tile.  One CTA owns 128 weight rows x one K range:
+// The decode path's own matvec ops cover M <= 32 with mma.sync; any M is taken here,
+// by one of two kernels (plan_for chooses).  Up to some 256 rows the problem is bound
+// by the weight's bytes, so the tile is laid out around the weight stream: the WEIGHT
+// rows are the 128-row "M" operand of tcgen05.mma and the activation rows are its "N"
+// operand (16..256 columns), i.e. the kernels compute C^T tile by tile.  More rows run
+// as CTA pairs on tiles of 256 weight rows (gemm_pair_sm100.cuh).  In the kernel of
+// this file one CTA owns 128 weight rows x one K range:
 //
 //   warp 0   TMA producer: per 64-wide K step one 128 x 64 weight box and one
 //            Mpad x 64 activation box (128-byte swizzle) into a ring of stages;
-//   warp 1   allocates tensor memory, issues tcgen05.mma (one thread), hands
-//            stages back with tcgen05.commit;
-//   warps 2-5 epilogue: tcgen05.ld of the fp32 accumulator (TMEM lane = weight
+//   warp 1   allocates tensor memory, issues tcgen05.mma (as a whole warp, one
+//            elected lane by predicate), hands stages back with tcgen05.commit;
+//   all warps epilogue: tcgen05.ld of the fp32 accumulator (TMEM lane = weight
 //            row, column = activation row) and bf16 stores.
 //
-// One SM cannot keep enough reads in flight to draw more than roughly 1/148 of the
-// HBM bandwidth, so a weight with few 128-row tiles is also split along K: the CTAs
-// of one output tile form a thread-block cluster, each leaves its fp32 partial tile
-// in its own shared memory (the stage ring is free by then), and after a cluster
-// barrier every CTA sums one slice of the rows over all peers through distributed
-// shared memory and stores it.  No global workspace and no atomics are involved.
+// One SM draws some 0.16 MB/us through its stages (85 CTAs 3.4 TB/s of HBM, 72 with
+// fewer activation rows a step 5.1), and a K step takes 0.2 us at least, so a weight
+// with few 128-row tiles is also split along K: the CTAs of one output tile form a
+// thread-block cluster, each leaves its fp32 partial tile in its own shared memory
+// (the stage ring is free by then), and after a cluster barrier every CTA sums one
+// slice of the rows over all peers through distributed shared memory and stores it.
+// No global workspace and no atomics are involved.
 //
 // Takes the place of the reference's GemmSm100Op (src/machete/kernels/gemm/
 // gemm_sm100.py:56-658), which tiles (S, N) with a double-buffered K loop inside

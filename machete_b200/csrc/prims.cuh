@@ -166,9 +166,6 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1,
 // from the shared-space address: the compiler may then schedule them freely
 // between the barriers (which are asm volatile with a memory clobber) instead
 // of keeping every load in program order, as it must for asm volatile loads.
-// Explicit ld.shared / st.shared with 32-bit shared-space addresses.  They are
-// asm volatile (ordered against the barrier waits, which clobber memory); the
-// hot loops therefore issue their loads in batches ahead of the mma's by hand.
 // Packed 16-bit arithmetic, every result rounded once.
 __device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
   uint32_t d;
@@ -185,6 +182,9 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
   asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
 }
+// Explicit ld.shared / st.shared with 32-bit shared-space addresses.  They are
+// asm volatile (ordered against the barrier waits, which clobber memory); the
+// hot loops therefore issue their loads in batches ahead of the mma's by hand.
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));

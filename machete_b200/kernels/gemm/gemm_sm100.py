@@ -11,7 +11,7 @@ returns the scheduled-op record (tile grid, tensor metadata) and ``GemmSm100Op.l
 from __future__ import annotations
 
 import ctypes as C
-from typing import Dict, Optional, Tuple
+from typing import Dict, Optional
 
 import torch
 
@@ -22,8 +22,7 @@ TILE_N = 128     # weight rows per CTA
 TILE_M = 256     # activation rows per CTA
 TILE_K = 64
 
-_WORKSPACE_BYTES = 256     # what mk_gemm_bf16_workspace_bytes answers
-_workspaces: Dict[Tuple[int, int], torch.Tensor] = {}
+_workspaces: Dict[int, torch.Tensor] = {}     # by device: the status block has the same size for every product
 
 
 def _check(rc: int, what: str) -> None:
@@ -34,14 +33,14 @@ def _check(rc: int, what: str) -> None:
 
 
 def gemm_workspace(M: int, N_out: int, K: int, device) -> torch.Tensor:
-    """A zeroed workspace for ``gemm_sm100`` (cached per device and size; the kernel leaves it zero)."""
-    need = int(N.lib().mk_gemm_bf16_workspace_bytes(M, N_out, K))    # the status block: the same for every size
+    """A zeroed workspace for ``gemm_sm100`` (cached per device; the kernel leaves it zero)."""
+    need = int(N.lib().mk_gemm_bf16_workspace_bytes(M, N_out, K))
     dev = torch.device(device)
-    key = (dev.index if dev.index is not None else torch.cuda.current_device(), need)
-    ws = _workspaces.get(key)
-    if ws is None:
+    idx = dev.index if dev.index is not None else torch.cuda.current_device()
+    ws = _workspaces.get(idx)
+    if ws is None or ws.numel() < need + 256:
         ws = torch.zeros(need + 256, dtype=torch.uint8, device=dev)
-        _workspaces[key] = ws
+        _workspaces[idx] = ws
     return ws
 
 
@@ -99,7 +98,7 @@ def gemm_sm100(a: torch.Tensor, b, c: torch.Tensor, *, activation=None, split_k:
     M, lda = _rows(a, K)
     _, ldc = _rows(c, n_out)
     idx = a.device.index
-    ws = workspace if workspace is not None else _workspaces.get((idx, _WORKSPACE_BYTES))
+    ws = workspace if workspace is not None else _workspaces.get(idx)
     if ws is None:
         ws = gemm_workspace(M, n_out, K, a.device)
     ptr = ws.data_ptr()
@@ -160,7 +159,8 @@ class GemmSm100Op(Op):
     @classmethod
     def schedule(cls, tile_sizes=None, page_size=DEFAULT_PAGE_SIZE, activation=None, **tensors):
         """``tile_sizes`` (``S`` in {64, 128, 256}, ``N``, ``K``) shape the scheduled-op record as in the
-        reference; the kernel's own tile is fixed (128 weight rows x up to 256 activation rows x 64)."""
+        reference; the kernels choose their own tiles (128 or, as CTA pairs, 256 weight rows x up to 256
+        activation rows x 64)."""
         if activation not in ACTIVATIONS:
             raise ValueError(f"Unknown activation: {activation}")
         ts = dict(tile_sizes or {})

@@ -93,7 +93,8 @@ def lower_program(ops: List[ScheduledOp], ctx: LowerCtx) -> List[NativeOp]:
                 i += 2
                 continue
         if ctx.fuse and out and i + 1 < len(ops):
-            # (a program of these two ops alone has no decode step beside it and keeps them as they are)
+            # (a program that begins with the pair, a final stage by itself, keeps the two ops of its schedule: it has
+            # no decode step before it whose matvecs and attention would gain from the smaller kernel variant)
             head = _fuse_final_add(sop, ops[i + 1], ctx)
             if head is not None:
                 out.append(head)
