@@ -135,7 +135,8 @@ enum {
   MK_AT_CAUSAL, MK_AT_MT, MK_AT_TS /* tokens per split */, MK_AT_O_T,
   /* MK_OP_ATTN_SPLIT only: 1 = the unit that completes a (batch, kv head,
    * query tile) group also combines the group's splits into o / lse, so no
-   * separate MK_OP_ATTN_COMBINE op (and no dependency stage) is needed */
+   * separate MK_OP_ATTN_COMBINE op (and no dependency stage) is needed (the
+   * library makes it 2 in its own record where one trip fetches the lse values) */
   MK_AT_FUSE_COMBINE,
   /* MK_OP_ATTN_SPLIT only: 1 = q and the cache row MK_AT_NEW_TOK of k hold
    * UNROTATED projections; the op applies the per-head RMSNorm (weights

@@ -156,6 +156,12 @@ static int encode_kv_map(CUtensorMap* out, uint64_t base, int D, int HKV, int N,
 static int build_op_maps(mk_op_t& op, CUtensorMap* maps, uint64_t dev_maps, int page_bytes) {
   if (op.opcode == MK_OP_ATTN_SPLIT || op.opcode == MK_OP_ATTN_COMBINE)
     op.i[MK_AT_GROUP] = op.i[MK_AT_H] / op.i[MK_AT_HKV];   // validated: H a positive multiple of HKV
+  if (op.opcode == MK_OP_ATTN_SPLIT && op.i[MK_AT_FUSE_COMBINE]) {
+    // 2: the combine fetches the lse values of a pass (the rows that a warp takes together) in one trip, four a lane.
+    // Decided here: the product and the compare in the kernel cost an 8B-shape step 0.4 % (2842 -> 2856 us).
+    const int rows = std::min(op.i[MK_AT_GROUP], 256 / op.i[MK_AT_D]);
+    op.i[MK_AT_FUSE_COMBINE] = op.i[MK_AT_M] == 1 && rows * op.i[MK_AT_SPLITS] <= 128 ? 2 : 1;
+  }
   if (op.opcode == MK_OP_ATTN_SPLIT) {
     const int D = op.i[MK_AT_D];
     const uint32_t tn = (uint32_t)at_page_tokens(D, page_bytes);

@@ -141,7 +141,7 @@ __device__ __forceinline__ void at_combine_group(Ctx& c, const mk_op_t* op, cons
         }
       }
       if (s0 == 0) {
-        if (M == 1 && nr * S <= 128) {
+        if (op->i[MK_AT_FUSE_COMBINE] == 2) {
           // one query token: the group's lse values are contiguous, (row, split) -> row * S + split, and four a
           // lane share one trip (more of them take the loop below)
           const float* l0 = lpart + ((int64_t)u.b * H + (int64_t)u.kvh * G + u.mt * 16 + r0) * S;
