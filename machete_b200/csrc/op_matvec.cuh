@@ -43,6 +43,11 @@ __device__ __forceinline__ uint32_t mv_half_bytes(int wfmt, int Kc) {
   return mv_is_fp4(wfmt) ? (uint32_t)(Kc / 256) * 1024u : (uint32_t)(Kc / 64) * 1024u;
 }
 
+// Row stride of the staged activations, bytes.  The eight lanes of a shared-memory phase read two rows (g, g + 1) at
+// four 16-byte chunks, 32 bytes apart with bf16 / fp16 weights: an odd multiple of 16 bytes from row to row makes the
+// eight distinct (64 bytes, pairs of them on the same banks: 1B-shape step at 16 rows 2060 us against 2018).
+__device__ __forceinline__ uint32_t mv_row_stride(int K, bool fp4) { return (uint32_t)K * 2u + (fp4 ? 64u : 16u); }
+
 // What the loader needs to issue the pages of one unit (from the instruction record).
 struct MvLoad {
   const void* tm_a;
@@ -159,7 +164,8 @@ __device__ __forceinline__ void mv_stage(Ctx& c, const mk_op_t* op, bool stage, 
   const int at = WFC == 0 ? (int)MK_T_BF16 : (WFC == 2 ? (int)MK_T_FP16 : mv_act_type(op));
   // a bf16 kernel always takes the RMSNorm scale in the epilogue: the second pass is not even compiled
   const bool fused = WFC == 0 ? pro != MK_PRO_NONE : (WFC != 2 && mv_rstd_in_epilogue(op));
-  const uint32_t xs = (uint32_t)K * 2u + 64u;
+  const bool fp4 = WFC == 0 ? false : (WFC == 2 ? true : mv_is_fp4(op->i[MK_MV_WFMT]));
+  const uint32_t xs = mv_row_stride(K, fp4);
   const int chunks = K >> 3;
   const uint16_t* x = reinterpret_cast<const uint16_t*>(op->p[MK_MV_P_X]);
   const uint16_t* ri = reinterpret_cast<const uint16_t*>(op->p[MK_MV_P_RES_IN]);
@@ -514,7 +520,7 @@ __device__ __forceinline__ bool mv_unit(Ctx& c, const mk_op_t* op, const UnitArg
   const int K = op->i[MK_MV_K], Kc = op->i[MK_MV_KC], M = op->i[MK_MV_M];
   const int wfmt = WFC == 0 ? (int)MK_W_BF16 : op->i[MK_MV_WFMT];
   const bool dense = WFC == 0 ? true : (WFC == 2 ? false : (wfmt == MK_W_BF16 || wfmt == MK_W_FP16));
-  const uint32_t xs = (uint32_t)K * 2u + 64u;
+  const uint32_t xs = mv_row_stride(K, !dense);
   const uint32_t half = mv_half_bytes(wfmt, Kc);
   const int NPG = c.pv->n_pages;
   if (part == 0 && op->i[MK_MV_EPI] == MK_EPI_RESIDUAL && op->i[MK_MV_S] == 1) {
@@ -556,11 +562,13 @@ __device__ __forceinline__ bool mv_unit(Ctx& c, const mk_op_t* op, const UnitArg
       // One K-tile = 64 K-values = 8 chunks of 16 B per row; this thread takes
       // chunks 2t and 2t+1 of rows g (half A) and g (half B): with the 128-byte
       // swizzle the 8 lanes of a shared-memory phase then hit 8 distinct chunks.
-      // The mma wrappers are asm volatile, which the compiler does not move
-      // loads across, so the software pipeline is written out by hand: tiles
-      // are handled two at a time and (for one activation n-tile) the
-      // fragments of the next pair are requested before the mma's of the
-      // current pair are issued.
+      // Tiles are handled in pairs.  A warp issues in order, a 16-byte shared load
+      // costs it 13 cycles and a product 11 to 15 (one warp on its scheduler; 32 from
+      // one product to the next on the same accumulator), so all loads of a pair
+      // followed by all its products take the sum of both.  The loads of the next
+      // pair are therefore dealt out between the products of this one (1B-shape step, one row: 866 -> 830 us; one
+      // 4096 -> 14336 product 25.4 -> 24.2).
+      // Rows past M read row 0: their columns of the accumulators are never stored.
       const int tiles = kc >> 6;
       const uint32_t off0 = (uint32_t)g * 128u + (uint32_t)(((2 * t) ^ g) << 4);      // chunk 2t of row g
       const uint32_t off1 = (uint32_t)g * 128u + (uint32_t)(((2 * t + 1) ^ g) << 4);  // chunk 2t+1
@@ -568,68 +576,70 @@ __device__ __forceinline__ bool mv_unit(Ctx& c, const mk_op_t* op, const UnitArg
       struct Frag {
         uint4 wa[2][2], wb[2][2], x[NT][2][2];   // [tile of the pair][chunk j]
       };
+      constexpr int kLoads = 8 + 4 * NT, kProducts = 8 * NT;
+      auto load_one = [&](Frag& f, int kt, int i) {   // load i of the pair's kLoads, in the order of use
+        const int per = 4 + 2 * NT, u = i / per, r = i % per;
+        const uint32_t ta = page + (uint32_t)(kt + u) * 1024u, tb = ta + half;
+        if (r == 0) f.wa[u][0] = lds128(ta + off0);
+        else if (r == 1) f.wb[u][0] = lds128(tb + off0);
+        else if (r < 2 + NT) f.x[r - 2][u][0] = lds128(xrow[r - 2] + xo0 + (uint32_t)(kt + u) * 128u);
+        else if (r == 2 + NT) f.wa[u][1] = lds128(ta + off1);
+        else if (r == 3 + NT) f.wb[u][1] = lds128(tb + off1);
+        else f.x[r - 4 - NT][u][1] = lds128(xrow[r - 4 - NT] + xo0 + (uint32_t)(kt + u) * 128u + 16u);
+      };
       auto load_pair = [&](Frag& f, int kt) {
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const uint32_t ta = page + (uint32_t)(kt + u) * 1024u, tb = ta + half;
-          f.wa[u][0] = lds128(ta + off0);
-          f.wa[u][1] = lds128(ta + off1);
-          f.wb[u][0] = lds128(tb + off0);
-          f.wb[u][1] = lds128(tb + off1);
-#pragma unroll
-          for (int nt = 0; nt < NT; ++nt) {
-            // always load (rows past M read row 0 and are zeroed): no branch in the hot loop
-            const uint4 x0 = lds128(xrow[nt] + xo0 + (uint32_t)(kt + u) * 128u);
-            const uint4 x1 = lds128(xrow[nt] + xo0 + (uint32_t)(kt + u) * 128u + 16u);
-            const uint32_t keep = xok[nt] ? 0xffffffffu : 0u;
-            f.x[nt][u][0] = make_uint4(x0.x & keep, x0.y & keep, x0.z & keep, x0.w & keep);
-            f.x[nt][u][1] = make_uint4(x1.x & keep, x1.y & keep, x1.z & keep, x1.w & keep);
-          }
+        for (int i = 0; i < kLoads; ++i) load_one(f, kt, i);
+      };
+      // Product i of a pair.  The two products on one 16-byte chunk feed the same accumulator; the
+      // first halves of all chunks come before the second halves, which keeps them several issue
+      // slots apart.  (The order on each accumulator fixes the bits of the result.)
+      auto mma_one = [&](const Frag& f, int i, int valid, auto is_bf16) {
+        const int hf = i / (4 * NT), u = i / (2 * NT) % 2, j = i / NT % 2, nt = i % NT, a = (u * 2 + j) % NA;
+        if (u < valid) {
+          const uint32_t a0 = hf ? f.wa[u][j].z : f.wa[u][j].x, a1 = hf ? f.wb[u][j].z : f.wb[u][j].x;
+          const uint32_t a2 = hf ? f.wa[u][j].w : f.wa[u][j].y, a3 = hf ? f.wb[u][j].w : f.wb[u][j].y;
+          const uint32_t b0 = hf ? f.x[nt][u][j].z : f.x[nt][u][j].x;
+          const uint32_t b1 = hf ? f.x[nt][u][j].w : f.x[nt][u][j].y;
+          if constexpr (decltype(is_bf16)::value)
+            mma_bf16(acc[a][nt], a0, a1, a2, a3, b0, b1);
+          else
+            mma_f16(acc[a][nt], a0, a1, a2, a3, b0, b1);
         }
       };
-      // The two mma's on one 16-byte chunk feed the same accumulator; issuing
-      // the first halves of all chunks before the second halves keeps dependent
-      // mma's several issue slots apart.
       auto mma_pair = [&](const Frag& f, int valid, auto is_bf16) {
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
+        for (int i = 0; i < kProducts; ++i) mma_one(f, i, valid, is_bf16);
+      };
+      auto step = [&](const Frag& f, Frag& next, int kt_next, auto is_bf16) {
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            if (u < valid) {
+        for (int i = 0; i < kProducts; ++i) {
 #pragma unroll
-              for (int j = 0; j < 2; ++j) {
-                constexpr int kSets = NA;
-                const int a = (u * 2 + j) % kSets;
-#pragma unroll
-                for (int nt = 0; nt < NT; ++nt) {
-                  const uint32_t a0 = half ? f.wa[u][j].z : f.wa[u][j].x, a1 = half ? f.wb[u][j].z : f.wb[u][j].x;
-                  const uint32_t a2 = half ? f.wa[u][j].w : f.wa[u][j].y, a3 = half ? f.wb[u][j].w : f.wb[u][j].y;
-                  const uint32_t b0 = half ? f.x[nt][u][j].z : f.x[nt][u][j].x;
-                  const uint32_t b1 = half ? f.x[nt][u][j].w : f.x[nt][u][j].y;
-                  if constexpr (decltype(is_bf16)::value)
-                    mma_bf16(acc[a][nt], a0, a1, a2, a3, b0, b1);
-                  else
-                    mma_f16(acc[a][nt], a0, a1, a2, a3, b0, b1);
-                }
-              }
-            }
-          }
+          for (int l = i * kLoads / kProducts; l < (i + 1) * kLoads / kProducts; ++l) load_one(next, kt_next, l);
+          mma_one(f, i, 2, is_bf16);
         }
       };
       // A page always holds whole tiles up to its capacity (TMA zero-fills past
       // K), so reading the second tile of the last pair is safe even when odd.
       auto run_page = [&](auto is_bf16) {
-        if constexpr (NT == 1) {
+        if constexpr (NT <= 2) {
           Frag f0, f1;
           load_pair(f0, 0);
+          int kt = 0;
 #pragma unroll 1
-          for (int kt = 0; kt < tiles; kt += 4) {
-            if (kt + 2 < tiles) load_pair(f1, kt + 2);
-            mma_pair(f0, min(2, tiles - kt), is_bf16);
-            if (kt + 2 < tiles) {
-              if (kt + 4 < tiles) load_pair(f0, kt + 4);
-              mma_pair(f1, min(2, tiles - kt - 2), is_bf16);
+          for (;;) {
+            if (kt + 2 >= tiles) {
+              mma_pair(f0, tiles - kt, is_bf16);
+              break;
             }
+            step(f0, f1, kt + 2, is_bf16);
+            kt += 2;
+            if (kt + 2 >= tiles) {
+              mma_pair(f1, tiles - kt, is_bf16);
+              break;
+            }
+            step(f1, f0, kt + 2, is_bf16);
+            kt += 2;
           }
         } else {
           Frag f;
