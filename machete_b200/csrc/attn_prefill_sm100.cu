@@ -7,8 +7,9 @@
 // sm_100.py:88-…, dispatch attention/__init__.py:16-130) as a launch of its own, so that a prompt can
 // fill the KV cache the decode kernel then reads.
 //
-// One CTA = one (batch, query head, tile of 128 query rows); KV tiles of 64 tokens; two CTAs share an SM
-// (<= 97 KB of shared memory and 256 tensor-memory columns each):
+// One CTA = one (batch, tile of 128 query rows), the rows being 128 / g queries of the g query heads that share a KV
+// head (the power of two in the group); KV tiles of 64 tokens; two CTAs share an SM (<= 97 KB of shared memory and 256
+// tensor-memory columns each; three at head dim 64 where that saves a round, see the launch):
 //
 //   warp 0     TMA: Q once, then K and V tiles (both double-buffered, K one tile ahead of V) as
 //              64-column boxes, 128-byte swizzle;
@@ -46,7 +47,13 @@
 
 namespace mkp {
 
-constexpr int kThreads = 192;
+// The kernel has two forms: two S accumulators, two CTAs to an SM, a warp for the loads, one for the products and four
+// of row threads; and (head dim 64) one S accumulator, three CTAs to an SM, one warp for loads and products, so that
+// the SM's 15 warps are four to a scheduler and a thread may use 128 registers (with 18 it is 96).
+template <int SB>
+constexpr int kThreads = SB == 1 ? 160 : 192;
+template <int SB>
+constexpr int kCtasPerSm = SB == 1 ? 3 : 2;
 constexpr int kBM = 128;   // query rows per CTA
 constexpr int kBN = 64;    // tokens per KV tile
 constexpr uint32_t kBox = 128 * 64 * 2;   // one 128-row x 64-column bf16 box
@@ -58,6 +65,7 @@ struct Params {
   int64_t o_sb, o_sh, o_sm;
   int B, H, Hkv, M, N, D;
   int causal;
+  int pack, pack_log2;   // query heads of a KV head in one tile: row r is query r >> pack_log2 of head r & (pack - 1)
   int next_early;        // the kernel behind this one may be placed from the start (else: with the last load)
   float scale_log2;      // scale * log2(e)
   uint64_t timeout_ns;
@@ -267,8 +275,9 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 
-template <int D>
-__global__ void __launch_bounds__(kThreads, 2)
+// SB = S accumulators.  (The barriers k_empty, v_empty and all second ones belong to the form with two.)
+template <int D, int SB>
+__global__ void __launch_bounds__(kThreads<SB>, kCtasPerSm<SB>)
 prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                const __grid_constant__ CUtensorMap map_v, const Params p) {
   constexpr int NB = D / 64;                       // 64-column boxes per row tile
@@ -286,16 +295,20 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   // Blocks are handed out in the order x, y, z: the query tile is the slowest index and runs from the LAST tile
   // down, so that under a causal mask the tiles with the most KV tiles start first and the short ones fill the
   // tail (longest job first).
-  const int mt = (int)(gridDim.z - 1 - blockIdx.z), h = blockIdx.x, b = blockIdx.y;
-  const int kvh = h / (p.H / p.Hkv);
-  const int m0 = mt * kBM;
+  // The tile's 128 rows are 128 / pack queries of `pack` heads that share a KV head: a prompt of 777 queries and four
+  // heads a KV head is 25 tiles, not 4 x 7, and fewer pairs lie behind the diagonal (32 / 8 heads, causal, us before and
+  // after: 2190 x 2190 head dim 128 45.2 / 40.5, 64 39.6 / 35.5; 1960 of 2045, four sequences, 159.5 / 146.6 and
+  // 133.2 / 118.3; 4096 x 4096 128.3 / 125.5 and 107.2 / 103.7).
+  const int mt = (int)(gridDim.z - 1 - blockIdx.z), h0 = blockIdx.x * p.pack, b = blockIdx.y;
+  const int kvh = h0 / (p.H / p.Hkv);
+  const int tile_m = kBM >> p.pack_log2;
+  const int m0 = mt * tile_m;
   // tokens this query tile can see: all N, or (causal) up to the diagonal of its last row
-  const int n_vis = p.causal ? min(p.N, p.N - p.M + m0 + kBM) : p.N;
+  const int n_vis = p.causal ? min(p.N, p.N - p.M + m0 + tile_m) : p.N;
   const int n_tiles = n_vis > 0 ? (n_vis + kBN - 1) / kBN : 0;
-  // 256 tensor-memory columns and at most ~100 KB of shared memory per CTA, so that TWO CTAs share an SM.
-  // Two S accumulators at columns [0, 64) / [64, 128) (P, as bf16 pairs, overwrites the first 32 columns of
-  // the accumulator it was computed from), O at [128, 128 + D).
-  constexpr uint32_t kOCol = 2 * kBN, kCols = 256;
+  // The S accumulators of 64 columns come first (P, as bf16 pairs, overwrites the first 32 columns of the accumulator
+  // it was computed from), O behind them.
+  constexpr uint32_t kOCol = SB * kBN, kCols = SB == 1 ? 128 : 256;
   static_assert(kOCol + D <= kCols, "accumulators must fit the allocation");
 
   if (threadIdx.x == 0) {
@@ -312,7 +325,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     sh->abort_flag = 0;
     mk::fence_mbar_init();
   }
-  if (warp == 1) tmem_alloc(mk::smem_u32(&sh->tmem_base), kCols);
+  constexpr int kMmaWarp = SB == 1 ? 0 : 1;
+  __syncwarp();
+  if (warp == kMmaWarp) tmem_alloc(mk::smem_u32(&sh->tmem_base), kCols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -321,11 +336,77 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   if (p.next_early) mk::next_may_start();
 
   // Tile j uses slot j & 1 of every double-buffered resource; its barrier phase is (j >> 1) & 1.
-  if (warp == 0) {
+  if (SB == 1 && warp == 0) {
+    // Loads and products from one warp: S(0), then for every tile P V(j) and S(j + 1) once P(j) is there.  When it is,
+    // S(j) and P V(j - 1) are finished (the row threads read S(j), which was issued behind P V(j - 1)), so K(j + 2) and
+    // V(j + 1) may follow into their slots with no barrier of their own.
+    const uint32_t id_s = idesc_bf16(kBN, false), id_o = idesc_bf16(D, true);
+    const bool one = elect_one();
+    const uint32_t elected = one ? 1u : 0u;
+    auto load_kv = [&](int j, bool is_v) {
+      if (j >= n_tiles) return;
+      const uint32_t fb = mk::smem_u32(is_v ? &sh->v_full[j & 1] : &sh->k_full[j & 1]);
+      const uint32_t dst = (is_v ? v_s : k_s) + (uint32_t)(j & 1) * kKVTile;
+      if (one) {
+        mk::mbar_arrive_expect_tx(fb, kKVTile);
+        for (int x = 0; x < NB; ++x) tma_load_4d(dst + x * kKVBox, is_v ? &map_v : &map_k, x * 64, j * kBN, kvh, b, fb);
+      }
+    };
+    if (one) {
+      const uint32_t qb = mk::smem_u32(&sh->q_full);
+      mk::mbar_arrive_expect_tx(qb, kTile);
+      for (int x = 0; x < NB; ++x) tma_load_4d(q_s + x * kBox, &map_q, x * 64, h0, m0, b, qb);
+    }
+    load_kv(0, false);
+    load_kv(0, true);
+    load_kv(1, false);
+    bool ok = wait_bar_warp(p, sh, mk::smem_u32(&sh->q_full), 0, PF_ST_TIMEOUT_FULL, -1);
+    auto issue_s = [&](int j) -> bool {
+      const int s = j & 1;
+      if (!wait_bar_warp(p, sh, mk::smem_u32(&sh->k_full[s]), (uint32_t)(j >> 1) & 1u, PF_ST_TIMEOUT_FULL, j)) return false;
+      tc_fence_after();
+#pragma unroll
+      for (int k = 0; k < D / 16; ++k) {
+        const uint32_t in_box = (uint32_t)(k & 3) * 32u;
+        tc_mma(tmem, desc_kmajor(q_s + (uint32_t)(k >> 2) * kBox + in_box),
+               desc_kmajor(k_s + s * kKVTile + (uint32_t)(k >> 2) * kKVBox + in_box), id_s, k > 0 ? 1u : 0u, elected);
+      }
+      tc_commit(mk::smem_u32(&sh->s_ready[0]), elected);
+      return true;
+    };
+    if (ok && n_tiles > 0) ok = issue_s(0);
+    for (int j = 0; j < n_tiles && ok; ++j) {
+      const int s = j & 1;
+      ok = wait_bar_warp(p, sh, mk::smem_u32(&sh->p_ready[0]), (uint32_t)j & 1u, PF_ST_TIMEOUT_P, j);
+      if (!ok) break;
+      load_kv(j + 2, false);
+      load_kv(j + 1, true);
+      if (j + 2 >= n_tiles) mk::next_may_start();
+      ok = wait_bar_warp(p, sh, mk::smem_u32(&sh->v_full[s]), (uint32_t)(j >> 1) & 1u, PF_ST_TIMEOUT_FULL, j);
+      if (!ok) break;
+      tc_fence_after();
+#pragma unroll
+      for (int k = 0; k < kBN / 16; ++k) {
+        // P: 16 tokens = 8 tensor-memory columns of bf16 pairs; V: MN-major, 16 tokens = 16 rows of 128 bytes
+        const uint64_t dv = desc_mnmajor(v_s + (uint32_t)s * kKVTile + (uint32_t)k * 2048u, kKVBox);
+        tc_mma_ts(tmem + kOCol, tmem + (uint32_t)k * 8u, dv, id_o, (j > 0 || k > 0) ? 1u : 0u, elected);
+      }
+      // (the tensor cores run the products in this order: S(j + 1) overwrites P(j) behind P V(j))
+      if (j + 1 < n_tiles) ok = issue_s(j + 1);
+      else tc_commit(mk::smem_u32(&sh->pv_done[0]), elected);
+    }
+    mk::next_may_start();
+    if (*reinterpret_cast<volatile int32_t*>(&sh->abort_flag)) {
+      // shared memory must outlive the copies in flight: a bounded wait for whatever was issued last
+      const uint64_t t0 = mk::globaltimer_ns();
+      while (mk::globaltimer_ns() - t0 < 20000ull) {
+      }
+    }
+  } else if (SB == 2 && warp == 0) {
     if (lane == 0) {
       const uint32_t qb = mk::smem_u32(&sh->q_full);
       mk::mbar_arrive_expect_tx(qb, kTile);
-      for (int x = 0; x < NB; ++x) tma_load_4d(q_s + x * kBox, &map_q, x * 64, m0, h, b, qb);
+      for (int x = 0; x < NB; ++x) tma_load_4d(q_s + x * kBox, &map_q, x * 64, h0, m0, b, qb);
       auto load_kv = [&](int j, bool is_v) -> bool {
         const int s = j & 1;
         const uint32_t ph = (uint32_t)(j >> 1) & 1u;
@@ -352,7 +433,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         }
       }
     }
-  } else if (warp == 1) {
+  } else if (SB == 2 && warp == 1) {
     // Head dim 64 issues as a whole warp (see tc_mma).  At 128 the tensor pipe is the bound either way and one lane
     // that waits and issues is the lighter neighbour: 0.9 % faster on average over fifteen prompts that fill the
     // device, 2.3 % over three that do not (2190 x 2190 causal 52.5 us against 54.5, 1637 x 1637 61.9 against 61.3).
@@ -407,21 +488,21 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     // row threads: warp w may touch tensor-memory lanes 32 * (w % 4) ..
     const int qd = warp & 3;
     const int row = qd * 32 + lane;                 // query row inside the tile = TMEM lane
-    const int m = m0 + row;
+    const int m = m0 + (row >> p.pack_log2), h = h0 + (row & (p.pack - 1));
     const int lim = p.causal ? (p.N - p.M + m) : (p.N - 1);   // last visible token of this row
     const uint32_t lane_addr = tmem + ((uint32_t)(qd * 32) << 16);
     const uint64_t scale2 = pack2(p.scale_log2, p.scale_log2);
     float mx = -INFINITY, sum = 0.f;
     bool ok = true;
     for (int j = 0; j < n_tiles; ++j) {
-      ok = wait_bar(p, sh, mk::smem_u32(&sh->s_ready[j & 1]), (uint32_t)(j >> 1) & 1u, PF_ST_TIMEOUT_S, j);
+      ok = wait_bar(p, sh, mk::smem_u32(&sh->s_ready[j & (SB - 1)]), (uint32_t)(j / SB) & 1u, PF_ST_TIMEOUT_S, j);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
       // Only the tiles on the causal diagonal and the last one of a ragged cache need the per-score
       // mask: `open` is true (for the whole warp) everywhere else.
       const bool open = __all_sync(0xffffffffu, (j * kBN + kBN - 1 <= lim) && (j * kBN + kBN <= p.N));
-      const uint32_t s_addr = lane_addr + (uint32_t)(j & 1) * kBN;
+      const uint32_t s_addr = lane_addr + (uint32_t)(j & (SB - 1)) * kBN;
       uint32_t r[kBN];                               // this row of S, then of P (bf16 pairs in r[0 .. 32))
       tmem_ld64(s_addr, r);
       if (!open) {
@@ -447,11 +528,14 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       }
       if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
         // O is free only after the previous P V has finished with it.  S(j) was issued after P V(j - 2), so
-        // that phase of this barrier is behind us and the parity is unambiguous.
-        ok = wait_bar(p, sh, mk::smem_u32(&sh->pv_done[(j - 1) & 1]), (uint32_t)((j - 1) >> 1) & 1u, PF_ST_TIMEOUT_O, j);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        tc_fence_after();
+        // that phase of this barrier is behind us and the parity is unambiguous.  (With one accumulator S(j) was
+        // issued after P V(j - 1), and its commit covers both.)
+        if (SB == 2) {
+          ok = wait_bar(p, sh, mk::smem_u32(&sh->pv_done[(j - 1) & 1]), (uint32_t)((j - 1) >> 1) & 1u, PF_ST_TIMEOUT_O, j);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          tc_fence_after();
+        }
 #pragma unroll 1
         for (int c = 0; c < D; c += 32) {
           uint32_t o[32];
@@ -497,12 +581,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       tmem_st32(s_addr, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
       tmem_wait_st();
       tc_fence_before();
-      mk::mbar_arrive(mk::smem_u32(&sh->p_ready[j & 1]));
+      mk::mbar_arrive(mk::smem_u32(&sh->p_ready[j & (SB - 1)]));
     }
     // epilogue: O / sum -> bf16
     if (ok && n_tiles > 0) {
-      ok = wait_bar(p, sh, mk::smem_u32(&sh->pv_done[(n_tiles - 1) & 1]), (uint32_t)((n_tiles - 1) >> 1) & 1u,
-                    PF_ST_TIMEOUT_O, n_tiles);
+      ok = wait_bar(p, sh, mk::smem_u32(&sh->pv_done[(n_tiles - 1) & (SB - 1)]),
+                    SB == 1 ? 0u : (uint32_t)((n_tiles - 1) >> 1) & 1u, PF_ST_TIMEOUT_O, n_tiles);
       ok = __all_sync(0xffffffffu, ok);
     }
     tc_fence_after();
@@ -539,7 +623,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   }
   __syncthreads();
   tc_fence_after();
-  if (warp == 1) tmem_dealloc(tmem, kCols);
+  if (warp == kMmaWarp) tmem_dealloc(tmem, kCols);
 }
 
 static std::string g_err;
@@ -567,8 +651,28 @@ static EncodeTiledFn encode_fn() {
   fn = reinterpret_cast<EncodeTiledFn>(sym);
   return fn;
 }
+// The query rows with the heads inside: dims (D, heads, rows, batch), one box = 64 columns x `pack` heads x 128 / pack
+// queries, which lands as 128 rows of 128 bytes, the heads of a query one behind the other.
+static int encode_query_map(CUtensorMap* out, const void* base, int D, int rows, int heads, int batch, int64_t s_r,
+                            int64_t s_h, int64_t s_b, int pack) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail(-5, "cuTensorMapEncodeTiled is not available from this driver");
+  if (((uint64_t)base & 15) || (s_r * 2) % 16 || (s_h * 2) % 16 || (s_b * 2) % 16 || s_r <= 0 || s_h <= 0 || s_b <= 0)
+    return fail(-2, "mk_flash_prefill_bf16: q must be 16-byte aligned with positive row / head / batch strides that are "
+                    "multiples of 8 elements");
+  cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)heads, (cuuint64_t)rows, (cuuint64_t)batch};
+  cuuint64_t strides[3] = {(cuuint64_t)s_h * 2, (cuuint64_t)s_r * 2, (cuuint64_t)s_b * 2};
+  cuuint32_t box[4] = {64, (cuuint32_t)pack, (cuuint32_t)(kBM / pack), 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(-5, "cuTensorMapEncodeTiled (q) failed with CUresult %d", (int)r);
+  return 0;
+}
+
 // [batch][head][row][D] with element strides (s_b, s_h, s_r), D contiguous: dims (D, rows, heads, batch),
-// one box = 64 columns x 128 rows of one head of one batch entry.
+// one box = 64 columns x `box_rows` rows of one head of one batch entry.
 static int encode_rows_map(CUtensorMap* out, const void* base, int D, int rows, int heads, int batch, int64_t s_r,
                            int64_t s_h, int64_t s_b, int box_rows, const char* what) {
   EncodeTiledFn fn = encode_fn();
@@ -607,8 +711,9 @@ static const Device* device_facts(int dev) {
           cudaDeviceGetAttribute(&d.cc, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess)
         return nullptr;
       if (d.cc == 10 &&
-          (cudaFuncSetAttribute(prefill_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem_optin) != cudaSuccess ||
-           cudaFuncSetAttribute(prefill_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem_optin) != cudaSuccess))
+          (cudaFuncSetAttribute(prefill_kernel<64, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem_optin) != cudaSuccess ||
+           cudaFuncSetAttribute(prefill_kernel<64, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem_optin) != cudaSuccess ||
+           cudaFuncSetAttribute(prefill_kernel<128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem_optin) != cudaSuccess))
         return nullptr;
       facts[dev] = d;
       known[dev].store(true, std::memory_order_release);
@@ -646,7 +751,10 @@ int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, 
   const int smem_optin = d->smem_optin;
   const int bn = kBN;                              // tokens per KV tile
   CUtensorMap mq, mkk, mv;
-  int rc = encode_rows_map(&mq, q, D, M, H, B, q_strides[2], q_strides[1], q_strides[0], kBM, "q");
+  // the largest power of two that divides the group, as long as the tiles fit the grid
+  int pack = (H / Hkv) & -(H / Hkv);
+  while (pack > kBM || (pack > 1 && (M + kBM / pack - 1) / (kBM / pack) > 65535)) pack >>= 1;
+  int rc = encode_query_map(&mq, q, D, M, H, B, q_strides[2], q_strides[1], q_strides[0], pack);
   if (rc) return rc;
   rc = encode_rows_map(&mkk, k, D, N, Hkv, B, k_strides[2], k_strides[1], k_strides[0], bn, "k");
   if (rc) return rc;
@@ -662,18 +770,28 @@ int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, 
   p.o_sb = o_strides[0], p.o_sh = o_strides[1], p.o_sm = o_strides[2];
   p.B = B, p.H = H, p.Hkv = Hkv, p.M = M, p.N = N, p.D = D;
   p.causal = causal ? 1 : 0;
+  p.pack = pack;
+  p.pack_log2 = 0;
+  while ((1 << p.pack_log2) < pack) ++p.pack_log2;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.timeout_ns = (uint64_t)(timeout_ms > 0 ? timeout_ms : 1000) * 1000000ull;
-  const dim3 grid(H, B, (M + kBM - 1) / kBM);
+  const int tile_m = kBM / pack;
+  const dim3 grid(H / pack, B, (M + tile_m - 1) / tile_m);
   // Where this grid leaves slots empty (two CTAs an SM), the next one is let in late: its CTAs would pile up on the
   // SMs that are free now (the average over six such prompts at head dim 64 11 % faster, three at 128 3.5 %).  With
   // every slot taken nothing piles up, and at head dim 64 (1960 behind 2045 tokens 84.8 us early, 86.7 late) the
   // last load is too short before the end to hide the placement; at 128 (0.4 % faster late) it is not.
-  p.next_early = D == 64 && (int64_t)grid.x * grid.y * grid.z >= 2 * (int64_t)d->sms ? 1 : 0;
+  const int64_t tiles = (int64_t)grid.x * grid.y * grid.z;
+  // Three CTAs an SM do no more per time than two (4096 x 4096, 1024 tiles: 109 us, 104), but each tile then takes half
+  // as long again (1024 x 1024, 256 tiles: 19.6 us, 14.1): they are taken where all tiles are on the device at once
+  // and with two a second round would follow (777 behind 2223 tokens, two sequences, 400 tiles: 59.4 us, 73.9 as
+  // 448 tiles of one head each in two rounds).
+  const bool three = D == 64 && tiles > 2 * (int64_t)d->sms && tiles <= 3 * (int64_t)d->sms;
+  p.next_early = D == 64 && !three && tiles >= 2 * (int64_t)d->sms ? 1 : 0;
   // the kernel may be placed while the one before it in the stream drains (it waits before it touches memory)
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
-  cfg.blockDim = dim3(kThreads);
+  cfg.blockDim = dim3(three ? kThreads<1> : kThreads<2>);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = reinterpret_cast<cudaStream_t>(cuda_stream);
   cudaLaunchAttribute attr[1];
@@ -681,8 +799,9 @@ int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = D == 64 ? cudaLaunchKernelEx(&cfg, prefill_kernel<64>, mq, mkk, mv, p)
-                          : cudaLaunchKernelEx(&cfg, prefill_kernel<128>, mq, mkk, mv, p);
+  cudaError_t e = three ? cudaLaunchKernelEx(&cfg, prefill_kernel<64, 1>, mq, mkk, mv, p)
+                  : D == 64 ? cudaLaunchKernelEx(&cfg, prefill_kernel<64, 2>, mq, mkk, mv, p)
+                            : cudaLaunchKernelEx(&cfg, prefill_kernel<128, 2>, mq, mkk, mv, p);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return fail(-(int)e - 1000, "mk_flash_prefill_bf16 launch: %s", cudaGetErrorString(e));
   return 0;
