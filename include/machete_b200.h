@@ -68,7 +68,12 @@ enum { MK_MV_PLAIN = 0, MK_MV_PAIR = 1, MK_MV_ROPE = 2 };
 /* matvec prologues */
 enum { MK_PRO_NONE = 0, MK_PRO_RMS = 1, MK_PRO_ADD_RMS = 2 };
 /* matvec epilogues */
-enum { MK_EPI_STORE = 0, MK_EPI_RESIDUAL = 1, MK_EPI_TOP1 = 2 };
+enum { MK_EPI_STORE = 0, MK_EPI_RESIDUAL = 1, MK_EPI_TOP1 = 2,
+       /* one of MK_MV_KBLOCKS ops that hold a K block each of one product and run side by side: a unit leaves its sums
+        * (times the global scale) in p[MK_MV_P_KPART], and the last of the MK_MV_KBLOCKS units of the same rows adds
+        * them in block order, rounded to the output type after every block, and stores.  The result of the chain
+        * "y = block 0; y = y + block 1; ..." in one dependency stage. */
+       MK_EPI_KSUM = 3 };
 /* matvec transforms applied to the accumulators before the epilogue */
 enum { MK_TR_NONE = 0, MK_TR_ROPE = 1, MK_TR_SILU_MUL = 2, MK_TR_RELU = 3, MK_TR_SILU = 4 };
 /* weight formats */
@@ -105,7 +110,9 @@ enum {
    * one-token buffer (q) sets the first bit only.  The reference bakes the
    * position into the schedule and re-schedules per token
    * (kernels/decode_matvec/sm100.py:116, 704-709). */
-  MK_MV_DYNPOS
+  MK_MV_DYNPOS,
+  /* MK_EPI_KSUM: number of blocks, and this op's index among them */
+  MK_MV_KBLOCKS, MK_MV_KBLOCK
 };
 enum { MK_MV_DYN_TABLES = 1, MK_MV_DYN_OUT = 2 };
 /* GSCALE / GSCALE1: fp32 global scale of W0 / of W1 (MK_MV_PAIR; block-scaled NVFP4 only) */
@@ -118,6 +125,9 @@ enum {
    * filled in by mk_create and mk_update_op, callers leave them zero */
   MK_MV_P_TM_W0, MK_MV_P_TM_W1, MK_MV_P_TM_SC0, MK_MV_P_TM_SC1
 };
+/* MK_EPI_KSUM (no prologue): fp32[n_units][MK_MV_KBLOCKS][n-tiles of 8 rows][128] and int32[n_units] arrival counters,
+ * zero before the first launch (the kernel leaves them zero); the ops of one product share both */
+enum { MK_MV_P_KPART = MK_MV_P_RES_IN, MK_MV_P_KARRIVE = MK_MV_P_RES_OUT };
 enum {
   MK_MV_S_WROW = 0,   /* weight row stride, bytes                         */
   MK_MV_S_X_B, MK_MV_S_X_S,           /* x strides, elements              */

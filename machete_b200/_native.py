@@ -23,17 +23,18 @@ OP_NOP, OP_MATVEC, OP_ATTN_SPLIT, OP_ATTN_COMBINE, OP_RMSNORM, OP_ROPE, OP_QKNOR
     OP_TOP1_FINAL, OP_ALLREDUCE = range(11)
 MV_PLAIN, MV_PAIR, MV_ROPE = range(3)
 PRO_NONE, PRO_RMS, PRO_ADD_RMS = range(3)
-EPI_STORE, EPI_RESIDUAL, EPI_TOP1 = range(3)
+EPI_STORE, EPI_RESIDUAL, EPI_TOP1, EPI_KSUM = range(4)
 TR_NONE, TR_ROPE, TR_SILU_MUL, TR_RELU, TR_SILU = range(5)
 W_BF16, W_FP16, W_NVFP4_F16S32, W_NVFP4_E4M3S16 = range(4)
 T_BF16, T_FP16, T_FP32 = range(3)
 
 (MV_O, MV_K, MV_M, MV_S, MV_MODE, MV_PRO, MV_EPI, MV_TR, MV_HD, MV_D2, MV_POS, MV_WFMT, MV_KC, MV_OUT_T,
- MV_X_T, MV_ROWS_PER_UNIT, MV_SPLIT, MV_IDX0, MV_DYNPOS) = range(19)
+ MV_X_T, MV_ROWS_PER_UNIT, MV_SPLIT, MV_IDX0, MV_DYNPOS, MV_KBLOCKS, MV_KBLOCK) = range(21)
 MV_DYN_TABLES, MV_DYN_OUT = 1, 2
 MV_F_EPS, MV_F_GSCALE, MV_F_GSCALE1 = range(3)
 (MV_P_W0, MV_P_W1, MV_P_X, MV_P_RES_IN, MV_P_NORM_W, MV_P_RES_OUT, MV_P_OUT, MV_P_EPI_RES, MV_P_COS,
  MV_P_SIN, MV_P_SC0, MV_P_SC1) = range(12)
+MV_P_KPART, MV_P_KARRIVE = MV_P_RES_IN, MV_P_RES_OUT
 (MV_S_WROW, MV_S_X_B, MV_S_X_S, MV_S_RI_B, MV_S_RI_S, MV_S_RO_B, MV_S_RO_S, MV_S_O_B, MV_S_O_S, MV_S_O_H,
  MV_S_ER_B, MV_S_ER_S, MV_S_COS, MV_S_SCROW) = range(14)
 

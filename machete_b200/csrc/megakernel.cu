@@ -330,6 +330,13 @@ static int validate_op(const mk_op_t& op, int idx, int page_bytes, int act_bytes
     }
     if (op.i[MK_MV_TR] == MK_TR_ROPE && mode != MK_MV_ROPE) return fail(-2, "op %d: rope transform needs rope mode", idx);
     if (op.i[MK_MV_TR] == MK_TR_SILU_MUL && mode != MK_MV_PAIR) return fail(-2, "op %d: silu-mul needs pair mode", idx);
+    if (op.i[MK_MV_EPI] == MK_EPI_KSUM) {
+      const int n = op.i[MK_MV_KBLOCKS], b = op.i[MK_MV_KBLOCK];
+      if (n < 2 || b < 0 || b >= n || mode != MK_MV_PLAIN || op.i[MK_MV_PRO] != MK_PRO_NONE || op.i[MK_MV_TR] != MK_TR_NONE)
+        return fail(-2, "op %d: a K block is one of at least two plain products without prologue and transform", idx);
+      if (!op.p[MK_MV_P_KPART] || (op.p[MK_MV_P_KPART] & 3) || !op.p[MK_MV_P_KARRIVE] || (op.p[MK_MV_P_KARRIVE] & 3))
+        return fail(-2, "op %d: K blocks need the partial sums' buffer and the arrival counters", idx);
+    }
     if (op.i[MK_MV_EPI] == MK_EPI_RESIDUAL && !op.p[MK_MV_P_EPI_RES]) return fail(-2, "op %d: epilogue residual missing", idx);
     if (op.n_units != units) return fail(-2, "op %d: expected %d units, got %d", idx, units, op.n_units);
   } else if (op.opcode == MK_OP_ATTN_SPLIT || op.opcode == MK_OP_ATTN_COMBINE) {

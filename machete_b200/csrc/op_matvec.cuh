@@ -368,7 +368,8 @@ __device__ __forceinline__ void mv_epilogue(Ctx& c, const mk_op_t* op, const MvO
   const int xt = WFC == 0 ? (int)MK_T_BF16 : op->i[MK_MV_X_T];
   const int ot = op->i[MK_MV_OUT_T];
   // block-scaled NVFP4: one fp32 scale per matrix (rows a and b come from two matrices in pair mode)
-  const bool gscaled = WFC != 0 && op->i[MK_MV_WFMT] == MK_W_NVFP4_E4M3S16;
+  // (K blocks: the parts were scaled before they were added)
+  const bool gscaled = WFC != 0 && op->i[MK_MV_WFMT] == MK_W_NVFP4_E4M3S16 && epi != MK_EPI_KSUM;
   const float gs = gscaled ? op->f[MK_MV_F_GSCALE] : 1.f;
   const float gsb = (gscaled && mode == MK_MV_PAIR) ? op->f[MK_MV_F_GSCALE1] : gs;
   const bool fused = WFC == 0 ? op->i[MK_MV_PRO] != MK_PRO_NONE : (WFC != 2 && mv_rstd_in_epilogue(op));
@@ -496,6 +497,55 @@ __device__ __forceinline__ void e2m1x8_scaled(uint32_t w, uint32_t scale, uint32
 // Swizzled address of 16-byte chunk `c` of row `r` (0-7) inside a 1 KB tile.
 __device__ __forceinline__ uint32_t tile_chunk(uint32_t tile, int r, int c) {
   return tile + (uint32_t)r * 128u + (uint32_t)((c ^ r) << 4);
+}
+
+// The K blocks of one product (MK_EPI_KSUM).  A block's sums go to global memory; the unit that completes the rows (one
+// acq_rel atomic, as for the attention splits) replaces `acc` by the sum of all blocks in block order, rounded to the
+// output type after each, which is what the chain of stores and residual adds computes.  Returns whether this unit
+// was the last.  A chain of n ops is n dependency stages, each with a staging on all CTAs, for 1/n of the bytes:
+// the down projection of the 1B shape at 16 rows took 41 us of a layer's 117 as four ops, 15 so.
+__device__ __forceinline__ float mv_round(float v, int ot) {
+  return ot == MK_T_BF16 ? bf16_round(v) : (ot == MK_T_FP16 ? f16lo(pack_f16(v, 0.f)) : v);
+}
+template <int NT, int WFC>
+__device__ __forceinline__ bool mv_kblock_sum(Ctx& c, const mk_op_t* op, int unit, float (&acc)[NT][4]) {
+  constexpr int R = NT * 4;
+  const int n = op->i[MK_MV_KBLOCKS], ot = op->i[MK_MV_OUT_T];
+  const float gs = WFC != 0 && op->i[MK_MV_WFMT] == MK_W_NVFP4_E4M3S16 ? op->f[MK_MV_F_GSCALE] : 1.f;
+  float* parts = reinterpret_cast<float*>(op->p[MK_MV_P_KPART]) + (size_t)unit * n * (R * 32) + c.lane;
+  float* mine = parts + op->i[MK_MV_KBLOCK] * (R * 32);
+#pragma unroll
+  for (int i = 0; i < R; ++i) mine[i * 32] = __fmul_rn(acc[i >> 2][i & 3], gs);
+  __syncwarp();
+  int last = 0;
+  if (c.lane == 0) {
+    int32_t* arrive = reinterpret_cast<int32_t*>(op->p[MK_MV_P_KARRIVE]) + unit;
+    int32_t old;
+    asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(old) : "l"(arrive) : "memory");
+    last = old == n - 1;
+    if (last) *arrive = 0;   // ready for the next launch
+  }
+  last = __shfl_sync(0xffffffffu, last, 0);
+  if (!last) return false;
+  constexpr int G = NT <= 2 ? 4 : 2;   // blocks fetched together
+#pragma unroll 1
+  for (int b0 = 0; b0 < n; b0 += G) {
+    float v[G][R];
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+#pragma unroll
+      for (int i = 0; i < R; ++i) v[g][i] = b0 + g < n ? __ldcg(parts + ((b0 + g) * R + i) * 32) : 0.f;
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      if (b0 + g >= n) break;
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        float& a = acc[i >> 2][i & 3];
+        a = mv_round(b0 + g == 0 ? v[g][i] : __fadd_rn(v[g][i], a), ot);
+      }
+    }
+  }
+  return true;
 }
 
 // NT = n-tiles of 8 activation rows; NA = independent accumulator sets (the
@@ -763,6 +813,7 @@ __device__ __forceinline__ bool mv_unit(Ctx& c, const mk_op_t* op, const UnitArg
     }
   }
   trace(c, TRC_MV_REDUCED, ord);
+  if (op->i[MK_MV_EPI] == MK_EPI_KSUM && !mv_kblock_sum<NT, WFC>(c, op, u.unit, acc[0])) return true;
   MvOut r;
   r.rowA0 = ins_field(u.mine->row_a, u.idx);
   r.rowB0 = ins_field(u.mine->row_b, u.idx);

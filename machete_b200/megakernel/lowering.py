@@ -91,6 +91,10 @@ class NativeOp:
     kind: str = ""         # free-form tag used by peephole rules and tests
     # an op that follows the device-resident cache position: first position its tensors do not hold
     pos_limit: Optional[int] = None
+    # ops that share this object write the same memory in any order (the K blocks of one product)
+    commutes: Optional[object] = None
+    # (i, n): the units go to every n-th CTA, the i-th of them first (ops that run side by side)
+    cta_share: Optional[Tuple[int, int]] = None
     # scratch that must be zero when a launch starts; the kernel leaves it zero unless a launch aborted
     zero_on_reset: list = field(default_factory=list)
 
@@ -134,6 +138,8 @@ class LowerCtx:
     kc_bf16: int = 1024
     kc_fp4: int = 2048
     fuse: bool = True
+    # scratch that fused ops of the program share, by what it is (the ops' regions order its use)
+    scratch: dict = field(default_factory=dict)
     # shortest bf16 K-slice to pick for ops with few units per CTA (0 = never shorten).  Off by default:
     # on B200 the extra pages cost more than the extra warps per unit gain (931 vs 916 us per Llama-1B step)
     small_op_kc: int = 0

@@ -61,9 +61,18 @@ class BackwardScheduler(TileScheduler):
     def place(self, ops, num_ctas):
         out, rr = [], 0
         for op in ops:
-            out.append(((np.arange(op.n_units, dtype=np.int64) + rr) % num_ctas).astype(np.int32))
+            mine = shared_ctas(op, (np.arange(num_ctas) + rr) % num_ctas)
+            out.append(mine[np.arange(op.n_units) % len(mine)].astype(np.int32))
             rr = (rr + op.n_units) % num_ctas
         return out
+
+
+def shared_ctas(op: NativeOp, order: np.ndarray) -> np.ndarray:
+    """The CTAs of ``order`` that may hold units of ``op`` (``NativeOp.cta_share``), in that order."""
+    if op.cta_share is None or op.cta_share[1] > len(order):
+        return order
+    i, n = op.cta_share
+    return order[order % n == i]
 
 
 class OverlapTileScheduler(TileScheduler):
@@ -103,8 +112,8 @@ class OverlapTileScheduler(TileScheduler):
         load = np.zeros(num_ctas, dtype=np.int64)
         out = []
         for op in ops:
-            order = np.argsort(load, kind="stable").astype(np.int32)
-            a = order[np.arange(op.n_units) % num_ctas].astype(np.int32)
+            order = shared_ctas(op, np.argsort(load, kind="stable").astype(np.int32))
+            a = order[np.arange(op.n_units) % len(order)].astype(np.int32)
             for u in range(op.n_units):
                 # a unit with no streamed bytes still costs a little time
                 load[a[u]] += max(op.bytes_of(u), 2048)
@@ -130,21 +139,22 @@ def infer_dependencies(ops: Sequence[NativeOp]) -> List[OpDeps]:
     result: List[OpDeps] = []
     for j, op in enumerate(ops):
         found: Dict[int, bool] = {}  # producer -> needed by a loader-side read?
+        side = set() if op.commutes is None else {i for i in range(j) if ops[i].commutes is op.commutes}
         act_version: List[int] = []
         for r in op.reads:
             latest = -1
             for i, w in writes_by_storage.get(r.meta.storage_ptr, ()):
-                if i != j and r.overlaps(w):
+                if i != j and i not in side and r.overlaps(w):
                     found[i] = found.get(i, False) or r.loader
                     latest = max(latest, i)
             if r.act:
                 act_version.append(latest)
         for w in op.writes:
             for i, w2 in writes_by_storage.get(w.meta.storage_ptr, ()):
-                if i != j and w.overlaps(w2):
+                if i != j and i not in side and w.overlaps(w2):
                     found.setdefault(i, False)
             for i, r2 in reads_by_storage.get(w.meta.storage_ptr, ()):
-                if i != j and w.overlaps(r2):
+                if i != j and i not in side and w.overlaps(r2):
                     found.setdefault(i, False)
         # transitive reduction: drop i when another kept producer already implies it
         cand = sorted(found, reverse=True)
