@@ -84,6 +84,16 @@ __device__ __forceinline__ LoaderInstr bcast_loader_instr(const LoaderInstr& m, 
   return r;
 }
 
+// Which kernels take the forms for whole decode steps of several rows or NVFP4 weights: a loader that issues under
+// elect_one, units found by one vote (see consumer_loop), attention states in the staging buffer (see at_unit).
+// Together, on one GPU: 8B shape, NVFP4, one row, KV 8192 2866 -> 2754 us a step, 8 rows, KV 4096 4925 -> 4706; 1B shape,
+// 16 rows, KV 1931 1627 -> 1529.  Programs of projections alone (bf16 1 x 4096 -> 14336 24.7 us, 25.4 so; NVFP4 4 rows
+// 19.5, 19.9) and bf16 steps of up to 8 rows (829 us, 840) lose by them: their few units a CTA are found in a step or
+// two, and a page is two copies for twice the bytes.
+template <int NTC, int WFC, int FEAT>
+constexpr bool kWideStep = NTC >= 0 && (NTC != 1 || WFC != 0) && (FEAT & (MK_F_AT64 | MK_F_AT128)) != 0;
+
+template <bool ELECT>
 static __device__ void loader_loop(Ctx& c, int ibeg, int iend) {
   const ProgramView& pv = *c.pv;
   const int NP = pv.n_pages;
@@ -116,7 +126,7 @@ static __device__ void loader_loop(Ctx& c, int ibeg, int iend) {
         trace(c, TRC_LWAIT_DONE, base + i);
       }
       if (ins.maps == 0) continue;   // only units with tensor maps stream pages
-      // Pages are issued by lane 0 alone in a tight loop from the fields of the
+      // Pages are issued by one lane alone in a tight loop from the fields of the
       // instruction record (no op-table read on this path; a one-thread wait
       // needs no vote).  Fill k of a slot needs fill k-1 handed back:
       // empty-barrier phase k-1.  A split-KV attention page is one K box and one
@@ -124,8 +134,8 @@ static __device__ void loader_loop(Ctx& c, int ibeg, int iend) {
       // (plus two scale boxes for NVFP4).
       const bool attn = (ins.flags & MK_LDF_ATTN) != 0;
       if (attn && need_wait) fence_proxy_async_all();   // the awaited K/V rows were written by plain stores
-      int issued = 0;
-      if (c.lane == 0) {
+      int issued = 0, leader = 0;
+      if (ELECT ? elect_one(leader) : c.lane == 0) {
         const uint8_t* maps = reinterpret_cast<const uint8_t*>(ins.maps);
         const bool pair = (ins.flags & MK_LDF_PAIR) != 0;
         MvLoad ml;
@@ -153,7 +163,7 @@ static __device__ void loader_loop(Ctx& c, int ibeg, int iend) {
           trace(c, TRC_LOAD_ISSUED, seq + issued);
         }
       }
-      issued = __shfl_sync(0xffffffffu, issued, 0);
+      issued = __shfl_sync(0xffffffffu, issued, leader);
       if (issued < n_pages) c.dead = true;   // lane 0 gave up (abort flag is already raised)
       ring_advance(rp, issued, NP);
       seq += (uint32_t)issued;
@@ -183,7 +193,7 @@ __device__ __forceinline__ bool run_unit(Ctx& c, const mk_op_t* op, const UnitAr
     if (opcode == MK_OP_MATVEC) return mv_dispatch<NTC, WFC, FEAT>(c, op, u);
   }
   if constexpr ((FEAT & (MK_F_AT64 | MK_F_AT128)) != 0) {
-    if (opcode == MK_OP_ATTN_SPLIT) return at_dispatch<FEAT>(c, op, u);
+    if (opcode == MK_OP_ATTN_SPLIT) return at_dispatch<FEAT, kWideStep<NTC, WFC, FEAT>>(c, op, u);
   }
   if constexpr ((FEAT & MK_F_COMBINE) != 0) {
     if (opcode == MK_OP_ATTN_COMBINE) {
@@ -238,8 +248,9 @@ __device__ void consumer_loop(Ctx& c, int ibeg, int iend, int ebeg, int eend) {
   // not shared), and a consumer that becomes free draws the next ticket, so a
   // warp that is held up (by an epilogue, by a page that is late) never has
   // a fixed share of later work waiting behind it.  Tickets rise, so each
-  // consumer walks the instruction list forward only; passing an op-entry
+  // consumer moves through the instruction list forward only; passing an op-entry
   // event on the way means taking part in it.
+  constexpr bool kVote = kWideStep<NTC, WFC, FEAT>;
   int i = ibeg;          // instruction under the cursor
   int base = ibeg;       // `mine` holds the records of [base, base + 32)
   uint32_t first_slot = 0;  // ticket of the first slot of instruction i
@@ -247,7 +258,58 @@ __device__ void consumer_loop(Ctx& c, int ibeg, int iend, int ebeg, int eend) {
   rp_i.slot = 0;
   rp_i.k = 0;
   InsRegs mine = empty_instr();
-  if (base + c.lane < iend) mine = load_instr(pv.instrs + base + c.lane);
+  // kVote: every lane also holds what the records before its own add up to, and the unit that owns a ticket is found
+  // with one vote.  (Walking the list record by record takes a warp 1.8 us from unit to unit of a long op, as long as
+  // the work on one NVFP4 page.)
+  uint32_t first = 0, seq = 0, mvs = 0, ats = 0;      // tickets, ring pages, shared matvec and attention units
+  auto tickets_of = [&]() -> uint32_t {               // of this lane's unit (0: no record)
+    const uint32_t split = (uint32_t)(mine.flags >> MK_LDF_SPLIT_SHIFT) & MK_LDF_SPLIT_MASK;
+    return base + c.lane >= iend ? 0u : ((mine.flags & kInsMatvec) != 0 ? split : 1u);
+  };
+  auto load_window = [&](uint32_t t0, uint32_t s0, uint32_t m0, uint32_t a0) {
+    mine = empty_instr();
+    if (base + c.lane < iend) mine = load_instr(pv.instrs + base + c.lane);
+    if (mine.flags & MK_LDF_DYN) {
+      // the pages in use, and with them the participants, follow the device-resident position
+      mine.n_pages = at_dyn_pages(mine.row_a, mine.n_pages,
+                                  at_page_tokens((mine.flags & MK_LDF_D128) ? 128 : 64, pv.page_bytes),
+                                  c.ctrl->pos[(mine.row_b >> 16) & 31] + 1);
+      const int split = max(1, min((mine.flags >> MK_LDF_SPLIT_SHIFT) & MK_LDF_SPLIT_MASK, mine.n_pages));
+      mine.flags = (mine.flags & ~(MK_LDF_SPLIT_MASK << MK_LDF_SPLIT_SHIFT)) | (split << MK_LDF_SPLIT_SHIFT);
+    }
+    // tickets | shared matvec units << 16 | shared attention units << 24, and ring pages
+    const uint32_t tk = tickets_of();
+    const uint32_t own = tk | (tk > 1 ? ((mine.flags & MK_LDF_ATTN) ? 1u << 24 : 1u << 16) : 0u);
+    uint32_t sum = own, sum_s = (uint32_t)mine.n_pages;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, sum, o), w2 = __shfl_up_sync(0xffffffffu, sum_s, o);
+      if (c.lane >= o) {
+        sum += v;
+        sum_s += w2;
+      }
+    }
+    sum -= own;
+    first = t0 + (sum & 0xffffu);
+    mvs = m0 + ((sum >> 16) & 0xffu);
+    ats = a0 + (sum >> 24);
+    seq = s0 + sum_s - (uint32_t)mine.n_pages;
+  };
+  // the window that begins at instruction `at` of this one (at <= 32)
+  auto move_window = [&](int at) {
+    const bool end = at == 32;
+    const uint32_t tk = end ? tickets_of() : 0u;
+    const bool attn = (mine.flags & MK_LDF_ATTN) != 0;
+    const int src = end ? 31 : at;
+    const uint32_t t0 = __shfl_sync(0xffffffffu, first + tk, src);
+    const uint32_t s0 = __shfl_sync(0xffffffffu, seq + (end ? (uint32_t)mine.n_pages : 0u), src);
+    const uint32_t m0 = __shfl_sync(0xffffffffu, mvs + (tk > 1 && !attn ? 1u : 0u), src);
+    const uint32_t a0 = __shfl_sync(0xffffffffu, ats + (tk > 1 && attn ? 1u : 0u), src);
+    base += at;
+    load_window(t0, s0, m0, a0);
+  };
+  if constexpr (kVote) load_window(0, 0, 0, 0);
+  else if (base + c.lane < iend) mine = load_instr(pv.instrs + base + c.lane);
 
   // An event record is held one word per lane (mk_event_t is 16 words); its
   // position alone is kept in a register of its own.
@@ -277,9 +339,13 @@ __device__ void consumer_loop(Ctx& c, int ibeg, int iend, int ebeg, int eend) {
     const int nxt_w = load_ev(ev + 1);
     // refill the instruction window here, off the critical path, when it is half used
     if (i - base >= 16) {
-      base = i;
-      mine = empty_instr();
-      if (base + c.lane < iend) mine = load_instr(pv.instrs + base + c.lane);
+      if constexpr (kVote) {
+        move_window(i - base);
+      } else {
+        base = i;
+        mine = empty_instr();
+        if (base + c.lane < iend) mine = load_instr(pv.instrs + base + c.lane);
+      }
     }
     // The first warp to arrive polls the producers' counters while the others
     // finish their units of the previous op.
@@ -302,6 +368,7 @@ __device__ void consumer_loop(Ctx& c, int ibeg, int iend, int ebeg, int eend) {
     bulk_done = &c.ctrl->bulk_done[k & 1];
     cached_op = e_op;
     cached_rec = op;
+    if (kWideStep<NTC, WFC, FEAT> && op->opcode == MK_OP_ATTN_SPLIT) staged_key = 0;   // its states go to the staging buffer
     if constexpr (NTC >= 0) {
       if (op->opcode == MK_OP_MATVEC) {
         const bool need = (op->act_key == 0) || (op->act_key != staged_key);
@@ -329,40 +396,68 @@ __device__ void consumer_loop(Ctx& c, int ibeg, int iend, int ebeg, int eend) {
     ticket = __shfl_sync(0xffffffffu, ticket, 0);
     bool found = false;
     int n_pages = 0, lflags = 0;
-    for (;;) {
-      // events due before instruction i; the ones behind the last instruction are
-      // taken when the cursor reaches the end of the list (every event position is
-      // at most the length of the list), so this is the only place events run
-      while (cur_pos <= i - ibeg) do_event();
-      if (i >= iend) break;
-      if (i - base >= 32) {
-        base = i;
-        mine = empty_instr();
-        if (base + c.lane < iend) mine = load_instr(pv.instrs + base + c.lane);
+    if constexpr (kVote) {
+      for (;;) {
+        // the record that owns the ticket, or the end of the window
+        const int at = __ffs(__ballot_sync(0xffffffffu, ticket - first < tickets_of())) - 1;
+        const bool here = at >= 0;
+        const int target = here ? base + at : min(base + 32, iend);
+        // events due before it; the ones behind the last instruction are taken when the window
+        // reaches the end of the list
+        if (cur_pos <= target - ibeg) {
+          i = ibeg + cur_pos;
+          do_event();
+          continue;
+        }
+        if (here) {
+          found = true;
+          i = target;
+          n_pages = __shfl_sync(0xffffffffu, mine.n_pages, at);
+          lflags = __shfl_sync(0xffffffffu, mine.flags, at);
+          first_slot = __shfl_sync(0xffffffffu, first, at);
+          mv_ord = __shfl_sync(0xffffffffu, (mine.flags & MK_LDF_ATTN) ? ats : mvs, at);
+          rp_i = ring_at(__shfl_sync(0xffffffffu, seq, at), NP);
+          break;
+        }
+        if (base + 32 >= iend) break;
+        move_window(32);
       }
-      n_pages = __shfl_sync(0xffffffffu, mine.n_pages, i - base);
-      lflags = __shfl_sync(0xffffffffu, mine.flags, i - base);
-      const bool shared = (lflags & kInsMatvec) != 0;
-      int split = (lflags >> MK_LDF_SPLIT_SHIFT) & MK_LDF_SPLIT_MASK;
-      if (lflags & MK_LDF_DYN) {
-        // an attention unit whose window follows the device-resident position: the pages in use, and
-        // with them the participants, are a function of the position (the same on every warp)
-        const int t_begin = __shfl_sync(0xffffffffu, mine.row_a, i - base);
-        const int brow = (__shfl_sync(0xffffffffu, mine.row_b, i - base) >> 16) & 31;
-        n_pages = at_dyn_pages(t_begin, n_pages, at_page_tokens((lflags & MK_LDF_D128) ? 128 : 64, pv.page_bytes),
-                               c.ctrl->pos[brow] + 1);
-        split = max(1, min(split, n_pages));
-        lflags = (lflags & ~(MK_LDF_SPLIT_MASK << MK_LDF_SPLIT_SHIFT)) | (split << MK_LDF_SPLIT_SHIFT);
+    } else {
+      for (;;) {
+        // events due before instruction i; the ones behind the last instruction are
+        // taken when the cursor reaches the end of the list (every event position is
+        // at most the length of the list), so this is the only place events run
+        while (cur_pos <= i - ibeg) do_event();
+        if (i >= iend) break;
+        if (i - base >= 32) {
+          base = i;
+          mine = empty_instr();
+          if (base + c.lane < iend) mine = load_instr(pv.instrs + base + c.lane);
+        }
+        n_pages = __shfl_sync(0xffffffffu, mine.n_pages, i - base);
+        lflags = __shfl_sync(0xffffffffu, mine.flags, i - base);
+        const bool shared = (lflags & kInsMatvec) != 0;
+        int split = (lflags >> MK_LDF_SPLIT_SHIFT) & MK_LDF_SPLIT_MASK;
+        if (lflags & MK_LDF_DYN) {
+          // an attention unit whose window follows the device-resident position: the pages in use, and
+          // with them the participants, are a function of the position (the same on every warp)
+          const int t_begin = __shfl_sync(0xffffffffu, mine.row_a, i - base);
+          const int brow = (__shfl_sync(0xffffffffu, mine.row_b, i - base) >> 16) & 31;
+          n_pages = at_dyn_pages(t_begin, n_pages, at_page_tokens((lflags & MK_LDF_D128) ? 128 : 64, pv.page_bytes),
+                                 c.ctrl->pos[brow] + 1);
+          split = max(1, min(split, n_pages));
+          lflags = (lflags & ~(MK_LDF_SPLIT_MASK << MK_LDF_SPLIT_SHIFT)) | (split << MK_LDF_SPLIT_SHIFT);
+        }
+        const uint32_t slots = shared ? (uint32_t)split : 1u;
+        if (ticket < first_slot + slots) {
+          found = true;
+          break;
+        }
+        first_slot += slots;
+        ring_advance(rp_i, n_pages, NP);
+        if (shared && split > 1) ++mv_ord;
+        ++i;
       }
-      const uint32_t slots = shared ? (uint32_t)split : 1u;
-      if (ticket < first_slot + slots) {
-        found = true;
-        break;
-      }
-      first_slot += slots;
-      ring_advance(rp_i, n_pages, NP);
-      if (shared && split > 1) ++mv_ord;
-      ++i;
     }
     if (!found) break;
     if (!c.dead) {
@@ -410,7 +505,8 @@ __global__ void __launch_bounds__(kThreads, 1) mk_persistent_kernel(const __grid
   c.pages = smem + kCtrlBytes + pv.act_bytes;
   c.act_u32 = smem_u32(c.act);
   c.pages_u32 = smem_u32(c.pages);
-  c.warp = threadIdx.x >> 5;
+  // (the shuffle makes the warp number known to be uniform)
+  c.warp = kWideStep<NTC, WFC, FEAT> ? __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0) : (int)(threadIdx.x >> 5);
   c.lane = threadIdx.x & 31;
   c.instr_idx = -1;
   c.dead = false;
@@ -422,7 +518,8 @@ __global__ void __launch_bounds__(kThreads, 1) mk_persistent_kernel(const __grid
       mbar_init(smem_u32(&c.ctrl->empty[i]), 1);
     }
     for (int i = 0; i < kMaxPages; ++i) c.ctrl->released[i] = 0;
-    for (int i = 0; i < 4; ++i) c.ctrl->mv_arrive[i] = c.ctrl->mv_done[i] = 0;
+    for (int i = 0; i < 4; ++i)
+      c.ctrl->mv_arrive[i] = c.ctrl->mv_done[i] = c.ctrl->at_arrive[i] = c.ctrl->at_done[i] = 0;
     c.ctrl->abort_flag = 0;
     c.ctrl->is_last = 0;
     c.ctrl->ticket = 0;
@@ -453,7 +550,7 @@ __global__ void __launch_bounds__(kThreads, 1) mk_persistent_kernel(const __grid
   if (bad_pos) {
     if (threadIdx.x == 0) report(c, MK_ST_BAD_POSITION, c.ctrl->pos[bad_pos - 1], pv.pos_limit);
   } else if (c.warp == 0) {
-    loader_loop(c, ibeg, iend);
+    loader_loop<kWideStep<NTC, WFC, FEAT>>(c, ibeg, iend);
   } else {
     consumer_loop<NTC, WFC, FEAT>(c, ibeg, iend, ebeg, eend);
   }

@@ -21,6 +21,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -213,6 +214,13 @@ static int attn_pages(const mk_op_t& op, int unit, int page_bytes) {
   return (te - tb + tn - 1) / tn;
 }
 
+// Consumer warps that share an attention unit of `pages` pages.  (Where the states are left in the ring, each keeps
+// one page until they are merged: two stay for the stream.  The number fixes the order of the sums, so it does not
+// depend on where the states are left.)
+static int at_participants(int pages, int n_ring_pages) {
+  return std::max(1, std::min(std::min((int)kConsumerWarps, pages), n_ring_pages - 2));
+}
+
 // Everything the device would otherwise derive per unit with divisions or
 // op-table reads: the loader's tensor-map address, first rows and tiles per
 // page, the participant count, and the finisher's output offsets.
@@ -231,9 +239,7 @@ static void fill_instr_fast_path(mk_instr_t& in, const mk_op_t& op, uint64_t dev
     in.out_off_a = sp;
     in.out_off_b = mt;
     in.ld_tiles = at_page_tokens(op.i[MK_AT_D], page_bytes);
-    // every participant keeps one ring page until the unit's states are merged:
-    // leave at least two pages for the stream
-    const int split = std::max(1, std::min(std::min((int)kConsumerWarps, in.n_pages), n_ring_pages - 2));
+    const int split = at_participants(in.n_pages, n_ring_pages);
     in.ld_flags = MK_LDF_ATTN | (op.i[MK_AT_D] == 128 ? MK_LDF_D128 : 0) | (split << MK_LDF_SPLIT_SHIFT) |
                   (op.i[MK_AT_DYNPOS] ? MK_LDF_DYN : 0);
     if (in.n_pages == 0) in.ld_maps = 0;   // an empty split: nothing to load, one consumer writes the empty partial
@@ -516,6 +522,7 @@ struct mk_handle_s {
   int feat;                          // features of the kernel in use
   std::vector<mk_op_t> ops;          // host copy of the op records (as uploaded)
   std::vector<mk_instr_t> instrs;    // host copy of the instruction table (as uploaded)
+  bool states_may_stage;             // no matvec unit relies on activations staged before an attention op
   int n_ctas;
   int smem_bytes;
   int smem_optin;
@@ -546,6 +553,42 @@ static void classify_op(const mk_op_t& op, int* ntc, int* wfc, int* feat) {
   *ntc = m <= 8 ? 1 : (m <= 16 ? 2 : 4);
   *wfc = wf == MK_W_BF16 ? 0 : (wf >= MK_W_NVFP4_F16S32 ? 2 : 1);
   if (op.i[MK_MV_EPI] == MK_EPI_TOP1) *feat = mk::MK_F_TOP1;
+  if (op.i[MK_MV_EPI] == MK_EPI_KSUM) *feat = mk::MK_F_KSUM;
+}
+
+// The staging buffer is free between an attention op's event and the next matvec's, unless a matvec unit behind an
+// attention unit has no event of its own and reads what an earlier event staged.
+static bool states_may_stage(const mk_program_t* p) {
+  for (int cta = 0; cta < p->n_ctas; ++cta) {
+    const int ib = p->cta_instr_begin[cta], ie = p->cta_instr_begin[cta + 1];
+    int e = p->cta_event_begin[cta];
+    const int ee = p->cta_event_begin[cta + 1];
+    bool overwritten = false;
+    for (int j = ib; j < ie; ++j) {
+      for (; e < ee && p->events[e].pos <= j - ib; ++e) {
+        if (p->ops[p->events[e].op].opcode == MK_OP_MATVEC) overwritten = false;
+        if (p->ops[p->events[e].op].opcode == MK_OP_ATTN_SPLIT) overwritten = true;
+      }
+      const int opcode = p->ops[p->instrs[j].op].opcode;
+      if (opcode == MK_OP_MATVEC && overwritten) return false;
+      // an attention unit without an event of its op runs beside units of the op before it
+      if (opcode == MK_OP_ATTN_SPLIT && !overwritten) return false;
+    }
+  }
+  return true;
+}
+
+// Where the participants of attention units leave their states (ProgramView::at_sets).
+static void place_states(mk_handle_s* h) {
+  int bytes = 0;
+  for (const mk_instr_t& in : h->instrs) {
+    const mk_op_t& op = h->ops[in.op];
+    if (op.opcode != MK_OP_ATTN_SPLIT) continue;
+    bytes = std::max(bytes, mk::at_participants(in.n_pages, h->pv.n_pages) * (op.i[MK_AT_D] / 8 + 1) * 512);
+  }
+  const int sets = bytes && h->states_may_stage ? h->pv.act_bytes / bytes : 0;
+  h->pv.at_set_bytes = sets ? bytes : 0;
+  h->pv.at_sets = sets == 0 || sets >= 4 ? 4 : (sets >= 2 ? 2 : 1);
 }
 
 // Pick the smallest kernel that covers the program: its matvec ops' tile class
@@ -589,6 +632,7 @@ static int select_kernel(mk_handle_s* h) {
   h->pv.mv_sets = 4;
   for (int n : h->op_ntc)
     if (n > 0) h->pv.mv_sets = std::min(h->pv.mv_sets, n == 1 ? 4 : (n == 2 ? 2 : 1));
+  place_states(h);
   // The dynamic shared-memory limit is a property of the kernel function, shared by
   // every handle that runs this variant: always raise it to the device's opt-in
   // maximum, so that a later, smaller program never lowers it under a live one.
@@ -730,6 +774,7 @@ static int create_program(const mk_program_t* prog, mk_handle_t* out, bool strea
   h->op_wfc.resize(prog->n_ops);
   h->op_feat.resize(prog->n_ops);
   for (int i = 0; i < prog->n_ops; ++i) classify_op(prog->ops[i], &h->op_ntc[i], &h->op_wfc[i], &h->op_feat[i]);
+  h->states_may_stage = states_may_stage(prog);
   rc = select_kernel(h);
   if (rc) return rc;
   h->device = prog->device;

@@ -269,12 +269,15 @@ __device__ __forceinline__ void at_fix_k_row(Ctx& c, const mk_op_t* op, const At
 // The unit's pages (blocks of tn tokens) are dealt round-robin to `parts`
 // consumer warps; each keeps its own online-softmax state (row max, row sum,
 // unnormalised output).  A participant parks its state in the last page it
-// consumed instead of handing that page back; the last one to arrive merges
-// the states in participant order, writes the normalised partial and then
-// releases everybody's parked page.  Returns true for the warp that finished
-// the unit.
+// consumed instead of handing that page back, or (STG, where the buffer is large
+// enough) in the staging buffer, which is idle from an attention op's event to
+// the next matvec's; the last one to arrive merges the states in participant
+// order, writes the normalised partial and then releases everybody's parked
+// page.  Returns true for the warp that finished the unit.  (With every state in
+// a page, the units of a batch held up to all but two pages of a short ring from
+// their first participant's end to the merge.)
 // QMODE 0: the fused q/k norm is compiled out (kernels for bf16-only programs); 1: decided per op.
-template <int D, int QMODE>
+template <int D, int QMODE, bool STG>
 __device__ __forceinline__ bool at_unit(Ctx& c, const mk_op_t* op, const UnitArgs& ua) {
   constexpr int KS = D / 16;   // k-steps of Q·K^T
   constexpr int ND = D / 8;    // n-tiles of the output
@@ -299,6 +302,8 @@ __device__ __forceinline__ bool at_unit(Ctx& c, const mk_op_t* op, const UnitArg
   const int tn = at_page_tokens(D, c.pv->page_bytes);
   const uint32_t tile_bytes = (uint32_t)tn * (uint32_t)D * 2u;
   const int NPG = c.pv->n_pages;
+  const bool staged_states = STG && c.pv->at_set_bytes > 0;
+  constexpr uint32_t kStateBytes = (ND + 1) * 512;
 
   // rows of this thread: r0 = mt*16 + g, r1 = r0 + 8 -> (m, head)
   int rm[2], rh[2];
@@ -395,7 +400,7 @@ __device__ __forceinline__ bool at_unit(Ctx& c, const mk_op_t* op, const UnitArg
 
   const int np = ua.n_pages;
   RingPos rp = ua.rp;
-  uint32_t park = 0;            // address of the page this warp keeps for its state
+  uint32_t park = 0;            // where this warp's state goes
   for (int p = part; p < np; p += parts, ring_advance(rp, parts, NPG)) {
     uint32_t page;
     if (!page_acquire(c, rp, page)) return false;
@@ -490,17 +495,20 @@ __device__ __forceinline__ bool at_unit(Ctx& c, const mk_op_t* op, const UnitArg
       }
     }
     trace(c, TRC_PAGE_DONE, rp.k * (uint32_t)NPG + rp.slot);
-    if (parts > 1 && p + parts >= np)
+    if (parts > 1 && p + parts >= np && !staged_states)
       park = page;              // the last page of this participant: keep it
     else
       page_release(c, rp);
   }
 
   if (parts > 1) {
-    // park (o, m, l) in the kept page: 16-byte record (i*32 + lane) holds o[i][0..3], the last one (m, m, l, l)
-    const int sets_log2 = __ffs(c.pv->mv_sets) - 1;                      // 1, 2 or 4 slot sets
-    const uint32_t set = ord & (uint32_t)(c.pv->mv_sets - 1), gen = ord >> sets_log2;
-    if (!wait_smem_ge(c, &c.ctrl->mv_done[set], gen, (int)ord)) return false;
+    // park (o, m, l): 16-byte record (i*32 + lane) holds o[i][0..3], the last one (m, m, l, l)
+    const int sets = STG ? c.pv->at_sets : c.pv->mv_sets;                // 1, 2 or 4
+    uint32_t *arrive = STG ? c.ctrl->at_arrive : c.ctrl->mv_arrive, *done = STG ? c.ctrl->at_done : c.ctrl->mv_done;
+    const uint32_t set = ord & (uint32_t)(sets - 1), gen = ord >> (__ffs(sets) - 1);
+    if (!wait_smem_ge(c, &done[set], gen, (int)ord)) return false;
+    const uint32_t states = c.act_u32 + set * (uint32_t)c.pv->at_set_bytes;
+    if (staged_states) park = states + (uint32_t)part * kStateBytes;
     __syncwarp();
 #pragma unroll
     for (int i = 0; i < ND; ++i)
@@ -514,7 +522,7 @@ __device__ __forceinline__ bool at_unit(Ctx& c, const mk_op_t* op, const UnitArg
     int last = 0;
     if (c.lane == 0) {
       __threadfence_block();
-      last = atomicAdd(&c.ctrl->mv_arrive[set], 1u) == (uint32_t)(parts - 1);
+      last = atomicAdd(&arrive[set], 1u) == (uint32_t)(parts - 1);
       __threadfence_block();
     }
     last = __shfl_sync(0xffffffffu, last, 0);
@@ -531,10 +539,12 @@ __device__ __forceinline__ bool at_unit(Ctx& c, const mk_op_t* op, const UnitArg
     const int lq = (np - 1) / parts, lr = (np - 1) - lq * parts;
 #pragma unroll 1
     for (int j = 0; j < parts; ++j) {
-      const int pl = j + (j <= lr ? lq : lq - 1) * parts;
-      RingPos rj = ua.rp0;
-      ring_advance(rj, pl, NPG);
-      const uint32_t src = c.pages_u32 + rj.slot * (uint32_t)c.pv->page_bytes;
+      uint32_t src = states + (uint32_t)j * kStateBytes;
+      if (!staged_states) {
+        RingPos rj = ua.rp0;
+        ring_advance(rj, j + (j <= lr ? lq : lq - 1) * parts, NPG);
+        src = c.pages_u32 + rj.slot * (uint32_t)c.pv->page_bytes;
+      }
       float wa[2], wb[2];
       // all of a participant's records are requested before the first is used
       const uint4 ml = lds128_sync(src + (uint32_t)(ND * 32 + c.lane) * 16u);
@@ -563,17 +573,19 @@ __device__ __forceinline__ bool at_unit(Ctx& c, const mk_op_t* op, const UnitArg
     // hand the parked pages back (generic-proxy writes before the next TMA fill)
     __syncwarp();
     if (c.lane == 0) {
-      fence_proxy_async();
-      for (int j = 0; j < parts; ++j) {
-        const int pl = j + (j <= lr ? lq : lq - 1) * parts;
-        RingPos rj = ua.rp0;
-        ring_advance(rj, pl, NPG);
-        mbar_arrive(empty_bar(c, rj.slot));
-        *reinterpret_cast<volatile uint32_t*>(&c.ctrl->released[rj.slot]) = rj.k + 1u;
+      if (!staged_states) {
+        fence_proxy_async();
+        for (int j = 0; j < parts; ++j) {
+          const int pl = j + (j <= lr ? lq : lq - 1) * parts;
+          RingPos rj = ua.rp0;
+          ring_advance(rj, pl, NPG);
+          mbar_arrive(empty_bar(c, rj.slot));
+          *reinterpret_cast<volatile uint32_t*>(&c.ctrl->released[rj.slot]) = rj.k + 1u;
+        }
       }
-      c.ctrl->mv_arrive[set] = 0;
+      arrive[set] = 0;
       __threadfence_block();
-      *reinterpret_cast<volatile uint32_t*>(&c.ctrl->mv_done[set]) = gen + 1u;
+      *reinterpret_cast<volatile uint32_t*>(&done[set]) = gen + 1u;
     }
   }
 
@@ -619,28 +631,28 @@ __device__ __forceinline__ bool at_unit(Ctx& c, const mk_op_t* op, const UnitArg
   return true;
 }
 
-template <int D, int QMODE>
+template <int D, int QMODE, bool STG>
 __device__ __forceinline__ UnitResult at_unit_call(Ctx c, const mk_op_t* op, const UnitArgs& ua) {
   UnitResult r;
-  r.signal = at_unit<D, QMODE>(c, op, ua);
+  r.signal = at_unit<D, QMODE, STG>(c, op, ua);
   r.dead = c.dead;
   r.trace_n = c.trace_n;
   return r;
 }
 
-template <int FEAT>
+template <int FEAT, bool STG>
 __device__ __forceinline__ bool at_dispatch(Ctx& c, const mk_op_t* op, const UnitArgs& ua) {
   constexpr int QMODE = (FEAT & MK_F_QKNORM) ? 1 : 0;
   UnitResult r;
   if constexpr ((FEAT & MK_F_AT64) && (FEAT & MK_F_AT128)) {
     if (op->i[MK_AT_D] == 64)
-      r = at_unit_call<64, QMODE>(c, op, ua);
+      r = at_unit_call<64, QMODE, STG>(c, op, ua);
     else
-      r = at_unit_call<128, QMODE>(c, op, ua);
+      r = at_unit_call<128, QMODE, STG>(c, op, ua);
   } else if constexpr ((FEAT & MK_F_AT64) != 0) {
-    r = at_unit_call<64, QMODE>(c, op, ua);
+    r = at_unit_call<64, QMODE, STG>(c, op, ua);
   } else {
-    r = at_unit_call<128, QMODE>(c, op, ua);
+    r = at_unit_call<128, QMODE, STG>(c, op, ua);
   }
   c.dead = r.dead;
   c.trace_n = r.trace_n;

@@ -35,7 +35,8 @@ enum {
   MK_F_AR = 32,      // the in-kernel all-reduce (tensor parallel)
   MK_F_TOP1 = 64,    // top-1 epilogue and its finalise op
   MK_F_TRACE = 128,  // event trace
-  MK_F_ALL = 255
+  MK_F_KSUM = 256,   // K blocks of one product side by side
+  MK_F_ALL = 511
 };
 
 // Device status codes (status[0]).
@@ -72,6 +73,10 @@ struct ProgramView {
   int32_t n_pages;
   int32_t page_bytes;
   int32_t act_bytes;
+  // where the participants of a shared attention unit leave their states (kernels with staged states): in the staging
+  // buffer, at_set_bytes a unit, or (0) in their last pages; at_sets units (1, 2 or 4) may be between states and merge
+  int32_t at_sets;
+  int32_t at_set_bytes;
   uint64_t timeout_ns;
   // optional event trace: per (CTA, warp) a ring of trace_cap records, then
   // one record count per (CTA, warp) after all rings; null = tracing off
@@ -120,6 +125,9 @@ struct Ctrl {
   // the set have finished their epilogue.
   uint32_t mv_arrive[4];
   uint32_t mv_done[4];
+  // the same for attention units (kernels with staged states; the others use the sets above)
+  uint32_t at_arrive[4];
+  uint32_t at_done[4];
   // units of an op finished on this CTA (bulk signalling); one word per op-record slot
   uint32_t bulk_done[2];
   uint32_t ticket;     // next consumer slot of the CTA (see consumer_loop)
@@ -178,7 +186,7 @@ struct UnitArgs {
   int idx;              // lane of the window that holds this unit's record
   int op, unit, n_pages, flags;
   int part;             // this consumer's participant index within the unit
-  uint32_t ord;         // shared units before this one on the CTA (selects the split-K slot set)
+  uint32_t ord;         // shared units (staged states: of its kind) before this one on the CTA: selects the slot set
   RingPos rp0;          // ring position of the unit's first page
   RingPos rp;           // ring position of this participant's first page
 };

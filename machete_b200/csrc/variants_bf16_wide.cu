@@ -5,8 +5,8 @@
 using namespace mk;
 
 static const mk_variant kVariants[] = {
-    {2, 0, MK_F_AT64 | MK_F_TOP1, mk::mk_persistent_kernel<2, 0, MK_F_AT64 | MK_F_TOP1>},
-    {4, 0, MK_F_AT64 | MK_F_TOP1, mk::mk_persistent_kernel<4, 0, MK_F_AT64 | MK_F_TOP1>},
+    {2, 0, MK_F_AT64 | MK_F_TOP1 | MK_F_KSUM, mk::mk_persistent_kernel<2, 0, MK_F_AT64 | MK_F_TOP1 | MK_F_KSUM>},
+    {4, 0, MK_F_AT64 | MK_F_TOP1 | MK_F_KSUM, mk::mk_persistent_kernel<4, 0, MK_F_AT64 | MK_F_TOP1 | MK_F_KSUM>},
     {2, 0, MK_F_TOP1, mk::mk_persistent_kernel<2, 0, MK_F_TOP1>},
     {4, 0, MK_F_TOP1, mk::mk_persistent_kernel<4, 0, MK_F_TOP1>},
 };

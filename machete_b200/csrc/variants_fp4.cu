@@ -5,10 +5,10 @@
 using namespace mk;
 
 static const mk_variant kVariants[] = {
-    {1, 2, MK_F_AT128 | MK_F_QKNORM | MK_F_TOP1, mk::mk_persistent_kernel<1, 2, MK_F_AT128 | MK_F_QKNORM | MK_F_TOP1>},
-    {1, 2, MK_F_AT128 | MK_F_QKNORM | MK_F_TOP1 | MK_F_TRACE, mk::mk_persistent_kernel<1, 2, MK_F_AT128 | MK_F_QKNORM | MK_F_TOP1 | MK_F_TRACE>},
+    {1, 2, MK_F_AT128 | MK_F_QKNORM | MK_F_TOP1 | MK_F_KSUM, mk::mk_persistent_kernel<1, 2, MK_F_AT128 | MK_F_QKNORM | MK_F_TOP1 | MK_F_KSUM>},
+    {1, 2, MK_F_AT128 | MK_F_QKNORM | MK_F_TOP1 | MK_F_KSUM | MK_F_TRACE, mk::mk_persistent_kernel<1, 2, MK_F_AT128 | MK_F_QKNORM | MK_F_TOP1 | MK_F_KSUM | MK_F_TRACE>},
     {1, 2, MK_F_TOP1, mk::mk_persistent_kernel<1, 2, MK_F_TOP1>},
-    {1, 2, MK_F_AT64 | MK_F_AT128 | MK_F_QKNORM | MK_F_TOP1 | MK_F_EW, mk::mk_persistent_kernel<1, 2, MK_F_AT64 | MK_F_AT128 | MK_F_QKNORM | MK_F_TOP1 | MK_F_EW>},
+    {1, 2, MK_F_AT64 | MK_F_AT128 | MK_F_QKNORM | MK_F_TOP1 | MK_F_KSUM | MK_F_EW, mk::mk_persistent_kernel<1, 2, MK_F_AT64 | MK_F_AT128 | MK_F_QKNORM | MK_F_TOP1 | MK_F_KSUM | MK_F_EW>},
 };
 
 extern "C" const mk_variant* mk_variants_fp4(int* n) {

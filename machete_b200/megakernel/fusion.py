@@ -80,8 +80,8 @@ def _parallel_kblocks(ops: List[ScheduledOp], start: int, ctx: LowerCtx) -> List
 
     Each block keeps its own op, with its own K slice to stage, on every n-th CTA; the last block to finish a unit's
     rows adds the blocks' fp32 sums in block order and rounds after each (``MK_EPI_KSUM``): the bits of the chain, in one
-    dependency stage instead of n.  16-layer 1B shape, 16 rows, KV 1931 (4 blocks): 1959 -> 1566 us a step; 36-layer 8B
-    shape with NVFP4 weights, 8 rows, KV 4096 (2 blocks): 4861 -> 4692.
+    dependency stage instead of n.  16-layer 1B shape, 16 rows, KV 1931 (4 blocks): 2020 -> 1627 us a step; 36-layer 8B
+    shape with NVFP4 weights, 8 rows, KV 4096 (2 blocks): 5034 -> 4925.
     """
     first = ops[start]
     added = _ADDED_BLOCK.get(first.op_cls.__name__)

@@ -385,6 +385,10 @@ class InstructionStreamBuilder:
             # one counter for the whole op: each CTA signals its units in bulk
             per_cta = np.bincount(np.asarray(where[:op.n_units], dtype=np.int64), minlength=num_ctas)
             bulk = op.n_groups == 1
+            if op.opcode == N.OP_ATTN_SPLIT:
+                # attention units may leave their partial states in the staging buffer
+                for c in set(int(c) for c in where[:op.n_units]):
+                    cta_staged[c] = 0
             for u in range(op.n_units):
                 cta = int(where[u])
                 if cta not in seen_cta:
