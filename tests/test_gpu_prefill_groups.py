@@ -50,3 +50,18 @@ def test_row_maxima_that_keep_growing(D, M):
     o = torch.zeros_like(q)
     flash_prefill(q, k, v, o, causal=True, check_status=True)
     assert_parity(o, _reference(q, k, v, True)[0], f"growing maxima D={D}")
+
+
+# two tiles' boundaries at the edges of a 32-query block, prefixes that are multiples of 32 and not; the last of 400 tiles
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("batch,H,Hkv,M,N", [(1, 8, 2, 100, 100), (1, 8, 2, 97, 360), (2, 32, 8, 777, 1000), (1, 6, 1, 65, 80),
+                                             (1, 64, 1, 40, 99), (1, 16, 2, 33, 1055)])
+def test_the_grouping_of_heads_leaves_the_bits(D, batch, H, Hkv, M, N):
+    g = torch.Generator(device="cuda").manual_seed(M * N)
+    q = torch.randn(batch, H, M, D, generator=g, device="cuda").to(BF)
+    k, v = (torch.randn(batch, Hkv, N, D, generator=g, device="cuda").to(BF) for _ in range(2))
+    packed, single = torch.zeros_like(q), torch.zeros_like(q)
+    flash_prefill(q, k, v, packed, causal=True, check_status=True)
+    each = (t.repeat_interleave(H // Hkv, dim=1).contiguous() for t in (k, v))      # a KV head of its own for every head
+    flash_prefill(q, *each, single, causal=True, check_status=True)
+    assert torch.equal(packed, single)
