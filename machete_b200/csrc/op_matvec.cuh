@@ -697,7 +697,10 @@ __device__ __forceinline__ bool mv_unit(Ctx& c, const mk_op_t* op, const UnitArg
 #pragma unroll 1
           for (int kt = 0; kt < tiles; kt += 2) {
             load_pair(f, kt);
-            mma_pair(f, min(2, tiles - kt), is_bf16);
+            // the number of tiles is a constant at each product: a test there and the products no longer follow one
+            // another (24 x 2048 -> 8192 34.1 us, 25.9 so; 4-layer 1B-shape step of 24 rows, KV 700 869 and 680)
+            if (kt + 2 <= tiles) mma_pair(f, 2, is_bf16);
+            else mma_pair(f, 1, is_bf16);
           }
         }
       };
