@@ -119,7 +119,7 @@ EXPORTS = [
     "mk_flash_decode_noalloc", "mk_flash_decode_noalloc_status",
     "mk_gemm_bf16_workspace_bytes", "mk_gemm_bf16", "mk_gemm_bf16_packed", "mk_gemm_bf16_status", "mk_gemm_bf16_plan",
     "mk_gemm_last_error",
-    "mk_flash_prefill_bf16", "mk_flash_prefill_status", "mk_flash_prefill_last_error",
+    "mk_flash_prefill_bf16", "mk_flash_prefill_plan", "mk_flash_prefill_status", "mk_flash_prefill_last_error",
 ]
 
 _lib = None
@@ -207,6 +207,8 @@ def _declare(h: C.CDLL) -> None:
     h.mk_flash_prefill_bf16.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp, vp, vp, f32, i32,
                                         vp, u64, i32, vp]
     h.mk_flash_prefill_bf16.restype = C.c_int
+    h.mk_flash_prefill_plan.argtypes = [i32] * 8 + [C.POINTER(i32)]
+    h.mk_flash_prefill_plan.restype = C.c_int
     h.mk_flash_prefill_status.argtypes = [vp, C.POINTER(i32)]
     h.mk_flash_prefill_status.restype = C.c_int
     h.mk_flash_prefill_last_error.restype = C.c_char_p

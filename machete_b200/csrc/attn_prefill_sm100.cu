@@ -37,6 +37,7 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 #include <string>
@@ -727,6 +728,48 @@ static const Device* device_facts(int dev) {
 
 }  // namespace mkp
 
+namespace mkp {
+
+// How a call is cut.
+struct Plan {
+  int pack;         // query heads of a KV head in one tile
+  int row_tiles;
+  int64_t tiles;    // of all heads and batch entries
+  bool three;       // the form with one S accumulator, three CTAs to an SM
+};
+
+static Plan plan(int B, int H, int Hkv, int M, int N, int D, bool causal, int sms) {
+  Plan r;
+  // the largest power of two that divides the group, as long as the tiles fit the grid
+  r.pack = (H / Hkv) & -(H / Hkv);
+  while (r.pack > kBM || (r.pack > 1 && (M + kBM / r.pack - 1) / (kBM / r.pack) > 65535)) r.pack >>= 1;
+  const int tile_m = kBM / r.pack;
+  const int64_t per_row = (int64_t)(H / r.pack) * B;
+  r.row_tiles = (M + tile_m - 1) / tile_m;
+  r.tiles = per_row * r.row_tiles;
+  // Three CTAs an SM do no more per time than two, and a tile then takes a quarter longer (every one: 1.2 us a KV tile,
+  // with two 0.9 beside another CTA and less alone).  Where all tiles fit the device at once so and two an SM need a
+  // second round, that round is the two shortest of a slot's tiles, one behind the other: it must be the longer way by
+  // more than the longest tile's loss.  Under a causal mask from the first token it never is.
+  // us with two / three, 32 / 8 heads, in brackets KV tiles of the slot against 1.4 times those of the longest tile:
+  //   causal 1185 x 1185 18.9 / 23.3 (2, 27), 1408 21.5 / 27.0 (8, 31), 1760 25.5 / 33.7 (19, 39), two sequences of 864
+  //   16.2 / 19.0 (10, 20); 1400 behind 600 tokens 30.9 / 38.9 (27, 45), behind 1600 54.8 / 57.2 (58, 66), behind 2600
+  //   81.5 / 77.0 (90, 88); two sequences of 777 behind 1223 46.6 / 41.5 (46, 45), behind 2223 71.3 / 59.8 (78, 66);
+  //   no mask, 1300 x 1300 35.9 / 32.5 (42, 29), 1760 x 4096 95.4 / 88.2 (128, 90).
+  r.three = false;
+  const int64_t slots = 2 * (int64_t)sms;
+  if (D == 64 && r.tiles > slots && r.tiles <= 3 * (int64_t)sms) {
+    auto kv_tiles = [&](int64_t rank) {   // of the rank-th tile, the longest first
+      const int64_t rows_end = (r.row_tiles - rank / per_row) * tile_m;
+      return ((causal ? std::min<int64_t>(N, N - M + rows_end) : N) + kBN - 1) / kBN;
+    };
+    r.three = 5 * (kv_tiles(slots - 1) + kv_tiles(slots)) > 7 * kv_tiles(0);
+  }
+  return r;
+}
+
+}  // namespace mkp
+
 extern "C" {
 
 const char* mk_flash_prefill_last_error(void) { return mkp::g_err.c_str(); }
@@ -754,9 +797,8 @@ int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, 
   const int smem_optin = d->smem_optin;
   const int bn = kBN;                              // tokens per KV tile
   CUtensorMap mq, mkk, mv;
-  // the largest power of two that divides the group, as long as the tiles fit the grid
-  int pack = (H / Hkv) & -(H / Hkv);
-  while (pack > kBM || (pack > 1 && (M + kBM / pack - 1) / (kBM / pack) > 65535)) pack >>= 1;
+  const Plan pl = plan(B, H, Hkv, M, N, D, causal != 0, d->sms);
+  const int pack = pl.pack;
   int rc = encode_query_map(&mq, q, D, M, H, B, q_strides[2], q_strides[1], q_strides[0], pack);
   if (rc) return rc;
   rc = encode_rows_map(&mkk, k, D, N, Hkv, B, k_strides[2], k_strides[1], k_strides[0], bn, "k");
@@ -778,23 +820,16 @@ int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, 
   while ((1 << p.pack_log2) < pack) ++p.pack_log2;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.timeout_ns = (uint64_t)(timeout_ms > 0 ? timeout_ms : 1000) * 1000000ull;
-  const int tile_m = kBM / pack;
-  const dim3 grid(H / pack, B, (M + tile_m - 1) / tile_m);
+  const dim3 grid(H / pack, B, pl.row_tiles);
   // Where this grid leaves slots empty (two CTAs an SM), the next one is let in late: its CTAs would pile up on the
   // SMs that are free now (the average over six such prompts at head dim 64 11 % faster, three at 128 3.5 %).  With
   // every slot taken nothing piles up, and at head dim 64 (1960 behind 2045 tokens 84.8 us early, 86.7 late) the
   // last load is too short before the end to hide the placement; at 128 (0.4 % faster late) it is not.
-  const int64_t tiles = (int64_t)grid.x * grid.y * grid.z;
-  // Three CTAs an SM do no more per time than two (4096 x 4096, 1024 tiles: 109 us, 104), but each tile then takes half
-  // as long again (1024 x 1024, 256 tiles: 19.6 us, 14.1): they are taken where all tiles are on the device at once
-  // and with two a second round would follow (777 behind 2223 tokens, two sequences, 400 tiles: 59.4 us, 73.9 as
-  // 448 tiles of one head each in two rounds).
-  const bool three = D == 64 && tiles > 2 * (int64_t)d->sms && tiles <= 3 * (int64_t)d->sms;
-  p.next_early = D == 64 && !three && tiles >= 2 * (int64_t)d->sms ? 1 : 0;
+  p.next_early = D == 64 && !pl.three && pl.tiles >= 2 * (int64_t)d->sms ? 1 : 0;
   // the kernel may be placed while the one before it in the stream drains (it waits before it touches memory)
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
-  cfg.blockDim = dim3(three ? kThreads<1> : kThreads<2>);
+  cfg.blockDim = dim3(pl.three ? kThreads<1> : kThreads<2>);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = reinterpret_cast<cudaStream_t>(cuda_stream);
   cudaLaunchAttribute attr[1];
@@ -802,11 +837,21 @@ int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = three ? cudaLaunchKernelEx(&cfg, prefill_kernel<64, 1>, mq, mkk, mv, p)
+  cudaError_t e = pl.three ? cudaLaunchKernelEx(&cfg, prefill_kernel<64, 1>, mq, mkk, mv, p)
                   : D == 64 ? cudaLaunchKernelEx(&cfg, prefill_kernel<64, 2>, mq, mkk, mv, p)
                             : cudaLaunchKernelEx(&cfg, prefill_kernel<128, 2>, mq, mkk, mv, p);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return fail(-(int)e - 1000, "mk_flash_prefill_bf16 launch: %s", cudaGetErrorString(e));
+  return 0;
+}
+
+int mk_flash_prefill_plan(int B, int H, int Hkv, int M, int N, int D, int causal, int sms, int32_t out[4]) {
+  using namespace mkp;
+  if (!out || B < 1 || H < 1 || Hkv < 1 || M < 1 || N < 1 || H % Hkv || (D != 64 && D != 128) || (causal && M > N) || sms < 1)
+    return fail(-2, "mk_flash_prefill_plan: bad sizes");
+  const Plan pl = plan(B, H, Hkv, M, N, D, causal != 0, sms);
+  out[0] = pl.three ? kCtasPerSm<1> : kCtasPerSm<2>, out[1] = pl.pack, out[2] = pl.row_tiles;
+  out[3] = (int32_t)std::min<int64_t>(pl.tiles, INT32_MAX);
   return 0;
 }
 
