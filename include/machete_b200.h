@@ -217,7 +217,8 @@ enum { MK_AR_S_INBOX = 0, MK_AR_S_FLAGS };
 typedef struct mk_op {
   int32_t opcode;
   int32_t n_units;        /* work units                                      */
-  int32_t act_key;        /* ops with equal non-zero key share staged input  */
+  int32_t act_key;        /* ops with equal non-zero key share staged input: the same rows and prologue, staged as
+                             bf16 (bf16 weights) or as fp16 (fp16 and NVFP4 weights) */
   int32_t reserved;
   int32_t i[24];
   float f[4];

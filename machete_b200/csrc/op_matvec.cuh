@@ -46,7 +46,10 @@ __device__ __forceinline__ uint32_t mv_half_bytes(int wfmt, int Kc) {
 // Row stride of the staged activations, bytes.  The eight lanes of a shared-memory phase read two rows (g, g + 1) at
 // four 16-byte chunks, 32 bytes apart with bf16 / fp16 weights: an odd multiple of 16 bytes from row to row makes the
 // eight distinct (64 bytes, pairs of them on the same banks: 1B-shape step at 16 rows 2060 us against 2018).
-__device__ __forceinline__ uint32_t mv_row_stride(int K, bool fp4) { return (uint32_t)K * 2u + (fp4 ? 64u : 16u); }
+// It follows the type the rows are staged in, not the weights': ops with one act_key read the same staged rows, and rows
+// staged as f16 serve fp16 and NVFP4 weights.  Those keep 64 bytes: NVFP4 steps of two and eight rows lose 0.8 and 0.3 %
+// by 16, fp16 products of 8 to 32 rows would gain 3 to 5 % (16 x 2048 -> 8192 19.2 us, 18.3).
+__device__ __forceinline__ uint32_t mv_row_stride(int K, bool bf16_rows) { return (uint32_t)K * 2u + (bf16_rows ? 16u : 64u); }
 
 // What the loader needs to issue the pages of one unit (from the instruction record).
 struct MvLoad {
@@ -164,8 +167,7 @@ __device__ __forceinline__ void mv_stage(Ctx& c, const mk_op_t* op, bool stage, 
   const int at = WFC == 0 ? (int)MK_T_BF16 : (WFC == 2 ? (int)MK_T_FP16 : mv_act_type(op));
   // a bf16 kernel always takes the RMSNorm scale in the epilogue: the second pass is not even compiled
   const bool fused = WFC == 0 ? pro != MK_PRO_NONE : (WFC != 2 && mv_rstd_in_epilogue(op));
-  const bool fp4 = WFC == 0 ? false : (WFC == 2 ? true : mv_is_fp4(op->i[MK_MV_WFMT]));
-  const uint32_t xs = mv_row_stride(K, fp4);
+  const uint32_t xs = mv_row_stride(K, at == MK_T_BF16);
   const int chunks = K >> 3;
   const uint16_t* x = reinterpret_cast<const uint16_t*>(op->p[MK_MV_P_X]);
   const uint16_t* ri = reinterpret_cast<const uint16_t*>(op->p[MK_MV_P_RES_IN]);
@@ -571,7 +573,7 @@ __device__ __forceinline__ bool mv_unit(Ctx& c, const mk_op_t* op, const UnitArg
   const int K = op->i[MK_MV_K], Kc = op->i[MK_MV_KC], M = op->i[MK_MV_M];
   const int wfmt = WFC == 0 ? (int)MK_W_BF16 : op->i[MK_MV_WFMT];
   const bool dense = WFC == 0 ? true : (WFC == 2 ? false : (wfmt == MK_W_BF16 || wfmt == MK_W_FP16));
-  const uint32_t xs = mv_row_stride(K, !dense);
+  const uint32_t xs = mv_row_stride(K, WFC == 0 || wfmt == MK_W_BF16);
   const uint32_t half = mv_half_bytes(wfmt, Kc);
   const int NPG = c.pv->n_pages;
   if (part == 0 && op->i[MK_MV_EPI] == MK_EPI_RESIDUAL && op->i[MK_MV_S] == 1) {

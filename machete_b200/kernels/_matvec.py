@@ -237,7 +237,7 @@ def lower_matvec(
         residual_in.data_ptr() if (pro == N.PRO_ADD_RMS) else 0,
         tuple(residual_in.stride()) if (pro == N.PRO_ADD_RMS) else (),
         norm_weight.data_ptr() if pro != N.PRO_NONE else 0, pro, float(eps), xt,
-        N.T_BF16 if w0.fmt == N.W_BF16 else N.T_FP16,
+        N.T_BF16 if w0.fmt == N.W_BF16 else N.T_FP16,      # the type the rows are staged in fixes their layout
     )
     return op
 
