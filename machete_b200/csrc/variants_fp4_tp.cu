@@ -4,6 +4,10 @@
 
 using namespace mk;
 
+// (the first kernel's features; none of the three takes the forms that spill here)
+static_assert(!kWideStep<1, 2, MK_F_AT128 | MK_F_QKNORM | MK_F_TOP1 | MK_F_AR>, "untimed in that form");
+static_assert(kWideStep<1, 2, MK_F_AT128 | MK_F_QKNORM | MK_F_TOP1> && kWideStep<0, -1, MK_F_ALL>, "timed in that form");
+
 static const mk_variant kVariants[] = {
     {1, 2, MK_F_AT128 | MK_F_QKNORM | MK_F_TOP1 | MK_F_AR, mk::mk_persistent_kernel<1, 2, MK_F_AT128 | MK_F_QKNORM | MK_F_TOP1 | MK_F_AR>},
     {2, 2, MK_F_AT128 | MK_F_QKNORM | MK_F_TOP1 | MK_F_AR, mk::mk_persistent_kernel<2, 2, MK_F_AT128 | MK_F_QKNORM | MK_F_TOP1 | MK_F_AR>},
