@@ -1,4 +1,4 @@
-"""Products of 17 to 32 rows: whole pairs of 64-value tiles, a single one behind them, pages that end in either."""
+"""Products at the edges of the row tiles: whole pairs of 64-value tiles, a single one behind them, pages that end in either."""
 
 import pytest
 import torch
@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("rows", [17, 24, 25, 32])
+@pytest.mark.parametrize("rows", [1, 8, 9, 16, 17, 24, 25, 32])
 @pytest.mark.parametrize("k", [64, 128, 192, 1024, 1088, 1152])
 def test_rows_and_tile_counts(dtype, rows, k):
     g = torch.Generator().manual_seed(rows * k)
