@@ -129,6 +129,8 @@ def lower_program(ops: List[ScheduledOp], ctx: LowerCtx) -> List[NativeOp]:
     from ..kernels._matvec import dense_weight, flat_out_strides, lower_matvec
 
     out: List[NativeOp] = []
+    # the kernels with the in-kernel all-reduce hold no sum of K blocks: a program with both would run the generic one
+    parallel = not any(sop.op_cls.__name__.startswith("AllReduce") for sop in ops)
     i = 0
     while i < len(ops):
         sop = ops[i]
@@ -142,7 +144,7 @@ def lower_program(ops: List[ScheduledOp], ctx: LowerCtx) -> List[NativeOp]:
                 out.append(nop)
                 i += n
                 continue
-            blocks = _parallel_kblocks(ops, i, ctx)
+            blocks = _parallel_kblocks(ops, i, ctx) if parallel else []
             if blocks:
                 out.extend(blocks)
                 i += len(blocks)

@@ -3,8 +3,10 @@
 import torch
 
 from machete_b200 import _native as N
+from machete_b200.kernels.allreduce import AllReduceSm100Op
 from machete_b200.kernels.decode_matvec import MatvecResidualSm100Op, MatvecSm100Op
 from machete_b200.megakernel import Megakernel, MegakernelConfig, OverlapTileScheduler
+from machete_b200.megakernel.peer import PeerBuffers
 from machete_b200.megakernel.scheduling import simulate
 
 BF = torch.bfloat16
@@ -49,3 +51,15 @@ def test_chains_that_read_their_own_output_stay_chains():
         mk = Megakernel(ops, config=MegakernelConfig(num_sms=16))
         assert all(op.commutes is None for op in mk.native_ops)
         assert mk.program.deps[1].coarse == ([0] if ops is inside else [])
+
+
+def test_programs_with_an_all_reduce_keep_their_chains():
+    # (no kernel has both but the generic one)
+    x, y = torch.zeros(16, 1, 4096, dtype=BF), torch.zeros(16, 1, 256, dtype=BF)
+    part, total = torch.zeros(16, 1, 256), torch.zeros(16, 1, 256, dtype=BF)
+    ops = chain(x, torch.zeros(256, 4096, dtype=BF), y, 4)
+    ops += MatvecSm100Op.schedule(a=y, weight=torch.zeros(256, 256, dtype=BF), y=part)
+    reduced = AllReduceSm100Op.schedule(peers=PeerBuffers(1 << 20, rank=0, world_size=2), x=part, y=total)
+    for with_reduce in (False, True):
+        mk = Megakernel(ops + (reduced if with_reduce else []), config=MegakernelConfig(num_sms=16))
+        assert [op.commutes is not None for op in mk.native_ops[:4]] == [not with_reduce] * 4
