@@ -127,6 +127,7 @@ static __device__ void loader_loop(Ctx& c, int ibeg, int iend) {
       }
       if (need_wait) {
         if (!wait_counters(c, ins.n_lwaits, ins.lwait_off)) break;
+        if (ELECT) __syncwarp();   // lane 0 saw the counters, another lane may issue
         trace(c, TRC_LWAIT_DONE, base + i);
       }
       if (ins.maps == 0) continue;   // only units with tensor maps stream pages
@@ -168,7 +169,7 @@ static __device__ void loader_loop(Ctx& c, int ibeg, int iend) {
         }
       }
       issued = __shfl_sync(0xffffffffu, issued, leader);
-      if (issued < n_pages) c.dead = true;   // lane 0 gave up (abort flag is already raised)
+      if (issued < n_pages) c.dead = true;   // the lane gave up (abort flag is already raised)
       ring_advance(rp, issued, NP);
       seq += (uint32_t)issued;
     }
@@ -514,7 +515,7 @@ __global__ void __launch_bounds__(kThreads, 1) mk_persistent_kernel(const __grid
   c.lane = threadIdx.x & 31;
   c.instr_idx = -1;
   c.dead = false;
-  trace_init<(FEAT & MK_F_TRACE) != 0>(c);
+  trace_init<(FEAT & MK_F_TRACE) != 0, kWideStep<NTC, WFC, FEAT>>(c);
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < pv.n_pages; ++i) {

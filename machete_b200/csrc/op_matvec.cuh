@@ -65,7 +65,7 @@ struct MvLoad {
 
 // Issue the copies of K-slice `p` into the page at `page` (shared address):
 // two tiled TMA copies (four with NVFP4 scales) and one arrival for the whole
-// loader warp.  Called by loader lane 0 only.
+// loader warp.  Called by one lane of it.
 __device__ __forceinline__ void mv_load_issue(const MvLoad& l, int p, uint32_t page, uint32_t bar, uint64_t policy) {
   const int kt0 = p * l.tiles_per_page;
   if (!l.fp4) {

@@ -163,7 +163,7 @@ struct Ctx {
   bool dead;          // a wait expired somewhere: skip work, keep barriers
   int trace_n;        // records this warp has written
   int trace_cap;
-  TraceRec* trace_base;  // this warp's trace ring (lane 0 only), null = off
+  TraceRec* trace_base;  // this warp's trace ring (one lane only, see trace_init), null = off
 };
 
 // The consumers' registers for one instruction record (one record per lane of
@@ -225,13 +225,20 @@ __device__ __forceinline__ void trace_sync_pair(Ctx& c) {
   }
   c.trace_n += 2;
 }
-template <bool TRACED>
+// One lane of a warp records: lane 0, and in a loader that issues under elect_one (ELECT) the lane that it elects (always
+// the same one for the same mask).
+template <bool TRACED, bool ELECT>
 __device__ __forceinline__ void trace_init(Ctx& c) {
   c.trace_n = 0;
   c.trace_cap = 0;
   c.trace_base = nullptr;   // stays null in a kernel built without tracing: every trace point folds away
   TraceRec* base = TRACED ? c.pv->trace : nullptr;
-  if (TRACED && base != nullptr && c.lane == 0) {
+  bool mine = c.lane == 0;
+  if (TRACED && ELECT && c.warp == 0) {
+    int leader;
+    mine = elect_one(leader);
+  }
+  if (TRACED && base != nullptr && mine) {
     prior_work_done();   // the launch before this one may still be writing its records
     c.trace_cap = c.pv->trace_cap - 2;   // room for the closing pair
     c.trace_base = base + ((size_t)blockIdx.x * (kConsumerWarps + 1) + c.warp) * c.pv->trace_cap;
