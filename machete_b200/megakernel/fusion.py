@@ -14,6 +14,7 @@ blocks run side by side instead (``_parallel_kblocks``).
 
 from __future__ import annotations
 
+from dataclasses import replace
 from typing import List
 
 import torch
@@ -75,6 +76,11 @@ _ADDED_BLOCK = {"MatvecSm100Op": "MatvecResidualSm100Op", "MatvecSm120Op": "Matv
 _MAX_PARALLEL_BLOCKS = 8
 
 
+def _row_class(rows: int) -> int:
+    """Rows that a kernel's accumulators hold for ``rows`` activation rows."""
+    return 8 if rows <= 8 else (16 if rows <= 16 else 32)
+
+
 def _parallel_kblocks(ops: List[ScheduledOp], start: int, ctx: LowerCtx) -> List[NativeOp]:
     """The chain ``y = a0 W0^T; y = y + a1 W1^T; ...`` as ops that run side by side ([] if it does not start here).
 
@@ -107,7 +113,7 @@ def _parallel_kblocks(ops: List[ScheduledOp], start: int, ctx: LowerCtx) -> List
     units = blocks[0].n_units
     if len(blocks) != n or any(b.n_units != units or b.i[N.MV_M] != blocks[0].i[N.MV_M] for b in blocks):
         return []
-    rows = 8 if blocks[0].i[N.MV_M] <= 8 else (16 if blocks[0].i[N.MV_M] <= 16 else 32)
+    rows = _row_class(blocks[0].i[N.MV_M])
     key = ("kblock parts", units * n * 16 * rows, y.data_ptr())   # (chunks of a batch have rows of their own)
     parts = ctx.scratch.get(key)
     if parts is None:
@@ -123,6 +129,38 @@ def _parallel_kblocks(ops: List[ScheduledOp], start: int, ctx: LowerCtx) -> List
         op.zero_on_reset = [*op.zero_on_reset, arrive]
         op.commutes, op.cta_share = group, (b, n)
     return blocks
+
+
+def in_place_of(old: NativeOp, new: NativeOp) -> NativeOp:
+    """``new`` as the record that replaces ``old`` of a compiled program.
+
+    The blocks of one product share the buffer of their sums and its counters, so a block that is replaced by itself has to
+    keep those of its program, and a product that stands alone in the program that lowered it has to become a block (a
+    block outside its group would wait for sums that nobody leaves).
+    """
+    if new.i.get(N.MV_EPI) == N.EPI_KSUM and new.opcode == N.OP_MATVEC:
+        # as the chain has it: the first block stores, the others add to what is there
+        alone = {N.MV_EPI: N.EPI_RESIDUAL if new.i[N.MV_KBLOCK] else N.EPI_STORE, N.MV_KBLOCKS: 0, N.MV_KBLOCK: 0}
+        shared = (N.MV_P_KPART, N.MV_P_KARRIVE)
+        new = replace(new, i={**new.i, **alone}, p={k: v for k, v in new.p.items() if k not in shared}, commutes=None,
+                      cta_share=None, zero_on_reset=[])
+    if old.i.get(N.MV_EPI) != N.EPI_KSUM or old.opcode != N.OP_MATVEC:
+        return new
+    block = old.i[N.MV_KBLOCK]
+    adds = new.i.get(N.MV_EPI) == N.EPI_RESIDUAL and new.p[N.MV_P_EPI_RES] == new.p[N.MV_P_OUT] and all(
+        new.s[r] == new.s[o] for r, o in ((N.MV_S_ER_B, N.MV_S_O_B), (N.MV_S_ER_S, N.MV_S_O_S)))
+    if new.opcode != N.OP_MATVEC or new.i[N.MV_MODE] != N.MV_PLAIN or new.i[N.MV_PRO] != N.PRO_NONE or \
+            new.i[N.MV_TR] != N.TR_NONE or not (adds if block else new.i[N.MV_EPI] == N.EPI_STORE):
+        raise ValueError(f"{old.name}: block {block} of {old.i[N.MV_KBLOCKS]} of a product can only become such a block: a plain "
+                         f"product that {'adds to its own output' if block else 'stores'} (compile with fuse=False otherwise)")
+    parts, arrive = old.p[N.MV_P_KPART], old.p[N.MV_P_KARRIVE]
+    room = next(t for t in old.keep if t.data_ptr() == parts).numel()
+    if old.n_units * old.i[N.MV_KBLOCKS] * 16 * _row_class(new.i[N.MV_M]) > room:
+        raise ValueError(f"{old.name}: {new.i[N.MV_M]} rows do not fit the sums' buffer of a product lowered for {old.i[N.MV_M]}")
+    return replace(new, i={**new.i, N.MV_EPI: N.EPI_KSUM, N.MV_KBLOCKS: old.i[N.MV_KBLOCKS], N.MV_KBLOCK: block},
+                   p={**new.p, N.MV_P_KPART: parts, N.MV_P_KARRIVE: arrive},
+                   keep=[*new.keep, *(t for t in old.keep if t.data_ptr() in (parts, arrive))],
+                   commutes=old.commutes, cta_share=old.cta_share, zero_on_reset=list(old.zero_on_reset))
 
 
 def lower_program(ops: List[ScheduledOp], ctx: LowerCtx) -> List[NativeOp]:

@@ -377,7 +377,10 @@ class Megakernel:
 
     def update_op(self, index: int, native_op: NativeOp, stream=None) -> None:
         """Replace op record ``index`` on the device (e.g. a new cache position)."""
+        from .fusion import in_place_of
+
         self.compile()
+        native_op = in_place_of(self.native_ops[index], native_op)
         rec = np.zeros(1, dtype=N.OP_DTYPE)
         rec[0] = native_op.record(int(self.program.ops[index]["act_key"]))
         handle = None if stream is None else C.c_void_p(getattr(stream, "cuda_stream", stream))

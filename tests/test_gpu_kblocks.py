@@ -72,3 +72,33 @@ def result(ops, rows, out, blocks, cfg, sched):
         y.fill_(float("nan"))
         mk.run()
     return y.clone(), z.clone()
+
+
+@pytest.mark.parametrize("from_chain", [True, False])
+def test_one_block_gets_other_weights(from_chain):
+    g = torch.Generator().manual_seed(3)
+    a = torch.randn(16, 1, 8192, generator=g).to(BF).cuda()
+    w, w2 = ((0.05 * torch.randn(256, 8192, generator=g)).to(BF).cuda() for _ in range(2))
+
+    def chain(weight, y):
+        ops = MatvecSm100Op.schedule(a=a[..., :2048], weight=weight[:, :2048], y=y)
+        for b in range(1, 4):
+            s = slice(b * 2048, (b + 1) * 2048)
+            ops += MatvecResidualSm100Op.schedule(a=a[..., s], weight=weight[:, s], residual_in=y, residual_out=y)
+        return ops
+
+    got = []
+    for fuse in (True, False):
+        cfg = MegakernelConfig(fuse=fuse)
+        y = torch.full((16, 1, 256), float("nan"), dtype=BF, device="cuda")
+        mk = Megakernel(chain(w, y), config=cfg)
+        mk.run()
+        fresh = Megakernel(chain(w2, y), config=MegakernelConfig(fuse=from_chain))
+        for block in (2, 0):
+            mk.update_op(block, fresh.native_ops[block])
+            for _ in range(2):
+                y.fill_(float("nan"))
+                mk.run()
+            got.append(y.clone())
+    assert torch.equal(got[0], got[2]) and torch.equal(got[1], got[3]) and not torch.equal(got[0], got[1])
+    assert not got[0].isnan().any()

@@ -1,11 +1,13 @@
 """K blocks side by side (CPU): who waits for whom, where the units go, and which chains stay chains."""
 
+import pytest
 import torch
 
 from machete_b200 import _native as N
 from machete_b200.kernels.allreduce import AllReduceSm100Op
 from machete_b200.kernels.decode_matvec import MatvecResidualSm100Op, MatvecSm100Op
 from machete_b200.megakernel import Megakernel, MegakernelConfig, OverlapTileScheduler
+from machete_b200.megakernel.fusion import in_place_of
 from machete_b200.megakernel.peer import PeerBuffers
 from machete_b200.megakernel.scheduling import simulate
 
@@ -63,3 +65,32 @@ def test_programs_with_an_all_reduce_keep_their_chains():
     for with_reduce in (False, True):
         mk = Megakernel(ops + (reduced if with_reduce else []), config=MegakernelConfig(num_sms=16))
         assert [op.commutes is not None for op in mk.native_ops[:4]] == [not with_reduce] * 4
+
+
+def test_a_replaced_block_keeps_its_place_in_the_group():
+    a, w, y = torch.zeros(16, 1, 4096, dtype=BF), torch.zeros(256, 4096, dtype=BF), torch.zeros(16, 1, 256, dtype=BF)
+    cfg = MegakernelConfig(num_sms=16)
+    mine = Megakernel(chain(a, w, y, 4), config=cfg).native_ops
+    w2 = torch.zeros(256, 4096, dtype=BF)
+    fresh = Megakernel(chain(a, w2, y, 4), config=cfg).native_ops                   # blocks of another program
+    plain = Megakernel(chain(a, w2, y, 4), config=MegakernelConfig(num_sms=16, fuse=False)).native_ops
+    for b in range(4):
+        for new in (fresh[b], plain[b]):
+            got = in_place_of(mine[b], new)
+            for slot in (N.MV_P_KPART, N.MV_P_KARRIVE):
+                assert got.p[slot] == mine[b].p[slot]
+            assert got.p[N.MV_P_W0] == w2[:, b * 1024:].data_ptr() and got.i[N.MV_EPI] == N.EPI_KSUM
+            assert (got.i[N.MV_KBLOCK], got.i[N.MV_KBLOCKS], got.commutes) == (b, 4, mine[0].commutes)
+            assert got.zero_on_reset == mine[b].zero_on_reset
+            assert in_place_of(got, got).record(1) == got.record(1)
+        # a block in a program of single ops is what the chain has
+        assert in_place_of(plain[b], fresh[b]).record(1) == plain[b].record(1)
+    # what is no block of the product is refused: another epilogue, another residual, more rows than the buffer holds
+    with pytest.raises(ValueError, match="block 0 of 4"):
+        in_place_of(mine[0], plain[1])
+    other = MatvecResidualSm100Op.schedule(a=a[..., :1024], weight=w[:, :1024], residual_in=torch.zeros_like(y), residual_out=y)
+    with pytest.raises(ValueError, match="block 1 of 4"):
+        in_place_of(mine[1], Megakernel(other, config=cfg).native_ops[0])
+    wide, wide_y = torch.zeros(17, 1, 1024, dtype=BF), torch.zeros(17, 1, 256, dtype=BF)
+    with pytest.raises(ValueError, match="17 rows do not fit"):
+        in_place_of(mine[0], Megakernel(MatvecSm100Op.schedule(a=wide, weight=w[:, :1024], y=wide_y), config=cfg).native_ops[0])
