@@ -385,6 +385,11 @@ int mk_reset(mk_handle_t h, void* cuda_stream);
  * the reference, which runs all ranks from one process
  * (megakernel/runtime_components.py:272-287). */
 int mk_launch_count(mk_handle_t h, int32_t* out);
+/* Where the participants of a shared attention unit leave their states in this program (kernels for whole decode steps of
+ * several rows or NVFP4 weights; others leave them in their last pages): out[0] bytes of a unit's states in the staging
+ * buffer, 0 = in the pages; [1] units that may be between states and merge (1, 2 or 4); [2] 0 = an op of the program relies
+ * on rows that were staged before an attention op, so the buffer is not used. */
+int mk_state_placement(mk_handle_t h, int32_t out[3]);
 int mk_set_launch_count(mk_handle_t h, int32_t count, void* cuda_stream);
 /* Replace op record `op_index` (new pointers, a new cache position, a longer
  * KV window).  The record is validated like mk_create does, the opcode and

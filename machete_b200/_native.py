@@ -113,7 +113,7 @@ class Program(C.Structure):
 
 EXPORTS = [
     "mk_abi_version", "mk_last_error", "mk_device_info", "mk_workspace_bytes", "mk_create", "mk_run",
-    "mk_status", "mk_workspace_status", "mk_set_trace", "mk_reset", "mk_launch_count", "mk_set_launch_count",
+    "mk_status", "mk_workspace_status", "mk_set_trace", "mk_reset", "mk_launch_count", "mk_state_placement", "mk_set_launch_count",
     "mk_update_op", "mk_read_counters", "mk_destroy",
     "mk_standalone_workspace_bytes", "mk_matvec_bf16", "mk_matvec_nvfp4", "mk_flash_decode",
     "mk_flash_decode_noalloc", "mk_flash_decode_noalloc_status",
@@ -178,6 +178,7 @@ def _declare(h: C.CDLL) -> None:
     h.mk_set_trace.restype = C.c_int
     h.mk_reset.argtypes = [vp, vp]
     h.mk_launch_count.argtypes = [vp, C.POINTER(i32)]
+    h.mk_state_placement.argtypes = [vp, C.POINTER(i32)]
     h.mk_set_launch_count.argtypes = [vp, i32, vp]
     h.mk_update_op.argtypes = [vp, i32, vp, vp]
     h.mk_read_counters.argtypes = [vp, C.POINTER(i32), i32]

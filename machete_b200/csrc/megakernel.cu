@@ -861,6 +861,12 @@ int mk_launch_count(mk_handle_t h, int32_t* out) {
   return 0;
 }
 
+int mk_state_placement(mk_handle_t h, int32_t out[3]) {
+  if (!h || !out) return mk::fail(-1, "null argument");
+  out[0] = h->pv.at_set_bytes, out[1] = h->pv.at_sets, out[2] = h->states_may_stage ? 1 : 0;
+  return 0;
+}
+
 int mk_set_launch_count(mk_handle_t h, int32_t count, void* cuda_stream) {
   using namespace mk;
   if (!h) return fail(-1, "null handle");
