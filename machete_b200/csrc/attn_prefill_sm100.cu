@@ -491,9 +491,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     const int row = qd * 32 + lane;                 // query row inside the tile = TMEM lane
     const int m = m0 + (row >> p.pack_log2), h = h0 + (row & (p.pack - 1));
     const int lim = p.causal ? (p.N - p.M + m) : (p.N - 1);   // last visible token of this row
-    // Open tiles take another mix of exponentials (see p_pass), so which tiles are open is a matter of results: it goes
-    // by blocks of 32 queries, whatever the heads in a tile.  (Every row of a warp is in one block.)
-    const int open_lim = p.causal ? (p.N - p.M + (m & ~31)) : (p.N - 1);
+    // Only the tiles on the causal diagonal and the last one of a ragged cache need the per-score mask; the first n_open
+    // do not.  They take another mix of exponentials (see p_pass), so which they are is a matter of results: it goes by
+    // blocks of 32 queries, whatever the heads in a tile.  (Every row of a warp is in one block.)
+    const int n_open = min(p.causal ? p.N - p.M + (m & ~31) + 1 : p.N, p.N) / kBN;
     const uint32_t lane_addr = tmem + ((uint32_t)(qd * 32) << 16);
     const uint64_t scale2 = pack2(p.scale_log2, p.scale_log2);
     float mx = -INFINITY, sum = 0.f;
@@ -503,9 +504,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      // Only the tiles on the causal diagonal and the last one of a ragged cache need the per-score
-      // mask: `open` is true (for the whole warp) everywhere else.
-      const bool open = __all_sync(0xffffffffu, (j * kBN + kBN - 1 <= open_lim) && (j * kBN + kBN <= p.N));
+      const bool open = __all_sync(0xffffffffu, j < n_open);   // (the vote makes it known to be uniform)
       const uint32_t s_addr = lane_addr + (uint32_t)(j & (SB - 1)) * kBN;
       uint32_t r[kBN];                               // this row of S, then of P (bf16 pairs in r[0 .. 32))
       tmem_ld64(s_addr, r);
