@@ -435,9 +435,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       }
     }
   } else if (SB == 2 && warp == 1) {
-    // Head dim 64 issues as a whole warp (see tc_mma).  At 128 the tensor pipe is the bound either way and one lane
-    // that waits and issues is the lighter neighbour: 0.9 % faster on average over fifteen prompts that fill the
-    // device, 2.3 % over three that do not (2190 x 2190 causal 52.5 us against 54.5, 1637 x 1637 61.9 against 61.3).
+    // Head dim 64 issues as a whole warp (see tc_mma).  At 128 one lane that waits and issues is the lighter neighbour
+    // where prompts fill the device (causal, 32 / 8 heads, 2190 x 2190 42.2 us against 45.2, 4096 x 4096 145.7 against
+    // 150.3).  A tile that has its SM to itself would be quicker by the warp (512 x 512 10.4 us, 9.9 so; 300 behind 1700
+    // tokens 28.1, 26.7).
     constexpr bool kOneLane = D == 128;
     if (!kOneLane || lane == 0) {
       auto wait_mma = [&](uint32_t bar, uint32_t parity, int code, int aux) -> bool {
@@ -821,9 +822,11 @@ int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, 
   p.timeout_ns = (uint64_t)(timeout_ms > 0 ? timeout_ms : 1000) * 1000000ull;
   const dim3 grid(H / pack, B, pl.row_tiles);
   // Where this grid leaves slots empty (two CTAs an SM), the next one is let in late: its CTAs would pile up on the
-  // SMs that are free now (the average over six such prompts at head dim 64 11 % faster, three at 128 3.5 %).  With
-  // every slot taken nothing piles up, and at head dim 64 (1960 behind 2045 tokens 84.8 us early, 86.7 late) the
-  // last load is too short before the end to hide the placement; at 128 (0.4 % faster late) it is not.
+  // SMs that are free now (causal, 32 / 8 heads, head dim 64, early / late: 777 x 777, 200 tiles 12.1 us / 11.2, 1024 x 1024,
+  // 256 tiles 16.3 / 13.5).  With the slots taken several times over it makes no difference up to 62 us a pass (2048 x 2048
+  // to two sequences of 2045), then early is 0.7 % faster (4096 x 4096 109.7 / 110.4); just above one round late would
+  // still be the better one (1185 x 1185, 304 tiles 18.5 / 16.0, 1500 x 1500, 376 tiles 22.2 / 20.4).  At 128 late is
+  // never behind by more than a run's noise.
   p.next_early = D == 64 && !pl.three && pl.tiles >= 2 * (int64_t)d->sms ? 1 : 0;
   // the kernel may be placed while the one before it in the stream drains (it waits before it touches memory)
   cudaLaunchConfig_t cfg = {};

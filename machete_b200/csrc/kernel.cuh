@@ -86,13 +86,14 @@ __device__ __forceinline__ LoaderInstr bcast_loader_instr(const LoaderInstr& m, 
 
 // Which kernels take the forms for whole decode steps of several rows or NVFP4 weights: a loader that issues under
 // elect_one, units found by one vote (see consumer_loop), attention states in the staging buffer (see at_unit).
-// Together, on one GPU: 8B shape, NVFP4, one row, KV 8192 2866 -> 2754 us a step, 8 rows, KV 4096 4925 -> 4706; 1B shape,
-// 16 rows, KV 1931 1627 -> 1529.  Programs of projections alone (bf16 1 x 4096 -> 14336 24.7 us, 25.4 so; NVFP4 4 rows
-// 19.5, 19.9) and bf16 steps of up to 8 rows (829 us, 840) lose by them: their few units a CTA are found in a step or
-// two, and a page is two copies for twice the bytes.  The NVFP4 kernels with the in-kernel all-reduce, which wants several
-// GPUs, have been timed in neither form; with these they spill 44 bytes instead of 36 (the 8B kernel above lost its gain to
-// 44), so they keep the others.  The generic kernels, all-reduce or not, take them (4 layers, us: bf16, one row of a program
-// that has other rows too, KV 4000 340 -> 250, NVFP4, 8 rows, KV 2000 882 -> 649, with the product loop dealt out).
+// us a step without one of them / with all three: 8B shape, NVFP4, one row, KV 8192 2832 / 2746 (loader), 2790 (lookup),
+// 2745 (states); 8 rows, KV 4096 4743, 4766, 4799 / 4692; 1B shape, 16 rows, KV 1931 1524, 1548, 1562 / 1509.
+// Programs of projections alone (bf16 1 x 4096 -> 14336 24.7 us, 25.4 so; NVFP4 4 rows 19.5, 19.9) and bf16 steps of up
+// to 8 rows (829 us, 840) lose by them: their few units a CTA are found in a step or two, and a page is two copies for
+// twice the bytes.  The NVFP4 kernels with the in-kernel all-reduce, which wants several GPUs, have been timed in neither
+// form; with these they spill 44 bytes instead of 36 (the 8B kernel above lost its gain to 44), so they keep the others.
+// The generic kernels, all-reduce or not, take them (4 layers, us: bf16, one row of a program that has other rows too,
+// KV 4000 340 -> 250, NVFP4, 8 rows, KV 2000 882 -> 649, with the product loop dealt out).
 template <int NTC, int WFC, int FEAT>
 constexpr bool kWideStep = NTC >= 0 && (NTC != 1 || WFC != 0) && (FEAT & (MK_F_AT64 | MK_F_AT128)) != 0 &&
                            ((FEAT & MK_F_AR) == 0 || WFC == -1);

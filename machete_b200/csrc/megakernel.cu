@@ -296,7 +296,7 @@ static int validate_op(const mk_op_t& op, int idx, int page_bytes, int act_bytes
       return fail(-2, "op %d: NVFP4 matvec needs K < 2048 or K %% 2048 == 0, got %d", idx, K);
     const uint64_t need = mv_page_need(wf, Kc);
     if (need > (uint64_t)page_bytes) return fail(-2, "op %d: K slice %d does not fit a %d-byte page", idx, Kc, page_bytes);
-    if ((uint64_t)M * ((uint64_t)K * 2 + 64) > (uint64_t)act_bytes)
+    if ((uint64_t)M * ((uint64_t)K * 2 + 64) > (uint64_t)act_bytes)   // (the wider of the two row strides)
       return fail(-2, "op %d: %d x %d activations exceed the %d-byte staging buffer", idx, M, K, act_bytes);
     if (!aligned16(op.p[MK_MV_P_W0]) || !op.p[MK_MV_P_W0] || (op.s[MK_MV_S_WROW] & 15))
       return fail(-2, "op %d: weight pointer / row stride must be 16-byte aligned", idx);

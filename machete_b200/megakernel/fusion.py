@@ -24,7 +24,7 @@ from .lowering import LowerCtx, NativeOp, Region, meta_of
 from .ops import ScheduledOp, tensor_meta_overlaps
 
 
-# Bytes of staged activations (rows x (K * 2 + 64)) that still leave six 18 KB / three 32 KB weight
+# Bytes of staged activations (rows x (K * 2 + 64), the wider of the two row strides) that still leave six 18 KB / three 32 KB weight
 # pages in shared memory: a matvec op stages its whole input, so batch x K is bounded by this.
 STAGING_BUDGET = 100 * 1024
 
