@@ -74,6 +74,10 @@ def _kblock_chain(ops: List[ScheduledOp], start: int):
 _ADDED_BLOCK = {"MatvecSm100Op": "MatvecResidualSm100Op", "MatvecSm120Op": "MatvecResidualSm120Op",
                 "MatvecNvfp4Sm120Op": "MatvecResidualNvfp4Sm120Op"}
 _MAX_PARALLEL_BLOCKS = 8
+# What a unit costs besides its K values, in K values: blocks of different lengths get CTAs by length + this.  1-row NVFP4
+# product of 8192 + 2048 -> 14336 values 35.7 us as a chain, 45.0 on half the CTAs each, 34.8 so; bf16, 8 rows, 4096 + 512
+# 39.9, 37.8, 31.5; NVFP4, 8 rows, 6144 + 256 -> 4096 21.2, 24.3, 20.1 (by length alone 33.6: short units are not free).
+_UNIT_COST = 1280
 
 
 def _row_class(rows: int) -> int:
@@ -84,7 +88,7 @@ def _row_class(rows: int) -> int:
 def _parallel_kblocks(ops: List[ScheduledOp], start: int, ctx: LowerCtx) -> List[NativeOp]:
     """The chain ``y = a0 W0^T; y = y + a1 W1^T; ...`` as ops that run side by side ([] if it does not start here).
 
-    Each block keeps its own op, with its own K slice to stage, on every n-th CTA; the last block to finish a unit's
+    Each block keeps its own op, with its own K slice to stage, on its part of the CTAs; the last block to finish a unit's
     rows adds the blocks' fp32 sums in block order and rounds after each (``MK_EPI_KSUM``): the bits of the chain, in one
     dependency stage instead of n.  16-layer 1B shape, 16 rows, KV 1931 (4 blocks): 2020 -> 1627 us a step; 36-layer 8B
     shape with NVFP4 weights, 8 rows, KV 4096 (2 blocks): 5034 -> 4925.
@@ -120,6 +124,7 @@ def _parallel_kblocks(ops: List[ScheduledOp], start: int, ctx: LowerCtx) -> List
         parts = ctx.scratch[key] = torch.empty(units * n * 16 * rows, dtype=torch.float32, device=y.device)
     arrive = torch.zeros(units, dtype=torch.int32, device=y.device)
     group = object()
+    costs = tuple(op.i[N.MV_K] + _UNIT_COST for op in blocks)
     for b, op in enumerate(blocks):
         op.i.update({N.MV_EPI: N.EPI_KSUM, N.MV_KBLOCKS: n, N.MV_KBLOCK: b})
         op.p.update({N.MV_P_KPART: parts.data_ptr(), N.MV_P_KARRIVE: arrive.data_ptr()})
@@ -127,7 +132,7 @@ def _parallel_kblocks(ops: List[ScheduledOp], start: int, ctx: LowerCtx) -> List
         op.writes = [*op.writes, Region(meta_of(parts, "kblock parts"))]
         op.keep += [parts, arrive]
         op.zero_on_reset = [*op.zero_on_reset, arrive]
-        op.commutes, op.cta_share = group, (b, n)
+        op.commutes, op.cta_share = group, (b, costs)
     return blocks
 
 

@@ -93,8 +93,8 @@ class NativeOp:
     pos_limit: Optional[int] = None
     # ops that share this object write the same memory in any order (the K blocks of one product)
     commutes: Optional[object] = None
-    # (i, n): the units go to every n-th CTA, the i-th of them first (ops that run side by side)
-    cta_share: Optional[Tuple[int, int]] = None
+    # (i, costs): ops of these costs run side by side, each on its part of the CTAs; this one is the i-th
+    cta_share: Optional[Tuple[int, Tuple[int, ...]]] = None
     # scratch that must be zero when a launch starts; the kernel leaves it zero unless a launch aborted
     zero_on_reset: list = field(default_factory=list)
 

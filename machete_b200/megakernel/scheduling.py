@@ -25,6 +25,7 @@ and every wait refers to an earlier op of that order.
 from __future__ import annotations
 
 from dataclasses import dataclass, field
+from functools import lru_cache
 from typing import Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -67,12 +68,25 @@ class BackwardScheduler(TileScheduler):
         return out
 
 
+@lru_cache(maxsize=64)
+def share_out(costs: Tuple[int, ...], num_ctas: int) -> np.ndarray:
+    """Owner of every CTA when each of ``costs`` gets its part of them, spread evenly (equal costs: CTA modulo their number)."""
+    owner, given, total = np.empty(num_ctas, dtype=np.int32), [0] * len(costs), sum(costs)
+    for cta in range(num_ctas):
+        due = [cost * (cta + 1) - total * had for cost, had in zip(costs, given)]
+        owner[cta] = due.index(max(due))
+        given[owner[cta]] += 1
+    return owner
+
+
 def shared_ctas(op: NativeOp, order: np.ndarray) -> np.ndarray:
     """The CTAs of ``order`` that may hold units of ``op`` (``NativeOp.cta_share``), in that order."""
-    if op.cta_share is None or op.cta_share[1] > len(order):
+    if op.cta_share is None:
         return order
-    i, n = op.cta_share
-    return order[order % n == i]
+    i, costs = op.cta_share
+    owner = share_out(costs, len(order))
+    # too few CTAs to give each block one: every block uses all
+    return order[owner[order] == i] if len(set(owner.tolist())) == len(costs) else order
 
 
 class OverlapTileScheduler(TileScheduler):

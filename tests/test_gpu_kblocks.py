@@ -102,3 +102,18 @@ def test_one_block_gets_other_weights(from_chain):
             got.append(y.clone())
     assert torch.equal(got[0], got[2]) and torch.equal(got[1], got[3]) and not torch.equal(got[0], got[1])
     assert not got[0].isnan().any()
+
+
+@pytest.mark.parametrize("rows,edges,out", [(1, (0, 1024, 1088), 700), (8, (0, 6144, 6656, 8192), 64), (16, (0, 512, 3072), 2400)])
+def test_blocks_of_different_lengths_equal_the_chain(rows, edges, out):
+    g = torch.Generator().manual_seed(rows)
+    a = torch.randn(rows, 1, edges[-1], generator=g).to(BF).cuda()
+    w = (0.05 * torch.randn(out, edges[-1], generator=g)).to(BF).cuda()
+
+    def ops(y, h, z):
+        chain = MatvecSm100Op.schedule(a=a[..., :edges[1]], weight=w[:, :edges[1]], y=y)
+        for lo, hi in zip(edges[1:-1], edges[2:]):
+            chain += MatvecResidualSm100Op.schedule(a=a[..., lo:hi], weight=w[:, lo:hi], residual_in=y, residual_out=y)
+        return chain
+
+    compare(ops, rows, out, len(edges) - 1)

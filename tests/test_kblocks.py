@@ -9,7 +9,7 @@ from machete_b200.kernels.decode_matvec import MatvecResidualSm100Op, MatvecSm10
 from machete_b200.megakernel import Megakernel, MegakernelConfig, OverlapTileScheduler
 from machete_b200.megakernel.fusion import in_place_of
 from machete_b200.megakernel.peer import PeerBuffers
-from machete_b200.megakernel.scheduling import simulate
+from machete_b200.megakernel.scheduling import share_out, simulate
 
 BF = torch.bfloat16
 
@@ -94,3 +94,31 @@ def test_a_replaced_block_keeps_its_place_in_the_group():
     wide, wide_y = torch.zeros(17, 1, 1024, dtype=BF), torch.zeros(17, 1, 256, dtype=BF)
     with pytest.raises(ValueError, match="17 rows do not fit"):
         in_place_of(mine[0], Megakernel(MatvecSm100Op.schedule(a=wide, weight=w[:, :1024], y=wide_y), config=cfg).native_ops[0])
+
+
+def test_ctas_are_dealt_out_by_what_the_blocks_cost():
+    assert share_out((7, 7, 7, 7), 14).tolist() == [c % 4 for c in range(14)]        # equal blocks: every n-th
+    for costs, ctas in (((8192, 2048), 148), ((1, 1000), 148), ((3, 1, 4, 1, 5), 148), ((6144, 256, 6144), 7)):
+        owner = share_out(costs, ctas)
+        for i, cost in enumerate(costs):
+            assert abs((owner == i).sum() - ctas * cost / sum(costs)) <= 1
+        first = [owner.tolist().index(i) for i in range(len(costs)) if (owner == i).any()]
+        assert max(first) - min(first) <= max(len(costs), sum(costs) // min(costs))  # spread out, not in runs
+
+
+@pytest.mark.parametrize("edges", [(0, 3072, 4096), (0, 64, 4096), (0, 2048, 4096)])
+@pytest.mark.parametrize("sched", [None, OverlapTileScheduler()])
+def test_long_blocks_get_more_ctas(edges, sched):
+    a, w, y = torch.zeros(16, 1, 4096, dtype=BF), torch.zeros(1024, 4096, dtype=BF), torch.zeros(16, 1, 1024, dtype=BF)
+    ops = MatvecSm100Op.schedule(a=a[..., :edges[1]], weight=w[:, :edges[1]], y=y)
+    ops += MatvecResidualSm100Op.schedule(a=a[..., edges[1]:], weight=w[:, edges[1]:], residual_in=y, residual_out=y)
+    for ctas in (1, 2, 16):
+        mk = Megakernel(ops, config=MegakernelConfig(num_sms=ctas), scheduler=sched)
+        where = [set(int(c) for c in mk.program.placement[j]) for j in (0, 1)]
+        if ctas == 1 or (ctas == 2 and edges[1] == 64):
+            assert where[0] == where[1] == set(range(ctas))                          # no CTA left for the shorter one
+        else:
+            assert not where[0] & where[1] and len(where[0] | where[1]) == ctas
+            assert abs(len(where[0]) - ctas * (edges[1] + 1280) / (4096 + 2 * 1280)) <= 1
+        final = simulate(mk.program)
+        assert (final == mk.program.counter_expected[:len(final)]).all()
