@@ -472,6 +472,17 @@ static int validate_program(const mk_program_t* p, int smem_optin, int num_sms, 
       else if (op.opcode == MK_OP_ATTN_SPLIT) pages = attn_pages(op, in.unit, p->page_bytes);
       if (in.n_pages != pages) return fail(-3, "instr %d: expected %d pages, got %d", j, pages, in.n_pages);
     }
+    // A fused combine keeps its weights in the split-K slots, so an event, behind which all units before it are complete,
+    // has to stand between it and matvec units of several participants.
+    bool slots = false, combine = false;
+    for (int j = ib, e = eb; j < ie; ++j) {
+      for (; e < ee && p->events[e].pos <= j - ib; ++e) slots = combine = false;
+      const mk_op_t& op = p->ops[p->instrs[j].op];
+      slots |= op.opcode == MK_OP_MATVEC && op.i[MK_MV_SPLIT] != 1 && p->instrs[j].n_pages > 1;
+      combine |= op.opcode == MK_OP_ATTN_SPLIT && op.i[MK_AT_FUSE_COMBINE];
+      if (slots && combine)
+        return fail(-3, "instr %d: no event between a fused combine and a matvec unit of several pages on CTA %d", j, cta);
+    }
     int last = -1;
     for (int e = eb; e < ee; ++e) {
       const mk_event_t& ev = p->events[e];

@@ -108,7 +108,7 @@ __device__ __forceinline__ void at_combine_group(Ctx& c, const mk_op_t* op, cons
   const float* lpart = reinterpret_cast<const float*>(op->p[MK_AT_P_LSEPART]);
   float* lse_out = reinterpret_cast<float*>(op->p[MK_AT_P_LSE]);
   const int ot = op->i[MK_AT_O_T];
-  // this warp's 2 KB of the split-K slot area (no matvec unit runs beside an attention op's units)
+  // this warp's 2 KB of the split-K slot area (no matvec unit of several participants runs beside: see validate_program)
   float* scratch = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(c.ctrl) + kCtrlStructBytes) + (c.warp - 1) * 512;
   const int rows = min(16, M * G - u.mt * 16);
   const int row = c.lane / LPR, dch = (c.lane % LPR) * 8;

@@ -400,7 +400,8 @@ class InstructionStreamBuilder:
             per_cta = np.bincount(np.asarray(where[:op.n_units], dtype=np.int64), minlength=num_ctas)
             bulk = op.n_groups == 1
             if op.opcode == N.OP_ATTN_SPLIT:
-                # attention units may leave their partial states in the staging buffer
+                # Attention units may leave their partial states in the staging buffer, and a fused combine keeps its
+                # weights in the split-K slots: the next matvec has an event, a barrier behind them, in any case.
                 for c in set(int(c) for c in where[:op.n_units]):
                     cta_staged[c] = 0
             for u in range(op.n_units):

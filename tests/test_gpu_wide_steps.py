@@ -89,34 +89,63 @@ def test_every_place_of_the_states_gives_the_same_bits(batch):
     assert not any(t.isnan().any() for t in got[0])
 
 
-def test_rows_staged_before_attention_keep_the_buffer():
-    """A projection behind attention that finds its rows staged and has no event: the states must not go there."""
+def two_projections_of_one_input(fuse):
+    """Projection of x, attention, another projection of x: the program, its op records without the second one's events."""
     ops, outs, keep = step(2, 500)
     g = torch.Generator().manual_seed(2)
     x = torch.randn(2, 1, 10240, generator=g).to(BF).cuda()
     ys = [torch.full((2, 1, 512), float("nan"), dtype=BF, device="cuda") for _ in range(2)]
     ws = [packed(512, 10240, g) for _ in range(2)]
-    # x's first projection, Q projection without its staging (another CTA's), attention, x's second projection
-    mk = Megakernel(project(x, ws[0], ys[0]) + ops[1:-1] + project(x, ws[1], ys[1]), config=MegakernelConfig(num_sms=8, num_pages=4))
-    for t in keep[0], outs[0]:
-        t.normal_()
+    outs[0].copy_(torch.randn(2, 1, 512, generator=g))
+    mk = Megakernel(project(x, ws[0], ys[0]) + ops[1:-1] + project(x, ws[1], ys[1]),
+                    config=MegakernelConfig(num_sms=8, num_pages=4, fuse=fuse))
+    want = [x[:, 0].float() @ dequantize_nvfp4_weight(w).float().t() for w in ws]
+    return mk, ys, want, (outs, keep, x, ws)
+
+
+def drop_events_of_the_last_op(mk):
     prog, last = mk.program, len(mk.native_ops) - 1
     assert prog.ops["act_key"][0] == prog.ops["act_key"][last] != 0
     drop = prog.events["op"] == last
-    assert drop.any() and not prog.events["n_waits"][drop].any()
+    assert drop.any()
+    prog.events["n_waits"][drop] = 0
     kept = np.concatenate([[0], np.cumsum(~drop)])
     prog.cta_event_begin[:] = kept[prog.cta_event_begin]
     prog.events = prog.events[~drop].copy()
+
+
+def test_projections_of_one_input_around_attention():
+    """The second projection must not start beside the attention units: their combine uses the slots of its partial sums."""
+    mk, ys, want, keep = two_projections_of_one_input(fuse=True)
+    first = None
+    for _ in range(100):
+        for y in ys:
+            y.fill_(float("nan"))
+        mk.run()
+        first = first or [y.clone() for y in ys]
+        assert all(torch.equal(a, b) for a, b in zip(first, ys))
+    for y, ref in zip(ys, want):
+        assert_parity(y[:, 0], ref, "projection")
+    # tables that would let them run side by side are refused
+    mk, ys, want, keep = two_projections_of_one_input(fuse=True)
+    drop_events_of_the_last_op(mk)
+    with pytest.raises(ValueError, match="no event between a fused combine"):
+        mk.compile()
+
+
+def test_rows_staged_before_attention_keep_the_buffer():
+    """Hand-made tables in which the second projection relies on the rows that the first one staged (and no combine is fused):
+    the states must not go there."""
+    mk, ys, want, keep = two_projections_of_one_input(fuse=False)
+    drop_events_of_the_last_op(mk)
     mk.compile()
     assert placement(mk) == [0, 4, 0]
-    mk.run()
-    for y, w in zip(ys, ws):
-        assert_parity(y[:, 0], x[:, 0].float() @ dequantize_nvfp4_weight(w).float().t(), "staged once")
-    assert not outs[1].isnan().any()
-    again, want, keep2 = step(2, 500)
-    want[0].copy_(outs[0])
-    Megakernel(again[1:-1], config=MegakernelConfig(num_sms=8, num_pages=4)).run()
-    assert_parity(outs[1], want[1], "attention")
+    for _ in range(20):
+        for y in ys:
+            y.fill_(float("nan"))
+        mk.run()
+        for y, ref in zip(ys, want):
+            assert_parity(y[:, 0], ref, "projection")
 
 
 @pytest.mark.parametrize("units", [(31, 1, 32), (32, 33, 1), (1, 30, 1, 32, 64, 5), (63, 1, 64, 2, 31), (16, 16, 17, 15, 33)])
