@@ -5,7 +5,7 @@ Headline workload (``config.workload``): the full 16-layer Llama-3.2-1B-shape
 decode step as one persistent kernel — hidden 2048, 32 query / 8 KV heads,
 head_dim 64, GLU intermediate 8192, tied 128256-vocab LM head with the greedy
 token computed in the kernel, random-init bf16 weights ~N(0, 0.02), decode
-batch 1, KV length 4096.  A "step" is one launch = one token per sequence.
+batch 1, KV length 4096.  A "step" is one run of the program = one token per sequence.
 
 One JSON line is printed by rank 0:
 
@@ -867,10 +867,11 @@ def main():
             "data": "synthetic", "config": workload_config(args, world, tp, w.tp_note),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "peak_kind": f"of {peak_kind}", "frac_of_nominal_8TBps": achieved / NOMINAL_HBM_GBS,
-                         "algorithmic_bytes_per_step": w.alg_bytes, "kernel": "mk_persistent_kernel",
+                         "algorithmic_bytes_per_step": w.alg_bytes,
+                         "kernel": "mk_persistent_kernel" if w.mk.launches_per_run == 1 else "mv_chain_kernel, at_chain_kernel",
                          "traffic": int(w.alg_bytes * NCU_TRAFFIC_RATIO),
                          "traffic_from": "ncu dram bytes of a 4-layer capture x layers (profiles/), not this run"},
-            "clocks": clocks, "e2e": e2e, "gpu_launches": args.steps * blocks,
+            "clocks": clocks, "e2e": e2e, "gpu_launches": args.steps * blocks * w.mk.launches_per_run,
             "kernel_config": {"ctas": mk.grid[0], "threads": mk.block[0], "smem": mk.smem_size, "pages": mk.num_pages,
                               "page_bytes": mk.page_bytes, "instructions": mk.total_tiles,
                               "counters": mk.num_barriers, "scheduler": args.scheduler},

@@ -294,6 +294,11 @@ typedef struct mk_wait {
   int32_t expected;       /* wait until counter >= expected                  */
 } mk_wait_t;
 
+/* mk_program_t.flags
+ * SINGLE_LAUNCH: mk_run is one launch, of the persistent kernel, for every program.  Without it a program whose ops all
+ *   have kernels of their own runs as a chain of launches (with the same results), unless a trace is attached. */
+enum { MK_PROG_SINGLE_LAUNCH = 1 };
+
 /* Host-side program description handed to mk_create (all arrays in HOST
  * memory; mk_create copies them into the device workspace). */
 typedef struct mk_program {
@@ -352,11 +357,14 @@ uint64_t mk_workspace_bytes(const mk_program_t* prog);
  * Replaces Megakernel.compile()'s metadata upload
  * (megakernel/megakernel.py:709-962); there is no JIT. */
 int mk_create(const mk_program_t* prog, mk_handle_t* out);
-/* Launch the persistent kernel on `cuda_stream` (a cudaStream_t; NULL = the
- * legacy default stream).  Asynchronous.  Counters are reset by the kernel
- * itself, so back-to-back launches and CUDA-graph replay are legal.
+/* Run the program on `cuda_stream` (a cudaStream_t; NULL = the legacy default
+ * stream): as a chain of kernels, or (see MK_PROG_SINGLE_LAUNCH) as one launch of
+ * the persistent kernel.  Asynchronous.  Counters are reset by the kernels
+ * themselves, so back-to-back runs and CUDA-graph replay are legal.
  * Replaces Megakernel.run() / launch_prepared (megakernel.py:2163-2204). */
 int mk_run(mk_handle_t h, void* cuda_stream);
+/* Kernel launches that one mk_run of this handle makes (0 for a null handle). */
+int mk_launches_per_run(mk_handle_t h);
 /* Copy the 16-word device status block to `out` (synchronises the device).
  * out[0] == 0 means no device-side error. */
 int mk_status(mk_handle_t h, int32_t out[16]);

@@ -57,6 +57,7 @@ AR_S_INBOX, AR_S_FLAGS = 0, 1
 AR_MAX_RANKS = 8
 EWF_RESIDUAL, EWF_GEMMA, EWF_FUSED_ADD, EWF_GATED, EWF_ROW_WEIGHT, EWF_FEEDBACK = 1, 2, 4, 8, 16, 32
 EVF_WRITE_RES_OUT, EVF_BULK_SIGNAL = 1, 2
+PROG_SINGLE_LAUNCH = 1
 
 # Device status codes (csrc/shell.cuh).
 STATUS_NAMES = {
@@ -112,7 +113,7 @@ class Program(C.Structure):
 
 
 EXPORTS = [
-    "mk_abi_version", "mk_last_error", "mk_device_info", "mk_workspace_bytes", "mk_create", "mk_run",
+    "mk_abi_version", "mk_last_error", "mk_device_info", "mk_workspace_bytes", "mk_create", "mk_run", "mk_launches_per_run",
     "mk_status", "mk_workspace_status", "mk_set_trace", "mk_reset", "mk_launch_count", "mk_state_placement", "mk_set_launch_count",
     "mk_update_op", "mk_read_counters", "mk_destroy",
     "mk_standalone_workspace_bytes", "mk_matvec_bf16", "mk_matvec_nvfp4", "mk_flash_decode",
@@ -172,6 +173,7 @@ def _declare(h: C.CDLL) -> None:
     h.mk_workspace_bytes.restype = u64
     h.mk_create.argtypes = [C.POINTER(Program), C.POINTER(vp)]
     h.mk_run.argtypes = [vp, vp]
+    h.mk_launches_per_run.argtypes = [vp]
     h.mk_status.argtypes = [vp, C.POINTER(i32)]
     h.mk_workspace_status.argtypes = [vp, C.POINTER(i32)]
     h.mk_set_trace.argtypes = [vp, vp, u64, i32]

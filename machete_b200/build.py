@@ -30,8 +30,8 @@ NVCC_FLAGS = [
 
 
 def _sources() -> list[Path]:
-    """The host side plus one translation unit per group of kernel variants."""
-    return [CSRC / "megakernel.cu", CSRC / "gemm_sm100.cu", CSRC / "attn_prefill_sm100.cu"] + sorted(CSRC.glob("variants_*.cu"))
+    """The host side plus one translation unit per group of kernels."""
+    return [CSRC / "megakernel.cu", CSRC / "gemm_sm100.cu", CSRC / "attn_prefill_sm100.cu"] + sorted(CSRC.glob("variants_*.cu")) + sorted(CSRC.glob("chain_*.cu"))
 
 
 def _deps() -> list[Path]:

@@ -22,9 +22,12 @@
 #include <string.h>
 
 #include <algorithm>
+#include <memory>
 #include <string>
 #include <vector>
 
+#include "chain_attn.cuh"
+#include "chain_ew.cuh"
 #include "kernel.cuh"
 
 namespace mk {
@@ -497,6 +500,8 @@ static int validate_program(const mk_program_t* p, int smem_optin, int num_sms, 
 
 }  // namespace mk
 
+#include "chain.inc"
+
 // The kernel variants are compiled in groups, one translation unit per group
 // (variants_*.cu), so that they build in parallel; each group hands out its
 // table.  Variants differ in <activation-tile class, weight family, features>.
@@ -541,6 +546,10 @@ struct mk_handle_s {
   int n_ops;
   uint8_t* ws;
   mk::Layout layout;
+  int num_sms;
+  bool single_launch;                // MK_PROG_SINGLE_LAUNCH
+  mk::ChainTables tables;
+  std::vector<mk::ChainStep> chain;  // the program as a chain of kernels; empty: the persistent kernel runs it
 };
 
 static void classify_op(const mk_op_t& op, int* ntc, int* wfc, int* feat) {
@@ -651,6 +660,11 @@ static int select_kernel(mk_handle_s* h) {
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, h->smem_optin);
   if (e != cudaSuccess) return mk::fail(-(int)e - 1000, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
   return 0;
+}
+
+static int plan_chain(mk_handle_s* h) {
+  if (h->single_launch) return 0;
+  return mk::build_chain(h->ops, h->tables, h->pv, h->ws + h->layout.tmaps, h->num_sms, h->smem_optin, &h->chain);
 }
 
 // Restores the caller's current device when an entry point returns.
@@ -788,10 +802,15 @@ static int create_program(const mk_program_t* prog, mk_handle_t* out, bool strea
   h->states_may_stage = states_may_stage(prog);
   rc = select_kernel(h);
   if (rc) return rc;
+  h->num_sms = num_sms;
+  h->single_launch = (prog->flags & MK_PROG_SINGLE_LAUNCH) != 0;
+  if (!h->single_launch) h->tables = read_chain_tables(prog);
   h->device = prog->device;
   h->n_ops = prog->n_ops;
   h->ws = ws;
   h->layout = l;
+  rc = plan_chain(h);
+  if (rc) return rc;
   guard.h = nullptr;
   *out = h;
   return 0;
@@ -802,6 +821,7 @@ int mk_create(const mk_program_t* prog, mk_handle_t* out) { return create_progra
 int mk_run(mk_handle_t h, void* cuda_stream) {
   using namespace mk;
   if (!h) return fail(-1, "null handle");
+  if (!h->chain.empty() && h->pv.trace == nullptr) return run_chain(h->chain, reinterpret_cast<cudaStream_t>(cuda_stream));
   // The launch may be placed while the kernel before it in the stream drains: its CTAs set up their shared
   // memory and wait (prior_work_done) before they touch global memory.
   cudaLaunchConfig_t cfg = {};
@@ -816,6 +836,11 @@ int mk_run(mk_handle_t h, void* cuda_stream) {
   cfg.numAttrs = 1;
   CUDA_TRY(cudaLaunchKernelEx(&cfg, h->kernel, h->pv));
   return 0;
+}
+
+int mk_launches_per_run(mk_handle_t h) {
+  if (!h) return 0;
+  return h->chain.empty() || h->pv.trace != nullptr ? 1 : (int)h->chain.size();
 }
 
 int mk_status(mk_handle_t h, int32_t out[16]) {
@@ -929,7 +954,8 @@ int mk_update_op(mk_handle_t h, int32_t op_index, const mk_op_t* op, void* cuda_
   h->ops[op_index] = rec;
   // a changed batch size or weight format may need another kernel variant
   classify_op(rec, &h->op_ntc[op_index], &h->op_wfc[op_index], &h->op_feat[op_index]);
-  return select_kernel(h);
+  rc = select_kernel(h);
+  return rc ? rc : plan_chain(h);
 }
 
 int mk_read_counters(mk_handle_t h, int32_t* out, int32_t n) {

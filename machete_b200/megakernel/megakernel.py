@@ -6,9 +6,12 @@ Host runtime behind the reference's public entry point
 ``bench_spec`` :2206, ``create_megakernel`` :2293).  The constructor lowers
 every ``ScheduledOp`` through its op class, infers dependencies and builds the
 tables; ``compile()`` uploads them through the C ABI (``mk_create``);
-``run()`` is one kernel launch (``mk_run``) with no per-launch host work: the
-kernel resets its own counters, so launches can be queued back to back or
-captured in a CUDA graph.
+``run()`` is one call of ``mk_run``: a chain of kernels, one for each op or
+group of ops that need nothing from one another, or one launch of the
+persistent kernel (programs with an all-reduce, a trace attached, or
+``single_launch``).  There is no other per-run host work: the kernels reset
+their own counters, so runs can be queued back to back or captured in a CUDA
+graph.
 """
 
 from __future__ import annotations
@@ -70,6 +73,7 @@ class MegakernelConfig:
     native_kc_fp4: Optional[int] = None  # K columns per NVFP4 weight page (default 2048)
     timeout_ms: int = 1000               # bound of every device-side wait
     fuse: bool = True                    # allow peephole fusion of op chains
+    single_launch: bool = False          # run() is one launch for every program, never a chain of kernels
     # Device-resident cache position: a one-element int32 CUDA tensor that ops scheduled with a
     # dynamic position read at the start of every launch and that the token-feedback form of the
     # top-1 head advances at the end (consecutive launches decode consecutive tokens).
@@ -240,6 +244,7 @@ class Megakernel:
         prog.act_bytes = self._act_bytes
         prog.timeout_ms = int(self.config.timeout_ms)
         prog.device = dev
+        prog.flags = N.PROG_SINGLE_LAUNCH if self.config.single_launch else 0
         prog.ops = arrays["ops"].ctypes.data
         prog.instrs = arrays["instrs"].ctypes.data
         prog.cta_instr_begin = arrays["ib"].ctypes.data
@@ -321,6 +326,12 @@ class Megakernel:
         N.check(N.lib().mk_run(state["handle"], C.c_void_p(int(handle))), "mk_run")
         if sync:
             self.wait()
+
+    @property
+    def launches_per_run(self) -> int:
+        """Kernel launches that one :meth:`run` makes."""
+        self.compile()
+        return int(N.lib().mk_launches_per_run(self._handle))
 
     def launch_count(self) -> int:
         """Launches this handle has completed (aborted ones included); see ``mk_launch_count``."""

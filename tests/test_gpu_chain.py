@@ -1,0 +1,176 @@
+"""A program as a chain of kernels against the same program as one launch: the same sums in the same order, so the same bits."""
+
+import pytest
+import torch
+
+from machete_b200.kernels.attention import flash_decoding_schedule
+from machete_b200.kernels.decode_matvec import (MatvecNvfp4Sm120Op, MatvecResidualNvfp4Sm120Op, MatvecResidualSm100Op,
+                                                MatvecSm100Op, RmsGateUpSiluNvfp4Sm120Op, RmsGateUpSiluSm100Op,
+                                                schedule_decode_layer_sm100)
+from machete_b200.kernels.decode_matvec.nvfp4_model import schedule_decode_layer_nvfp4_sm100
+from machete_b200.megakernel import Megakernel, MegakernelConfig, OverlapTileScheduler
+from machete_b200.quantization import quantize_nvfp4_weight
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+
+
+class Values:
+    def __init__(self, seed):
+        self.g = torch.Generator(device="cuda").manual_seed(seed)
+
+    def __call__(self, *shape, std=1.0, dtype=BF):
+        return (torch.randn(*shape, generator=self.g, device="cuda") * std).to(dtype)
+
+    def weight(self, fmt, o, k):
+        w = self(o, k, std=0.02, dtype=torch.float16 if fmt == "fp16" else BF)
+        return w if fmt in ("bf16", "fp16") else quantize_nvfp4_weight(w, group_size=16 if fmt == "nvfp4" else 32)
+
+
+def equal_forms(ops, outs, **config):
+    """Both forms, three launches each (the arrival counts and slots they leave behind included), from the same buffers."""
+    start, got = [t.clone() for t in outs], []
+    for single in (True, False):
+        for t, s in zip(outs, start):
+            t.copy_(s)
+        mk = Megakernel(ops, config=MegakernelConfig(single_launch=single, **config), scheduler=OverlapTileScheduler()).compile()
+        for _ in range(3):
+            mk.run()
+        assert mk.launch_count() == 3 and not mk.read_counters().any()
+        got.append([t.clone() for t in outs])
+    for a, b in zip(*got):
+        assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+    return got[1]
+
+
+# rows at the edges of the kernels' row classes; outputs at those of a unit's 16 rows; K of one tile, of a ragged last page, of
+# odd numbers of tiles, of as many pages as participants and of more
+@pytest.mark.parametrize("fmt,rows,k,out", [
+    ("bf16", 1, 64, 1), ("bf16", 1, 1088, 16), ("bf16", 1, 14336, 40), ("bf16", 2, 832, 4096), ("bf16", 8, 6144, 100),
+    ("bf16", 9, 2880, 33), ("bf16", 16, 1024, 1024), ("bf16", 17, 1600, 15), ("bf16", 32, 1536, 5000),
+    ("fp16", 1, 2048, 64), ("fp16", 5, 960, 200), ("fp16", 16, 1152, 17), ("fp16", 32, 512, 48),
+    ("nvfp4", 1, 256, 1), ("nvfp4", 1, 14336, 1000), ("nvfp4", 4, 4096, 14336), ("nvfp4", 8, 1792, 24),
+    ("nvfp4", 9, 2048, 520), ("nvfp4", 16, 768, 31), ("nvfp4", 25, 1280, 4096),
+    ("nvfp4-g32", 1, 4096, 6144), ("nvfp4-g32", 3, 512, 16), ("nvfp4-g32", 12, 1024, 100), ("nvfp4-g32", 32, 256, 8)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_products(fmt, rows, k, out, residual):
+    v = Values(rows * k + out)
+    dtype = torch.float16 if fmt == "fp16" else BF
+    # sequences of several tokens where the rows divide so, with strides of their own
+    b, s = (rows // 2, 2) if rows % 2 == 0 else (rows, 1)
+    x, y = v(b, s, k + 8, dtype=dtype)[..., :k], torch.zeros(b, s + 1, out + 8, dtype=dtype, device="cuda")[:, 1:, :out]
+    r, w = v(b, s, out, dtype=dtype), v.weight(fmt, out, k)
+    if fmt.startswith("nvfp4"):
+        kw = dict(a=x, weight_packed=w.packed, weight_scales=w.scales, group_size=w.group_size, global_scale=w.global_scale)
+        ops = MatvecResidualNvfp4Sm120Op.schedule(residual_in=r, residual_out=y, **kw) if residual else \
+            MatvecNvfp4Sm120Op.schedule(y=y, **kw)
+    else:
+        ops = MatvecResidualSm100Op.schedule(a=x, weight=w, residual_in=r, residual_out=y) if residual else \
+            MatvecSm100Op.schedule(a=x, weight=w, y=y)
+    assert equal_forms(ops, [y])[0].float().abs().sum() > 0
+
+
+@pytest.mark.parametrize("fmt,rows,k,inter", [("bf16", 1, 2048, 8), ("bf16", 8, 4096, 104), ("bf16", 16, 1024, 2048), ("bf16", 32, 832, 24),
+                                              ("nvfp4", 1, 4096, 12288), ("nvfp4", 7, 6144, 16), ("nvfp4-g32", 16, 2048, 1000),
+                                              ("nvfp4", 32, 768, 2048)])
+def test_normalised_rows_and_pairs(fmt, rows, k, inter):
+    v = Values(rows + k)
+    x, y, n = v(rows, 1, k), torch.zeros(rows, 1, inter, dtype=BF, device="cuda"), 1 + v(k, std=0.02)
+    g, u = v.weight(fmt, inter, k), v.weight(fmt, inter, k)
+    if fmt == "bf16":
+        ops = RmsGateUpSiluSm100Op.schedule(x=x, norm_weight=n, gate_weight=g, up_weight=u, y=y)
+    else:
+        ops = RmsGateUpSiluNvfp4Sm120Op.schedule(x=x, norm_weight=n, gate_packed=g.packed, gate_scales=g.scales, up_packed=u.packed,
+                                                 up_scales=u.scales, group_size=g.group_size, global_scale=g.global_scale,
+                                                 up_global_scale=u.global_scale, y=y)
+    assert equal_forms(ops, [y])[0].float().abs().sum() > 0
+
+
+@pytest.mark.parametrize("batch,kv,heads,kv_heads,dim,splits,causal,m", [
+    (1, 1, 8, 8, 64, 0, False, 1), (1, 300, 32, 8, 64, 0, False, 1), (2, 65, 16, 1, 128, 3, False, 1), (3, 1930, 32, 4, 128, 0, False, 1),
+    (1, 2000, 8, 2, 64, 128, False, 1), (1, 700, 8, 4, 128, 40, True, 16), (2, 130, 4, 4, 64, 64, True, 5), (8, 4096, 32, 8, 128, 0, False, 1)])
+@pytest.mark.parametrize("fuse", [True, False])
+def test_attention(batch, kv, heads, kv_heads, dim, splits, causal, m, fuse):
+    v = Values(kv + dim)
+    q, o = v(batch, m, heads, dim), torch.zeros(batch, m, heads, dim, dtype=BF, device="cuda")
+    k, vv = v(batch, kv + 3, kv_heads, dim)[:, :kv], v(batch, kv, kv_heads, dim)
+    ops, _ = flash_decoding_schedule(q, k, vv, o, num_splits=splits, causal=causal, kv_group_size=heads // kv_heads)
+    lse = ops[1].tensor_refs["lse"]
+    assert equal_forms(ops, [o, lse], fuse=fuse)[0].float().abs().sum() > 0
+
+
+def layer_weights(v, fmt, hidden, inter, heads, kv_heads, dim, kv):
+    w = {"cos": v(kv, dim // 2), "sin": v(kv, dim // 2), "layer.0.attn_norm": 1 + v(hidden, std=0.02), "layer.0.mlp_norm": 1 + v(hidden, std=0.02)}
+    if fmt != "bf16":
+        w["layer.0.q_norm"], w["layer.0.k_norm"] = 1 + v(dim, std=0.02), 1 + v(dim, std=0.02)
+    for name, o, i in (("q", heads * dim, hidden), ("k", kv_heads * dim, hidden), ("v", kv_heads * dim, hidden), ("o", hidden, heads * dim),
+                       ("gate", inter, hidden), ("up", inter, hidden), ("down", hidden, inter)):
+        p = v.weight(fmt, o, i)
+        if fmt == "bf16":
+            w[f"layer.0.W_{name}"] = p
+        else:
+            w[f"layer.0.W_{name}.packed"], w[f"layer.0.W_{name}.scales"], w[f"layer.0.W_{name}.global_scale"] = p.packed, p.scales, float(p.global_scale)
+    return w
+
+
+# a whole layer: rows appended to the cache in the launch before the attention that reads them, whose other pages are
+# fetched before that launch has finished; 16 rows: the down projection's K blocks side by side
+@pytest.mark.parametrize("fmt,batch,seq,kv,pos", [("bf16", 1, 1, 700, 699), ("bf16", 3, 1, 130, 64), ("bf16", 2, 3, 70, 61), ("bf16", 16, 1, 300, 250),
+                                                  ("nvfp4", 1, 1, 1000, 999), ("nvfp4", 8, 1, 66, 32), ("nvfp4", 2, 1, 40, 0)])
+@pytest.mark.parametrize("moving", [False, True])
+def test_layer(fmt, batch, seq, kv, pos, moving):
+    if moving and seq > 1:
+        pytest.skip("a moving position takes one token a sequence")
+    hidden, inter, heads, kv_heads, dim = (2048, 8192, 16, 4, 64) if fmt == "bf16" else (2048, 6144, 8, 2, 128)
+    v = Values(batch + kv)
+    w = layer_weights(v, fmt, hidden, inter, heads, kv_heads, dim, kv)
+    z = lambda n: torch.zeros(batch, seq, n, dtype=BF, device="cuda")      # noqa: E731
+    kc, vc = v(batch, kv, kv_heads, dim), v(batch, kv, kv_heads, dim)
+    x, r, xo, ro, q, at, h = v(batch, seq, hidden), v(batch, seq, hidden), z(hidden), z(hidden), z(heads * dim), z(heads * dim), z(inter)
+    kw = dict(layer_idx=0, batch=batch, seq_len=seq, weights=w, k_cache=kc, v_cache=vc, x_in=x, residual_in=r, x_out=xo, residual_out=ro,
+              q_buf=q, attn_out_buf=at, mlp_h_buf=h, eps=1e-5, num_q_heads=heads, num_kv_heads=kv_heads, head_dim=dim)
+    config = {}
+    if moving:
+        config["position"] = torch.tensor([pos], dtype=torch.int32, device="cuda")
+        kw.update(cache_pos=0, dynamic_position=True)
+    else:
+        kw["cache_pos"] = pos
+    if fmt == "bf16":
+        ops = schedule_decode_layer_sm100(hidden_size=hidden, intermediate_size=inter, **kw).ops
+    else:
+        ops = schedule_decode_layer_nvfp4_sm100(**kw).ops
+    assert equal_forms(ops, [xo, ro, q, at, h, kc, vc], **config)[0].float().abs().sum() > 0
+
+
+def test_a_position_outside_the_cache_runs_nothing():
+    v = Values(5)
+    w = layer_weights(v, "bf16", 512, 1024, 8, 2, 64, 64)
+    z = lambda n: torch.zeros(1, 1, n, dtype=BF, device="cuda")      # noqa: E731
+    kc, vc, pos = v(1, 64, 2, 64), v(1, 64, 2, 64), torch.tensor([64], dtype=torch.int32, device="cuda")
+    before, xo = kc.clone(), z(512)
+    ops = schedule_decode_layer_sm100(layer_idx=0, batch=1, seq_len=1, cache_pos=0, dynamic_position=True, weights=w, k_cache=kc, v_cache=vc,
+                                      x_in=v(1, 1, 512), residual_in=z(512), x_out=xo, residual_out=z(512), q_buf=z(512),
+                                      attn_out_buf=z(512), mlp_h_buf=z(1024), eps=1e-5, hidden_size=512, intermediate_size=1024,
+                                      num_q_heads=8, num_kv_heads=2, head_dim=64).ops
+    mk = Megakernel(ops, config=MegakernelConfig(position=pos)).compile()
+    with pytest.raises(RuntimeError, match="position"):
+        mk.run()
+    assert torch.equal(kc, before) and not xo.any()
+    pos.fill_(3)
+    mk.run()
+    assert xo.any()
+
+
+def test_replaced_records_change_the_chain():
+    v = Values(9)
+    x, w, w2 = v(3, 1, 1024), v(64, 1024, std=0.02), v(64, 1024, std=0.02)
+    y = torch.zeros(3, 1, 64, dtype=BF, device="cuda")
+    mk = Megakernel(MatvecSm100Op.schedule(a=x, weight=w, y=y)).compile()
+    other = Megakernel(MatvecSm100Op.schedule(a=x, weight=w2, y=y)).compile()
+    other.run()
+    want = y.clone()
+    mk.run()
+    assert not torch.equal(y, want)
+    mk.update_op(0, other.native_ops[0])
+    mk.run()
+    assert torch.equal(y, want)
