@@ -124,7 +124,6 @@ __global__ void __launch_bounds__(kAtChainThreads, 2) at_chain_kernel(const __gr
   __syncthreads();
   const bool early = (L.flags & kChainEarlyLoads) != 0;
   if (!early) prior_work_done();
-  next_may_start();
   const mk_op_t* op = &c.ctrl->op_cache[0];
 
   AtUnit u = at_decode(op, (int)blockIdx.x);
@@ -244,6 +243,7 @@ __global__ void __launch_bounds__(kAtChainThreads, 2) at_chain_kernel(const __gr
       }
     }
     named_bar_sync(kConsumerBarrier, kConsumerWarps * 32);
+    next_may_start();     // (not before: the next launch's weights would stand in the way of the query rows)
   }
 
   // ---- this participant's pages
@@ -383,31 +383,39 @@ __global__ void __launch_bounds__(kAtChainThreads, 2) at_chain_kernel(const __gr
   for (int i = 0; i < MT; ++i) om[i][0] = om[i][1] = om[i][2] = om[i][3] = 0.f;
   mrow[0] = mrow[1] = -INFINITY;
   lrow[0] = lrow[1] = 0.f;
-#pragma unroll 2
-  for (int j = 0; j < parts; ++j) {
-    const uint32_t src = c.pages_u32 + (uint32_t)j * kStateBytes + (uint32_t)c.lane * 16u;
-    const uint4 ml = lds128_sync(src + (uint32_t)ND * 512u);
-    uint4 v[MT];
+  {
+    // everything that is read is requested first; the running maximum and the weights do not depend on the values
+    uint4 ml[kConsumerWarps], v[kConsumerWarps][MT];
 #pragma unroll
-    for (int i = 0; i < MT; ++i) v[i] = lds128_sync(src + (uint32_t)(c.warp + 8 * i) * 512u);
-    const float mj[2] = {__uint_as_float(ml.x), __uint_as_float(ml.y)};
-    const float lj[2] = {__uint_as_float(ml.z), __uint_as_float(ml.w)};
-    float wa[2], wb[2];
+    for (int j = 0; j < kConsumerWarps; ++j) {
+      if (j >= parts) break;
+      const uint32_t src = c.pages_u32 + (uint32_t)j * kStateBytes + (uint32_t)c.lane * 16u;
+      ml[j] = lds128_sync(src + (uint32_t)ND * 512u);
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const float mnew = fmaxf(mrow[e], mj[e]);
-      const float muse = (mnew == -INFINITY) ? 0.f : mnew;
-      wa[e] = fast_exp2((mrow[e] - muse) * c2);
-      wb[e] = fast_exp2((mj[e] - muse) * c2);
-      mrow[e] = mnew;
-      lrow[e] = lrow[e] * wa[e] + lj[e] * wb[e];
+      for (int i = 0; i < MT; ++i) v[j][i] = lds128_sync(src + (uint32_t)(c.warp + 8 * i) * 512u);
     }
 #pragma unroll
-    for (int i = 0; i < MT; ++i) {
-      om[i][0] = om[i][0] * wa[0] + __uint_as_float(v[i].x) * wb[0];
-      om[i][1] = om[i][1] * wa[0] + __uint_as_float(v[i].y) * wb[0];
-      om[i][2] = om[i][2] * wa[1] + __uint_as_float(v[i].z) * wb[1];
-      om[i][3] = om[i][3] * wa[1] + __uint_as_float(v[i].w) * wb[1];
+    for (int j = 0; j < kConsumerWarps; ++j) {
+      if (j >= parts) break;
+      const float mj[2] = {__uint_as_float(ml[j].x), __uint_as_float(ml[j].y)};
+      const float lj[2] = {__uint_as_float(ml[j].z), __uint_as_float(ml[j].w)};
+      float wa[2], wb[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const float mnew = fmaxf(mrow[e], mj[e]);
+        const float muse = (mnew == -INFINITY) ? 0.f : mnew;
+        wa[e] = fast_exp2((mrow[e] - muse) * c2);
+        wb[e] = fast_exp2((mj[e] - muse) * c2);
+        mrow[e] = mnew;
+        lrow[e] = lrow[e] * wa[e] + lj[e] * wb[e];
+      }
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        om[i][0] = om[i][0] * wa[0] + __uint_as_float(v[j][i].x) * wb[0];
+        om[i][1] = om[i][1] * wa[0] + __uint_as_float(v[j][i].y) * wb[0];
+        om[i][2] = om[i][2] * wa[1] + __uint_as_float(v[j][i].z) * wb[1];
+        om[i][3] = om[i][3] * wa[1] + __uint_as_float(v[j][i].w) * wb[1];
+      }
     }
   }
   // normalised partial + lse
@@ -441,10 +449,29 @@ __global__ void __launch_bounds__(kAtChainThreads, 2) at_chain_kernel(const __gr
   }
   __syncthreads();
   if (!c.ctrl->is_last) return;
-  // As at_combine_group, with a pair of values a thread: splits are added in order.  Row r's weights: comb[r * S + s].
+  // As at_combine_group, with a pair of values a thread: splits are added in order.  Row r's weights: comb[r * S + s].  The
+  // first splits' values are requested before the weights are worked out.
+  constexpr int UN = 18;
   float* comb = reinterpret_cast<float*>(smem + L.comb_off);
   float* inv_of = reinterpret_cast<float*>(c.ctrl->red);
   const int rows = min(16, M * G - u.mt * 16);
+  auto pair_at = [&](int i, int64_t& off) -> const float* {   // the pair's partial values, and where its result goes
+    const int r0 = i / (D / 2), d = (i % (D / 2)) * 2;
+    const int r = u.mt * 16 + r0, m = M != 1 ? r / G : 0, h = u.kvh * G + (M != 1 ? r % G : r);
+    off = u.b * op->s[MK_AT_S_O_B] + m * op->s[MK_AT_S_O_M] + h * op->s[MK_AT_S_O_H] + d;
+    return op_ + ((((int64_t)u.b * H + h) * S) * M + m) * D + d;
+  };
+  const int64_t stride = (int64_t)M * D;
+  float2 v[UN];
+  auto fetch_pairs = [&](const float* base, int s0) {
+#pragma unroll
+    for (int k = 0; k < UN; ++k)
+      v[k] = s0 + k < S ? __ldcg(reinterpret_cast<const float2*>(base + (s0 + k) * stride)) : make_float2(0.f, 0.f);
+  };
+  int pair = threadIdx.x;
+  int64_t off = 0;
+  const float* base = pair < rows * (D / 2) ? pair_at(pair, off) : nullptr;
+  if (base) fetch_pairs(base, 0);
   for (int r0 = c.warp; r0 < rows; r0 += 8) {
     const int r = u.mt * 16 + r0, m = M != 1 ? r / G : 0, h = u.kvh * G + (M != 1 ? r % G : r);
     const float* ls = lp_ + ((int64_t)u.b * H + h) * S * M + m;
@@ -471,34 +498,30 @@ __global__ void __launch_bounds__(kAtChainThreads, 2) at_chain_kernel(const __gr
   }
   __syncthreads();
   const int ot = op->i[MK_AT_O_T];
-  for (int i = threadIdx.x; i < rows * (D / 2); i += kAtChainThreads) {
-    constexpr int UN = 9;
-    const int r0 = i / (D / 2), d = (i % (D / 2)) * 2;
-    const int r = u.mt * 16 + r0, m = M != 1 ? r / G : 0, h = u.kvh * G + (M != 1 ? r % G : r);
-    const float* base = op_ + ((((int64_t)u.b * H + h) * S) * M + m) * D + d;
-    const int64_t stride = (int64_t)M * D;
-    const float inv = inv_of[r0];
-    const float* w = comb + r0 * S;
+#pragma unroll 1
+  while (base) {
+    const float inv = inv_of[pair / (D / 2)];
+    const float* w = comb + pair / (D / 2) * S;
     float a0 = 0.f, a1 = 0.f;
 #pragma unroll 1
-    for (int s0 = 0; s0 < S; s0 += UN) {
-      float2 v[UN];
-#pragma unroll
-      for (int k = 0; k < UN; ++k)
-        v[k] = s0 + k < S ? __ldcg(reinterpret_cast<const float2*>(base + (s0 + k) * stride)) : make_float2(0.f, 0.f);
+    for (int s0 = 0;;) {
 #pragma unroll
       for (int k = 0; k < UN; ++k) {
-        if (s0 + k >= S) break;
-        const float ws = w[s0 + k] * inv;
+        const float ws = s0 + k < S ? w[s0 + k] * inv : 0.f;
         a0 += ws * v[k].x;
         a1 += ws * v[k].y;
       }
+      s0 += UN;
+      if (s0 >= S) break;
+      fetch_pairs(base, s0);
     }
-    const int64_t off = u.b * op->s[MK_AT_S_O_B] + m * op->s[MK_AT_S_O_M] + h * op->s[MK_AT_S_O_H] + d;
     if (ot == MK_T_FP32)
       *reinterpret_cast<float2*>(reinterpret_cast<float*>(op->p[MK_AT_P_O]) + off) = make_float2(a0, a1);
     else
       *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(op->p[MK_AT_P_O]) + off) = ot == MK_T_BF16 ? pack_bf16(a0, a1) : pack_f16(a0, a1);
+    pair += kAtChainThreads;
+    base = pair < rows * (D / 2) ? pair_at(pair, off) : nullptr;
+    if (base) fetch_pairs(base, 0);
   }
 }
 

@@ -31,6 +31,7 @@ enum { kChainEarlyLoads = 1,   // the weights may be read before the kernel befo
 struct ChainHead {             // what the loader needs to know of an op: it does not wait for the records
   int64_t out_h;                 // output stride of a head
   int32_t mode, hd, d2, tiles;   // row mapping, head dim, its half, K-tiles of a page
+  int32_t rows, flags;           // output rows; kEpi...
 };
 struct MvLaunch {
   ProgramView pv;                  // status block, time limit, cache position, op records (from first_op on)
@@ -39,6 +40,7 @@ struct MvLaunch {
   int32_t unit_end[kChainOps];     // units of ops 0..i
   int32_t cta_end[kChainOps];      // K blocks: CTAs of blocks 0..i; zero where the ops share the CTAs and what they stage
   int32_t pages[kChainOps], parts[kChainOps];   // pages of a unit, and the partial sums they meet in
+  int32_t spread;                               // the partial sums of a unit are dealt to different warps
   int32_t n_ops, flags, res_op, first_op;       // res_op: the op whose residual_out this launch writes, or -1
   int32_t stages, page_bytes, sets_log2;        // ring slots, and sets of slots for partial sums
   int32_t slot_off, act_off, page_off;          // shared memory, bytes
@@ -56,8 +58,11 @@ struct ChainIn {
 };
 struct ChainUnit {
   int32_t op, rowA0, rowB0, offA, offB, chunk;   // op of the launch, and MvOut
-  int32_t pad[2];
+  int32_t flags, valid;                          // kChainEpi...; valid rows of the two halves, nA | nB << 8
 };
+// What an op's epilogue does, in one word that comes with the unit.
+enum { kEpiNormed = 1, kEpiScaled = 2, kEpiPair = 4, kEpiRope = 8, kEpiSiluMul = 16, kEpiRelu = 32, kEpiSilu = 64, kEpiResidual = 128,
+       kEpiTop1 = 256, kEpiFp32 = 512, kEpiFp16 = 1024, kEpiKsum = 2048 };
 __device__ __forceinline__ int small_div(int n, int magic) { return (int)(((uint32_t)n * (uint32_t)magic) >> 20); }
 constexpr int kChainUnits = 32;   // units between the loader's and the last finisher's: at most 12 pages + 4 slot sets
 struct ChainTab {
@@ -518,7 +523,9 @@ __device__ __forceinline__ ChainUnit chain_unit(const MvLaunch& L, int op0, int 
     r.offA = (int)((int64_t)qa * op.out_h + (r.rowA0 - qa * op.hd));
     r.offB = (int)((int64_t)qb * op.out_h + (r.rowB0 - qb * op.hd));
   }
-  r.pad[0] = r.pad[1] = 0;
+  r.flags = op.flags;
+  const int na = op.mode == MK_MV_ROPE ? 8 : clamp8(op.rows - r.rowA0), nb = op.mode == MK_MV_ROPE ? 8 : clamp8(op.rows - r.rowB0);
+  r.valid = na | nb << 8;
   return r;
 }
 
@@ -536,22 +543,20 @@ __device__ __forceinline__ ChainRow chain_row(const mk_op_t* op, int b, int t, i
 // and hold no branch: one warp runs this for a unit, and for a launch of a unit or two a CTA it is the launch's end (a branch
 // a row and choice: some 350 cycles a row of every lane).
 template <int ROWS, int WF>
-__device__ __forceinline__ void chain_epilogue(Ctx& c, const mk_op_t* op, const ChainRow* rows, const MvOut& r,
+__device__ __forceinline__ void chain_epilogue(Ctx& c, const mk_op_t* op, const ChainRow* rows, const ChainUnit& r,
                                                const float (&sum)[chain_nt(ROWS)][4]) {
   constexpr int Q = ROWS == 1 ? 1 : 2 * chain_nt(ROWS);   // rows of a lane
   const int g = c.lane >> 2, t = c.lane & 3;
-  const int O = op->i[MK_MV_O], M = ROWS == 1 ? 1 : op->i[MK_MV_M], mode = op->i[MK_MV_MODE], tr = op->i[MK_MV_TR];
-  const int ot = op->i[MK_MV_OUT_T];
+  const int M = ROWS == 1 ? 1 : op->i[MK_MV_M];
+  const int fl = r.flags;
   constexpr bool bf = WF != 1;   // the activations' type
-  const bool residual = op->i[MK_MV_EPI] == MK_EPI_RESIDUAL;
-  const bool va = g < (mode == MK_MV_ROPE ? 8 : clamp8(O - r.rowA0));
-  const bool vb = g < (mode == MK_MV_ROPE ? 8 : clamp8(O - r.rowB0)) && tr != MK_TR_SILU_MUL;
+  const bool va = g < (r.valid & 255), vb = g < (r.valid >> 8) && !(fl & kEpiSiluMul);
   auto row_of = [&](int q) { return (q >> 1) * 8 + 2 * t + (q & 1); };
   auto value = [&](uint32_t v) { return bf ? bf16lo(v) : f16lo(v); };
   float a[Q], b[Q];
 #pragma unroll
   for (int q = 0; q < Q; ++q) a[q] = sum[q >> 1][q & 1], b[q] = sum[q >> 1][2 + (q & 1)];
-  if (WF == 0 && op->i[MK_MV_PRO] != MK_PRO_NONE) {
+  if (WF == 0 && (fl & kEpiNormed)) {
     // the rows' RMSNorm scales, from the sums of squares that the staging left
     const float k = (float)op->i[MK_MV_K], eps = op->f[MK_MV_F_EPS];
 #pragma unroll
@@ -565,12 +570,12 @@ __device__ __forceinline__ void chain_epilogue(Ctx& c, const mk_op_t* op, const 
       b[q] *= scale;
     }
   }
-  if (WF == 2 && op->i[MK_MV_WFMT] == MK_W_NVFP4_E4M3S16 && op->i[MK_MV_EPI] != MK_EPI_KSUM) {   // (K blocks: the parts were scaled)
-    const float gs = op->f[MK_MV_F_GSCALE], gsb = mode == MK_MV_PAIR ? op->f[MK_MV_F_GSCALE1] : gs;
+  if (WF == 2 && (fl & kEpiScaled)) {
+    const float gs = op->f[MK_MV_F_GSCALE], gsb = fl & kEpiPair ? op->f[MK_MV_F_GSCALE1] : gs;
 #pragma unroll
     for (int q = 0; q < Q; ++q) a[q] *= gs, b[q] *= gsb;
   }
-  if (tr == MK_TR_ROPE) {
+  if (fl & kEpiRope) {
     const uint16_t* cs = reinterpret_cast<const uint16_t*>(op->p[MK_MV_P_COS]) + r.chunk * 8 + g;
     const uint16_t* sn = reinterpret_cast<const uint16_t*>(op->p[MK_MV_P_SIN]) + r.chunk * 8 + g;
     uint16_t cq[Q], sq[Q];
@@ -588,17 +593,17 @@ __device__ __forceinline__ void chain_epilogue(Ctx& c, const mk_op_t* op, const 
       a[q] = a2;
       b[q] = b2;
     }
-  } else if (tr == MK_TR_SILU_MUL) {
+  } else if (fl & kEpiSiluMul) {
 #pragma unroll
     for (int q = 0; q < Q; ++q) a[q] = silu_f(a[q]) * b[q];
-  } else if (tr == MK_TR_RELU) {
+  } else if (fl & kEpiRelu) {
 #pragma unroll
     for (int q = 0; q < Q; ++q) a[q] = fmaxf(a[q], 0.f), b[q] = fmaxf(b[q], 0.f);
-  } else if (tr == MK_TR_SILU) {
+  } else if (fl & kEpiSilu) {
 #pragma unroll
     for (int q = 0; q < Q; ++q) a[q] = silu_f(a[q]), b[q] = silu_f(b[q]);
   }
-  if (residual) {
+  if (fl & kEpiResidual) {
     const uint16_t* er = reinterpret_cast<const uint16_t*>(op->p[MK_MV_P_EPI_RES]) + g;
     uint16_t ra[Q], rb[Q];
 #pragma unroll
@@ -611,7 +616,7 @@ __device__ __forceinline__ void chain_epilogue(Ctx& c, const mk_op_t* op, const 
 #pragma unroll
     for (int q = 0; q < Q; ++q) a[q] += value(ra[q]), b[q] += value(rb[q]);
   }
-  if (op->i[MK_MV_EPI] == MK_EPI_TOP1) {
+  if (fl & kEpiTop1) {
     const int idx0 = op->i[MK_MV_IDX0];
     unsigned long long* keys = reinterpret_cast<unsigned long long*>(op->p[MK_MV_P_OUT]);
 #pragma unroll 1
@@ -630,7 +635,7 @@ __device__ __forceinline__ void chain_epilogue(Ctx& c, const mk_op_t* op, const 
     return;
   }
   char* out = reinterpret_cast<char*>(op->p[MK_MV_P_OUT]);
-  if (ot == MK_T_FP32) {
+  if (fl & kEpiFp32) {
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
       if (row_of(q) >= M) continue;
@@ -643,7 +648,7 @@ __device__ __forceinline__ void chain_epilogue(Ctx& c, const mk_op_t* op, const 
     for (int q = 0; q < Q; ++q) {
       const bool ok = row_of(q) < M;
       uint16_t* o = reinterpret_cast<uint16_t*>(out) + (ok ? rows[row_of(q)].out : 0) + g;
-      const uint32_t v = ot == MK_T_BF16 ? pack_bf16(a[q], b[q]) : pack_f16(a[q], b[q]);
+      const uint32_t v = fl & kEpiFp16 ? pack_f16(a[q], b[q]) : pack_bf16(a[q], b[q]);
       if (ok && va) o[r.offA] = (uint16_t)v;
       if (ok && vb) o[r.offB] = (uint16_t)(v >> 16);
     }
@@ -653,11 +658,10 @@ __device__ __forceinline__ void chain_epilogue(Ctx& c, const mk_op_t* op, const 
 // All partial sums of a unit are in: add them in the order of mv_unit (a participant's accumulators, then the participants),
 // free the slot set and store.
 template <int ROWS, int WF, int NA, bool KS>
-__device__ __forceinline__ void chain_finish(Ctx& c, const mk_op_t* ops, const ChainRow* rows, const ChainUnit& cu, int unit,
+__device__ __forceinline__ void chain_finish(Ctx& c, const mk_op_t* ops, const ChainRow* rows, const ChainUnit cu, int unit,
                                              const float4* mine, int parts, uint32_t set, uint32_t gen) {
   constexpr int NT = chain_nt(ROWS);
   const mk_op_t* op = ops + cu.op;
-  const MvOut r = {cu.rowA0, cu.rowB0, cu.offA, cu.offB, cu.chunk};
   float sum[NT][4];
 #pragma unroll
   for (int n = 0; n < NT; ++n) sum[n][0] = sum[n][1] = sum[n][2] = sum[n][3] = 0.f;
@@ -683,9 +687,26 @@ __device__ __forceinline__ void chain_finish(Ctx& c, const mk_op_t* ops, const C
     *reinterpret_cast<volatile uint32_t*>(&c.ctrl->mv_done[set]) = gen + 1u;
   }
   if constexpr (KS) {
-    if (op->i[MK_MV_EPI] == MK_EPI_KSUM && !mv_kblock_sum<NT, WF == 1 ? -1 : WF>(c, op, unit, sum)) return;
+    if ((cu.flags & kEpiKsum) && !mv_kblock_sum<NT, WF == 1 ? -1 : WF>(c, op, unit, sum)) return;
   }
-  chain_epilogue<ROWS, WF>(c, op, rows + cu.op * 32, r, sum);
+  chain_epilogue<ROWS, WF>(c, op, rows + cu.op * 32, cu, sum);
+}
+
+// Waits until the ring's slot holds its k-th page: when all `handed_back` shares of the earlier ones are in, and only then,
+// the barrier's parity says which page is there.  One vote for both.
+__device__ __forceinline__ bool chain_acquire(Ctx& c, uint32_t slot, uint32_t k, uint32_t handed_back) {
+  volatile uint32_t* released = &c.ctrl->released[slot];
+  const uint32_t bar = full_bar(c, slot);
+  uint64_t t0 = 0;
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 64; ++i)
+      if (__all_sync(0xffffffffu, *released >= handed_back && mbar_try_wait(bar, k & 1u))) return true;
+    if (give_up_check(c, t0, MK_ST_TIMEOUT_PAGE_FULL, (int)slot, (int)k)) {
+      c.dead = true;
+      return false;
+    }
+  }
 }
 
 template <int ROWS, int WF, int AS, bool KS>
@@ -720,11 +741,10 @@ __global__ void __launch_bounds__(kChainThreads, ROWS <= 8 ? 2 : 1) mv_chain_ker
   }
   const int units = local < total ? (total - local + count - 1) / count : 0;
   const int P = L.pages[op0], parts = L.parts[op0];
+  // pages of a unit go to AS warps each, or all of them to the same AS
+  const int step = L.spread ? AS : 0, arrivals = L.spread ? parts * AS : AS, last_pages = L.spread ? parts : 1;
 
-  // (launches behind the first start only when all CTAs of this one have passed here: the first launch waits before, so
-  // all that ran before the program is visible to every load of the later ones, early or not)
   const bool early = (L.flags & kChainEarlyLoads) != 0;
-  if (early) next_may_start();
   if (c.warp == kChainWarps) {
     // ---- loader
     if (c.lane < L.stages) {
@@ -821,7 +841,6 @@ __global__ void __launch_bounds__(kChainThreads, ROWS <= 8 ? 2 : 1) mv_chain_ker
   }
   named_bar_sync(kChainBarrier, kChainWarps * 32);
   prior_work_done();
-  if (!early) next_may_start();
   if ((L.flags & kChainLast) && blockIdx.x == 0 && threadIdx.x == 0) L.pv.state->launches += 1;
   if (units > 0) {
     const mk_op_t* res_op = L.res_op >= 0 && blockIdx.x == 0 ? ops + L.res_op : nullptr;
@@ -834,6 +853,10 @@ __global__ void __launch_bounds__(kChainThreads, ROWS <= 8 ? 2 : 1) mv_chain_ker
     }
   }
   named_bar_sync(kChainBarrier, kChainWarps * 32);
+  // The next launch starts, and begins to fetch its weights, only now: its copies would stand in the way of this launch's
+  // activations.  (No launch behind the first starts before all CTAs of this one have come here, behind the wait: what ran
+  // before the program is visible to every load of the later launches, early or not.)
+  next_may_start();
   if (c.ctrl->pos_bad) {
     // a position outside the caches: nothing runs
     // (the report raises the abort flag, at which the loader stops)
@@ -856,21 +879,20 @@ __global__ void __launch_bounds__(kChainThreads, ROWS <= 8 ? 2 : 1) mv_chain_ker
     int part = 0;
 #pragma unroll 1
     for (int p = 0; p < P; ++p) {
-      const int h = (turn - part * AS) & (kChainWarps - 1);
+      const int h = (turn - part * step) & (kChainWarps - 1);
       if (h < AS) {
         const uint32_t page = c.pages_u32 + slot * page_bytes;
         // (only when all earlier pages of the slot are handed back does the barrier's parity say which page is there)
-        if (k > 0 && !wait_smem_ge(c, &c.ctrl->released[slot], k * AS, (int)slot)) break;
-        if (!wait_mbar(c, full_bar(c, slot), k & 1u, MK_ST_TIMEOUT_PAGE_FULL, (int)slot)) break;
+        if (!chain_acquire(c, slot, k, k * AS)) break;
         const ChainUnit& cu = tab.unit[u & (kChainUnits - 1)];
-        if (p == 0 && h == 0 && c.lane < M) {
+        if (p == 0 && h == 0 && (cu.flags & (kEpiRope | kEpiResidual)) && c.lane < M) {
           // what the unit's epilogue reads: into L1 now
           const mk_op_t* op = ops + cu.op;
           const ChainRow& row = rows[cu.op * 32 + c.lane];
-          if (op->i[MK_MV_TR] == MK_TR_ROPE) {
+          if (cu.flags & kEpiRope) {
             asm volatile("prefetch.global.L1 [%0];" ::"l"(op->p[MK_MV_P_COS] + (uint64_t)(row.tab + cu.chunk * 8) * 2u));
             asm volatile("prefetch.global.L1 [%0];" ::"l"(op->p[MK_MV_P_SIN] + (uint64_t)(row.tab + cu.chunk * 8) * 2u));
-          } else if (op->i[MK_MV_EPI] == MK_EPI_RESIDUAL) {
+          } else {
             asm volatile("prefetch.global.L1 [%0];" ::"l"(op->p[MK_MV_P_EPI_RES] + (uint64_t)(row.er + cu.rowA0) * 2u));
           }
         }
@@ -906,23 +928,20 @@ __global__ void __launch_bounds__(kChainThreads, ROWS <= 8 ? 2 : 1) mv_chain_ker
           mbar_arrive(empty_bar(c, slot));
           atomicAdd(&c.ctrl->released[slot], 1u);
         }
-        if (!entered) {
-          // the set's previous user must have been summed
-          if (!wait_smem_ge(c, &c.ctrl->mv_done[set], gen, u)) break;
-          entered = true;
-        }
+        if (!entered && gen > 0 && !wait_smem_ge(c, &c.ctrl->mv_done[set], gen, u)) break;   // the set's previous user must have been summed
+        entered = true;
 #pragma unroll
         for (int a = 0; a < AN; ++a)
 #pragma unroll
           for (int n = 0; n < NN; ++n) rec(a, n) = make_float4(acc[a][n][0], acc[a][n][1], acc[a][n][2], acc[a][n][3]);
-        if (p + parts >= P) {
-          // the partial sum's last page
+        if (p + last_pages >= P) {
+          // this warp's last page of the partial sum, or of the unit
           __syncwarp();
           int last = 0;
           if (c.lane == 0) {
-            __threadfence_block();
-            last = atomicAdd(&c.ctrl->mv_arrive[set], 1u) == (uint32_t)(parts * AS - 1);
-            __threadfence_block();
+            uint32_t old;
+            asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(old) : "r"(smem_u32(&c.ctrl->mv_arrive[set])) : "memory");
+            last = old == (uint32_t)(arrivals - 1);
           }
           last = __shfl_sync(0xffffffffu, last, 0);
           if (last) chain_finish<ROWS, WF, NA, KS>(c, ops, rows, cu, local + u * count, mine, parts, set, gen);
@@ -934,7 +953,8 @@ __global__ void __launch_bounds__(kChainThreads, ROWS <= 8 ? 2 : 1) mv_chain_ker
         ++k;
       }
     }
-    turn = (turn - parts * AS) & (kChainWarps - 1);
+    // (dealt out: one more, as the warps of a unit's last page arrive last and one of them adds the unit up)
+    turn = (turn - (L.spread ? arrivals + 1 : AS)) & (kChainWarps - 1);
   }
 }
 

@@ -22,7 +22,9 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -550,6 +552,9 @@ struct mk_handle_s {
   bool single_launch;                // MK_PROG_SINGLE_LAUNCH
   mk::ChainTables tables;
   std::vector<mk::ChainStep> chain;  // the program as a chain of kernels; empty: the persistent kernel runs it
+  std::unique_ptr<mk::ChainGraph> chain_graph;   // the same as a graph, where it is long
+  std::atomic<bool> chain_stale;     // a record was replaced: planned again by the next run
+  std::mutex planning;
 };
 
 static void classify_op(const mk_op_t& op, int* ntc, int* wfc, int* feat) {
@@ -662,9 +667,18 @@ static int select_kernel(mk_handle_s* h) {
   return 0;
 }
 
-static int plan_chain(mk_handle_s* h) {
-  if (h->single_launch) return 0;
-  return mk::build_chain(h->ops, h->tables, h->pv, h->ws + h->layout.tmaps, h->num_sms, h->smem_optin, &h->chain);
+// Plans the program's launches.  A replaced record mostly changes what the device reads (pointers, a position) and no launch:
+// the graph is kept then.
+static void plan_chain(mk_handle_s* h) {
+  h->chain_stale = false;
+  if (h->single_launch) return;
+  std::vector<mk::ChainStep> steps;
+  mk::build_chain(h->ops, h->tables, h->pv, h->ws + h->layout.tmaps, h->num_sms, h->smem_optin, &steps);
+  const bool same = steps.size() == h->chain.size() &&
+                    std::equal(steps.begin(), steps.end(), h->chain.begin(), [](const auto& a, const auto& b) { return a.same(b); });
+  if (same) return;
+  h->chain = std::move(steps);
+  h->chain_graph = mk::build_chain_graph(h->chain);
 }
 
 // Restores the caller's current device when an entry point returns.
@@ -809,8 +823,7 @@ static int create_program(const mk_program_t* prog, mk_handle_t* out, bool strea
   h->n_ops = prog->n_ops;
   h->ws = ws;
   h->layout = l;
-  rc = plan_chain(h);
-  if (rc) return rc;
+  plan_chain(h);
   guard.h = nullptr;
   *out = h;
   return 0;
@@ -821,7 +834,12 @@ int mk_create(const mk_program_t* prog, mk_handle_t* out) { return create_progra
 int mk_run(mk_handle_t h, void* cuda_stream) {
   using namespace mk;
   if (!h) return fail(-1, "null handle");
-  if (!h->chain.empty() && h->pv.trace == nullptr) return run_chain(h->chain, reinterpret_cast<cudaStream_t>(cuda_stream));
+  if (h->chain_stale) {
+    std::lock_guard<std::mutex> one(h->planning);
+    if (h->chain_stale) plan_chain(h);
+  }
+  if (!h->chain.empty() && h->pv.trace == nullptr)
+    return run_chain(h->chain, h->chain_graph.get(), reinterpret_cast<cudaStream_t>(cuda_stream));
   // The launch may be placed while the kernel before it in the stream drains: its CTAs set up their shared
   // memory and wait (prior_work_done) before they touch global memory.
   cudaLaunchConfig_t cfg = {};
@@ -954,8 +972,8 @@ int mk_update_op(mk_handle_t h, int32_t op_index, const mk_op_t* op, void* cuda_
   h->ops[op_index] = rec;
   // a changed batch size or weight format may need another kernel variant
   classify_op(rec, &h->op_ntc[op_index], &h->op_wfc[op_index], &h->op_feat[op_index]);
-  rc = select_kernel(h);
-  return rc ? rc : plan_chain(h);
+  h->chain_stale = true;
+  return select_kernel(h);
 }
 
 int mk_read_counters(mk_handle_t h, int32_t* out, int32_t n) {
