@@ -27,8 +27,9 @@ class Values:
         return w if fmt in ("bf16", "fp16") else quantize_nvfp4_weight(w, group_size=16 if fmt == "nvfp4" else 32)
 
 
-def equal_forms(ops, outs, **config):
-    """Both forms, three launches each (the arrival counts and slots they leave behind included), from the same buffers."""
+def equal_forms(ops, outs, launches=1, **config):
+    """Both forms, three launches each (the arrival counts and slots they leave behind included), from the same buffers.
+    `launches`: at least so many kernels in the chain (one may be the persistent kernel, for what a chain cannot run)."""
     start, got = [t.clone() for t in outs], []
     for single in (True, False):
         for t, s in zip(outs, start):
@@ -36,6 +37,7 @@ def equal_forms(ops, outs, **config):
         mk = Megakernel(ops, config=MegakernelConfig(single_launch=single, **config), scheduler=OverlapTileScheduler()).compile()
         for _ in range(3):
             mk.run()
+        assert mk.launches_per_run == 1 if single else mk.launches_per_run >= launches
         assert mk.launch_count() == 3 and not mk.read_counters().any()
         got.append([t.clone() for t in outs])
     for a, b in zip(*got):
@@ -139,7 +141,7 @@ def test_layer(fmt, batch, seq, kv, pos, moving):
         ops = schedule_decode_layer_sm100(hidden_size=hidden, intermediate_size=inter, **kw).ops
     else:
         ops = schedule_decode_layer_nvfp4_sm100(**kw).ops
-    assert equal_forms(ops, [xo, ro, q, at, h, kc, vc], **config)[0].float().abs().sum() > 0
+    assert equal_forms(ops, [xo, ro, q, at, h, kc, vc], launches=5, **config)[0].float().abs().sum() > 0
 
 
 def test_a_position_outside_the_cache_runs_nothing():
@@ -174,3 +176,67 @@ def test_replaced_records_change_the_chain():
     mk.update_op(0, other.native_ops[0])
     mk.run()
     assert torch.equal(y, want)
+
+
+def dependent_products(ws, first, last):
+    """Projections, each on the rows of the one before it: as many launches, one graph from eight on."""
+    ops, x = [], first
+    for w in ws:
+        y = last if w is ws[-1] else torch.zeros_like(first)
+        ops += MatvecSm100Op.schedule(a=x, weight=w, y=y)
+        x = y
+    return ops
+
+
+@pytest.mark.parametrize("n", [7, 8, 20])
+def test_long_chains(n):
+    v = Values(n)
+    y = torch.zeros(2, 1, 256, dtype=BF, device="cuda")
+    ops = dependent_products([v(256, 256, std=0.08) for _ in range(n)], v(2, 1, 256), y)
+    assert equal_forms(ops, [y], launches=n)[0].float().abs().sum() > 0
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_replaced_records_change_a_long_chain(captured):
+    v = Values(11)
+    x, x2, y = v(2, 1, 256), v(2, 1, 256), torch.zeros(2, 1, 256, dtype=BF, device="cuda")
+    ws = [v(256, 256, std=0.08) for _ in range(9)]
+    ops = dependent_products(ws, x, y)
+    mk = Megakernel(ops).compile()
+    mk.run()
+    old = y.clone()
+    first_y = ops[0].tensor_refs["y"]
+    other = Megakernel(MatvecSm100Op.schedule(a=x2, weight=ws[0], y=first_y)).compile()
+    mk.update_op(0, other.native_ops[0])
+    if captured:      # planned again while the caller's stream is captured
+        stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=stream):
+            mk.run(sync=False)
+        graph.replay()
+    else:
+        mk.run()
+    torch.cuda.synchronize()
+    want = torch.zeros_like(y)
+    Megakernel(dependent_products(ws, x2, want), config=MegakernelConfig(single_launch=True)).compile().run()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want) and not torch.equal(y, old)
+
+
+# every row class and number of warps: two dependent projections are two kernels (one would be the persistent kernel)
+@pytest.mark.parametrize("fmt", ["bf16", "fp16", "nvfp4"])
+@pytest.mark.parametrize("rows,k,out", [(1, 1024, 1024), (2, 4096, 4096), (8, 2048, 256), (8, 6144, 2048), (9, 1024, 6144), (16, 2048, 2048),
+                                        (16, 1792, 512), (17, 1024, 1024), (32, 1024, 256)])
+def test_every_row_class_has_its_kernel(fmt, rows, k, out):
+    v = Values(rows + k)
+    dtype = torch.float16 if fmt == "fp16" else BF
+    x, y, z = v(rows, 1, k, dtype=dtype), *(torch.zeros(rows, 1, n, dtype=dtype, device="cuda") for n in (out, 64))
+    ops = []
+    for a, b, o, i in ((x, y, out, k), (y, z, 64, out)):
+        w = v.weight(fmt, o, i)
+        if fmt == "nvfp4":
+            ops += MatvecNvfp4Sm120Op.schedule(a=a, weight_packed=w.packed, weight_scales=w.scales, group_size=w.group_size,
+                                               global_scale=w.global_scale, y=b)
+        else:
+            ops += MatvecSm100Op.schedule(a=a, weight=w, y=b)
+    assert equal_forms(ops, [y, z], launches=2)[1].float().abs().sum() > 0
