@@ -12,7 +12,7 @@ struct EwLaunch {
   int32_t flags, index;
 };
 
-static __global__ void __launch_bounds__(kChainWarps * 32) ew_chain_kernel(const __grid_constant__ EwLaunch L) {
+static __global__ void __launch_bounds__(kEwWarps * 32) ew_chain_kernel(const __grid_constant__ EwLaunch L) {
   __shared__ Ctrl ctrl;
   __shared__ mk_op_t rec;
   Ctx c;
@@ -43,7 +43,7 @@ static __global__ void __launch_bounds__(kChainWarps * 32) ew_chain_kernel(const
     if (threadIdx.x == 0) report(c, MK_ST_BAD_POSITION, ctrl.pos[ctrl.pos_bad - 1], L.pv.pos_limit);
     return;
   }
-  const int unit = (int)blockIdx.x * kChainWarps + c.warp;
+  const int unit = (int)blockIdx.x * kEwWarps + c.warp;
   const mk_op_t* op = &rec;
   if (unit >= op->n_units) return;
   switch (op->opcode) {

@@ -17,8 +17,10 @@
 
 namespace mk {
 
-constexpr int kChainWarps = 8;                              // consumers; one more warp loads
-constexpr int kChainThreads = (kChainWarps + 1) * 32;
+// A kernel's W consumer warps, and one more that loads.
+template <int W>
+constexpr int kChainThreads = (W + 1) * 32;
+constexpr int kEwWarps = 8;                                 // row-wise ops: a unit each
 // A kernel's ROWS: one activation row, or up to 8, 16 or 32; its n-tiles of 8 rows.
 __host__ __device__ constexpr int chain_nt(int rows) { return rows <= 8 ? 1 : rows / 8; }
 constexpr uint32_t kChainBarrier = 1, kChainReady = 2;   // named barriers: the consumers'; all threads', once
@@ -44,7 +46,7 @@ struct MvLaunch {
   int32_t n_ops, flags, res_op, first_op;       // res_op: the op whose residual_out this launch writes, or -1
   int32_t stages, page_bytes, sets_log2;        // ring slots, and sets of slots for partial sums
   int32_t slot_off, act_off, page_off;          // shared memory, bytes
-  // n / d as (n * magic) >> 20 for the small numbers here: rows by tokens a sequence, threads by 16-byte chunks of a row
+  // n / d as (n * magic) >> 22 for the small numbers here: rows by tokens a sequence, threads by 16-byte chunks of a row
   int32_t s_magic, chunk_magic[kChainOps];
 };
 
@@ -63,7 +65,7 @@ struct ChainUnit {
 // What an op's epilogue does, in one word that comes with the unit.
 enum { kEpiNormed = 1, kEpiScaled = 2, kEpiPair = 4, kEpiRope = 8, kEpiSiluMul = 16, kEpiRelu = 32, kEpiSilu = 64, kEpiResidual = 128,
        kEpiTop1 = 256, kEpiFp32 = 512, kEpiFp16 = 1024, kEpiKsum = 2048 };
-__device__ __forceinline__ int small_div(int n, int magic) { return (int)(((uint32_t)n * (uint32_t)magic) >> 20); }
+__device__ __forceinline__ int small_div(int n, int magic) { return (int)(((uint32_t)n * (uint32_t)magic) >> 22); }
 constexpr int kChainUnits = 32;   // units between the loader's and the last finisher's: at most 12 pages + 4 slot sets
 struct ChainTab {
   ChainIn in[32];
@@ -93,7 +95,7 @@ __device__ __forceinline__ uint32_t chain_chunk(int m, int ch) {
 // The sums of squares are those of mv_stage: its 224 threads take chunks tid, tid + 224, ... of a row, and a warp's sum
 // goes to red[row * 7 + warp].  Here (row, one of those seven warps) is a job, and the eight warps take jobs in turn, R at
 // a time, so that a batch's rows are requested together.
-template <int ROWS, int WF, int R, int H>
+template <int ROWS, int WF, int R, int H, int W>
 __device__ __forceinline__ void chain_stage_rms(Ctx& c, const mk_op_t* op, const ChainIn* in, const mk_op_t* res_op) {
   constexpr int T = kConsumerWarps * 32;
   constexpr bool fused = WF == 0;
@@ -108,13 +110,13 @@ __device__ __forceinline__ void chain_stage_rms(Ctx& c, const mk_op_t* op, const
   const int jobs = kConsumerWarps * M;
   const uint4 z = make_uint4(0, 0, 0, 0);
 #pragma unroll 1
-  for (int j0 = c.warp; j0 < jobs; j0 += R * kChainWarps) {
+  for (int j0 = c.warp; j0 < jobs; j0 += R * W) {
     int row[R], ch0[R];
     ChainIn at[R];
     float sum[R];
 #pragma unroll
     for (int j = 0; j < R; ++j) {
-      const int job = j0 + j * kChainWarps;
+      const int job = j0 + j * W;
       row[j] = job < jobs ? (ROWS == 1 ? 0 : job / kConsumerWarps) : -1;
       const int m = max(row[j], 0);
       ch0[j] = row[j] < 0 ? chunks : (job - m * kConsumerWarps) * 32 + c.lane;   // (a missing job has no chunks)
@@ -157,15 +159,15 @@ __device__ __forceinline__ void chain_stage_rms(Ctx& c, const mk_op_t* op, const
 #pragma unroll
     for (int j = 0; j < R; ++j) {
       const float t = warp_sum(sum[j]);
-      if (c.lane == 0 && row[j] >= 0) c.ctrl->red[j0 + j * kChainWarps] = t;   // = row * 7 + the job's warp
+      if (c.lane == 0 && row[j] >= 0) c.ctrl->red[j0 + j * W] = t;   // = row * 7 + the job's warp
     }
   }
   if constexpr (!fused) {
     // second pass over the chunks that this thread wrote: normalise and convert to the products' type
-    named_bar_sync(kChainBarrier, kChainWarps * 32);
+    named_bar_sync(kChainBarrier, W * 32);
     const float eps = op->f[MK_MV_F_EPS];
 #pragma unroll 1
-    for (int j0 = c.warp; j0 < jobs; j0 += kChainWarps) {
+    for (int j0 = c.warp; j0 < jobs; j0 += W) {
       const int m = ROWS == 1 ? 0 : j0 / kConsumerWarps;
       float tot = 0.f;
 #pragma unroll
@@ -322,7 +324,7 @@ __device__ __forceinline__ void chain_page_dense(float (&acc)[ChainCut<NT, AS>::
   };
   // a warp of one tile a pair has (tiles - u0) / 2 of them, rounded up; one of both may end with a pair of one tile
   const int pairs = UN == 1 ? (tiles - u0 + 1) >> 1 : tiles >> 1;
-  if constexpr (NT == 4 && NN * UN * JN > 4) {   // (two sets of fragments would not fit the registers)
+  if constexpr (NT > 1 && NN * UN * JN >= 4) {   // (two sets of fragments would not fit the registers)
     Frag f;
 #pragma unroll 1
     for (int i = 0; i < pairs; ++i) {
@@ -470,7 +472,7 @@ __device__ __forceinline__ void chain_page_fp4(float (&acc)[ChainCut<NT, AS>::AN
         for (int i = 0; i < QN; ++i) px[n][j][i] += by * 512u;
     }
   };
-  if constexpr (NT == 4 && NN * QN > 4) {   // (two sets of fragments would not fit the registers)
+  if constexpr (NT > 1 && NN * QN >= 4) {   // (two sets of fragments would not fit the registers)
     Frag f;
 #pragma unroll 1
     for (int kt = 0; kt < tiles; ++kt) {
@@ -709,8 +711,9 @@ __device__ __forceinline__ bool chain_acquire(Ctx& c, uint32_t slot, uint32_t k,
   }
 }
 
-template <int ROWS, int WF, int AS, bool KS>
-__global__ void __launch_bounds__(kChainThreads, ROWS <= 8 ? 2 : 1) mv_chain_kernel(const __grid_constant__ MvLaunch L) {
+template <int ROWS, int WF, int AS, bool KS, int W>
+__global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
+    mv_chain_kernel(const __grid_constant__ MvLaunch L) {
   constexpr int NT = chain_nt(ROWS);
   using Cut = ChainCut<NT, AS>;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -745,7 +748,7 @@ __global__ void __launch_bounds__(kChainThreads, ROWS <= 8 ? 2 : 1) mv_chain_ker
   const int step = L.spread ? AS : 0, arrivals = L.spread ? parts * AS : AS, last_pages = L.spread ? parts : 1;
 
   const bool early = (L.flags & kChainEarlyLoads) != 0;
-  if (c.warp == kChainWarps) {
+  if (c.warp == W) {
     // ---- loader
     if (c.lane < L.stages) {
       mbar_init(smem_u32(&c.ctrl->full[c.lane]), 32);
@@ -755,7 +758,7 @@ __global__ void __launch_bounds__(kChainThreads, ROWS <= 8 ? 2 : 1) mv_chain_ker
     if (c.lane < 4) c.ctrl->mv_arrive[c.lane] = c.ctrl->mv_done[c.lane] = 0;
     if (c.lane == 0) c.ctrl->abort_flag = c.ctrl->pos_bad = 0;
     fence_mbar_init();
-    named_bar_arrive(kChainReady, kChainThreads);
+    named_bar_arrive(kChainReady, kChainThreads<W>);
     __syncwarp();
     int leader;
     if (elect_one(leader)) {
@@ -808,9 +811,9 @@ __global__ void __launch_bounds__(kChainThreads, ROWS <= 8 ? 2 : 1) mv_chain_ker
   }
 
   // ---- consumers
-  for (int i = threadIdx.x; i < L.n_ops * (int)(sizeof(mk_op_t) / 16); i += kChainWarps * 32)
+  for (int i = threadIdx.x; i < L.n_ops * (int)(sizeof(mk_op_t) / 16); i += W * 32)
     reinterpret_cast<uint4*>(ops)[i] = ldcg128(reinterpret_cast<const uint4*>(L.pv.ops + L.first_op) + i);
-  named_bar_sync(kChainReady, kChainThreads);      // the records, and the loader's barriers
+  named_bar_sync(kChainReady, kChainThreads<W>);      // the records, and the loader's barriers
   const mk_op_t* sop = ops + op0;
   const int K = sop->i[MK_MV_K], M = ROWS == 1 ? 1 : sop->i[MK_MV_M], Kc = sop->i[MK_MV_KC], pro = sop->i[MK_MV_PRO];
   ChainWalk walk;
@@ -826,7 +829,7 @@ __global__ void __launch_bounds__(kChainThreads, ROWS <= 8 ? 2 : 1) mv_chain_ker
     }
     const int b = ROWS == 1 ? 0 : small_div(m, L.s_magic), t = ROWS == 1 ? 0 : m - b * sop->i[MK_MV_S];
 #pragma unroll 1
-    for (int o = tid >> 5; o < L.n_ops; o += kChainWarps)
+    for (int o = tid >> 5; o < L.n_ops; o += W)
       if (m < M) rows[o * 32 + m] = chain_row(ops + o, b, t, pos);
     if (tid < M) {
       const mk_op_t* ro = ops + max(L.res_op, 0);
@@ -836,10 +839,10 @@ __global__ void __launch_bounds__(kChainThreads, ROWS <= 8 ? 2 : 1) mv_chain_ker
     }
     walk.m0 = small_div(tid, L.chunk_magic[op0]);
     walk.ch0 = tid - walk.m0 * chunks;
-    walk.dm = small_div(kChainWarps * 32, L.chunk_magic[op0]);
-    walk.dch = kChainWarps * 32 - walk.dm * chunks;
+    walk.dm = small_div(W * 32, L.chunk_magic[op0]);
+    walk.dch = W * 32 - walk.dm * chunks;
   }
-  named_bar_sync(kChainBarrier, kChainWarps * 32);
+  named_bar_sync(kChainBarrier, W * 32);
   prior_work_done();
   if ((L.flags & kChainLast) && blockIdx.x == 0 && threadIdx.x == 0) L.pv.state->launches += 1;
   if (units > 0) {
@@ -848,11 +851,11 @@ __global__ void __launch_bounds__(kChainThreads, ROWS <= 8 ? 2 : 1) mv_chain_ker
       chain_stage_plain<WF>(c, sop, M, tab.in, walk);
     } else if constexpr (WF != 1) {
       // rows' parts, and chunks of each, requested together
-      constexpr int R = ROWS == 1 ? 1 : (WF == 0 && NT != 1 ? 4 : 2), H = ROWS == 1 || WF == 2 ? 3 : (NT == 1 ? 2 : 1);
-      chain_stage_rms<ROWS, WF, R, H>(c, sop, tab.in, res_op);
+      constexpr int R = ROWS == 1 ? 1 : (WF == 0 && NT != 1 ? 3 : 2), H = ROWS == 1 || WF == 2 ? 3 : (NT == 1 ? 2 : 1);
+      chain_stage_rms<ROWS, WF, R, H, W>(c, sop, tab.in, res_op);
     }
   }
-  named_bar_sync(kChainBarrier, kChainWarps * 32);
+  named_bar_sync(kChainBarrier, W * 32);
   // The next launch starts, and begins to fetch its weights, only now: its copies would stand in the way of this launch's
   // activations.  (No launch behind the first starts before all CTAs of this one have come here, behind the wait: what ran
   // before the program is visible to every load of the later launches, early or not.)
@@ -879,7 +882,7 @@ __global__ void __launch_bounds__(kChainThreads, ROWS <= 8 ? 2 : 1) mv_chain_ker
     int part = 0;
 #pragma unroll 1
     for (int p = 0; p < P; ++p) {
-      const int h = (turn - part * step) & (kChainWarps - 1);
+      const int h = (turn - part * step) & (W - 1);
       if (h < AS) {
         const uint32_t page = c.pages_u32 + slot * page_bytes;
         // (only when all earlier pages of the slot are handed back does the barrier's parity say which page is there)
@@ -954,28 +957,31 @@ __global__ void __launch_bounds__(kChainThreads, ROWS <= 8 ? 2 : 1) mv_chain_ker
       }
     }
     // (dealt out: one more, as the warps of a unit's last page arrive last and one of them adds the unit up)
-    turn = (turn - (L.spread ? arrivals + 1 : AS)) & (kChainWarps - 1);
+    turn = (turn - (L.spread ? arrivals + 1 : AS)) & (W - 1);
   }
 }
 
 }  // namespace mk
 
-// One compiled kernel: <activation rows, weight family (0 bf16, 1 fp16, 2 NVFP4), warps a page, with the sum of K blocks>.
+// One compiled kernel: <activation rows, weight family (0 bf16, 1 fp16, 2 NVFP4), warps a page, with the sum of K blocks,
+// consumer warps>.
 typedef void (*mk_chain_fn)(const mk::MvLaunch);
 struct mk_chain_variant {
-  int rows, as, ks;
+  int rows, as, ks, warps;
   mk_chain_fn fn;
 };
-#define MK_CHAIN_TABLE(name, WF)                                                                    \
-  extern "C" const mk_chain_variant* name(int* n) {                                                 \
-    static const mk_chain_variant v[] = {                                                           \
-        {1, 2, 0, mk::mv_chain_kernel<1, WF, 2, false>},   {1, 4, 0, mk::mv_chain_kernel<1, WF, 4, false>},   \
-        {8, 2, 0, mk::mv_chain_kernel<8, WF, 2, false>},   {8, 4, 0, mk::mv_chain_kernel<8, WF, 4, false>},   \
-        {16, 2, 0, mk::mv_chain_kernel<16, WF, 2, false>}, {16, 4, 0, mk::mv_chain_kernel<16, WF, 4, false>}, \
-        {32, 2, 0, mk::mv_chain_kernel<32, WF, 2, false>}, {32, 4, 0, mk::mv_chain_kernel<32, WF, 4, false>}, \
-        {8, 2, 1, mk::mv_chain_kernel<8, WF, 2, true>},    {16, 2, 1, mk::mv_chain_kernel<16, WF, 2, true>},  \
-        {32, 2, 1, mk::mv_chain_kernel<32, WF, 2, true>},                                           \
-    };                                                                                              \
-    *n = (int)(sizeof(v) / sizeof(v[0]));                                                           \
-    return v;                                                                                       \
+#define MK_CHAIN_KERNEL(ROWS, WF, AS, KS, W) {ROWS, AS, KS, W, mk::mv_chain_kernel<ROWS, WF, AS, KS, W>}
+#define MK_CHAIN_TABLE(name, WF)                                                                          \
+  extern "C" const mk_chain_variant* name(int* n) {                                                       \
+    static const mk_chain_variant v[] = {                                                                 \
+        MK_CHAIN_KERNEL(1, WF, 2, false, 8),   MK_CHAIN_KERNEL(1, WF, 4, false, 8),                       \
+        MK_CHAIN_KERNEL(8, WF, 2, false, 8),   MK_CHAIN_KERNEL(8, WF, 4, false, 8),                       \
+        MK_CHAIN_KERNEL(8, WF, 2, false, 16),  MK_CHAIN_KERNEL(8, WF, 4, false, 16),                      \
+        MK_CHAIN_KERNEL(16, WF, 2, false, 16), MK_CHAIN_KERNEL(16, WF, 4, false, 16),                     \
+        MK_CHAIN_KERNEL(32, WF, 2, false, 8),  MK_CHAIN_KERNEL(32, WF, 4, false, 8),                      \
+        MK_CHAIN_KERNEL(8, WF, 2, true, 8),    MK_CHAIN_KERNEL(8, WF, 2, true, 16),                       \
+        MK_CHAIN_KERNEL(16, WF, 2, true, 16),  MK_CHAIN_KERNEL(32, WF, 2, true, 8),                       \
+    };                                                                                                    \
+    *n = (int)(sizeof(v) / sizeof(v[0]));                                                                 \
+    return v;                                                                                             \
   }
