@@ -15,7 +15,12 @@
 
 namespace mk {
 
-constexpr int kAtChainThreads = 256;      // seven participants, one loader
+// Participants and a loader.  Seven participants, of which two CTAs share a multiprocessor; or four, and three or four CTAs, for
+// launches of many units of few pages (see chain_attn_step).
+template <int PARTS>
+constexpr int kAtChainThreads = (PARTS + 1) * 32;
+// Shared memory of each: 228 KB a multiprocessor, 1 KB of a CTA's the system's.
+constexpr int at_chain_smem(int ctas) { return (228 / ctas - 1) * 1024; }
 constexpr int kAtChainMaxStages = 16;
 
 struct AtLaunch {
@@ -91,8 +96,9 @@ __device__ __forceinline__ void at_norm_query(const mk_op_t* op, const uint32_t 
   }
 }
 
-template <int D, bool QNORM>
-__global__ void __launch_bounds__(kAtChainThreads, 2) at_chain_kernel(const __grid_constant__ AtLaunch L) {
+// PARTS: participants; one more warp loads.  CTAS: that share a multiprocessor.
+template <int D, bool QNORM, int PARTS, int CTAS>
+__global__ void __launch_bounds__(kAtChainThreads<PARTS>, CTAS) at_chain_kernel(const __grid_constant__ AtLaunch L) {
   constexpr int KS = D / 16, ND = D / 8, TN = (D == 64) ? 64 : 32, NS = TN / 8;
   constexpr uint32_t kStateBytes = (ND + 1) * 512;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -108,6 +114,7 @@ __global__ void __launch_bounds__(kAtChainThreads, 2) at_chain_kernel(const __gr
   c.trace_base = nullptr;
   c.trace_n = c.trace_cap = 0;
   const int NPG = L.pv.n_pages;
+  static_assert(!QNORM || PARTS >= KS / 2, "a warp for each pair of query fragments");
   if (threadIdx.x == 0) {
     for (int i = 0; i < NPG; ++i) {
       mbar_init(smem_u32(&c.ctrl->full[i]), 32);
@@ -165,7 +172,7 @@ __global__ void __launch_bounds__(kAtChainThreads, 2) at_chain_kernel(const __gr
     rh[e] = u.kvh * G + (rv[e] ? (M != 1 ? r % G : r) : 0);
   }
 
-  if (c.warp == kConsumerWarps) {
+  if (c.warp == PARTS) {
     // ---- loader
     int leader;
     if (elect_one(leader)) {
@@ -211,7 +218,7 @@ __global__ void __launch_bounds__(kAtChainThreads, 2) at_chain_kernel(const __gr
     if constexpr (QNORM) {
       if (c.warp < KS / 2) tb = at_query_tables<D>(op, c.warp, t, tab_off);
       // (and what the new k row wants, close by)
-      if (c.warp == kConsumerWarps - 1 && c.lane < D / 64)
+      if (c.warp == PARTS - 1 && c.lane < D / 64)
         asm volatile("prefetch.global.L1 [%0];" ::"l"(op->p[MK_AT_P_KNW] + (uint64_t)c.lane * 128u));
     }
     const uint16_t* q = reinterpret_cast<const uint16_t*>(op->p[MK_AT_P_Q]) + u.b * op->s[MK_AT_S_Q_B];
@@ -236,13 +243,13 @@ __global__ void __launch_bounds__(kAtChainThreads, 2) at_chain_kernel(const __gr
       }
     } else {
 #pragma unroll 1
-      for (int ks = c.warp; ks < KS; ks += kConsumerWarps) {
+      for (int ks = c.warp; ks < KS; ks += PARTS) {
         uint32_t f[4];
         fetch(ks, f);
         sts128(qf_at + (uint32_t)ks * 512u, make_uint4(f[0], f[1], f[2], f[3]));
       }
     }
-    named_bar_sync(kConsumerBarrier, kConsumerWarps * 32);
+    named_bar_sync(kConsumerBarrier, PARTS * 32);
     next_may_start();     // (not before: the next launch's weights would stand in the way of the query rows)
   }
 
@@ -365,7 +372,7 @@ __global__ void __launch_bounds__(kAtChainThreads, 2) at_chain_kernel(const __gr
     }
   }
 
-  // ---- states, merged in participant order; a warp takes n-tiles warp, warp + 8, ... of the output
+  // ---- states, merged in participant order; a warp takes every W-th n-tile of the output
   __syncthreads();      // all pages are consumed: the ring is free
   if (c.warp < parts) {
     const uint32_t park = c.pages_u32 + (uint32_t)c.warp * kStateBytes;
@@ -377,7 +384,7 @@ __global__ void __launch_bounds__(kAtChainThreads, 2) at_chain_kernel(const __gr
                                                                  __float_as_uint(lrow[0]), __float_as_uint(lrow[1])));
   }
   __syncthreads();
-  constexpr int MT = (ND + 7) / 8;
+  constexpr int W = PARTS + 1, MT = (ND + PARTS) / W;
   float om[MT][4];
 #pragma unroll
   for (int i = 0; i < MT; ++i) om[i][0] = om[i][1] = om[i][2] = om[i][3] = 0.f;
@@ -385,17 +392,18 @@ __global__ void __launch_bounds__(kAtChainThreads, 2) at_chain_kernel(const __gr
   lrow[0] = lrow[1] = 0.f;
   {
     // everything that is read is requested first; the running maximum and the weights do not depend on the values
-    uint4 ml[kConsumerWarps], v[kConsumerWarps][MT];
+    uint4 ml[PARTS], v[PARTS][MT];
 #pragma unroll
-    for (int j = 0; j < kConsumerWarps; ++j) {
+    for (int j = 0; j < PARTS; ++j) {
       if (j >= parts) break;
       const uint32_t src = c.pages_u32 + (uint32_t)j * kStateBytes + (uint32_t)c.lane * 16u;
       ml[j] = lds128_sync(src + (uint32_t)ND * 512u);
 #pragma unroll
-      for (int i = 0; i < MT; ++i) v[j][i] = lds128_sync(src + (uint32_t)(c.warp + 8 * i) * 512u);
+      for (int i = 0; i < MT; ++i)
+        if (c.warp + W * i < ND) v[j][i] = lds128_sync(src + (uint32_t)(c.warp + W * i) * 512u);
     }
 #pragma unroll
-    for (int j = 0; j < kConsumerWarps; ++j) {
+    for (int j = 0; j < PARTS; ++j) {
       if (j >= parts) break;
       const float mj[2] = {__uint_as_float(ml[j].x), __uint_as_float(ml[j].y)};
       const float lj[2] = {__uint_as_float(ml[j].z), __uint_as_float(ml[j].w)};
@@ -432,7 +440,8 @@ __global__ void __launch_bounds__(kAtChainThreads, 2) at_chain_kernel(const __gr
     float* dst = op_ + base * D;
 #pragma unroll
     for (int i = 0; i < MT; ++i)
-      *reinterpret_cast<float2*>(dst + (c.warp + 8 * i) * 8 + 2 * t) = make_float2(om[i][2 * e] * inv, om[i][2 * e + 1] * inv);
+      if (c.warp + W * i < ND)
+        *reinterpret_cast<float2*>(dst + (c.warp + W * i) * 8 + 2 * t) = make_float2(om[i][2 * e] * inv, om[i][2 * e + 1] * inv);
     if (t == 0 && c.warp == 0) lp_[base] = l > 0.f ? mrow[e] * sc + __logf(l) : -INFINITY;
   }
   if (!op->i[MK_AT_FUSE_COMBINE]) return;
@@ -472,7 +481,7 @@ __global__ void __launch_bounds__(kAtChainThreads, 2) at_chain_kernel(const __gr
   int64_t off = 0;
   const float* base = pair < rows * (D / 2) ? pair_at(pair, off) : nullptr;
   if (base) fetch_pairs(base, 0);
-  for (int r0 = c.warp; r0 < rows; r0 += 8) {
+  for (int r0 = c.warp; r0 < rows; r0 += W) {
     const int r = u.mt * 16 + r0, m = M != 1 ? r / G : 0, h = u.kvh * G + (M != 1 ? r % G : r);
     const float* ls = lp_ + ((int64_t)u.b * H + h) * S * M + m;
     float* w = comb + r0 * S;
@@ -519,7 +528,7 @@ __global__ void __launch_bounds__(kAtChainThreads, 2) at_chain_kernel(const __gr
       *reinterpret_cast<float2*>(reinterpret_cast<float*>(op->p[MK_AT_P_O]) + off) = make_float2(a0, a1);
     else
       *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(op->p[MK_AT_P_O]) + off) = ot == MK_T_BF16 ? pack_bf16(a0, a1) : pack_f16(a0, a1);
-    pair += kAtChainThreads;
+    pair += kAtChainThreads<PARTS>;
     base = pair < rows * (D / 2) ? pair_at(pair, off) : nullptr;
     if (base) fetch_pairs(base, 0);
   }
@@ -529,6 +538,6 @@ __global__ void __launch_bounds__(kAtChainThreads, 2) at_chain_kernel(const __gr
 
 typedef void (*mk_chain_attn_fn)(const mk::AtLaunch);
 struct mk_chain_attn_variant {
-  int d, qnorm;
+  int d, qnorm, parts, ctas;
   mk_chain_attn_fn fn;
 };

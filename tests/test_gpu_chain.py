@@ -90,7 +90,10 @@ def test_normalised_rows_and_pairs(fmt, rows, k, inter):
 
 @pytest.mark.parametrize("batch,kv,heads,kv_heads,dim,splits,causal,m", [
     (1, 1, 8, 8, 64, 0, False, 1), (1, 300, 32, 8, 64, 0, False, 1), (2, 65, 16, 1, 128, 3, False, 1), (3, 1930, 32, 4, 128, 0, False, 1),
-    (1, 2000, 8, 2, 64, 128, False, 1), (1, 700, 8, 4, 128, 40, True, 16), (2, 130, 4, 4, 64, 64, True, 5), (8, 4096, 32, 8, 128, 0, False, 1)])
+    (1, 2000, 8, 2, 64, 128, False, 1), (1, 700, 8, 4, 128, 40, True, 16), (2, 130, 4, 4, 64, 64, True, 5), (8, 4096, 32, 8, 128, 0, False, 1),
+    # units of one to four pages in one, two and more waves of two, three and four CTAs a multiprocessor
+    (13, 500, 8, 8, 64, 4, False, 1), (11, 701, 32, 8, 64, 8, False, 1), (16, 1931, 16, 8, 64, 8, False, 1), (20, 250, 16, 8, 64, 2, True, 2),
+    (12, 380, 32, 8, 128, 4, False, 1), (16, 129, 8, 8, 128, 4, False, 1)])
 @pytest.mark.parametrize("fuse", [True, False])
 def test_attention(batch, kv, heads, kv_heads, dim, splits, causal, m, fuse):
     v = Values(kv + dim)
