@@ -73,9 +73,9 @@ QWEN3_8B = dict(name="qwen3-8b-shape", hidden=4096, inter=12288, nq=32, nkv=8, h
 MODELS = {"llama1b": LLAMA1B, "qwen3-8b": QWEN3_8B}
 FALLBACK_HBM_GBS = 6650.0
 # dram read + write bytes per algorithmic byte, from one ncu capture of a 4-layer + LM-head case
-# of the same kernel (profiles/mk_persistent_kernel_llama1b_decode.md); DRAM traffic is
+# of the same kernels (profiles/chain_kernels_llama1b_decode.md); DRAM traffic is
 # proportional to the layers streamed, so the ratio carries over to the full workload.
-NCU_TRAFFIC_RATIO = 1.006
+NCU_TRAFFIC_RATIO = 1.002
 NOMINAL_HBM_GBS = 8000.0
 MIN_TIMED_SECONDS = 0.5
 L2_BYTES = 126 << 20

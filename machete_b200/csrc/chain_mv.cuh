@@ -9,8 +9,9 @@
 //   * a page is shared by AS warps.  The persistent kernel's warp rotates its products over independent accumulators
 //     (so that no product waits for the one before); here those accumulators are dealt to different warps, which keeps
 //     the order of every sum and takes the time of a page by AS;
-//   * 9 warps of at most 96 registers and at most 113 KB of shared memory: two CTAs share an SM, the second one being
-//     the next launch's, with its ring full, or another of this one where that has units enough.  (8 warps of 128 registers
+//   * 9 warps of at most 96 registers and, where that is room enough, at most 113 KB of shared memory: two CTAs share an SM,
+//     the second one being the next launch's or another of this one where that has units enough; 17 warps where the rows
+//     leave room for one CTA only (see chain_matvec_step).  (8 warps of 128 registers
 //     of which the one that handed a page back last requested the next: some 0.8 us a page on the products' path.)
 #pragma once
 #include "op_matvec.cuh"
