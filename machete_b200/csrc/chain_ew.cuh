@@ -36,6 +36,12 @@ static __global__ void __launch_bounds__(kEwWarps * 32) ew_chain_kernel(const __
       if (c.lane < L.pv.pos_count && (uint32_t)v >= (uint32_t)L.pv.pos_limit) ctrl.pos_bad = 1 + c.lane;
       ctrl.pos[c.lane] = v;
     }
+    // A wait that ran out in a launch before: no token is chosen or fed back and the position stays, as in the persistent
+    // kernel, where this op would not have run (a row of which no unit has left a maximum would name token -1).
+    if (rec.opcode == MK_OP_TOP1_FINAL) {
+      const int failed = *reinterpret_cast<volatile int32_t*>(&L.pv.state->abort_flag);
+      if (failed && c.lane == 0) ctrl.abort_flag = 1;
+    }
     if ((L.flags & kChainLast) && blockIdx.x == 0 && c.lane == 0) L.pv.state->launches += 1;
   }
   __syncthreads();
@@ -43,6 +49,7 @@ static __global__ void __launch_bounds__(kEwWarps * 32) ew_chain_kernel(const __
     if (threadIdx.x == 0) report(c, MK_ST_BAD_POSITION, ctrl.pos[ctrl.pos_bad - 1], L.pv.pos_limit);
     return;
   }
+  if (ctrl.abort_flag) return;
   const int unit = (int)blockIdx.x * kEwWarps + c.warp;
   const mk_op_t* op = &rec;
   if (unit >= op->n_units) return;

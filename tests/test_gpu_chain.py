@@ -8,6 +8,7 @@ from machete_b200.kernels.decode_matvec import (MatvecNvfp4Sm120Op, MatvecResidu
                                                 MatvecSm100Op, RmsGateUpSiluNvfp4Sm120Op, RmsGateUpSiluSm100Op,
                                                 schedule_decode_layer_sm100)
 from machete_b200.kernels.decode_matvec.nvfp4_model import schedule_decode_layer_nvfp4_sm100
+from machete_b200.kernels.llama1b import schedule_decode_model_sm100
 from machete_b200.megakernel import Megakernel, MegakernelConfig, OverlapTileScheduler
 from machete_b200.quantization import quantize_nvfp4_weight
 
@@ -243,3 +244,29 @@ def test_every_row_class_has_its_kernel(fmt, rows, k, out):
         else:
             ops += MatvecSm100Op.schedule(a=a, weight=w, y=b)
     assert equal_forms(ops, [y, z], launches=2)[1].float().abs().sum() > 0
+
+
+def test_no_token_is_fed_back_after_a_failed_launch():
+    """The status and the abort flag that a wait which ran out leaves, written by the host: the last op leaves position,
+    token and input row alone, the error is raised, and the next step runs."""
+    hidden, nq, nkv, hd, inter, vocab, T, start = 512, 8, 2, 64, 1024, 1024, 128, 40
+    v = Values(21)
+    w = layer_weights(v, "bf16", hidden, inter, nq, nkv, hd, T)
+    z = lambda n: torch.zeros(1, 1, n, dtype=BF, device="cuda")      # noqa: E731
+    x_in, position = v(1, 1, hidden), torch.tensor([start], dtype=torch.int32, device="cuda")
+    tv, ti = torch.zeros(1, 1, device="cuda"), torch.full((1, 1), 7, dtype=torch.int32, device="cuda")
+    ops, _keep = schedule_decode_model_sm100(
+        batch=1, cache_pos=0, weights=w, k_cache=[v(1, T, nkv, hd)], v_cache=[v(1, T, nkv, hd)], x_buffers=[z(hidden), z(hidden)],
+        residual_buffers=[z(hidden), z(hidden)], q_buf=z(nq * hd), attn_out_buf=z(nq * hd), mlp_h_buf=z(inter),
+        final_norm=1 + v(hidden, std=0.02), lm_head=v(vocab, hidden, std=0.05), top_values=tv, top_indices=ti, num_layers=1, x_in=x_in,
+        residual_in=z(hidden), position=position, hidden_size=hidden, intermediate_size=inter, num_q_heads=nq, num_kv_heads=nkv, head_dim=hd)
+    mk = Megakernel(ops, config=MegakernelConfig(position=position), scheduler=OverlapTileScheduler()).compile()
+    assert mk.launches_per_run > 1
+    before, at = x_in.clone(), -mk._workspace.data_ptr() % 256
+    state = mk._workspace[at:at + 128].view(torch.int32)      # status[16], abort flag, ...
+    state[0] = state[16] = 1
+    with pytest.raises(RuntimeError, match="aborted"):
+        mk.run()
+    assert int(position) == start and int(ti) == 7 and torch.equal(x_in, before)
+    mk.run()
+    assert int(position) == start + 1 and not torch.equal(x_in, before)
