@@ -151,18 +151,25 @@ class TensorMeta:
         return (self.data_ptr, self.data_ptr + hi * self.element_size)
 
 
-def _axis_starts(meta: TensorMeta) -> Optional[Tuple[int, ...]]:
-    """Per-axis start indices of a view inside its storage lattice."""
-    remaining = meta.storage_offset
-    starts = []
-    for axis, stride in enumerate(meta.strides):
-        if stride <= 0:
+def _axis_starts(meta: TensorMeta, *views: TensorMeta) -> Optional[Tuple[int, ...]]:
+    """Per-axis start indices of a view inside its storage lattice, the largest stride first whatever the order of the axes.
+
+    ``None`` where the indices do not tell the view's values from others': a stride that does not pass over all that the smaller
+    ones reach (sliding windows).  ``views``: others of the same strides, which take part in the choice among axes of one
+    stride (all but the longest hold one index).
+    """
+    if any(stride <= 0 for stride in meta.strides):
+        return None
+    longest = [max(v.shape[i] for v in (meta, *views)) for i in range(meta.ndim)]
+    order = sorted(range(meta.ndim), key=lambda i: (-meta.strides[i], -longest[i], i))
+    remaining, starts = meta.storage_offset, [0] * meta.ndim
+    for i in order:
+        starts[i], remaining = divmod(remaining, meta.strides[i])
+    reach = remaining
+    for i in reversed(order):
+        if starts[i] + meta.shape[i] > 1 and meta.strides[i] <= reach:
             return None
-        if axis == meta.ndim - 1:
-            starts.append(remaining // stride if stride else 0)
-            break
-        starts.append(remaining // stride)
-        remaining %= stride
+        reach += (starts[i] + meta.shape[i] - 1) * meta.strides[i]
     return tuple(starts)
 
 
@@ -181,7 +188,7 @@ def tensor_meta_overlaps(a: TensorMeta, b: TensorMeta) -> bool:
         return False
     if (a.storage_ptr == b.storage_ptr and a.ndim == b.ndim and a.strides == b.strides
             and a.element_size == b.element_size):
-        sa, sb = _axis_starts(a), _axis_starts(b)
+        sa, sb = _axis_starts(a, b), _axis_starts(b, a)
         if sa is not None and sb is not None:
             return all(
                 max(sa[i], sb[i]) < min(sa[i] + a.shape[i], sb[i] + b.shape[i]) for i in range(a.ndim)
