@@ -365,6 +365,27 @@ int mk_create(const mk_program_t* prog, mk_handle_t* out);
 int mk_run(mk_handle_t h, void* cuda_stream);
 /* Kernel launches that one mk_run of this handle makes (0 for a null handle). */
 int mk_launches_per_run(mk_handle_t h);
+/* One launch of a program that runs as a chain. */
+enum { MK_LAUNCH_ROWWISE = 0, MK_LAUNCH_MATVEC = 1, MK_LAUNCH_ATTENTION = 2 };
+typedef struct mk_launch {
+  int32_t kind;                     /* MK_LAUNCH_* */
+  int32_t first_op, n_ops;          /* ops [first_op, first_op + n_ops) of the program */
+  int32_t grid, threads, smem;
+  int32_t rows;                     /* matvec: activation rows that its kernel holds */
+  int32_t warps;                    /* consumer warps (attention: participants of a unit at most) */
+  int32_t per_page;                 /* matvec: warps that share a page */
+  int32_t per_sm;                   /* attention: CTAs that share a multiprocessor */
+  int32_t stages;                   /* ring slots */
+  int32_t residual_op;              /* matvec: the op whose residual_out it writes, or -1 */
+  int32_t early;                    /* 1: weights or cache pages are loaded before the launch before has finished, ... */
+  int32_t wait_lo, wait_hi;         /* ... but those that hold cache tokens [wait_lo, wait_hi) are not; */
+  int32_t wait_dyn;                 /* 1: the device-resident position is added to both */
+} mk_launch_t;
+/* The launches that mk_run makes, in order, into out[0..max): returns how many there are, 0 where the persistent kernel runs
+ * the program, or a negative error.  mk_plan_launches tells it without a device, for one of `num_sms` multiprocessors and
+ * `smem_optin` bytes of shared memory a CTA; pointers in the program are not followed but for its tables. */
+int mk_launch_plan(mk_handle_t h, mk_launch_t* out, int32_t max);
+int mk_plan_launches(const mk_program_t* prog, int32_t num_sms, int32_t smem_optin, mk_launch_t* out, int32_t max);
 /* Copy the 16-word device status block to `out` (synchronises the device).
  * out[0] == 0 means no device-side error. */
 int mk_status(mk_handle_t h, int32_t out[16]);

@@ -159,7 +159,8 @@ static int encode_kv_map(CUtensorMap* out, uint64_t base, int D, int HKV, int N,
   return 0;
 }
 
-static int build_op_maps(mk_op_t& op, CUtensorMap* maps, uint64_t dev_maps, int page_bytes) {
+// The record's fields that are the library's own.
+static void fill_derived(mk_op_t& op) {
   if (op.opcode == MK_OP_ATTN_SPLIT || op.opcode == MK_OP_ATTN_COMBINE)
     op.i[MK_AT_GROUP] = op.i[MK_AT_H] / op.i[MK_AT_HKV];   // validated: H a positive multiple of HKV
   if (op.opcode == MK_OP_ATTN_SPLIT && op.i[MK_AT_FUSE_COMBINE]) {
@@ -168,6 +169,10 @@ static int build_op_maps(mk_op_t& op, CUtensorMap* maps, uint64_t dev_maps, int 
     const int rows = std::min(op.i[MK_AT_GROUP], 256 / op.i[MK_AT_D]);
     op.i[MK_AT_FUSE_COMBINE] = op.i[MK_AT_M] == 1 && rows * op.i[MK_AT_SPLITS] <= 128 ? 2 : 1;
   }
+}
+
+static int build_op_maps(mk_op_t& op, CUtensorMap* maps, uint64_t dev_maps, int page_bytes) {
+  fill_derived(op);
   if (op.opcode == MK_OP_ATTN_SPLIT) {
     const int D = op.i[MK_AT_D];
     const uint32_t tn = (uint32_t)at_page_tokens(D, page_bytes);
@@ -677,6 +682,7 @@ static void plan_chain(mk_handle_s* h) {
   const bool same = steps.size() == h->chain.size() &&
                     std::equal(steps.begin(), steps.end(), h->chain.begin(), [](const auto& a, const auto& b) { return a.same(b); });
   if (same) return;
+  if (mk::prepare_chain(steps, h->smem_optin)) steps.clear();
   h->chain = std::move(steps);
   h->chain_graph = mk::build_chain_graph(h->chain);
 }
@@ -854,6 +860,38 @@ int mk_run(mk_handle_t h, void* cuda_stream) {
   cfg.numAttrs = 1;
   CUDA_TRY(cudaLaunchKernelEx(&cfg, h->kernel, h->pv));
   return 0;
+}
+
+// Launches of a chain as the caller sees them.
+static int tell_launches(const std::vector<mk::ChainStep>& steps, mk_launch_t* out, int32_t max) {
+  for (int i = 0; i < (int)steps.size() && i < max; ++i) out[i] = steps[i].what;
+  return (int)steps.size();
+}
+
+int mk_launch_plan(mk_handle_t h, mk_launch_t* out, int32_t max) {
+  using namespace mk;
+  if (!h || (max > 0 && !out)) return fail(-1, "null argument");
+  return tell_launches(h->chain, out, max);
+}
+
+int mk_plan_launches(const mk_program_t* prog, int32_t num_sms, int32_t smem_optin, mk_launch_t* out, int32_t max) {
+  using namespace mk;
+  if (num_sms < 1 || smem_optin < 1 || (max > 0 && !out)) return fail(-1, "bad argument");
+  int smem_bytes = 0;
+  const int rc = validate_program(prog, smem_optin, num_sms, &smem_bytes);
+  if (rc) return rc;
+  std::vector<mk_op_t> ops(prog->ops, prog->ops + prog->n_ops);
+  for (mk_op_t& op : ops) fill_derived(op);
+  ProgramView pv;
+  memset(&pv, 0, sizeof(pv));
+  pv.n_pages = prog->n_pages;
+  pv.page_bytes = prog->page_bytes;
+  pv.dyn_pos = prog->position;
+  pv.pos_limit = prog->position_limit;
+  pv.pos_count = prog->position_count > 0 ? prog->position_count : 1;
+  std::vector<ChainStep> steps;
+  if (!(prog->flags & MK_PROG_SINGLE_LAUNCH)) build_chain(ops, read_chain_tables(prog), pv, nullptr, num_sms, smem_optin, &steps);
+  return tell_launches(steps, out, max);
 }
 
 int mk_launches_per_run(mk_handle_t h) {

@@ -220,12 +220,8 @@ class Megakernel:
         return self.program.total_bytes
 
     # -- compile / run ------------------------------------------------------------------------
-    def compile(self) -> "Megakernel":
-        """Upload the program tables to the device (idempotent)."""
-        if self._handle:
-            return self
-        lib = N.lib()
-        dev = _device_index(self._device)
+    def _tables(self):
+        """The program as ``mk_create`` takes it, and the arrays that it points to."""
         p = self.program
         arrays = {
             "ops": np.ascontiguousarray(p.ops), "instrs": np.ascontiguousarray(p.instrs),
@@ -243,7 +239,6 @@ class Megakernel:
         prog.n_pages = self._n_pages
         prog.act_bytes = self._act_bytes
         prog.timeout_ms = int(self.config.timeout_ms)
-        prog.device = dev
         prog.flags = N.PROG_SINGLE_LAUNCH if self.config.single_launch else 0
         prog.ops = arrays["ops"].ctypes.data
         prog.instrs = arrays["instrs"].ctypes.data
@@ -253,7 +248,7 @@ class Megakernel:
         prog.waits = arrays["waits"].ctypes.data
         pos = self.config.position
         if pos is not None:
-            if pos.dtype != torch.int32 or not 1 <= pos.numel() <= 32 or not pos.is_cuda or not pos.is_contiguous():
+            if pos.dtype != torch.int32 or not 1 <= pos.numel() <= 32 or not pos.is_contiguous():
                 raise ValueError("MegakernelConfig.position must be a contiguous int32 CUDA tensor with one element, "
                                  "or one per batch row (at most 32)")
             prog.position = pos.data_ptr()
@@ -264,6 +259,20 @@ class Megakernel:
             if not limits:
                 raise ValueError("MegakernelConfig.position is set but no op follows it (schedule with a dynamic position)")
             prog.position_limit = min(limits)
+        return prog, arrays
+
+    def compile(self) -> "Megakernel":
+        """Upload the program tables to the device (idempotent)."""
+        if self._handle:
+            return self
+        lib = N.lib()
+        dev = _device_index(self._device)
+        pos = self.config.position
+        if pos is not None and not pos.is_cuda:
+            raise ValueError("MegakernelConfig.position must be a contiguous int32 CUDA tensor with one element, "
+                             "or one per batch row (at most 32)")
+        prog, arrays = self._tables()
+        prog.device = dev
         nbytes = int(lib.mk_workspace_bytes(C.byref(prog)))
         self._workspace = torch.empty(nbytes + 256, dtype=torch.uint8, device=torch.device("cuda", dev))
         base = self._workspace.data_ptr()
@@ -332,6 +341,25 @@ class Megakernel:
         """Kernel launches that one :meth:`run` makes."""
         self.compile()
         return int(N.lib().mk_launches_per_run(self._handle))
+
+    def launch_plan(self) -> list:
+        """The launches of the chain that :meth:`run` makes, one dict each (see ``mk_launch_t``); empty where the persistent
+        kernel runs the program.  Before :meth:`compile`, those of a device of ``num_sms`` multiprocessors; needs none."""
+        lib = N.lib()
+        if self._handle:
+            def ask(out, n):
+                return lib.mk_launch_plan(self._handle, out, n)
+        else:
+            prog, arrays = self._tables()
+
+            def ask(out, n, keep=arrays):
+                return lib.mk_plan_launches(C.byref(prog), self.num_sms, self._smem_optin, out, n)
+        n = ask(None, 0)
+        if n < 0:
+            N.check(n, "launch_plan")
+        out = (N.Launch * max(1, n))()
+        ask(out, n)
+        return [{name: getattr(launch, name) for name, _ in N.Launch._fields_} for launch in out[:n]]
 
     def launch_count(self) -> int:
         """Launches this handle has completed (aborted ones included); see ``mk_launch_count``."""

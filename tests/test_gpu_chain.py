@@ -6,6 +6,7 @@ import torch
 from machete_b200.kernels.attention import flash_decoding_schedule
 from machete_b200.kernels.decode_matvec import (MatvecNvfp4Sm120Op, MatvecResidualNvfp4Sm120Op, MatvecResidualSm100Op,
                                                 MatvecSm100Op, RmsGateUpSiluNvfp4Sm120Op, RmsGateUpSiluSm100Op,
+                                                RmsKMatvecRopeCacheSm100Op, RmsQMatvecRopeSm100Op, RmsVMatvecCacheSm100Op,
                                                 schedule_decode_layer_sm100)
 from machete_b200.kernels.decode_matvec.nvfp4_model import schedule_decode_layer_nvfp4_sm100
 from machete_b200.kernels.llama1b import schedule_decode_model_sm100
@@ -146,6 +147,34 @@ def test_layer(fmt, batch, seq, kv, pos, moving):
     else:
         ops = schedule_decode_layer_nvfp4_sm100(**kw).ops
     assert equal_forms(ops, [xo, ro, q, at, h, kc, vc], launches=5, **config)[0].float().abs().sum() > 0
+
+
+# appends to one cache, to sequences one by one at positions of their own, to heads of a head-major cache: rows that lie somewhere
+# else than token `position` of sequence 0 are waited for as well
+@pytest.mark.parametrize("case", ["V alone", "K alone", "a later sequence", "sequences one by one", "later heads", "heads one by one"])
+@pytest.mark.parametrize("heads_first", [False, True])
+def test_appends_to_part_of_the_caches(case, heads_first):
+    hidden, heads, kv_heads, dim, batch, kv, pos = 2048, 16, 4, 64, 3, 700, 699
+    v = Values(len(case))
+    caches = v(2, batch, kv_heads, kv, dim).transpose(2, 3) if heads_first else v(2, batch, kv, kv_heads, dim)
+    k, vc = caches[0], caches[1]
+    x, r, n = v(batch, 1, hidden), v(batch, 1, hidden), 1 + v(hidden, std=0.02)
+    cos, sin, w = v(1, dim // 2), v(1, dim // 2), v(kv_heads * dim, hidden, std=0.05)
+    q, o = torch.zeros(batch, 1, heads * dim, dtype=BF, device="cuda"), torch.zeros(batch, 1, heads, dim, dtype=BF, device="cuda")
+    both = ((RmsKMatvecRopeCacheSm100Op, k), (RmsVMatvecCacheSm100Op, vc))
+    append = {"V alone": [(*both[1], 0, pos)], "K alone": [(*both[0], 0, pos)],
+              "a later sequence": [(c, t[1:2], 1, pos) for c, t in both],
+              "sequences one by one": [(c, t[b:b + 1], b, p) for b, p in enumerate((pos, 40, 300)) for c, t in both],
+              "later heads": [(c, t[:, :, 2:], 0, pos) for c, t in both],
+              "heads one by one": [(c, t[:, :, h:h + 1], 0, pos) for h in range(kv_heads) for c, t in both]}[case]
+    ops = RmsQMatvecRopeSm100Op.schedule(x=x, residual_in=r, residual_out=torch.zeros_like(x), norm_weight=n, q=q, cos=cos, sin=sin,
+                                         weight=v(heads * dim, hidden, std=0.05))
+    for cls, cache, first, at in append:
+        rows = slice(first, first + cache.shape[0])
+        ops += cls.schedule(x=x[rows], residual_in=r[rows], norm_weight=n, weight=w[:cache.shape[2] * dim], cos=cos, sin=sin, dst_cache=cache,
+                            cache_pos=at)
+    ops += flash_decoding_schedule(q.view(batch, 1, heads, dim), k, vc, o, kv_group_size=heads // kv_heads)[0]
+    assert equal_forms(ops, [o, q, caches], launches=2)[0].float().abs().sum() > 0
 
 
 def test_a_position_outside_the_cache_runs_nothing():
