@@ -168,7 +168,8 @@ enum {
    * used). */
   MK_AT_DYNPOS,
   /* query heads per KV head (H / Hkv): filled in by mk_create / mk_update_op, whatever the caller
-   * leaves here, so that the kernel does not divide */
+   * leaves here, so that the kernel does not divide.  MK_OP_ATTN_SPLIT: so are the three words behind it
+   * (the cache tokens whose pages wait for the ops before) */
   MK_AT_GROUP
 };
 enum { MK_AT_F_SCALE = 0, MK_AT_F_EPS };
@@ -424,7 +425,9 @@ int mk_set_launch_count(mk_handle_t h, int32_t count, void* cuda_stream);
  * KV window).  The record is validated like mk_create does, the opcode and
  * unit count must stay, the op's tensor maps are re-encoded and the
  * instruction rows derived from the record (pages per unit, loader and
- * finisher fast path) are recomputed and uploaded.  Synchronises
+ * finisher fast path) are recomputed and uploaded, and so are the cache tokens
+ * that attention ops wait for where the op, or one that appends to its caches,
+ * moved.  Synchronises
  * `cuda_stream`.  The reference re-schedules and recompiles for a new
  * position (kernels/decode_matvec/sm100.py:116, 704-709). */
 int mk_update_op(mk_handle_t h, int32_t op_index, const mk_op_t* op, void* cuda_stream);

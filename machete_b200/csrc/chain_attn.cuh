@@ -27,8 +27,6 @@ struct AtLaunch {
   ProgramView pv;               // n_pages: ring slots; page_bytes: a K and a V block
   int32_t flags, index;
   int32_t tn, most_parts;       // tokens a page; participants of a unit at most
-  int32_t wait_lo, wait_hi;     // tokens that the program appends before this op (with a device-resident position: relative to it)
-  int32_t wait_dyn;
   int32_t q_off, comb_off, page_off;   // shared memory, bytes: query fragments; combine weights; ring
   const uint8_t* maps;                 // the K and the V cache's tensor maps
 };
@@ -177,7 +175,7 @@ __global__ void __launch_bounds__(kAtChainThreads<PARTS>, CTAS) at_chain_kernel(
     int leader;
     if (elect_one(leader)) {
       const uint64_t policy = l2_evict_first_policy();
-      const int w0 = L.wait_lo + (L.wait_dyn ? pos : 0), w1 = L.wait_hi + (L.wait_dyn ? pos : 0);
+      const int moved = op->i[kAtWaitDyn] ? pos : 0, w0 = op->i[kAtWaitLo] + moved, w1 = op->i[kAtWaitHi] + moved;
       bool waited = !early;
       uint32_t slot = 0, k = 0;
       int p = 0;

@@ -687,6 +687,11 @@ static void plan_chain(mk_handle_s* h) {
   h->chain_graph = mk::build_chain_graph(h->chain);
 }
 
+static void set_windows(std::vector<mk_op_t>& ops, const mk::ChainTables& t, int pos_limit) {
+  for (int i = 0; i < (int)ops.size(); ++i)
+    if (ops[i].opcode == MK_OP_ATTN_SPLIT) mk::set_window(ops, t, i, pos_limit);
+}
+
 // Restores the caller's current device when an entry point returns.
 struct DeviceScope {
   int prev = -1;
@@ -769,6 +774,8 @@ static int create_program(const mk_program_t* prog, mk_handle_t* out, bool strea
                          (uint64_t)(ws + l.tmaps) + (uint64_t)i * kMapsPerOp * sizeof(CUtensorMap), prog->page_bytes);
       if (rc) return rc;
     }
+    h->tables = read_chain_tables(prog);
+    set_windows(h->ops, h->tables, prog->position_limit);
     CUDA_TRY(upload(ws + l.tmaps, maps.data(), maps.size() * sizeof(CUtensorMap)));
     CUDA_TRY(upload(ws + l.ops, h->ops.data(), h->ops.size() * sizeof(mk_op_t)));
   }
@@ -824,7 +831,6 @@ static int create_program(const mk_program_t* prog, mk_handle_t* out, bool strea
   if (rc) return rc;
   h->num_sms = num_sms;
   h->single_launch = (prog->flags & MK_PROG_SINGLE_LAUNCH) != 0;
-  if (!h->single_launch) h->tables = read_chain_tables(prog);
   h->device = prog->device;
   h->n_ops = prog->n_ops;
   h->ws = ws;
@@ -863,15 +869,26 @@ int mk_run(mk_handle_t h, void* cuda_stream) {
 }
 
 // Launches of a chain as the caller sees them.
-static int tell_launches(const std::vector<mk::ChainStep>& steps, mk_launch_t* out, int32_t max) {
-  for (int i = 0; i < (int)steps.size() && i < max; ++i) out[i] = steps[i].what;
+static int tell_launches(const std::vector<mk::ChainStep>& steps, const std::vector<mk_op_t>& ops, mk_launch_t* out, int32_t max) {
+  for (int i = 0; i < (int)steps.size() && i < max; ++i) {
+    out[i] = steps[i].what;
+    const mk_op_t& op = ops[out[i].first_op];
+    if (out[i].kind != MK_LAUNCH_ATTENTION || !out[i].early) continue;
+    if (op.i[mk::kAtWaitHi] == mk::kAllTokens) {
+      out[i].early = 0;
+      continue;
+    }
+    out[i].wait_lo = op.i[mk::kAtWaitLo];
+    out[i].wait_hi = op.i[mk::kAtWaitHi];
+    out[i].wait_dyn = op.i[mk::kAtWaitDyn];
+  }
   return (int)steps.size();
 }
 
 int mk_launch_plan(mk_handle_t h, mk_launch_t* out, int32_t max) {
   using namespace mk;
   if (!h || (max > 0 && !out)) return fail(-1, "null argument");
-  return tell_launches(h->chain, out, max);
+  return tell_launches(h->chain, h->ops, out, max);
 }
 
 int mk_plan_launches(const mk_program_t* prog, int32_t num_sms, int32_t smem_optin, mk_launch_t* out, int32_t max) {
@@ -889,9 +906,11 @@ int mk_plan_launches(const mk_program_t* prog, int32_t num_sms, int32_t smem_opt
   pv.dyn_pos = prog->position;
   pv.pos_limit = prog->position_limit;
   pv.pos_count = prog->position_count > 0 ? prog->position_count : 1;
+  const ChainTables tables = read_chain_tables(prog);
+  set_windows(ops, tables, prog->position_limit);
   std::vector<ChainStep> steps;
-  if (!(prog->flags & MK_PROG_SINGLE_LAUNCH)) build_chain(ops, read_chain_tables(prog), pv, nullptr, num_sms, smem_optin, &steps);
-  return tell_launches(steps, out, max);
+  if (!(prog->flags & MK_PROG_SINGLE_LAUNCH)) build_chain(ops, tables, pv, nullptr, num_sms, smem_optin, &steps);
+  return tell_launches(steps, ops, out, max);
 }
 
 int mk_launches_per_run(mk_handle_t h) {
@@ -998,19 +1017,33 @@ int mk_update_op(mk_handle_t h, int32_t op_index, const mk_op_t* op, void* cuda_
     lo = std::min(lo, j);
     hi = std::max(hi, j + 1);
   }
+  // Other launches where the record says something else than the kernels read from it; for a window of fewer or more pages
+  // the ones that there are would do, but not as well.
+  const mk_op_t before = h->ops[op_index];
+  h->ops[op_index] = rec;
+  bool replan = !chain_alike(before, rec);
+  if (rec.opcode == MK_OP_ATTN_SPLIT) replan |= most_pages_of(before, h->pv.page_bytes) != most_pages_of(rec, h->pv.page_bytes);
+  if (replan) h->chain_stale = true;
+  // the tokens that attention ops wait for: of this one, or of those that read what it writes
+  std::vector<int> changed(1, op_index);
+  for (int i = 0; i < h->n_ops; ++i) {
+    if (h->ops[i].opcode != MK_OP_ATTN_SPLIT) continue;
+    const std::vector<int>& writers = h->tables.load_deps[i];
+    if (i == op_index) set_window(h->ops, h->tables, i, h->pv.pos_limit);
+    else if (std::find(writers.begin(), writers.end(), op_index) != writers.end() && set_window(h->ops, h->tables, i, h->pv.pos_limit))
+      changed.push_back(i);
+  }
   cudaStream_t st = reinterpret_cast<cudaStream_t>(cuda_stream);
   CUDA_TRY(cudaMemcpyAsync(dev_maps, maps, sizeof(maps), cudaMemcpyHostToDevice, st));
-  CUDA_TRY(cudaMemcpyAsync(h->ws + h->layout.ops + (size_t)op_index * sizeof(mk_op_t), &rec, sizeof(mk_op_t),
-                           cudaMemcpyHostToDevice, st));
+  for (int i : changed)
+    CUDA_TRY(cudaMemcpyAsync(h->ws + h->layout.ops + (size_t)i * sizeof(mk_op_t), &h->ops[i], sizeof(mk_op_t), cudaMemcpyHostToDevice, st));
   if (hi > lo)
     CUDA_TRY(cudaMemcpyAsync(h->ws + h->layout.instrs + lo * sizeof(mk_instr_t), h->instrs.data() + lo,
                              (hi - lo) * sizeof(mk_instr_t), cudaMemcpyHostToDevice, st));
   // the host buffers above must outlive the copies
   CUDA_TRY(cudaStreamSynchronize(st));
-  h->ops[op_index] = rec;
   // a changed batch size or weight format may need another kernel variant
   classify_op(rec, &h->op_ntc[op_index], &h->op_wfc[op_index], &h->op_feat[op_index]);
-  h->chain_stale = true;
   return select_kernel(h);
 }
 

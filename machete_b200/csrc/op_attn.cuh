@@ -52,6 +52,12 @@ __device__ __forceinline__ AtUnit at_decode_fast(const mk_op_t* op, const UnitAr
   return u;
 }
 
+// Words of an attention record behind MK_AT_GROUP, the library's own: the cache tokens [lo, hi) that the program writes before the op
+// (kAtWaitDyn: the device-resident position is added to both), whose pages are not loaded before those writes.  They stand in the
+// record, where a replaced record of a writer or of the op changes them for launches that have been captured too.
+enum { kAtWaitLo = MK_AT_GROUP + 1, kAtWaitHi, kAtWaitDyn };
+constexpr int kAllTokens = 1 << 30;   // [0, kAllTokens): every page waits
+
 // Tokens per page for head dim D and a given page size: a K block and a V
 // block of `tn` rows each; tn is a multiple of the consumer's inner block
 // (64 tokens for D = 64, 32 for D = 128) and at most 64: a split of a few

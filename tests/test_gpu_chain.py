@@ -299,3 +299,61 @@ def test_no_token_is_fed_back_after_a_failed_launch():
     assert int(position) == start and int(ti) == 7 and torch.equal(x_in, before)
     mk.run()
     assert int(position) == start + 1 and not torch.equal(x_in, before)
+
+
+class MovingLayer:
+    """One layer with a position in its records; V lies in front of K.  `at(pos)`: its ops at a position, on the same buffers."""
+
+    def __init__(self, batch=2, length=600, seed=21):
+        self.hidden, self.inter, self.heads, self.kv_heads, self.dim = 2048, 4096, 16, 4, 64
+        self.batch, v = batch, Values(seed)
+        self.w = layer_weights(v, "bf16", self.hidden, self.inter, self.heads, self.kv_heads, self.dim, length)
+        z = lambda n: torch.zeros(batch, 1, n, dtype=BF, device="cuda")      # noqa: E731
+        self.caches, self.x, self.r = v(2, batch, length, self.kv_heads, self.dim), v(batch, 1, self.hidden), v(batch, 1, self.hidden)
+        self.xo, self.ro, self.q, self.a, self.h = z(self.hidden), z(self.hidden), z(self.heads * self.dim), z(self.heads * self.dim), z(self.inter)
+        self.outs = [self.xo, self.ro, self.q, self.a, self.h, self.caches]
+        self.start = [t.clone() for t in self.outs]
+
+    def at(self, pos):
+        return schedule_decode_layer_sm100(
+            layer_idx=0, batch=self.batch, seq_len=1, cache_pos=pos, weights=self.w, k_cache=self.caches[1], v_cache=self.caches[0], x_in=self.x,
+            residual_in=self.r, x_out=self.xo, residual_out=self.ro, q_buf=self.q, attn_out_buf=self.a, mlp_h_buf=self.h, eps=1e-5,
+            hidden_size=self.hidden, intermediate_size=self.inter, num_q_heads=self.heads, num_kv_heads=self.kv_heads, head_dim=self.dim,
+            fa_num_splits=4).ops
+
+    def after(self, step):
+        for t, s in zip(self.outs, self.start):
+            t.copy_(s)
+        step()
+        torch.cuda.synchronize()
+        return [t.clone() for t in self.outs]
+
+
+def same_bytes(a, b):
+    return all(torch.equal(p.view(torch.uint8), q.view(torch.uint8)) for p, q in zip(a, b))
+
+
+def captured(mk):
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.graph(graph, stream=stream):
+        mk.run(sync=False, validate=False)
+    return graph
+
+
+# over a page's boundary and a split's, several at a time, and back: the rows that attention waits for move with the records
+def test_replaced_positions_move_a_captured_step():
+    layer = MovingLayer()
+    mk = Megakernel(layer.at(100), scheduler=OverlapTileScheduler()).compile()
+    mk.run()
+    graph = captured(mk)
+    for pos in (101, 127, 128, 129, 300, 70, 511, 512, 599, 63):
+        fresh = Megakernel(layer.at(pos), scheduler=OverlapTileScheduler()).compile()
+        for i, record in enumerate(fresh.native_ops):
+            mk.update_op(i, record)
+        plan = mk.launch_plan()
+        assert [(p["early"], p["wait_lo"], p["wait_hi"]) for p in plan if p["kind"] == 2] == [(1, pos, pos + 1)]
+        want = layer.after(fresh.run)
+        for step in (graph.replay, mk.run, graph.replay):
+            assert same_bytes(layer.after(step), want), pos
+        mk.wait()
