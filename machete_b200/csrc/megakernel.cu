@@ -23,6 +23,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -78,8 +79,8 @@ static Layout layout_of(const mk_program_t* p) {
   o = align_up(o + (uint64_t)(p->n_events > 0 ? p->n_events : 1) * sizeof(mk_event_t), 256);
   l.ebegin = o;
   o = align_up(o + (uint64_t)(p->n_ctas + 1) * 4, 256);
-  l.waits = o;
-  o = align_up(o + (uint64_t)(p->n_waits > 0 ? p->n_waits : 1) * sizeof(mk_wait_t), 256);
+  l.waits = o;   // (twice the table: see gather_loader_lists)
+  o = align_up(o + (uint64_t)(p->n_waits > 0 ? 2 * (uint64_t)p->n_waits : 1) * sizeof(mk_wait_t), 256);
   l.tmaps = o;
   o = align_up(o + (uint64_t)p->n_ops * kMapsPerOp * sizeof(CUtensorMap), 256);
   l.total = o;
@@ -284,6 +285,38 @@ static void fill_instr_fast_path(mk_instr_t& in, const mk_op_t& op, uint64_t dev
   const int64_t sh = op.s[MK_MV_S_O_H];
   in.out_off_a = (int32_t)((int64_t)(in.ld_row_a / hd) * sh + in.ld_row_a % hd);
   in.out_off_b = (int32_t)((int64_t)(in.ld_row_b / hd) * sh + in.ld_row_b % hd);
+}
+
+// All that the loads of an attention op's units wait for, as one list of the wait table: what a unit waits for when a replaced
+// record moves the appended rows into its tokens.  (The tables give the list to the units that held those rows when the program was
+// scheduled.)  Lists that do not stand in `waits` yet are put behind it, as far as that at most doubles it.
+struct WaitList {
+  int n = 0, off = 0;
+};
+static std::vector<WaitList> gather_loader_lists(const mk_program_t* p, std::vector<mk_wait_t>* waits) {
+  std::vector<WaitList> lists(p->n_ops);
+  std::vector<std::vector<WaitList>> seen(p->n_ops);
+  for (int j = 0; j < p->n_instrs; ++j) {
+    const mk_instr_t& in = p->instrs[j];
+    if (in.n_lwaits == 0 || p->ops[in.op].opcode != MK_OP_ATTN_SPLIT) continue;
+    auto& of = seen[in.op];
+    if (std::none_of(of.begin(), of.end(), [&](const WaitList& w) { return w.n == in.n_lwaits && w.off == in.lwait_off; }))
+      of.push_back({in.n_lwaits, in.lwait_off});
+  }
+  for (int i = 0; i < p->n_ops; ++i) {
+    std::map<int, int> all;   // counter -> what it has to reach
+    for (const WaitList& w : seen[i])
+      for (int k = w.off; k < w.off + w.n; ++k) {
+        int& expected = all.emplace(p->waits[k].counter, 0).first->second;
+        expected = std::max(expected, p->waits[k].expected);
+      }
+    for (const WaitList& w : seen[i])
+      if (w.n == (int)all.size()) lists[i] = w;
+    if (lists[i].n || (int)(waits->size() + all.size()) > 2 * p->n_waits) continue;
+    lists[i] = {(int)all.size(), (int)waits->size()};
+    for (const auto& w : all) waits->push_back({w.first, w.second});
+  }
+  return lists;
 }
 
 static int validate_op(const mk_op_t& op, int idx, int page_bytes, int act_bytes) {
@@ -545,6 +578,7 @@ struct mk_handle_s {
   int feat;                          // features of the kernel in use
   std::vector<mk_op_t> ops;          // host copy of the op records (as uploaded)
   std::vector<mk_instr_t> instrs;    // host copy of the instruction table (as uploaded)
+  std::vector<mk::WaitList> loader_lists;   // per op, empty without waits
   bool states_may_stage;             // no matvec unit relies on activations staged before an attention op
   int n_ctas;
   int smem_bytes;
@@ -692,6 +726,31 @@ static void set_windows(std::vector<mk_op_t>& ops, const mk::ChainTables& t, int
     if (ops[i].opcode == MK_OP_ATTN_SPLIT) mk::set_window(ops, t, i, pos_limit);
 }
 
+// The instruction rows of op `i` from its record: page counts, the fast path, and for attention what the loads wait for, which
+// follows the rows that are appended.  [*lo, *hi): the span of the table that holds them.
+static void refresh_rows(mk_handle_s* h, int i, size_t* lo, size_t* hi) {
+  const mk_op_t& op = h->ops[i];
+  const mk::WaitList list = h->loader_lists.empty() ? mk::WaitList{} : h->loader_lists[i];
+  const bool attention = op.opcode == MK_OP_ATTN_SPLIT;
+  const bool moves = attention && list.n > 0 && h->tables.ok && !op.i[MK_AT_DYNPOS];   // (a device-resident position: the loader looks)
+  *lo = h->instrs.size(), *hi = 0;
+  for (size_t j = 0; j < h->instrs.size(); ++j) {
+    mk_instr_t& in = h->instrs[j];
+    if (in.op != i) continue;
+    if (op.opcode == MK_OP_MATVEC) in.n_pages = mk::matvec_pages(op);
+    else if (attention) in.n_pages = mk::attn_pages(op, in.unit, h->pv.page_bytes);
+    mk::fill_instr_fast_path(in, op, (uint64_t)(h->ws + h->layout.tmaps), h->pv.page_bytes, h->pv.n_pages);
+    if (moves) {
+      const int begin = (in.unit % op.i[MK_AT_SPLITS]) * op.i[MK_AT_TS], end = std::min(begin + op.i[MK_AT_TS], op.i[MK_AT_N]);
+      const bool waits = in.n_pages > 0 && begin < op.i[mk::kAtWaitHi] && end > op.i[mk::kAtWaitLo];
+      in.n_lwaits = waits ? list.n : 0;
+      in.lwait_off = waits ? list.off : 0;
+    }
+    *lo = std::min(*lo, j);
+    *hi = std::max(*hi, j + 1);
+  }
+}
+
 // Restores the caller's current device when an entry point returns.
 struct DeviceScope {
   int prev = -1;
@@ -799,7 +858,11 @@ static int create_program(const mk_program_t* prog, mk_handle_t* out, bool strea
     CUDA_TRY(upload(ws + l.events, events.data(), events.size() * sizeof(mk_event_t)));
   }
   CUDA_TRY(upload(ws + l.ebegin, prog->cta_event_begin, (size_t)(prog->n_ctas + 1) * 4));
-  if (prog->n_waits) CUDA_TRY(upload(ws + l.waits, prog->waits, (size_t)prog->n_waits * sizeof(mk_wait_t)));
+  if (prog->n_waits) {
+    std::vector<mk_wait_t> waits(prog->waits, prog->waits + prog->n_waits);
+    h->loader_lists = gather_loader_lists(prog, &waits);
+    CUDA_TRY(upload(ws + l.waits, waits.data(), waits.size() * sizeof(mk_wait_t)));
+  }
 
   h->pv.ops = reinterpret_cast<const mk_op_t*>(ws + l.ops);
   h->pv.instrs = reinterpret_cast<const mk_instr_t*>(ws + l.instrs);
@@ -1005,18 +1068,6 @@ int mk_update_op(mk_handle_t h, int32_t op_index, const mk_op_t* op, void* cuda_
   uint8_t* dev_maps = h->ws + h->layout.tmaps + (size_t)op_index * kMapsPerOp * sizeof(CUtensorMap);
   rc = build_op_maps(rec, maps, (uint64_t)dev_maps, h->pv.page_bytes);
   if (rc) return rc;
-  // Page counts and the per-unit fast path are derived from the record: recompute the
-  // op's instruction rows and upload the span of the table that holds them.
-  size_t lo = h->instrs.size(), hi = 0;
-  for (size_t j = 0; j < h->instrs.size(); ++j) {
-    mk_instr_t& in = h->instrs[j];
-    if (in.op != op_index) continue;
-    if (rec.opcode == MK_OP_MATVEC) in.n_pages = matvec_pages(rec);
-    else if (rec.opcode == MK_OP_ATTN_SPLIT) in.n_pages = attn_pages(rec, in.unit, h->pv.page_bytes);
-    fill_instr_fast_path(in, rec, (uint64_t)(h->ws + h->layout.tmaps), h->pv.page_bytes, h->pv.n_pages);
-    lo = std::min(lo, j);
-    hi = std::max(hi, j + 1);
-  }
   // Other launches where the record says something else than the kernels read from it; for a window of fewer or more pages
   // the ones that there are would do, but not as well.
   const mk_op_t before = h->ops[op_index];
@@ -1035,11 +1086,15 @@ int mk_update_op(mk_handle_t h, int32_t op_index, const mk_op_t* op, void* cuda_
   }
   cudaStream_t st = reinterpret_cast<cudaStream_t>(cuda_stream);
   CUDA_TRY(cudaMemcpyAsync(dev_maps, maps, sizeof(maps), cudaMemcpyHostToDevice, st));
-  for (int i : changed)
+  for (int i : changed) {
     CUDA_TRY(cudaMemcpyAsync(h->ws + h->layout.ops + (size_t)i * sizeof(mk_op_t), &h->ops[i], sizeof(mk_op_t), cudaMemcpyHostToDevice, st));
-  if (hi > lo)
-    CUDA_TRY(cudaMemcpyAsync(h->ws + h->layout.instrs + lo * sizeof(mk_instr_t), h->instrs.data() + lo,
-                             (hi - lo) * sizeof(mk_instr_t), cudaMemcpyHostToDevice, st));
+    // what the rows of the instruction table derive from the record: upload the span that holds them
+    size_t lo = 0, hi = 0;
+    refresh_rows(h, i, &lo, &hi);
+    if (hi > lo)
+      CUDA_TRY(cudaMemcpyAsync(h->ws + h->layout.instrs + lo * sizeof(mk_instr_t), h->instrs.data() + lo, (hi - lo) * sizeof(mk_instr_t),
+                               cudaMemcpyHostToDevice, st));
+  }
   // the host buffers above must outlive the copies
   CUDA_TRY(cudaStreamSynchronize(st));
   // a changed batch size or weight format may need another kernel variant

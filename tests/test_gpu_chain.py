@@ -342,9 +342,10 @@ def captured(mk):
 
 
 # over a page's boundary and a split's, several at a time, and back: the rows that attention waits for move with the records
-def test_replaced_positions_move_a_captured_step():
+@pytest.mark.parametrize("single", [False, True])
+def test_replaced_positions_move_a_captured_step(single):
     layer = MovingLayer()
-    mk = Megakernel(layer.at(100), scheduler=OverlapTileScheduler()).compile()
+    mk = Megakernel(layer.at(100), config=MegakernelConfig(single_launch=single), scheduler=OverlapTileScheduler()).compile()
     mk.run()
     graph = captured(mk)
     for pos in (101, 127, 128, 129, 300, 70, 511, 512, 599, 63):
@@ -352,7 +353,7 @@ def test_replaced_positions_move_a_captured_step():
         for i, record in enumerate(fresh.native_ops):
             mk.update_op(i, record)
         plan = mk.launch_plan()
-        assert [(p["early"], p["wait_lo"], p["wait_hi"]) for p in plan if p["kind"] == 2] == [(1, pos, pos + 1)]
+        assert [(p["early"], p["wait_lo"], p["wait_hi"]) for p in plan if p["kind"] == 2] == ([] if single else [(1, pos, pos + 1)])
         want = layer.after(fresh.run)
         for step in (graph.replay, mk.run, graph.replay):
             assert same_bytes(layer.after(step), want), pos
