@@ -364,7 +364,9 @@ int mk_create(const mk_program_t* prog, mk_handle_t* out);
  * themselves, so back-to-back runs and CUDA-graph replay are legal.
  * Replaces Megakernel.run() / launch_prepared (megakernel.py:2163-2204). */
 int mk_run(mk_handle_t h, void* cuda_stream);
-/* Kernel launches that one mk_run of this handle makes (0 for a null handle). */
+/* Kernel launches that one mk_run of this handle makes (0 for a null handle).  On a capturing stream a chain has one more: the
+ * persistent kernel, which ends at once unless mk_update_op has replaced a record since in a way that the captured launches
+ * cannot follow (other sizes, types, transforms or head strides). */
 int mk_launches_per_run(mk_handle_t h);
 /* One launch of a program that runs as a chain. */
 enum { MK_LAUNCH_ROWWISE = 0, MK_LAUNCH_MATVEC = 1, MK_LAUNCH_ATTENTION = 2 };
@@ -427,8 +429,9 @@ int mk_set_launch_count(mk_handle_t h, int32_t count, void* cuda_stream);
  * instruction rows derived from the record (pages per unit, loader and
  * finisher fast path) are recomputed and uploaded, and so are the cache tokens
  * that attention ops wait for where the op, or one that appends to its caches,
- * moved.  Synchronises
- * `cuda_stream`.  The reference re-schedules and recompiles for a new
+ * moved.  Synchronises `cuda_stream`.  Replays of a step that was captured
+ * before run the new record, as far as one kernel covers both (ops of at most
+ * 8, 16 or 32 rows, and their weight format).  The reference re-schedules and recompiles for a new
  * position (kernels/decode_matvec/sm100.py:116, 704-709). */
 int mk_update_op(mk_handle_t h, int32_t op_index, const mk_op_t* op, void* cuda_stream);
 /* Read back the dependency counters (n_counters words) — after a completed

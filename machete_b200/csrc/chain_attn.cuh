@@ -111,6 +111,10 @@ __global__ void __launch_bounds__(kAtChainThreads<PARTS>, CTAS) at_chain_kernel(
   c.dead = false;
   c.trace_base = nullptr;
   c.trace_n = c.trace_cap = 0;
+  if (!plan_in_force(L.pv)) {
+    prior_work_done();
+    return;
+  }
   const int NPG = L.pv.n_pages;
   static_assert(!QNORM || PARTS >= KS / 2, "a warp for each pair of query fragments");
   if (threadIdx.x == 0) {

@@ -24,6 +24,10 @@ static __global__ void __launch_bounds__(kEwWarps * 32) ew_chain_kernel(const __
   c.dead = false;
   c.trace_base = nullptr;
   c.trace_n = c.trace_cap = 0;
+  if (!plan_in_force(L.pv)) {
+    prior_work_done();
+    return;
+  }
   if (threadIdx.x == 0) ctrl.abort_flag = ctrl.pos_bad = 0;
   if (threadIdx.x < sizeof(mk_op_t) / 16)
     reinterpret_cast<uint4*>(&rec)[threadIdx.x] = ldcg128(reinterpret_cast<const uint4*>(L.pv.ops + L.index) + threadIdx.x);

@@ -732,6 +732,10 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
   c.dead = false;
   c.trace_base = nullptr;
   c.trace_n = c.trace_cap = 0;
+  if (!plan_in_force(L.pv)) {
+    prior_work_done();
+    return;
+  }
   const uint32_t page_bytes = (uint32_t)L.page_bytes;
 
   // this CTA's units: every `count`-th of `total` from `local` on, of ops [op0, ...)

@@ -593,6 +593,8 @@ struct mk_handle_s {
   std::vector<mk::ChainStep> chain;  // the program as a chain of kernels; empty: the persistent kernel runs it
   std::unique_ptr<mk::ChainGraph> chain_graph;   // the same as a graph, where it is long
   std::atomic<bool> chain_stale;     // a record was replaced: planned again by the next run
+  int plan;                          // counts the updates after which launches planned before do not run the program
+  bool fixed;                        // no record of it is replaced
   std::mutex planning;
 };
 
@@ -642,17 +644,18 @@ static bool states_may_stage(const mk_program_t* p) {
   return true;
 }
 
-// Where the participants of attention units leave their states (ProgramView::at_sets).
-static void place_states(mk_handle_s* h) {
+// Where the participants of attention units leave their states (ProgramView::at_sets); `any_window`: for whatever windows the
+// records may get.
+static void place_states(const mk_handle_s* h, bool any_window, mk::ProgramView* pv) {
   int bytes = 0;
   for (const mk_instr_t& in : h->instrs) {
     const mk_op_t& op = h->ops[in.op];
     if (op.opcode != MK_OP_ATTN_SPLIT) continue;
-    bytes = std::max(bytes, mk::at_participants(in.n_pages, h->pv.n_pages) * (op.i[MK_AT_D] / 8 + 1) * 512);
+    bytes = std::max(bytes, mk::at_participants(any_window ? 1 << 20 : in.n_pages, pv->n_pages) * (op.i[MK_AT_D] / 8 + 1) * 512);
   }
-  const int sets = bytes && h->states_may_stage ? h->pv.act_bytes / bytes : 0;
-  h->pv.at_set_bytes = sets ? bytes : 0;
-  h->pv.at_sets = sets == 0 || sets >= 4 ? 4 : (sets >= 2 ? 2 : 1);
+  const int sets = bytes && h->states_may_stage ? pv->act_bytes / bytes : 0;
+  pv->at_set_bytes = sets ? bytes : 0;
+  pv->at_sets = sets == 0 || sets >= 4 ? 4 : (sets >= 2 ? 2 : 1);
 }
 
 // Pick the smallest kernel that covers the program: its matvec ops' tile class
@@ -696,7 +699,7 @@ static int select_kernel(mk_handle_s* h) {
   h->pv.mv_sets = 4;
   for (int n : h->op_ntc)
     if (n > 0) h->pv.mv_sets = std::min(h->pv.mv_sets, n == 1 ? 4 : (n == 2 ? 2 : 1));
-  place_states(h);
+  place_states(h, false, &h->pv);
   // The dynamic shared-memory limit is a property of the kernel function, shared by
   // every handle that runs this variant: always raise it to the device's opt-in
   // maximum, so that a later, smaller program never lowers it under a live one.
@@ -906,6 +909,24 @@ static int create_program(const mk_program_t* prog, mk_handle_t* out, bool strea
 
 int mk_create(const mk_program_t* prog, mk_handle_t* out) { return create_program(prog, out, false, nullptr); }
 
+static int launch_persistent(mk_handle_s* h, const mk::ProgramView& pv, cudaStream_t stream) {
+  using namespace mk;
+  // The launch may be placed while the kernel before it in the stream drains: its CTAs set up their shared
+  // memory and wait (prior_work_done) before they touch global memory.
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)h->n_ctas);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = (size_t)h->smem_bytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  CUDA_TRY(cudaLaunchKernelEx(&cfg, h->kernel, pv));
+  return 0;
+}
+
 int mk_run(mk_handle_t h, void* cuda_stream) {
   using namespace mk;
   if (!h) return fail(-1, "null handle");
@@ -913,22 +934,22 @@ int mk_run(mk_handle_t h, void* cuda_stream) {
     std::lock_guard<std::mutex> one(h->planning);
     if (h->chain_stale) plan_chain(h);
   }
-  if (!h->chain.empty() && h->pv.trace == nullptr)
-    return run_chain(h->chain, h->chain_graph.get(), reinterpret_cast<cudaStream_t>(cuda_stream));
-  // The launch may be placed while the kernel before it in the stream drains: its CTAs set up their shared
-  // memory and wait (prior_work_done) before they touch global memory.
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)h->n_ctas);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = (size_t)h->smem_bytes;
-  cfg.stream = reinterpret_cast<cudaStream_t>(cuda_stream);
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  CUDA_TRY(cudaLaunchKernelEx(&cfg, h->kernel, h->pv));
-  return 0;
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(cuda_stream);
+  const bool persistent = h->chain.empty() || h->pv.trace != nullptr;
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  CUDA_TRY(cudaStreamIsCapturing(stream, &capturing));
+  if (capturing == cudaStreamCaptureStatusNone || h->fixed) {
+    if (persistent) return launch_persistent(h, h->pv, stream); return run_chain(h->chain, h->chain_graph.get(), stream);
+  }
+  // The records may be others when the captured step is replayed.
+  ProgramView pv = h->pv;
+  place_states(h, true, &pv);
+  if (persistent) return launch_persistent(h, pv, stream);
+  // a chain is its kernels, and the persistent kernel for records that those cannot run
+  pv.plan = h->plan;
+  pv.plan_now = &reinterpret_cast<DeviceState*>(h->ws + h->layout.state)->plan;
+  const int rc = launch_chain(h->chain, stream, pv.plan_now, pv.plan);
+  return rc ? rc : launch_persistent(h, pv, stream);
 }
 
 // Launches of a chain as the caller sees them.
@@ -1016,13 +1037,13 @@ int mk_reset(mk_handle_t h, void* cuda_stream) {
   using namespace mk;
   if (!h) return fail(-1, "null handle");
   // Status, abort flag, the count of finished CTAs and the dependency counters
-  // are cleared; the launch count is kept: the tensor-parallel exchange tags
+  // are cleared; the plan's number and the launch count are kept: the tensor-parallel exchange tags
   // its messages with it, and ranks stay in step only while every rank's count
   // advances once per launch.
   cudaStream_t st = reinterpret_cast<cudaStream_t>(cuda_stream);
   uint8_t* base = h->ws + h->layout.state;
   CUDA_TRY(cudaMemsetAsync(base, 0, offsetof(DeviceState, launches), st));
-  const size_t after = offsetof(DeviceState, launches) + sizeof(int32_t);
+  const size_t after = offsetof(DeviceState, plan) + sizeof(int32_t);
   CUDA_TRY(cudaMemsetAsync(base + after, 0, (h->layout.ops - h->layout.state) - after, st));
   return 0;
 }
@@ -1073,6 +1094,7 @@ int mk_update_op(mk_handle_t h, int32_t op_index, const mk_op_t* op, void* cuda_
   const mk_op_t before = h->ops[op_index];
   h->ops[op_index] = rec;
   bool replan = !chain_alike(before, rec);
+  if (replan) ++h->plan;
   if (rec.opcode == MK_OP_ATTN_SPLIT) replan |= most_pages_of(before, h->pv.page_bytes) != most_pages_of(rec, h->pv.page_bytes);
   if (replan) h->chain_stale = true;
   // the tokens that attention ops wait for: of this one, or of those that read what it writes
@@ -1095,6 +1117,7 @@ int mk_update_op(mk_handle_t h, int32_t op_index, const mk_op_t* op, void* cuda_
       CUDA_TRY(cudaMemcpyAsync(h->ws + h->layout.instrs + lo * sizeof(mk_instr_t), h->instrs.data() + lo, (hi - lo) * sizeof(mk_instr_t),
                                cudaMemcpyHostToDevice, st));
   }
+  CUDA_TRY(cudaMemcpyAsync(h->ws + h->layout.state + offsetof(DeviceState, plan), &h->plan, sizeof(int32_t), cudaMemcpyHostToDevice, st));
   // the host buffers above must outlive the copies
   CUDA_TRY(cudaStreamSynchronize(st));
   // a changed batch size or weight format may need another kernel variant

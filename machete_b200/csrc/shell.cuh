@@ -57,7 +57,8 @@ struct DeviceState {
   int32_t abort_flag;   // set by the first CTA that times out
   int32_t done_ctas;    // CTAs that finished this launch
   int32_t launches;     // completed launches
-  int32_t pad[13];
+  int32_t plan;         // see ProgramView::plan
+  int32_t pad[12];
 };
 
 struct ProgramView {
@@ -86,7 +87,15 @@ struct ProgramView {
   const int32_t* dyn_pos;  // device-resident cache position, or null
   int32_t pos_limit;       // positions >= this end the launch with MK_ST_BAD_POSITION before any op runs
   int32_t pos_count;       // entries behind dyn_pos: 1 (one position for every batch row) or one per row (<= 32)
+  // A chain that a caller captured holds the launches of one plan, and the persistent kernel behind them: where a replaced record has
+  // made another plan of the program since, the chain's launches end at once, else the persistent kernel does.
+  int32_t plan;             // this launch's
+  const int32_t* plan_now;  // the one in force; null: this launch runs
 };
+
+__device__ __forceinline__ bool plan_in_force(const ProgramView& pv) {
+  return pv.plan_now == nullptr || *reinterpret_cast<const volatile int32_t*>(pv.plan_now) == pv.plan;
+}
 
 // One trace event: a globaltimer stamp, an event code and an argument.
 struct TraceRec {

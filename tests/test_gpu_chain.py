@@ -358,3 +358,32 @@ def test_replaced_positions_move_a_captured_step(single):
         for step in (graph.replay, mk.run, graph.replay):
             assert same_bytes(layer.after(step), want), pos
         mk.wait()
+
+
+# records that the captured launches cannot follow: K slices of another length; caches with the heads in front of the tokens
+def test_replaced_sizes_and_strides_reach_a_captured_step():
+    layer = MovingLayer()
+    mk = Megakernel(layer.at(300), scheduler=OverlapTileScheduler()).compile()
+    mk.run()
+    graph = captured(mk)
+    rows = layer.caches
+    by_head = rows.new_zeros(2, layer.batch, layer.kv_heads, 600, layer.dim).transpose(2, 3)
+    by_head.copy_(rows)
+    other = MovingLayer(seed=22)
+    for name in ("x", "r", "w", "xo", "ro", "q", "a", "h"):
+        setattr(other, name, getattr(layer, name))
+    other.caches = by_head
+    layer.outs, layer.start = [*layer.outs, by_head], [*layer.start, by_head.clone()]
+    counted = mk.launch_count()
+    for at, config in ((layer.at, dict(native_kc=512)), (other.at, {}), (layer.at, {})):
+        fresh = Megakernel(at(300), config=MegakernelConfig(single_launch=True, **config), scheduler=OverlapTileScheduler()).compile()
+        for i, record in enumerate(fresh.native_ops):
+            mk.update_op(i, record)
+        want = layer.after(fresh.run)
+        assert same_bytes(layer.after(graph.replay), want)
+        assert same_bytes(layer.after(mk.run), want) and len(mk.launch_plan()) == 5
+        again = captured(mk)
+        assert same_bytes(layer.after(again.replay), want) and same_bytes(layer.after(graph.replay), want)
+        mk.wait()
+        counted += 4
+        assert mk.launch_count() == counted
