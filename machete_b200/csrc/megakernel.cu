@@ -22,7 +22,6 @@
 #include <string.h>
 
 #include <algorithm>
-#include <atomic>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -590,9 +589,8 @@ struct mk_handle_s {
   int num_sms;
   bool single_launch;                // MK_PROG_SINGLE_LAUNCH
   mk::ChainTables tables;
-  std::vector<mk::ChainStep> chain;  // the program as a chain of kernels; empty: the persistent kernel runs it
-  std::unique_ptr<mk::ChainGraph> chain_graph;   // the same as a graph, where it is long
-  std::atomic<bool> chain_stale;     // a record was replaced: planned again by the next run
+  std::shared_ptr<const mk::ChainPlan> chain;   // what a run launches; read and replaced under `planning`
+  bool chain_stale;                  // a record was replaced: planned again by the next run
   int plan;                          // counts the updates after which launches planned before do not run the program
   bool fixed;                        // no record of it is replaced
   std::mutex planning;
@@ -709,19 +707,46 @@ static int select_kernel(mk_handle_s* h) {
   return 0;
 }
 
-// Plans the program's launches.  A replaced record mostly changes what the device reads (pointers, a position) and no launch:
-// the graph is kept then.
-static void plan_chain(mk_handle_s* h) {
-  h->chain_stale = false;
-  if (h->single_launch) return;
-  std::vector<mk::ChainStep> steps;
-  mk::build_chain(h->ops, h->tables, h->pv, h->ws + h->layout.tmaps, h->num_sms, h->smem_optin, &steps);
-  const bool same = steps.size() == h->chain.size() &&
-                    std::equal(steps.begin(), steps.end(), h->chain.begin(), [](const auto& a, const auto& b) { return a.same(b); });
-  if (same) return;
-  if (mk::prepare_chain(steps, h->smem_optin)) steps.clear();
-  h->chain = std::move(steps);
-  h->chain_graph = mk::build_chain_graph(h->chain);
+// Restores the caller's current device when an entry point returns.
+struct DeviceScope {
+  int prev = -1;
+  ~DeviceScope() {
+    if (prev >= 0) cudaSetDevice(prev);
+  }
+};
+
+// The program's launches as its records stand.  The graph is kept where the launches are those of `before`.
+static std::shared_ptr<const mk::ChainPlan> make_plan(const mk_handle_s* h, const std::shared_ptr<const mk::ChainPlan>& before) {
+  auto plan = std::make_shared<mk::ChainPlan>();
+  if (h->single_launch) return plan;
+  mk::build_chain(h->ops, h->tables, h->pv, h->ws + h->layout.tmaps, h->num_sms, h->smem_optin, &plan->steps);
+  if (before && plan->steps.size() == before->steps.size() &&
+      std::equal(plan->steps.begin(), plan->steps.end(), before->steps.begin(), [](const auto& a, const auto& b) { return a.same(b); }))
+    return before;
+  DeviceScope scope;
+  if (cudaGetDevice(&scope.prev) != cudaSuccess || cudaSetDevice(h->device) != cudaSuccess || mk::prepare_chain(plan->steps, h->smem_optin))
+    plan->steps.clear();
+  plan->graph = mk::build_chain_graph(plan->steps);
+  return plan;
+}
+// The plan to run now.  Runs of one handle may come from several threads: whoever finds a replaced record plans, the others wait.
+static std::shared_ptr<const mk::ChainPlan> current_plan(mk_handle_s* h) {
+  std::lock_guard<std::mutex> one(h->planning);
+  if (h->chain_stale) {
+    h->chain = make_plan(h, h->chain);
+    h->chain_stale = false;
+  }
+  return h->chain;
+}
+
+// What an entry point answers when the host runs out of memory.
+template <class F>
+static int guarded(F f) {
+  try {
+    return f();
+  } catch (const std::exception& e) {
+    return mk::fail(-6, "%s", e.what());
+  }
 }
 
 static void set_windows(std::vector<mk_op_t>& ops, const mk::ChainTables& t, int pos_limit) {
@@ -753,14 +778,6 @@ static void refresh_rows(mk_handle_s* h, int i, size_t* lo, size_t* hi) {
     *hi = std::max(*hi, j + 1);
   }
 }
-
-// Restores the caller's current device when an entry point returns.
-struct DeviceScope {
-  int prev = -1;
-  ~DeviceScope() {
-    if (prev >= 0) cudaSetDevice(prev);
-  }
-};
 
 extern "C" {
 
@@ -901,7 +918,7 @@ static int create_program(const mk_program_t* prog, mk_handle_t* out, bool strea
   h->n_ops = prog->n_ops;
   h->ws = ws;
   h->layout = l;
-  plan_chain(h);
+  h->chain = make_plan(h, nullptr);
   guard.h = nullptr;
   *out = h;
   return 0;
@@ -927,19 +944,14 @@ static int launch_persistent(mk_handle_s* h, const mk::ProgramView& pv, cudaStre
   return 0;
 }
 
-int mk_run(mk_handle_t h, void* cuda_stream) {
+static int run_program(mk_handle_s* h, cudaStream_t stream) {
   using namespace mk;
-  if (!h) return fail(-1, "null handle");
-  if (h->chain_stale) {
-    std::lock_guard<std::mutex> one(h->planning);
-    if (h->chain_stale) plan_chain(h);
-  }
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(cuda_stream);
-  const bool persistent = h->chain.empty() || h->pv.trace != nullptr;
+  const std::shared_ptr<const ChainPlan> plan = current_plan(h);
+  const bool persistent = plan->steps.empty() || h->pv.trace != nullptr;
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   CUDA_TRY(cudaStreamIsCapturing(stream, &capturing));
   if (capturing == cudaStreamCaptureStatusNone || h->fixed) {
-    if (persistent) return launch_persistent(h, h->pv, stream); return run_chain(h->chain, h->chain_graph.get(), stream);
+    if (persistent) return launch_persistent(h, h->pv, stream); return run_chain(*plan, stream);
   }
   // The records may be others when the captured step is replayed.
   ProgramView pv = h->pv;
@@ -948,8 +960,13 @@ int mk_run(mk_handle_t h, void* cuda_stream) {
   // a chain is its kernels, and the persistent kernel for records that those cannot run
   pv.plan = h->plan;
   pv.plan_now = &reinterpret_cast<DeviceState*>(h->ws + h->layout.state)->plan;
-  const int rc = launch_chain(h->chain, stream, pv.plan_now, pv.plan);
+  const int rc = launch_chain(plan->steps, stream, pv.plan_now, pv.plan);
   return rc ? rc : launch_persistent(h, pv, stream);
+}
+
+int mk_run(mk_handle_t h, void* cuda_stream) {
+  if (!h) return mk::fail(-1, "null handle");
+  return guarded([&] { return run_program(h, reinterpret_cast<cudaStream_t>(cuda_stream)); });
 }
 
 // Launches of a chain as the caller sees them.
@@ -972,10 +989,10 @@ static int tell_launches(const std::vector<mk::ChainStep>& steps, const std::vec
 int mk_launch_plan(mk_handle_t h, mk_launch_t* out, int32_t max) {
   using namespace mk;
   if (!h || (max > 0 && !out)) return fail(-1, "null argument");
-  return tell_launches(h->chain, h->ops, out, max);
+  return guarded([&] { return tell_launches(current_plan(h)->steps, h->ops, out, max); });
 }
 
-int mk_plan_launches(const mk_program_t* prog, int32_t num_sms, int32_t smem_optin, mk_launch_t* out, int32_t max) {
+static int plan_launches(const mk_program_t* prog, int32_t num_sms, int32_t smem_optin, mk_launch_t* out, int32_t max) {
   using namespace mk;
   if (num_sms < 1 || smem_optin < 1 || (max > 0 && !out)) return fail(-1, "bad argument");
   int smem_bytes = 0;
@@ -997,9 +1014,13 @@ int mk_plan_launches(const mk_program_t* prog, int32_t num_sms, int32_t smem_opt
   return tell_launches(steps, ops, out, max);
 }
 
+int mk_plan_launches(const mk_program_t* prog, int32_t num_sms, int32_t smem_optin, mk_launch_t* out, int32_t max) {
+  return guarded([&] { return plan_launches(prog, num_sms, smem_optin, out, max); });
+}
+
 int mk_launches_per_run(mk_handle_t h) {
   if (!h) return 0;
-  return h->chain.empty() || h->pv.trace != nullptr ? 1 : (int)h->chain.size();
+  return guarded([&] { return h->pv.trace != nullptr ? 1 : std::max(1, (int)current_plan(h)->steps.size()); });
 }
 
 int mk_status(mk_handle_t h, int32_t out[16]) {
@@ -1073,9 +1094,8 @@ int mk_set_launch_count(mk_handle_t h, int32_t count, void* cuda_stream) {
   return 0;
 }
 
-int mk_update_op(mk_handle_t h, int32_t op_index, const mk_op_t* op, void* cuda_stream) {
+static int update_op(mk_handle_s* h, int32_t op_index, const mk_op_t* op, void* cuda_stream) {
   using namespace mk;
-  if (!h || !op) return fail(-1, "null argument");
   if (op_index < 0 || op_index >= h->n_ops) return fail(-1, "op index %d out of range", op_index);
   mk_op_t rec = *op;
   int rc = validate_op(rec, op_index, h->pv.page_bytes, h->pv.act_bytes);
@@ -1091,6 +1111,7 @@ int mk_update_op(mk_handle_t h, int32_t op_index, const mk_op_t* op, void* cuda_
   if (rc) return rc;
   // Other launches where the record says something else than the kernels read from it; for a window of fewer or more pages
   // the ones that there are would do, but not as well.
+  std::lock_guard<std::mutex> one(h->planning);
   const mk_op_t before = h->ops[op_index];
   h->ops[op_index] = rec;
   bool replan = !chain_alike(before, rec);
@@ -1123,6 +1144,11 @@ int mk_update_op(mk_handle_t h, int32_t op_index, const mk_op_t* op, void* cuda_
   // a changed batch size or weight format may need another kernel variant
   classify_op(rec, &h->op_ntc[op_index], &h->op_wfc[op_index], &h->op_feat[op_index]);
   return select_kernel(h);
+}
+
+int mk_update_op(mk_handle_t h, int32_t op_index, const mk_op_t* op, void* cuda_stream) {
+  if (!h || !op) return mk::fail(-1, "null argument");
+  return guarded([&] { return update_op(h, op_index, op, cuda_stream); });
 }
 
 int mk_read_counters(mk_handle_t h, int32_t* out, int32_t n) {

@@ -1,5 +1,7 @@
 """A program as a chain of kernels against the same program as one launch: the same sums in the same order, so the same bits."""
 
+import threading
+
 import pytest
 import torch
 
@@ -387,3 +389,36 @@ def test_replaced_sizes_and_strides_reach_a_captured_step():
         mk.wait()
         counted += 4
         assert mk.launch_count() == counted
+
+
+def test_two_threads_run_a_program_whose_record_was_replaced():
+    v = Values(31)
+    y = torch.zeros(2, 1, 256, dtype=BF, device="cuda")
+    ops = dependent_products([v(256, 256, std=0.08) for _ in range(9)], v(2, 1, 256), y)
+    mk = Megakernel(ops).compile()
+    mk.run()
+    want, rounds = y.clone(), 40
+    records = [Megakernel(ops, config=MegakernelConfig(native_kc=kc)).native_ops for kc in (64, 1024)]   # (other launches each time)
+    stream, errors = torch.cuda.Stream(), []
+
+    def runs(gate):
+        try:
+            gate.wait(30)
+            for _ in range(3):
+                mk.run(stream=stream, sync=False, validate=False)
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    for n in range(rounds):
+        mk.update_op(n % 9, records[(n // 9) % 2][n % 9])
+        y.zero_()
+        torch.cuda.synchronize()
+        gate = threading.Barrier(2)
+        threads = [threading.Thread(target=runs, args=(gate,)) for _ in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join(60)
+        mk.wait()
+        assert not errors and (y.float() - want.float()).abs().max() <= 0.02 * want.float().abs().max()
+    assert mk.launch_count() == 1 + 6 * rounds
