@@ -848,8 +848,15 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
     walk.dch = W * 32 - walk.dm * chunks;
   }
   named_bar_sync(kChainBarrier, W * 32);
+  const int bad = c.ctrl->pos_bad;
   prior_work_done();
   if ((L.flags & kChainLast) && blockIdx.x == 0 && threadIdx.x == 0) L.pv.state->launches += 1;
+  if (bad) {
+    // a position outside the caches: nothing runs, the residual output included
+    // (the report raises the abort flag, at which the loader stops)
+    if (threadIdx.x == 0) report(c, MK_ST_BAD_POSITION, c.ctrl->pos[bad - 1], L.pv.pos_limit);
+    return;
+  }
   if (units > 0) {
     const mk_op_t* res_op = L.res_op >= 0 && blockIdx.x == 0 ? ops + L.res_op : nullptr;
     if (pro == MK_PRO_NONE) {
@@ -865,12 +872,6 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
   // activations.  (No launch behind the first starts before all CTAs of this one have come here, behind the wait: what ran
   // before the program is visible to every load of the later launches, early or not.)
   next_may_start();
-  if (c.ctrl->pos_bad) {
-    // a position outside the caches: nothing runs
-    // (the report raises the abort flag, at which the loader stops)
-    if (threadIdx.x == 0) report(c, MK_ST_BAD_POSITION, c.ctrl->pos[c.ctrl->pos_bad - 1], L.pv.pos_limit);
-    return;
-  }
 
   const int g = c.lane >> 2;
   const uint32_t xs = chain_row_stride<WF>(K);

@@ -1,0 +1,62 @@
+"""What a chain of kernels does where a run of it cannot do all: positions outside the caches, launches behind one that failed, ops behind
+the one that moves the position; and records that only some of a launch's ops carry."""
+
+import pytest
+import torch
+
+from machete_b200.kernels.attention import flash_decoding_schedule
+from machete_b200.kernels.decode_matvec import schedule_decode_layer_sm100
+from machete_b200.megakernel import Megakernel, MegakernelConfig
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+
+
+def values(*shape, std=1.0, seed=3):
+    return (torch.randn(*shape, generator=torch.Generator().manual_seed(seed + sum(shape))) * std).to(BF).cuda()
+
+
+def positions(*at):
+    return torch.tensor(at, dtype=torch.int32, device="cuda")
+
+
+class Layer:
+    """A layer that follows a device-resident position; every buffer that it writes holds 7 before a run."""
+
+    def __init__(self, length=64, batch=2):
+        hidden, inter, dim = 512, 1024, 64
+        w = {"cos": values(length, 32), "sin": values(length, 32), "layer.0.attn_norm": values(hidden), "layer.0.mlp_norm": values(hidden)}
+        for name, o, i in (("q", hidden, hidden), ("k", 128, hidden), ("v", 128, hidden), ("o", hidden, hidden), ("gate", inter, hidden),
+                           ("up", inter, hidden), ("down", hidden, inter)):
+            w[f"layer.0.W_{name}"] = values(o, i, std=0.02)
+        z = lambda n: torch.empty(batch, 1, n, dtype=BF, device="cuda")      # noqa: E731
+        self.caches, self.xo, self.ro, self.q, self.a, self.h = values(2, batch, length, 2, dim), z(hidden), z(hidden), z(hidden), z(hidden), z(inter)
+        self.outs = [self.xo, self.ro, self.q, self.a, self.h]
+        self.caches_before = self.caches.clone()
+        self.ops = schedule_decode_layer_sm100(
+            layer_idx=0, batch=batch, seq_len=1, cache_pos=0, dynamic_position=True, weights=w, k_cache=self.caches[0], v_cache=self.caches[1],
+            x_in=values(batch, 1, hidden), residual_in=values(batch, 1, hidden, seed=5), x_out=self.xo, residual_out=self.ro, q_buf=self.q,
+            attn_out_buf=self.a, mlp_h_buf=self.h, eps=1e-5, hidden_size=hidden, intermediate_size=inter, num_q_heads=8, num_kv_heads=2,
+            head_dim=dim).ops
+
+    def clear(self):
+        for t in self.outs:
+            t.fill_(7)
+        self.caches.copy_(self.caches_before)
+
+    def untouched(self):
+        return all(bool((t == 7).all()) for t in self.outs) and torch.equal(self.caches, self.caches_before)
+
+
+@pytest.mark.parametrize("single", [False, True])
+@pytest.mark.parametrize("at", [(64,), (-1,), (3, 64)])
+def test_a_position_outside_the_cache_writes_nothing_and_is_counted(at, single):
+    layer, pos = Layer(), positions(*at)
+    mk = Megakernel(layer.ops, config=MegakernelConfig(position=pos, single_launch=single)).compile()
+    layer.clear()
+    with pytest.raises(RuntimeError, match="position"):
+        mk.run()
+    assert layer.untouched() and mk.launch_count() == 1
+    pos.fill_(3)
+    mk.run()
+    assert not any(bool((t == 7).all()) for t in layer.outs) and mk.launch_count() == 2
