@@ -144,11 +144,17 @@ __global__ void __launch_bounds__(kAtChainThreads<PARTS>, CTAS) at_chain_kernel(
     pos = reinterpret_cast<const volatile int32_t*>(L.pv.dyn_pos)[min(u.b, L.pv.pos_count - 1)];
     // every launch of the program sees a position outside the caches, and none runs
     bool bad = false;
-    for (int i = 0; i < L.pv.pos_count; ++i)
-      bad |= (uint32_t)reinterpret_cast<const volatile int32_t*>(L.pv.dyn_pos)[i] >= (uint32_t)L.pv.pos_limit;
+    int worst = 0;
+    for (int i = 0; i < L.pv.pos_count; ++i) {
+      const int v = reinterpret_cast<const volatile int32_t*>(L.pv.dyn_pos)[i];
+      if ((uint32_t)v >= (uint32_t)L.pv.pos_limit) bad = true, worst = v;
+    }
     if (bad) {
       prior_work_done();
-      if (threadIdx.x == 0) report(c, MK_ST_BAD_POSITION, pos, L.pv.pos_limit);
+      if (threadIdx.x == 0) {
+        if ((L.flags & kChainLast) && blockIdx.x == 0) L.pv.state->launches += 1;
+        report(c, MK_ST_BAD_POSITION, worst, L.pv.pos_limit);
+      }
       return;
     }
   }

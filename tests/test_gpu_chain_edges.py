@@ -60,3 +60,12 @@ def test_a_position_outside_the_cache_writes_nothing_and_is_counted(at, single):
     pos.fill_(3)
     mk.run()
     assert not any(bool((t == 7).all()) for t in layer.outs) and mk.launch_count() == 2
+
+
+def test_attention_alone_counts_a_run_that_found_a_bad_position():
+    q, o, k, pos = values(1, 1, 8, 64), torch.full((1, 1, 8, 64), 7, dtype=BF, device="cuda"), values(1, 64, 2, 64), positions(64)
+    ops = flash_decoding_schedule(q, k, k.clone(), o, kv_group_size=4, dynamic_len=True)[0]
+    mk = Megakernel(ops, config=MegakernelConfig(position=pos)).compile()
+    with pytest.raises(RuntimeError, match="position"):
+        mk.run()
+    assert mk.launch_count() == 1 and bool((o == 7).all())
