@@ -5,8 +5,9 @@ import pytest
 import torch
 
 from machete_b200.kernels.attention import flash_decoding_schedule
-from machete_b200.kernels.decode_matvec import schedule_decode_layer_sm100
-from machete_b200.megakernel import Megakernel, MegakernelConfig
+from machete_b200.kernels.decode_matvec import RmsVMatvecCacheSm100Op, schedule_decode_layer_sm100
+from machete_b200.kernels.decode_matvec.top1 import schedule_final_top1_sm100
+from machete_b200.megakernel import Megakernel, MegakernelConfig, OverlapTileScheduler
 
 pytestmark = pytest.mark.gpu
 BF = torch.bfloat16
@@ -69,3 +70,21 @@ def test_attention_alone_counts_a_run_that_found_a_bad_position():
     with pytest.raises(RuntimeError, match="position"):
         mk.run()
     assert mk.launch_count() == 1 and bool((o == 7).all())
+
+
+@pytest.mark.parametrize("single", [False, True])
+@pytest.mark.parametrize("start", [5, 15])
+def test_an_op_behind_the_feedback_sees_the_position_that_the_run_began_with(start, single):
+    hidden, vocab, length, dim = 256, 512, 16, 64
+    x, r, n, emb, pos = values(1, 1, hidden), values(1, 1, hidden, seed=4), values(hidden), values(vocab, hidden, std=0.05), positions(start)
+    tv, ti = torch.zeros(1, 1, device="cuda"), torch.zeros(1, 1, dtype=torch.int32, device="cuda")
+    ops = schedule_final_top1_sm100(x=x, residual_in=r, final_norm=n, lm_head=emb, top_values=tv, top_indices=ti, seq_len=1,
+                                    feedback=dict(embedding=emb, x_in=x, position=pos))
+    ops = list(ops[0] if isinstance(ops, tuple) else ops)
+    cache = torch.full((1, length, 2, dim), 7, dtype=BF, device="cuda")
+    ops += RmsVMatvecCacheSm100Op.schedule(x=x, residual_in=r, norm_weight=n, weight=values(2 * dim, hidden, std=0.05), cos=values(1, 32),
+                                           sin=values(1, 32), dst_cache=cache, dynamic_pos=True)
+    mk = Megakernel(ops, config=MegakernelConfig(position=pos, single_launch=single), scheduler=OverlapTileScheduler()).compile()
+    mk.run()
+    written = [t for t in range(length) if not bool((cache[0, t] == 7).all())]
+    assert written == [start] and int(pos.item()) == start + 1
