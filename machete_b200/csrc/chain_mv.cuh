@@ -824,15 +824,17 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
   ChainWalk walk;
   {
     const int tid = (int)threadIdx.x, m = tid & 31, chunks = K >> 3;
+    const int b = ROWS == 1 ? 0 : small_div(m, L.s_magic), t = ROWS == 1 ? 0 : m - b * sop->i[MK_MV_S];
     int pos = 0;
     if (L.pv.dyn_pos != nullptr) {
-      // one position per batch row, or one for all
+      // one position per sequence, or one for all; every launch looks at all of them
       prior_work_done();
-      pos = reinterpret_cast<const volatile int32_t*>(L.pv.dyn_pos)[min(m, L.pv.pos_count - 1)];
-      if (m < L.pv.pos_count && (uint32_t)pos >= (uint32_t)L.pv.pos_limit) c.ctrl->pos_bad = 1 + m;
-      if (tid < 32) c.ctrl->pos[m] = pos;
+      const volatile int32_t* at = reinterpret_cast<const volatile int32_t*>(L.pv.dyn_pos);
+      const int any = at[min(m, L.pv.pos_count - 1)];
+      pos = at[min(b, L.pv.pos_count - 1)];
+      if (m < L.pv.pos_count && (uint32_t)any >= (uint32_t)L.pv.pos_limit) c.ctrl->pos_bad = 1 + m;
+      if (tid < 32) c.ctrl->pos[m] = any;
     }
-    const int b = ROWS == 1 ? 0 : small_div(m, L.s_magic), t = ROWS == 1 ? 0 : m - b * sop->i[MK_MV_S];
 #pragma unroll 1
     for (int o = tid >> 5; o < L.n_ops; o += W)
       if (m < M) rows[o * 32 + m] = chain_row(ops + o, b, t, pos);

@@ -88,3 +88,15 @@ def test_an_op_behind_the_feedback_sees_the_position_that_the_run_began_with(sta
     mk.run()
     written = [t for t in range(length) if not bool((cache[0, t] == 7).all())]
     assert written == [start] and int(pos.item()) == start + 1
+
+
+@pytest.mark.parametrize("single", [False, True])
+def test_tokens_of_a_sequence_share_its_position(single):
+    hidden, length, dim = 256, 32, 64
+    x, r, n, pos = values(2, 3, hidden), values(2, 3, hidden, seed=4), values(hidden), positions(4, 20)
+    cache = torch.full((2, length, 2, dim), 7, dtype=BF, device="cuda")
+    ops = RmsVMatvecCacheSm100Op.schedule(x=x, residual_in=r, norm_weight=n, weight=values(2 * dim, hidden, std=0.05), cos=values(3, 32),
+                                          sin=values(3, 32), dst_cache=cache, dynamic_pos=True)
+    Megakernel(ops, config=MegakernelConfig(position=pos, single_launch=single)).run()
+    written = [[t for t in range(length) if not bool((cache[b, t] == 7).all())] for b in range(2)]
+    assert written == [[4, 5, 6], [20, 21, 22]]
