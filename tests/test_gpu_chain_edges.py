@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from machete_b200.kernels.attention import flash_decoding_schedule
-from machete_b200.kernels.decode_matvec import RmsVMatvecCacheSm100Op, schedule_decode_layer_sm100
+from machete_b200.kernels.decode_matvec import RmsQMatvecRopeSm100Op, RmsVMatvecCacheSm100Op, schedule_decode_layer_sm100
 from machete_b200.kernels.decode_matvec.top1 import schedule_final_top1_sm100
 from machete_b200.megakernel import Megakernel, MegakernelConfig, OverlapTileScheduler
 
@@ -100,3 +100,18 @@ def test_tokens_of_a_sequence_share_its_position(single):
     Megakernel(ops, config=MegakernelConfig(position=pos, single_launch=single)).run()
     written = [[t for t in range(length) if not bool((cache[b, t] == 7).all())] for b in range(2)]
     assert written == [[4, 5, 6], [20, 21, 22]]
+
+
+@pytest.mark.parametrize("single", [False, True])
+def test_every_op_of_a_group_leaves_its_residual(single):
+    hidden, dim = 256, 64
+    x, r, n, cos, sin = values(2, 1, hidden), values(2, 1, hidden, seed=4), values(hidden), values(1, 32), values(1, 32)
+    sums, q = torch.full((2, 2, 1, hidden), 7, dtype=BF, device="cuda"), torch.zeros(2, 2, 1, 2 * dim, dtype=BF, device="cuda")
+    cache = torch.zeros(2, 8, 2, dim, dtype=BF, device="cuda")
+    common = dict(x=x, residual_in=r, norm_weight=n, cos=cos, sin=sin)
+    ops = RmsVMatvecCacheSm100Op.schedule(weight=values(2 * dim, hidden), dst_cache=cache, cache_pos=3, **common)
+    for i in range(2):
+        ops += RmsQMatvecRopeSm100Op.schedule(weight=values(2 * dim, hidden), residual_out=sums[i], q=q[i], **common)
+    Megakernel(ops, config=MegakernelConfig(single_launch=single), scheduler=OverlapTileScheduler()).run()
+    want = (x.float() + r.float()).to(BF)
+    assert torch.equal(sums[0], want) and torch.equal(sums[1], want)
