@@ -125,6 +125,7 @@ __global__ void __launch_bounds__(kAtChainThreads<PARTS>, CTAS) at_chain_kernel(
     }
     c.ctrl->abort_flag = 0;
     c.ctrl->is_last = 0;
+    c.ctrl->pos_bad = launch_failed(L.pv);
     fence_mbar_init();
   }
   if (threadIdx.x < sizeof(mk_op_t) / 16)
@@ -133,6 +134,11 @@ __global__ void __launch_bounds__(kAtChainThreads<PARTS>, CTAS) at_chain_kernel(
   __syncthreads();
   const bool early = (L.flags & kChainEarlyLoads) != 0;
   if (!early) prior_work_done();
+  if (c.ctrl->pos_bad) {     // a launch before has failed
+    prior_work_done();
+    if ((L.flags & kChainLast) && blockIdx.x == 0 && threadIdx.x == 0) L.pv.state->launches += 1;
+    return;
+  }
   const mk_op_t* op = &c.ctrl->op_cache[0];
 
   AtUnit u = at_decode(op, (int)blockIdx.x);

@@ -28,7 +28,7 @@ static __global__ void __launch_bounds__(kEwWarps * 32) ew_chain_kernel(const __
     prior_work_done();
     return;
   }
-  if (threadIdx.x == 0) ctrl.abort_flag = ctrl.pos_bad = 0;
+  if (threadIdx.x == 0) ctrl.abort_flag = launch_failed(L.pv), ctrl.pos_bad = 0;
   if (threadIdx.x < sizeof(mk_op_t) / 16)
     reinterpret_cast<uint4*>(&rec)[threadIdx.x] = ldcg128(reinterpret_cast<const uint4*>(L.pv.ops + L.index) + threadIdx.x);
   __syncthreads();
@@ -40,12 +40,9 @@ static __global__ void __launch_bounds__(kEwWarps * 32) ew_chain_kernel(const __
       if (c.lane < L.pv.pos_count && (uint32_t)v >= (uint32_t)L.pv.pos_limit) ctrl.pos_bad = 1 + c.lane;
       ctrl.pos[c.lane] = v;
     }
-    // A wait that ran out in a launch before: no token is chosen or fed back and the position stays, as in the persistent
-    // kernel, where this op would not have run (a row of which no unit has left a maximum would name token -1).
-    if (rec.opcode == MK_OP_TOP1_FINAL) {
-      const int failed = *reinterpret_cast<volatile int32_t*>(&L.pv.state->abort_flag);
-      if (failed && c.lane == 0) ctrl.abort_flag = 1;
-    }
+    // The top-1 looks again, behind the wait: no token is chosen or fed back behind a launch that failed (a row of which no unit
+    // has left a maximum would name token -1)
+    if (rec.opcode == MK_OP_TOP1_FINAL && launch_failed(L.pv) && c.lane == 0) ctrl.abort_flag = 1;
     if ((L.flags & kChainLast) && blockIdx.x == 0 && c.lane == 0) L.pv.state->launches += 1;
   }
   __syncthreads();

@@ -81,6 +81,11 @@ __device__ __forceinline__ uint32_t lds64_lo_hi(uint32_t addr, uint32_t& hi) {
 }
 __device__ __forceinline__ uint4 ldcg128(const void* p) { return __ldcg(reinterpret_cast<const uint4*>(p)); }
 
+// Whether a wait has run out in a launch before: nothing runs any more then, as in the persistent kernel.  Every launch looks before it
+// waits for the one before, where it costs no time (behind that wait it cost a step 0.3 to 1 %); the launch that stands behind the
+// failed one already may have looked too early, and runs.  One thread of a CTA decides.
+__device__ __forceinline__ int launch_failed(const ProgramView& pv) { return *reinterpret_cast<const volatile int32_t*>(&pv.state->abort_flag); }
+
 // Row stride of the staged activations and the place of 16-byte chunk `ch` of row m.  Dense weights: as mv_row_stride.
 // NVFP4: the eight lanes of a shared-memory phase read two rows at four chunks that lie 128 bytes apart; the chunk
 // number's low bits, exclusive-or with which 128 bytes it lies in and with the row, keep the eight on different banks
@@ -816,9 +821,11 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
   }
 
   // ---- consumers
+  const int failed = threadIdx.x == 0 ? launch_failed(L.pv) : 0;
   for (int i = threadIdx.x; i < L.n_ops * (int)(sizeof(mk_op_t) / 16); i += W * 32)
     reinterpret_cast<uint4*>(ops)[i] = ldcg128(reinterpret_cast<const uint4*>(L.pv.ops + L.first_op) + i);
   named_bar_sync(kChainReady, kChainThreads<W>);      // the records, and the loader's barriers
+  if (failed) c.ctrl->pos_bad = -1;
   const mk_op_t* sop = ops + op0;
   const int K = sop->i[MK_MV_K], M = ROWS == 1 ? 1 : sop->i[MK_MV_M], Kc = sop->i[MK_MV_KC], pro = sop->i[MK_MV_PRO];
   ChainWalk walk;
@@ -854,9 +861,12 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
   prior_work_done();
   if ((L.flags & kChainLast) && blockIdx.x == 0 && threadIdx.x == 0) L.pv.state->launches += 1;
   if (bad) {
-    // a position outside the caches: nothing runs, the residual output included
+    // a position outside the caches, or a launch before has failed: nothing runs, the residual output included
     // (the report raises the abort flag, at which the loader stops)
-    if (threadIdx.x == 0) report(c, MK_ST_BAD_POSITION, c.ctrl->pos[bad - 1], L.pv.pos_limit);
+    if (threadIdx.x == 0) {
+      if (bad > 0) report(c, MK_ST_BAD_POSITION, c.ctrl->pos[bad - 1], L.pv.pos_limit);
+      else atomicExch(&c.ctrl->abort_flag, 1);
+    }
     return;
   }
   if (units > 0) {

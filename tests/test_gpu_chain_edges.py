@@ -5,7 +5,8 @@ import pytest
 import torch
 
 from machete_b200.kernels.attention import flash_decoding_schedule
-from machete_b200.kernels.decode_matvec import RmsQMatvecRopeSm100Op, RmsVMatvecCacheSm100Op, schedule_decode_layer_sm100
+from machete_b200.kernels.decode_matvec import (RmsKMatvecRopeCacheSm100Op, RmsQMatvecRopeSm100Op, RmsVMatvecCacheSm100Op,
+                                                schedule_decode_layer_sm100)
 from machete_b200.kernels.decode_matvec.top1 import schedule_final_top1_sm100
 from machete_b200.megakernel import Megakernel, MegakernelConfig, OverlapTileScheduler
 
@@ -115,3 +116,17 @@ def test_every_op_of_a_group_leaves_its_residual(single):
     Megakernel(ops, config=MegakernelConfig(single_launch=single), scheduler=OverlapTileScheduler()).run()
     want = (x.float() + r.float()).to(BF)
     assert torch.equal(sums[0], want) and torch.equal(sums[1], want)
+
+
+def test_nothing_runs_behind_a_launch_that_failed():
+    layer, pos = Layer(), positions(9)
+    mk = Megakernel(layer.ops, config=MegakernelConfig(position=pos)).compile()
+    layer.clear()
+    # a wait that ran out, as its launch leaves it: the status code and the abort flag (word 16) of the workspace
+    state = mk._workspace[(-mk._workspace.data_ptr()) % 256:][:256].view(torch.int32)
+    state[0], state[16] = 2, 1
+    with pytest.raises(RuntimeError, match="aborted"):
+        mk.run()
+    assert layer.untouched() and mk.launch_count() == 1
+    mk.run()
+    assert not any(bool((t == 7).all()) for t in layer.outs) and mk.launch_count() == 2
