@@ -119,7 +119,7 @@ class _RmsProjectionNvfp4Sm120Base(_Nvfp4Base):
         if dyn:
             nop.i[N.MV_DYNPOS] = (N.MV_DYN_TABLES if cls.apply_rope else 0) | (N.MV_DYN_OUT if cls.write_cache else 0)
             if cls.write_cache:
-                nop.pos_limit = int(t["dst_cache"].shape[1])
+                nop.pos_limit = int(t["dst_cache"].shape[1]) - int(t["x"].shape[1]) + 1     # (all of the S rows)
         if cls.write_cache:
             pos = int(sop.static_dims.get("cache_pos", 0))
             hi = int(t["dst_cache"].shape[1]) if dyn else pos + int(t["x"].shape[1])

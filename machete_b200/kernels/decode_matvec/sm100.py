@@ -126,7 +126,7 @@ class _RmsProjectionSm100Base(_DecodeMatvecSm100Base):
             # q lands in a one-token buffer: only its RoPE row follows the position
             nop.i[N.MV_DYNPOS] = N.MV_DYN_TABLES | (N.MV_DYN_OUT if cls.write_cache else 0)
             if cls.write_cache:
-                nop.pos_limit = int(t["dst_cache"].shape[1])
+                nop.pos_limit = int(t["dst_cache"].shape[1]) - int(t["x"].shape[1]) + 1     # (all of the S rows)
         if cls.write_cache:
             # only rows [cache_pos, cache_pos + S) of the cache are written (any row, with a dynamic position)
             pos = int(sop.static_dims.get("cache_pos", 0))

@@ -150,3 +150,12 @@ def test_the_layers_of_a_model_load_early():
     assert [p["kind"] for p in plan] == [N.LAUNCH_MATVEC, N.LAUNCH_ATTENTION] + 3 * [N.LAUNCH_MATVEC]
     assert [p["early"] for p in plan] == [0, 1, 1, 1, 1]
     assert (plan[1]["wait_lo"], plan[1]["wait_hi"], plan[1]["wait_dyn"]) == (90, 91, 0)
+
+
+@pytest.mark.parametrize("seq", [1, 3])
+def test_a_position_is_inside_only_if_every_token_of_the_step_is(seq):
+    x, cache = z(2, seq, HIDDEN), z(2, T, HKV, D)
+    ops = RmsVMatvecCacheSm100Op.schedule(x=x, residual_in=x.clone(), norm_weight=z(HIDDEN), weight=z(HKV * D, HIDDEN), cos=z(seq, D // 2),
+                                          sin=z(seq, D // 2), dst_cache=cache, dynamic_pos=True)
+    mk = Megakernel(ops, config=MegakernelConfig(position=torch.zeros(2, dtype=torch.int32)))
+    assert mk._tables()[0].position_limit == T - seq + 1
