@@ -989,7 +989,8 @@ struct mk_chain_variant {
   mk_chain_fn fn;
 };
 #define MK_CHAIN_KERNEL(ROWS, WF, AS, KS, W) {ROWS, AS, KS, W, mk::mv_chain_kernel<ROWS, WF, AS, KS, W>}
-#define MK_CHAIN_TABLE(name, WF)                                                                          \
+// (K blocks of up to 8 rows on eight warps: NVFP4 only, two CTAs a multiprocessor)
+#define MK_CHAIN_TABLE(name, WF, ...)                                                                     \
   extern "C" const mk_chain_variant* name(int* n) {                                                       \
     static const mk_chain_variant v[] = {                                                                 \
         MK_CHAIN_KERNEL(1, WF, 2, false, 8),   MK_CHAIN_KERNEL(1, WF, 4, false, 8),                       \
@@ -997,9 +998,8 @@ struct mk_chain_variant {
         MK_CHAIN_KERNEL(8, WF, 2, false, 16),  MK_CHAIN_KERNEL(8, WF, 4, false, 16),                      \
         MK_CHAIN_KERNEL(16, WF, 2, false, 16), MK_CHAIN_KERNEL(16, WF, 4, false, 16),                     \
         MK_CHAIN_KERNEL(32, WF, 2, false, 8),  MK_CHAIN_KERNEL(32, WF, 4, false, 8),                      \
-        MK_CHAIN_KERNEL(8, WF, 2, true, 8),    MK_CHAIN_KERNEL(8, WF, 2, true, 16),                       \
-        MK_CHAIN_KERNEL(16, WF, 2, true, 16),  MK_CHAIN_KERNEL(32, WF, 2, true, 8),                       \
-    };                                                                                                    \
+        MK_CHAIN_KERNEL(8, WF, 2, true, 16),   MK_CHAIN_KERNEL(16, WF, 2, true, 16),                      \
+        MK_CHAIN_KERNEL(32, WF, 2, true, 8),   ##__VA_ARGS__};                                            \
     *n = (int)(sizeof(v) / sizeof(v[0]));                                                                 \
     return v;                                                                                             \
   }
