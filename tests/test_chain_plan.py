@@ -7,7 +7,7 @@ import torch
 
 from machete_b200 import _native as N
 from machete_b200.kernels.attention import flash_decoding_schedule
-from machete_b200.kernels.decode_matvec import (RmsKMatvecRopeCacheSm100Op, RmsQMatvecRopeSm100Op, RmsVMatvecCacheSm100Op,
+from machete_b200.kernels.decode_matvec import (MatvecSm100Op, RmsKMatvecRopeCacheSm100Op, RmsQMatvecRopeSm100Op, RmsVMatvecCacheSm100Op,
                                                 schedule_decode_layer_sm100)
 from machete_b200.megakernel import Megakernel, MegakernelConfig, OverlapTileScheduler
 
@@ -159,3 +159,13 @@ def test_a_position_is_inside_only_if_every_token_of_the_step_is(seq):
                                           sin=z(seq, D // 2), dst_cache=cache, dynamic_pos=True)
     mk = Megakernel(ops, config=MegakernelConfig(position=torch.zeros(2, dtype=torch.int32)))
     assert mk._tables()[0].position_limit == T - seq + 1
+
+
+# eight dense rows that leave a ring of at most four pages, and of more, by their length and by the length of a page
+@pytest.mark.parametrize("rows,k,out,page_k,warps,ring", [(3, 14336, 4096, 1024, 8, 3), (8, 4608, 8192, 1024, 8, 4), (8, 3072, 8192, 1024, 16, 5),
+                                                          (3, 14336, 4096, 512, 16, 7), (1, 4096, 14336, 1024, 8, 6), (16, 1024, 1024, 1024, 16, 1),
+                                                          (17, 1024, 4096, 1024, 8, 2)])
+def test_warps_follow_the_ring(rows, k, out, page_k, warps, ring):
+    ops = MatvecSm100Op.schedule(a=z(1, rows, k), weight=z(out, k), y=z(1, rows, out))
+    launch, = Megakernel(ops, config=MegakernelConfig(native_kc=page_k)).launch_plan()
+    assert (launch["warps"], launch["stages"]) == (warps, ring)
