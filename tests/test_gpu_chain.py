@@ -5,6 +5,7 @@ import threading
 import pytest
 import torch
 
+from machete_b200 import _native as N
 from machete_b200.kernels.attention import flash_decoding_schedule
 from machete_b200.kernels.decode_matvec import (MatvecNvfp4Sm120Op, MatvecResidualNvfp4Sm120Op, MatvecResidualSm100Op,
                                                 MatvecSm100Op, RmsGateUpSiluNvfp4Sm120Op, RmsGateUpSiluSm100Op,
@@ -31,9 +32,9 @@ class Values:
         return w if fmt in ("bf16", "fp16") else quantize_nvfp4_weight(w, group_size=16 if fmt == "nvfp4" else 32)
 
 
-def equal_forms(ops, outs, launches=1, **config):
+def equal_forms(ops, outs, launches=1, attention=None, **config):
     """Both forms, three launches each (the arrival counts and slots they leave behind included), from the same buffers.
-    `launches`: at least so many kernels in the chain (one may be the persistent kernel, for what a chain cannot run)."""
+    `launches`: at least so many kernels in the chain; `attention`: participants and CTAs a multiprocessor of its attention launch."""
     start, got = [t.clone() for t in outs], []
     for single in (True, False):
         for t, s in zip(outs, start):
@@ -41,7 +42,10 @@ def equal_forms(ops, outs, launches=1, **config):
         mk = Megakernel(ops, config=MegakernelConfig(single_launch=single, **config), scheduler=OverlapTileScheduler()).compile()
         for _ in range(3):
             mk.run()
-        assert mk.launches_per_run == 1 if single else mk.launches_per_run >= launches
+        plan = mk.launch_plan()
+        assert mk.launches_per_run == max(1, len(plan)) and (len(plan) == 0 if single else len(plan) >= launches)
+        if attention and not single:
+            assert [(p["warps"], p["per_sm"]) for p in plan if p["kind"] == N.LAUNCH_ATTENTION] == [attention]
         assert mk.launch_count() == 3 and not mk.read_counters().any()
         got.append([t.clone() for t in outs])
     for a, b in zip(*got):
@@ -92,20 +96,35 @@ def test_normalised_rows_and_pairs(fmt, rows, k, inter):
     assert equal_forms(ops, [y])[0].float().abs().sum() > 0
 
 
-@pytest.mark.parametrize("batch,kv,heads,kv_heads,dim,splits,causal,m", [
-    (1, 1, 8, 8, 64, 0, False, 1), (1, 300, 32, 8, 64, 0, False, 1), (2, 65, 16, 1, 128, 3, False, 1), (3, 1930, 32, 4, 128, 0, False, 1),
-    (1, 2000, 8, 2, 64, 128, False, 1), (1, 700, 8, 4, 128, 40, True, 16), (2, 130, 4, 4, 64, 64, True, 5), (8, 4096, 32, 8, 128, 0, False, 1),
+# (participants, CTAs a multiprocessor) of the launch on 148 multiprocessors
+@pytest.mark.parametrize("batch,kv,heads,kv_heads,dim,splits,causal,m,form", [
+    (1, 1, 8, 8, 64, 0, False, 1, (7, 2)), (1, 300, 32, 8, 64, 0, False, 1, (7, 2)), (2, 65, 16, 1, 128, 3, False, 1, (7, 2)),
+    (3, 1930, 32, 4, 128, 0, False, 1, (7, 2)), (1, 2000, 8, 2, 64, 128, False, 1, (7, 2)), (1, 700, 8, 4, 128, 40, True, 16, (4, 3)),
+    (2, 130, 4, 4, 64, 64, True, 5, (7, 2)), (8, 4096, 32, 8, 128, 0, False, 1, (7, 2)),
     # units of one to four pages in one, two and more waves of two, three and four CTAs a multiprocessor
-    (13, 500, 8, 8, 64, 4, False, 1), (11, 701, 32, 8, 64, 8, False, 1), (16, 1931, 16, 8, 64, 8, False, 1), (20, 250, 16, 8, 64, 2, True, 2),
-    (12, 380, 32, 8, 128, 4, False, 1), (16, 129, 8, 8, 128, 4, False, 1)])
+    (13, 500, 8, 8, 64, 4, False, 1, (4, 3)), (11, 701, 32, 8, 64, 8, False, 1, (4, 3)), (16, 1931, 16, 8, 64, 8, False, 1, (4, 4)),
+    (20, 250, 16, 8, 64, 2, True, 2, (4, 3)), (12, 380, 32, 8, 128, 4, False, 1, (4, 3)), (16, 129, 8, 8, 128, 4, False, 1, (7, 2))])
 @pytest.mark.parametrize("fuse", [True, False])
-def test_attention(batch, kv, heads, kv_heads, dim, splits, causal, m, fuse):
+def test_attention(batch, kv, heads, kv_heads, dim, splits, causal, m, form, fuse):
     v = Values(kv + dim)
     q, o = v(batch, m, heads, dim), torch.zeros(batch, m, heads, dim, dtype=BF, device="cuda")
     k, vv = v(batch, kv + 3, kv_heads, dim)[:, :kv], v(batch, kv, kv_heads, dim)
     ops, _ = flash_decoding_schedule(q, k, vv, o, num_splits=splits, causal=causal, kv_group_size=heads // kv_heads)
     lse = ops[1].tensor_refs["lse"]
-    assert equal_forms(ops, [o, lse], fuse=fuse)[0].float().abs().sum() > 0
+    assert equal_forms(ops, [o, lse], attention=form, fuse=fuse)[0].float().abs().sum() > 0
+
+
+# every kernel with the fused q/k norm; the new token in the first page, a middle one and the last
+@pytest.mark.parametrize("batch,kv,heads,kv_heads,dim,splits,new,form", [
+    (2, 300, 32, 8, 64, 0, 299, (7, 2)), (13, 500, 8, 8, 64, 4, 0, (4, 3)), (16, 1931, 16, 8, 64, 8, 1000, (4, 4)),
+    (3, 1930, 32, 4, 128, 0, 1929, (7, 2)), (12, 380, 32, 8, 128, 4, 190, (4, 3))])
+def test_attention_that_normalises(batch, kv, heads, kv_heads, dim, splits, new, form):
+    v = Values(kv + dim)
+    q, o = v(batch, 1, heads, dim), torch.zeros(batch, 1, heads, dim, dtype=BF, device="cuda")
+    k, vv = v(batch, kv, kv_heads, dim), v(batch, kv, kv_heads, dim)
+    norm = dict(q_weight=1 + v(dim, std=0.02), k_weight=1 + v(dim, std=0.02), cos=v(dim // 2), sin=v(dim // 2), new_token=new)
+    ops, _ = flash_decoding_schedule(q, k, vv, o, num_splits=splits, kv_group_size=heads // kv_heads, qk_norm=norm)
+    assert equal_forms(ops, [o, k], attention=form)[0].float().abs().sum() > 0
 
 
 def layer_weights(v, fmt, hidden, inter, heads, kv_heads, dim, kv):
@@ -275,6 +294,28 @@ def test_every_row_class_has_its_kernel(fmt, rows, k, out):
         else:
             ops += MatvecSm100Op.schedule(a=a, weight=w, y=b)
     assert equal_forms(ops, [y, z], launches=2)[1].float().abs().sum() > 0
+
+
+# every kernel with the sum of K blocks: the blocks of a product in one launch; (activation rows, consumer warps) of its kernel
+@pytest.mark.parametrize("fmt,rows,k,out,form", [
+    ("bf16", 4, 28672, 520, (8, 16)), ("bf16", 12, 8192, 520, (16, 16)), ("bf16", 20, 4096, 520, (32, 8)),
+    ("fp16", 4, 28672, 520, (8, 16)), ("fp16", 12, 8192, 520, (16, 16)), ("fp16", 20, 4096, 520, (32, 8)),
+    ("nvfp4", 1, 4096, 520, (8, 16)), ("nvfp4", 4, 4096, 2400, (8, 8)), ("nvfp4", 12, 4096, 520, (16, 16)), ("nvfp4", 20, 4096, 520, (32, 8))])
+def test_k_blocks_side_by_side(fmt, rows, k, out, form):
+    v = Values(rows + k)
+    dtype = torch.float16 if fmt == "fp16" else BF
+    a, y, ops, step = v(rows, 1, k, dtype=dtype), torch.zeros(rows, 1, out, dtype=dtype, device="cuda"), [], k // 4
+    for b in range(4):
+        part, sums = a[..., b * step:(b + 1) * step], dict(residual_in=y, residual_out=y) if b else dict(y=y)
+        w = v.weight(fmt, out, step)
+        if fmt == "nvfp4":
+            cls = MatvecResidualNvfp4Sm120Op if b else MatvecNvfp4Sm120Op
+            ops += cls.schedule(a=part, weight_packed=w.packed, weight_scales=w.scales, group_size=16, global_scale=w.global_scale, **sums)
+        else:
+            ops += (MatvecResidualSm100Op if b else MatvecSm100Op).schedule(a=part, weight=w, **sums)
+    launch, = Megakernel(ops, scheduler=OverlapTileScheduler()).launch_plan()
+    assert launch["n_ops"] == 4 and (launch["rows"], launch["warps"]) == form
+    assert equal_forms(ops, [y])[0].float().abs().sum() > 0
 
 
 def test_no_token_is_fed_back_after_a_failed_launch():
