@@ -2,7 +2,8 @@
 """Benchmark of the decode-step megakernel.
 
 Headline workload (``config.workload``): the full 16-layer Llama-3.2-1B-shape
-decode step as one persistent kernel — hidden 2048, 32 query / 8 KV heads,
+decode step, run as a chain of kernels (tensor parallel: as one persistent
+kernel) — hidden 2048, 32 query / 8 KV heads,
 head_dim 64, GLU intermediate 8192, tied 128256-vocab LM head with the greedy
 token computed in the kernel, random-init bf16 weights ~N(0, 0.02), decode
 batch 1, KV length 4096.  A "step" is one run of the program = one token per sequence.
@@ -752,7 +753,7 @@ def main():
     mk, cfg, tp, B, bf = w.mk, w.cfg, w.tp, args.batch, torch.bfloat16
 
     if args.stage_trace:
-        # per-op timeline of ONE traced launch (tracing costs a few stores per page: the untraced time is
+        # per-op timeline of ONE traced launch, of the persistent kernel, which runs a program while a trace is attached (tracing costs a few stores per page: the untraced time is
         # printed beside it); rank 0 only
         for _ in range(5):
             mk.run()
@@ -872,6 +873,7 @@ def main():
                          "traffic": int(w.alg_bytes * NCU_TRAFFIC_RATIO),
                          "traffic_from": "ncu dram bytes of a 4-layer capture x layers (profiles/), not this run"},
             "clocks": clocks, "e2e": e2e, "gpu_launches": args.steps * blocks * w.mk.launches_per_run,
+            # of the program's single-launch form; a chain's kernels have their own (Megakernel.launch_plan)
             "kernel_config": {"ctas": mk.grid[0], "threads": mk.block[0], "smem": mk.smem_size, "pages": mk.num_pages,
                               "page_bytes": mk.page_bytes, "instructions": mk.total_tiles,
                               "counters": mk.num_barriers, "scheduler": args.scheduler},

@@ -6,8 +6,9 @@
  * `class Megakernel`, `.compile()` :1594, `.run()` :2183) and of the CuTe-DSL
  * op bodies it JIT-compiles.  Host code (Python via ctypes, or any C caller)
  * describes a decode step as a *program*: a table of op records, a per-CTA
- * instruction list, dependency-counter wait tables and op-entry events.  One
- * persistent kernel (one CTA per SM) executes the whole program per launch.
+ * instruction list, dependency-counter wait tables and op-entry events.  A run is
+ * a chain of kernels, one for each op or for ops that go together, or one launch
+ * of a persistent kernel (one CTA per SM) that executes the whole program.
  *
  * Ownership: the caller owns every buffer.  `mk_create` copies the program
  * tables into a caller-provided device workspace; no entry point allocates or
@@ -395,8 +396,9 @@ int mk_status(mk_handle_t h, int32_t out[16]);
 /* The same status block read straight from a workspace (it sits at offset
  * 0): for the standalone entry points, which hand out no handle. */
 int mk_workspace_status(const void* workspace, int32_t out[16]);
-/* Attach (or, with buffer == NULL, detach) a device buffer that the kernel
- * fills with 16-byte {globaltimer ns, code, arg} records, `records_per_warp`
+/* Attach (or, with buffer == NULL, detach) a device buffer that the persistent
+ * kernel, which runs every program while one is attached (a chain records
+ * nothing), fills with 16-byte {globaltimer ns, code, arg} records, `records_per_warp`
  * per warp of every CTA (9 warps: loader first), followed by one int32 record
  * count per warp.  Needs n_ctas * 9 * (records_per_warp * 16 + 4) bytes.
  * Takes the place of the reference's cutedsl-trace lanes

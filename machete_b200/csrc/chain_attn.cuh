@@ -4,7 +4,7 @@
 // What a launch of one token's attention is bound by, besides the cache's bytes, is what follows the last page: the states of
 // up to seven warps are merged, the partial goes to memory and the last CTA of a (batch, KV head) group combines the
 // group's splits.  The persistent kernel does each of these on one warp (12 us of a layer's 20 at head dim 128, 8192 tokens);
-// here all eight warps of the CTA share them: a merge takes n-tiles of the output in turn, a combine pairs of values, and
+// here all warps of the CTA, the loader's included, share them: a merge takes n-tiles of the output in turn, a combine pairs of values, and
 // neither changes the order of any sum.  The cache does not depend on the kernel before, except for the rows that it
 // appends: the loader fills the ring before it waits, and waits at the first page that holds such a row.  The query rows go
 // through shared memory, normalised and rotated once for all warps, which also leaves 128 registers a thread enough for

@@ -99,7 +99,7 @@ __device__ __forceinline__ uint32_t chain_chunk(int m, int ch) {
 
 // ---- staging -------------------------------------------------------------------------
 // The sums of squares are those of mv_stage: its 224 threads take chunks tid, tid + 224, ... of a row, and a warp's sum
-// goes to red[row * 7 + warp].  Here (row, one of those seven warps) is a job, and the eight warps take jobs in turn, R at
+// goes to red[row * 7 + warp].  Here (row, one of those seven warps) is a job, and the W warps take jobs in turn, R at
 // a time, so that a batch's rows are requested together.
 template <int ROWS, int WF, int R, int H, int W>
 __device__ __forceinline__ void chain_stage_rms(Ctx& c, const mk_op_t* op, const ChainIn* in, const mk_op_t* res_op) {
@@ -205,7 +205,7 @@ __device__ __forceinline__ void chain_stage_rms(Ctx& c, const mk_op_t* op, const
   }
 }
 
-// Without a prologue: thread `tid` takes 16-byte chunks tid, tid + 256, ... of all rows laid end to end: (m0, ch0) is its
+// Without a prologue: thread `tid` takes 16-byte chunks tid, tid + (the CTA's consumer threads), ... of all rows laid end to end: (m0, ch0) is its
 // first, and each step is (dm, dch) on.
 struct ChainWalk {
   int m0, ch0, dm, dch;
@@ -548,8 +548,7 @@ __device__ __forceinline__ ChainRow chain_row(const mk_op_t* op, int b, int t, i
 }
 
 // mv_epilogue for results that are stored.  What an op asks for is asked once, around loops over the rows that are unrolled
-// and hold no branch: one warp runs this for a unit, and for a launch of a unit or two a CTA it is the launch's end (a branch
-// a row and choice: some 350 cycles a row of every lane).
+// and hold no branch: one warp runs this for a unit, and for a launch of a unit or two a CTA it is the launch's end.
 template <int ROWS, int WF>
 __device__ __forceinline__ void chain_epilogue(Ctx& c, const mk_op_t* op, const ChainRow* rows, const ChainUnit& r,
                                                const float (&sum)[chain_nt(ROWS)][4]) {
@@ -892,7 +891,7 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
   constexpr int NA = Cut::NA, AN = Cut::AN, NN = Cut::NN;
   float4* slots = reinterpret_cast<float4*>(smem + L.slot_off);
   uint32_t slot = 0, k = 0;          // the page's place in the ring, and pages in its slot before it
-  int turn = c.warp;                 // this warp less the warp whose turn the unit's first page is, mod 8
+  int turn = c.warp;                 // this warp less the warp whose turn the unit's first page is, mod W
   for (int u = 0; u < units && !c.dead; ++u) {
     const uint32_t set = (uint32_t)u & ((1u << L.sets_log2) - 1u), gen = (uint32_t)u >> L.sets_log2;
     float4* mine = slots + (size_t)set * (uint32_t)(parts * NA * NT) * 32u + c.lane;

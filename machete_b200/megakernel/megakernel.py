@@ -111,7 +111,7 @@ def _device_index(device) -> int:
 
 
 class Megakernel:
-    """A decode-step program for the persistent sm_100a kernel.
+    """A decode-step program for the sm_100a kernels.
 
     Args:
         ops: list of ``ScheduledOp`` in program order.
@@ -432,7 +432,10 @@ class Megakernel:
                    6: "unit_end", 7: "event_begin", 8: "event_deps", 9: "event_end", 10: "lwait_done"}
 
     def enable_trace(self, records_per_warp: int = 4096) -> None:
-        """Record globaltimer-stamped events of every warp on the next launches.
+        """Record globaltimer-stamped events of every warp on the next launches, which are those of the persistent kernel.
+
+        A program that runs as a chain of kernels runs on the persistent kernel while a trace is attached: the records say
+        nothing of the chain (see :meth:`launch_plan` for its launches).
 
         The counterpart of ``MegakernelConfig.tracing`` in the reference
         (megakernel/tracing.py:51-153); costs a few global stores per page, so
@@ -506,7 +509,7 @@ class Megakernel:
             json.dump({"traceEvents": events}, fh)
 
     def stage_table(self) -> list:
-        """Where the last traced launch spent its time, op by op (microseconds from the first record).
+        """Where the last traced launch (of the persistent kernel) spent its time, op by op (microseconds from the first record).
 
         One dict per native op: ``begin`` = first unit started on any CTA, ``end`` = last unit
         signalled, ``gap`` = begin minus the latest end of any earlier op (negative when ops overlap),
