@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(kThreads, 1) mk_persistent_kernel(const __grid
   c.dead = false;
   trace_init<(FEAT & MK_F_TRACE) != 0, kWideStep<NTC, WFC, FEAT>>(c);
 
-  if (pv.plan_now != nullptr && plan_in_force(pv)) {   // the chain in front of this launch has run the program
+  if (pv.plan >= 0 && plan_in_force(pv)) {   // the chain in front of this launch has run the program
     prior_work_done();
     return;
   }

@@ -892,6 +892,8 @@ static int create_program(const mk_program_t* prog, mk_handle_t* out, bool strea
   h->pv.waits = reinterpret_cast<const mk_wait_t*>(ws + l.waits);
   h->pv.counters = reinterpret_cast<int32_t*>(ws + l.counters);
   h->pv.state = reinterpret_cast<DeviceState*>(ws + l.state);
+  h->pv.plan_now = &h->pv.state->plan;
+  h->pv.plan = -1;
   h->pv.n_counters = prog->n_counters;
   h->pv.n_pages = prog->n_pages;
   h->pv.page_bytes = prog->page_bytes;
@@ -959,8 +961,7 @@ static int run_program(mk_handle_s* h, cudaStream_t stream) {
   if (persistent) return launch_persistent(h, pv, stream);
   // a chain is its kernels, and the persistent kernel for records that those cannot run
   pv.plan = h->plan;
-  pv.plan_now = &reinterpret_cast<DeviceState*>(h->ws + h->layout.state)->plan;
-  const int rc = launch_chain(plan->steps, stream, pv.plan_now, pv.plan);
+  const int rc = launch_chain(plan->steps, stream, h->plan);
   return rc ? rc : launch_persistent(h, pv, stream);
 }
 

@@ -89,12 +89,12 @@ struct ProgramView {
   int32_t pos_count;       // entries behind dyn_pos: 1 (one position for every batch row) or one per row (<= 32)
   // A chain that a caller captured holds the launches of one plan, and the persistent kernel behind them: where a replaced record has
   // made another plan of the program since, the chain's launches end at once, else the persistent kernel does.
-  int32_t plan;             // this launch's
-  const int32_t* plan_now;  // the one in force; null: this launch runs
+  int32_t plan;             // this launch's; -1: it runs whatever the plan in force is
+  const int32_t* plan_now;  // the one in force; of every launch a valid address, so that a load that is moved in front of its test does no harm
 };
 
 __device__ __forceinline__ bool plan_in_force(const ProgramView& pv) {
-  return pv.plan_now == nullptr || *reinterpret_cast<const volatile int32_t*>(pv.plan_now) == pv.plan;
+  return pv.plan < 0 || *reinterpret_cast<const volatile int32_t*>(pv.plan_now) == pv.plan;
 }
 
 // One trace event: a globaltimer stamp, an event code and an argument.
