@@ -29,9 +29,7 @@ constexpr int kChainOps = 8;                          // ops of one launch: Q, K
 constexpr int kChainMaxStages = 12;
 
 enum { kChainEarlyLoads = 1,   // the weights may be read before the kernel before has finished
-       kChainLast = 2,         // the program's last launch: counts it
-       kChainSpread = 4,       // the partial sums of a unit are dealt to different warps
-       kChainResShift = 8 };
+       kChainLast = 2 };       // the program's last launch: counts it
 
 struct ChainHead {             // what the loader needs to know of an op: it does not wait for the records
   int64_t out_h;                 // output stride of a head
@@ -45,14 +43,18 @@ struct MvLaunch {
   int32_t unit_end[kChainOps];     // units of ops 0..i
   int32_t cta_end[kChainOps];      // K blocks: CTAs of blocks 0..i; zero where the ops share the CTAs and what they stage
   int32_t pages[kChainOps], parts[kChainOps];   // pages of a unit, and the partial sums they meet in
-  int32_t n_ops, flags, first_op;               // flags: kChain..., and from bit kChainResShift on 1 + the op whose residual_out this launch writes
+  int32_t spread;                               // the partial sums of a unit are dealt to different warps
+  int32_t n_ops, flags, res_op, first_op;       // res_op: the op whose residual_out this launch writes, or -1
   int32_t stages, page_bytes, sets_log2;        // ring slots, and sets of slots for partial sums
   int32_t slot_off, act_off, page_off;          // shared memory, bytes
   // n / d as (n * magic) >> 22 for the small numbers here: rows by tokens a sequence, threads by 16-byte chunks of a row
   int32_t s_magic, chunk_magic[kChainOps];
+  int32_t pad[12];
 };
 // What a launch costs the host goes by where its parameters end: 24 or 32 bytes behind a multiple of 64 2.0 us, elsewhere 2.4 (driver 580,
-// 488 to 768 bytes, the stream idle; 16 x 1024 -> 1024 through Megakernel.run 5.2 us a pass with 608 bytes, 5.7 with 616).
+// 488 to 768 bytes, the stream idle; 16 x 1024 -> 1024 through Megakernel.run 5.3 us a pass with 600 bytes, 5.7 with 616).  Hence the pad:
+// fields of 16 bits or in one word with the flags, which make it 608, cost the kernels registers (1B shape batch 1 689 to 694 us,
+// 8B NVFP4 batch 1 2250 to 2272).
 static_assert(sizeof(MvLaunch) % 64 == 24 || sizeof(MvLaunch) % 64 == 32, "a launch with these parameters costs the host 0.4 us more");
 
 // What a CTA works out once, while it waits for the kernel before, so that no division and no chain of loads stands on the
@@ -758,8 +760,7 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
   const int units = local < total ? (total - local + count - 1) / count : 0;
   const int P = L.pages[op0], parts = L.parts[op0];
   // pages of a unit go to AS warps each, or all of them to the same AS
-  const bool spread = (L.flags & kChainSpread) != 0;
-  const int step = spread ? AS : 0, arrivals = spread ? parts * AS : AS, last_pages = spread ? parts : 1;
+  const int step = L.spread ? AS : 0, arrivals = L.spread ? parts * AS : AS, last_pages = L.spread ? parts : 1;
 
   const bool early = (L.flags & kChainEarlyLoads) != 0;
   if (c.warp == W) {
@@ -850,7 +851,7 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
     for (int o = tid >> 5; o < L.n_ops; o += W)
       if (m < M) rows[o * 32 + m] = chain_row(ops + o, b, t, pos);
     if (tid < M) {
-      const mk_op_t* ro = ops + max((L.flags >> kChainResShift) - 1, 0);
+      const mk_op_t* ro = ops + max(L.res_op, 0);
       tab.in[m].x = b * sop->s[MK_MV_S_X_B] + t * sop->s[MK_MV_S_X_S];
       tab.in[m].ri = b * sop->s[MK_MV_S_RI_B] + t * sop->s[MK_MV_S_RI_S];
       tab.in[m].ro = b * ro->s[MK_MV_S_RO_B] + t * ro->s[MK_MV_S_RO_S];
@@ -874,7 +875,7 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
     return;
   }
   if (units > 0) {
-    const mk_op_t* res_op = (L.flags >> kChainResShift) > 0 && blockIdx.x == 0 ? ops + (L.flags >> kChainResShift) - 1 : nullptr;
+    const mk_op_t* res_op = L.res_op >= 0 && blockIdx.x == 0 ? ops + L.res_op : nullptr;
     if (pro == MK_PRO_NONE) {
       chain_stage_plain<WF>(c, sop, M, tab.in, walk);
     } else if constexpr (WF != 1) {
@@ -979,7 +980,7 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
       }
     }
     // (dealt out: one more, as the warps of a unit's last page arrive last and one of them adds the unit up)
-    turn = (turn - (spread ? arrivals + 1 : AS)) & (W - 1);
+    turn = (turn - (L.spread ? arrivals + 1 : AS)) & (W - 1);
   }
 }
 
