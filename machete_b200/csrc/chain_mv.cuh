@@ -51,8 +51,8 @@ struct MvLaunch {
   int32_t s_magic, chunk_magic[kChainOps];
   int32_t pad[12];
 };
-// What a launch costs the host goes by where its parameters end: 24 or 32 bytes behind a multiple of 64 2.0 us, elsewhere 2.4 (driver 580,
-// 488 to 768 bytes, the stream idle; 16 x 1024 -> 1024 through Megakernel.run 5.3 us a pass with 600 bytes, 5.7 with 616).  Hence the pad:
+// What a launch costs the host goes by where its parameters end: 24 or 32 bytes behind a multiple of 64 2.0 us, elsewhere 2.4 (NVIDIA
+// driver 580, 488 to 768 bytes, the stream idle; 16 x 1024 -> 1024 through Megakernel.run 5.3 us a pass with 600 bytes, 5.7 with 616).  Hence the pad:
 // fields of 16 bits or in one word with the flags, which make it 608, cost the kernels registers (1B shape batch 1 689 to 694 us,
 // 8B NVFP4 batch 1 2250 to 2272).
 static_assert(sizeof(MvLaunch) % 64 == 24 || sizeof(MvLaunch) % 64 == 32, "a launch with these parameters costs the host 0.4 us more");

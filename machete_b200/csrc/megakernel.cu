@@ -1115,6 +1115,7 @@ static int update_op(mk_handle_s* h, int32_t op_index, const mk_op_t* op, void* 
   std::lock_guard<std::mutex> one(h->planning);
   const mk_op_t before = h->ops[op_index];
   h->ops[op_index] = rec;
+  const int plan_before = h->plan;
   bool replan = !chain_alike(before, rec);
   if (replan) ++h->plan;
   if (rec.opcode == MK_OP_ATTN_SPLIT) replan |= most_pages_of(before, h->pv.page_bytes) != most_pages_of(rec, h->pv.page_bytes);
@@ -1139,7 +1140,8 @@ static int update_op(mk_handle_s* h, int32_t op_index, const mk_op_t* op, void* 
       CUDA_TRY(cudaMemcpyAsync(h->ws + h->layout.instrs + lo * sizeof(mk_instr_t), h->instrs.data() + lo, (hi - lo) * sizeof(mk_instr_t),
                                cudaMemcpyHostToDevice, st));
   }
-  CUDA_TRY(cudaMemcpyAsync(h->ws + h->layout.state + offsetof(DeviceState, plan), &h->plan, sizeof(int32_t), cudaMemcpyHostToDevice, st));
+  if (h->plan != plan_before)
+    CUDA_TRY(cudaMemcpyAsync(h->ws + h->layout.state + offsetof(DeviceState, plan), &h->plan, sizeof(int32_t), cudaMemcpyHostToDevice, st));
   // the host buffers above must outlive the copies
   CUDA_TRY(cudaStreamSynchronize(st));
   // a changed batch size or weight format may need another kernel variant
