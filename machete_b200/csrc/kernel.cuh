@@ -518,7 +518,10 @@ __global__ void __launch_bounds__(kThreads, 1) mk_persistent_kernel(const __grid
   c.dead = false;
   trace_init<(FEAT & MK_F_TRACE) != 0, kWideStep<NTC, WFC, FEAT>>(c);
 
-  if (pv.plan >= 0 && plan_in_force(pv)) {   // the chain in front of this launch has run the program
+  if (pv.plan >= 0 && plan_in_force(pv)) {
+    // The chain in front of this launch has run the program.  The next launch is let in at once (it waits for this one, and so for
+    // the chain): 16 x 1024 -> 1024, captured runs back to back, 6.1 us a run without, 5.0 so.
+    next_may_start();
     prior_work_done();
     return;
   }
