@@ -755,7 +755,8 @@ static void set_windows(std::vector<mk_op_t>& ops, const mk::ChainTables& t, int
 }
 
 // The instruction rows of op `i` from its record: page counts, the fast path, and for attention what the loads wait for, which
-// follows the rows that are appended.  [*lo, *hi): the span of the table that holds them.
+// follows the rows that are appended.  [*lo, *hi): the span of the table that holds those that changed (an op's rows lie all over a table
+// of megabytes, and a new position or pointer mostly changes none).
 static void refresh_rows(mk_handle_s* h, int i, size_t* lo, size_t* hi) {
   const mk_op_t& op = h->ops[i];
   const mk::WaitList list = h->loader_lists.empty() ? mk::WaitList{} : h->loader_lists[i];
@@ -765,6 +766,7 @@ static void refresh_rows(mk_handle_s* h, int i, size_t* lo, size_t* hi) {
   for (size_t j = 0; j < h->instrs.size(); ++j) {
     mk_instr_t& in = h->instrs[j];
     if (in.op != i) continue;
+    const mk_instr_t before = in;
     if (op.opcode == MK_OP_MATVEC) in.n_pages = mk::matvec_pages(op);
     else if (attention) in.n_pages = mk::attn_pages(op, in.unit, h->pv.page_bytes);
     mk::fill_instr_fast_path(in, op, (uint64_t)(h->ws + h->layout.tmaps), h->pv.page_bytes, h->pv.n_pages);
@@ -774,6 +776,7 @@ static void refresh_rows(mk_handle_s* h, int i, size_t* lo, size_t* hi) {
       in.n_lwaits = waits ? list.n : 0;
       in.lwait_off = waits ? list.off : 0;
     }
+    if (memcmp(&before, &in, sizeof(in)) == 0) continue;
     *lo = std::min(*lo, j);
     *hi = std::max(*hi, j + 1);
   }
@@ -1133,7 +1136,7 @@ static int update_op(mk_handle_s* h, int32_t op_index, const mk_op_t* op, void* 
   CUDA_TRY(cudaMemcpyAsync(dev_maps, maps, sizeof(maps), cudaMemcpyHostToDevice, st));
   for (int i : changed) {
     CUDA_TRY(cudaMemcpyAsync(h->ws + h->layout.ops + (size_t)i * sizeof(mk_op_t), &h->ops[i], sizeof(mk_op_t), cudaMemcpyHostToDevice, st));
-    // what the rows of the instruction table derive from the record: upload the span that holds them
+    // what the rows of the instruction table derive from the record
     size_t lo = 0, hi = 0;
     refresh_rows(h, i, &lo, &hi);
     if (hi > lo)
