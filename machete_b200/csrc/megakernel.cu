@@ -929,7 +929,9 @@ static int create_program(const mk_program_t* prog, mk_handle_t* out, bool strea
   return 0;
 }
 
-int mk_create(const mk_program_t* prog, mk_handle_t* out) { return create_program(prog, out, false, nullptr); }
+int mk_create(const mk_program_t* prog, mk_handle_t* out) {
+  return guarded([&] { return create_program(prog, out, false, nullptr); });
+}
 
 static int launch_persistent(mk_handle_s* h, const mk::ProgramView& pv, cudaStream_t stream) {
   using namespace mk;
@@ -955,9 +957,8 @@ static int run_program(mk_handle_s* h, cudaStream_t stream) {
   const bool persistent = plan->steps.empty() || h->pv.trace != nullptr;
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   CUDA_TRY(cudaStreamIsCapturing(stream, &capturing));
-  if (capturing == cudaStreamCaptureStatusNone || h->fixed) {
-    if (persistent) return launch_persistent(h, h->pv, stream); return run_chain(*plan, stream);
-  }
+  if (capturing == cudaStreamCaptureStatusNone || h->fixed)
+    return persistent ? launch_persistent(h, h->pv, stream) : run_chain(*plan, stream);
   // The records may be others when the captured step is replayed.
   ProgramView pv = h->pv;
   place_states(h, true, &pv);
