@@ -560,8 +560,8 @@ int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, 
                           const int64_t v_strides[3], const int64_t o_strides[3], float scale, int causal,
                           void* workspace, uint64_t workspace_bytes, int timeout_ms, void* cuda_stream);
 int mk_flash_prefill_status(const void* workspace, int32_t out[4]);
-/* How mk_flash_prefill_bf16 cuts a call of these sizes on a device of `sms` multiprocessors: out[0] CTAs an SM (2, or 3
- * in the form with one score accumulator); [1] query heads of a KV head in one tile of 128 rows; [2] row tiles;
+/* How mk_flash_prefill_bf16 cuts a call of these sizes on a device of `sms` multiprocessors: out[0] tiles that share an SM (2,
+ * a CTA each, or 3 in one CTA); [1] query heads of a KV head in one tile of 128 rows; [2] row tiles;
  * [3] tiles of all heads and batch entries. */
 int mk_flash_prefill_plan(int B, int H, int Hkv, int M, int N, int D, int causal, int sms, int32_t out[4]);
 const char* mk_flash_prefill_last_error(void);

@@ -7,25 +7,32 @@
 // sm_100.py:88-…, dispatch attention/__init__.py:16-130) as a launch of its own, so that a prompt can
 // fill the KV cache the decode kernel then reads.
 //
-// One CTA = one (batch, tile of 128 query rows), the rows being 128 / g queries of the g query heads that share a KV
-// head (the power of two in the group); KV tiles of 64 tokens; two CTAs share an SM (<= 97 KB of shared memory and 256
-// tensor-memory columns each; three at head dim 64 where that saves a round, see the launch):
+// A tile is 128 query rows of one batch entry, the rows being 128 / g queries of the g query heads that share a KV head (the
+// power of two in the group); KV tiles of 64 tokens.  Two forms:
+//   * one tile a CTA, two CTAs to an SM (<= 97 KB of shared memory and 256 tensor-memory columns each), two S accumulators;
+//   * (head dim 64) three tiles a CTA, one CTA to an SM, which share the K and V tiles: each tile has one S accumulator and
+//     room for P behind it (160 columns), and S(j + 1) is issued as soon as the row threads hold S(j).  Three row warps a
+//     scheduler hide more of one another's latencies than two (777 queries behind 2223 tokens, two sequences, us: three CTAs of
+//     one accumulator each, whose S waited for the P V before, 58.7; so 50.5; 4096 x 4096 102 / 90).
 //
-//   warp 0     TMA: Q once, then K and V tiles (both double-buffered, K one tile ahead of V) as
-//              64-column boxes, 128-byte swizzle;
-//   warp 1     tcgen05.mma issuer: S(j) = Q K(j)^T into one of two tensor-memory accumulators, one tile
-//              ahead of the softmax, and O += P(j) V(j) with P read FROM TENSOR MEMORY (the M x K
-//              operand) and V as the N operand in MN-major form (its head dimension is contiguous in
-//              shared memory exactly as the cache stores it);
-//   warps 2-5  one thread per query row (= tensor-memory lane): one tcgen05.ld of the row of S(j), mask,
-//              maximum, P = exp2(scale * s - reference) with packed f32x2 arithmetic, running sum in
-//              registers (no shuffles: a thread owns its row), P stored as bf16 pairs over the first half
-//              of the accumulator it came from (tcgen05.st), O rescaled in tensor memory only when a row
-//              maximum outgrew the exponent reference by 2^8; normalised bf16 store at the end.
+//   load warp     TMA: Q once, then K and V tiles (four each, at 128 two; K one tile ahead of V) as 64-column boxes, 128-byte
+//                 swizzle;
+//   product warps one a tile, tcgen05.mma: S(j) = Q K(j)^T one tile ahead of the softmax, and O += P(j) V(j) with P read
+//                 FROM TENSOR MEMORY (the M x K operand) and V as the N operand in MN-major form (its head dimension is
+//                 contiguous in shared memory exactly as the cache stores it);
+//   row warps     four a tile, one thread per query row (= tensor-memory lane): one tcgen05.ld of the row of S(j), mask,
+//                 maximum, P = exp2(scale * s - reference) with packed f32x2 arithmetic, running sum in
+//                 registers (no shuffles: a thread owns its row), P stored as bf16 pairs (tcgen05.st; with two accumulators
+//                 over the first half of the one it came from), O rescaled in tensor memory only when a row
+//                 maximum outgrew the exponent reference by 2^8; normalised bf16 store at the end.
 //
-// The row threads never wait for P V: while the tensor cores run P(j) V(j) and S(j + 2) they are already
-// on tile j + 1, so the exponentials (the scarce unit: 16 per clock and SM) and the products overlap inside
-// one CTA, and the second CTA of the SM fills what is left.
+// The row threads hardly wait for P V: while the tensor cores run P(j) V(j) and the next S they are already on tile j + 1, so the
+// exponentials (the scarce unit: 16 per clock and SM) and the products overlap inside one tile, and the other tiles of the
+// SM fill what is left.  What bounds it: at head dim 64 the row threads' instructions (some 360 a warp and KV tile; ncu on the
+// chunk above: issue slots 60 %, exp2 unit 50 %, fma 45 %, alu 40 %, tensor pipe 53 % of active cycles); at 128 the tensor pipe, whose
+// 64-wide S products are held up by shared memory.  Measured and left out: KV tiles of 128 tokens (4096 x 4096, head dim 64
+// 109 -> 116 us, 128 124 -> 141: the same instructions with more registers); the maximum taken beside the exponentials, and these
+// taken again where it grew (50.5 -> 55); one warp for all tiles' products (no change).
 //
 // Every wait is bounded; on expiry the CTA records a status, raises its abort flag, all roles fall
 // through to the common exit and tensor memory is freed.
@@ -48,14 +55,7 @@
 
 namespace mkp {
 
-// The kernel has two forms: two S accumulators, two CTAs to an SM, a warp for the loads, one for the products and four
-// of row threads; and (head dim 64) one S accumulator, three CTAs to an SM, one warp for loads and products, so that
-// the SM's 15 warps are four to a scheduler and a thread may use 128 registers (with 18 it is 96).
-template <int SB>
-constexpr int kThreads = SB == 1 ? 160 : 192;
-template <int SB>
-constexpr int kCtasPerSm = SB == 1 ? 3 : 2;
-constexpr int kBM = 128;   // query rows per CTA
+constexpr int kBM = 128;   // query rows of a tile
 constexpr int kBN = 64;    // tokens per KV tile
 constexpr uint32_t kBox = 128 * 64 * 2;   // one 128-row x 64-column bf16 box
 
@@ -66,6 +66,7 @@ struct Params {
   int64_t o_sb, o_sh, o_sm;
   int B, H, Hkv, M, N, D;
   int causal;
+  int row_tiles;
   int pack, pack_log2;   // query heads of a KV head in one tile: row r is query r >> pack_log2 of head r & (pack - 1)
   int next_early;        // the kernel behind this one may be placed from the start (else: with the last load)
   float scale_log2;      // scale * log2(e)
@@ -73,12 +74,6 @@ struct Params {
 };
 
 enum { PF_ST_TIMEOUT_EMPTY = 1, PF_ST_TIMEOUT_FULL = 2, PF_ST_TIMEOUT_S = 3, PF_ST_TIMEOUT_P = 4, PF_ST_TIMEOUT_O = 5 };
-
-struct Shared {
-  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_ready[2], p_ready[2], pv_done[2];
-  uint32_t tmem_base;
-  int32_t abort_flag;
-};
 
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* tmap, int c0, int c1, int c2, int c3, uint32_t bar) {
   asm volatile(
@@ -240,276 +235,279 @@ __device__ __forceinline__ uint32_t idesc_bf16(int n, bool b_mn) {
   return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn ? (1u << 16) : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
 }
 
-__device__ __forceinline__ void give_up(const Params& p, Shared* sh, int code, int aux) {
+__device__ __forceinline__ void give_up(const Params& p, int32_t* abort_flag, int code, int aux) {
   if (atomicCAS(&p.status[0], 0, code) == 0) {
     p.status[1] = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
     p.status[2] = threadIdx.x >> 5;
     p.status[3] = aux;
   }
-  atomicExch(&sh->abort_flag, 1);
+  atomicExch(abort_flag, 1);
   __threadfence();
 }
-__device__ __forceinline__ bool wait_bar(const Params& p, Shared* sh, uint32_t bar, uint32_t parity, int code, int aux) {
+__device__ __forceinline__ bool wait_bar(const Params& p, int32_t* abort_flag, uint32_t bar, uint32_t parity, int code, int aux) {
   uint64_t t0 = 0;
   for (uint32_t spin = 0;; ++spin) {
     if (mk::mbar_try_wait(bar, parity)) return true;
     if ((spin & 255u) == 255u) {
-      if (*reinterpret_cast<volatile int32_t*>(&sh->abort_flag)) return false;
+      if (*reinterpret_cast<volatile int32_t*>(abort_flag)) return false;
       const uint64_t now = mk::globaltimer_ns();
       if (t0 == 0) t0 = now;
       if (now - t0 > p.timeout_ns) {
-        give_up(p, sh, code, aux);
+        give_up(p, abort_flag, code, aux);
         return false;
       }
     }
   }
 }
 
-// The same wait for a whole warp: every lane polls, the outcome is the same for all.
-__device__ __forceinline__ bool wait_bar_warp(const Params& p, Shared* sh, uint32_t bar, uint32_t parity, int code, int aux) {
-  if (__all_sync(0xffffffffu, mk::mbar_try_wait(bar, parity))) return true;
-  return __all_sync(0xffffffffu, wait_bar(p, sh, bar, parity, code, aux));
-}
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
   return p != 0;
 }
 
-// SB = S accumulators.  (The barriers k_empty, v_empty and all second ones belong to the form with two.)
-template <int D, int SB>
-__global__ void __launch_bounds__(kThreads<SB>, kCtasPerSm<SB>)
+__device__ __forceinline__ void arrive_if(uint32_t bar, bool yes) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %1, 0;\n\t@q mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar), "r"((uint32_t)yes)
+               : "memory");
+}
+// The row threads' loop is longer than what a scheduler keeps of its instructions, so every taken branch in it waits for
+// an instruction fetch, some forty clocks: waits that find their phase complete, which most do, run straight on, and
+// what is rare stands out of line.  (A tile that has its SM to itself, 128 queries behind 3968 tokens, us with the slow paths in
+// the loop and so: head dim 64 42.2 / 38.4, 128 50.8 / 44.8; 777 queries behind 2223 tokens, two sequences, head dim 128 78.6 / 70.1.)
+__device__ __noinline__ bool wait_cold(const Params& p, int32_t* abort_flag, uint32_t bar, uint32_t parity, int code, int aux) {
+  return __all_sync(0xffffffffu, wait_bar(p, abort_flag, bar, parity, code, aux));
+}
+__device__ __forceinline__ bool wait_hot(const Params& p, int32_t* abort_flag, uint32_t bar, uint32_t parity, int code, int aux) {
+  if (__builtin_expect(__all_sync(0xffffffffu, mk::mbar_try_wait(bar, parity)), 1)) return true;
+#pragma unroll 1
+  for (int i = 0; i < 64; ++i)
+    if (mk::mbar_try_wait(bar, parity)) break;
+  if (__all_sync(0xffffffffu, mk::mbar_try_wait(bar, parity))) return true;
+  return wait_cold(p, abort_flag, bar, parity, code, aux);
+}
+// O of this thread's row times alpha, once the P V that `bar` tells of has finished with it.
+template <int D>
+__device__ __noinline__ bool rescale(const Params& p, int32_t* abort_flag, uint32_t o_addr, float alpha, uint32_t bar, uint32_t parity, int j) {
+  if (!wait_hot(p, abort_flag, bar, parity, PF_ST_TIMEOUT_O, j)) return false;
+  tc_fence_after();
+#pragma unroll 1
+  for (int c = 0; c < D; c += 32) {
+    uint32_t o[32];
+    tmem_ld32(o_addr + (uint32_t)c, o);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+    tmem_st32(o_addr + (uint32_t)c, o);
+  }
+  return true;
+}
+
+// A CTA's shape: T tiles of 128 query rows that share the K and V tiles, each with four warps of row threads and a warp that
+// issues its products, and a warp for the loads.
+template <int D, int T>
+struct Form {
+  static constexpr int kThreads = (5 * T + 1) * 32;
+  static constexpr int kPerSm = T == 1 ? 2 : 1;
+  static constexpr int NB = D / 64;                       // 64-column boxes of a row
+  static constexpr uint32_t kQTile = NB * kBox, kKVBox = kBN * 64 * 2, kKVTile = NB * kKVBox;
+  static constexpr int KS = D == 128 ? 2 : 4, VS = KS;   // K and V tiles in flight
+  // tensor memory of a tile: O, then two S accumulators of which P (bf16 pairs) takes the first half, or (three tiles) one and P behind it
+  static constexpr int SB = T == 1 ? 2 : 1;
+  static constexpr uint32_t kTileCols = D + (SB == 2 ? 2 * kBN : kBN + kBN / 2), kCols = T == 1 ? 256 : 512;
+  static_assert(T * kTileCols <= kCols, "accumulators must fit the allocation");
+  struct Shared {
+    uint64_t q_full[T], s_full[2 * T], s_free[T], p_ready[2 * T], pv_done[2 * T], k_full[KS], k_empty[KS], v_full[VS], v_empty[VS];
+    uint32_t tmem_base;
+    int32_t abort_flag;
+  };
+  static constexpr size_t kSmem = (size_t)T * kQTile + (size_t)(KS + VS) * kKVTile + sizeof(Shared);
+};
+
+template <int D, int T>
+__global__ void __launch_bounds__(Form<D, T>::kThreads, Form<D, T>::kPerSm)
 prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-               const __grid_constant__ CUtensorMap map_v, const Params p) {
-  constexpr int NB = D / 64;                       // 64-column boxes per row tile
-  constexpr uint32_t kTile = NB * kBox;            // the 128 x D query tile
-  constexpr uint32_t kKVBox = kBN * 64 * 2;        // one 64-token x 64-column box of K or V
-  constexpr uint32_t kKVTile = NB * kKVBox;
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t raw = mk::smem_u32(smem_raw);
-  const uint32_t base = (raw + 1023u) & ~1023u;
-  uint8_t* smem = smem_raw + (base - raw);
-  // layout: Q | K0 | K1 | V0 | V1 | control
-  const uint32_t q_s = base, k_s = q_s + kTile, v_s = k_s + 2 * kKVTile;
-  Shared* sh = reinterpret_cast<Shared*>(smem + kTile + 4 * kKVTile);
+               const __grid_constant__ CUtensorMap map_v, const __grid_constant__ Params p) {
+  using F = Form<D, T>;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t q_s = mk::smem_u32(smem), k_s = q_s + T * F::kQTile, v_s = k_s + F::KS * F::kKVTile;
+  typename F::Shared* sh = reinterpret_cast<typename F::Shared*>(smem + T * F::kQTile + (F::KS + F::VS) * F::kKVTile);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // Blocks are handed out in the order x, y, z: the query tile is the slowest index and runs from the LAST tile
+  constexpr int kLoadWarp = 5 * T;
+  // Blocks are handed out in the order x, y, z: the query tiles are the slowest index and run from the LAST tile
   // down, so that under a causal mask the tiles with the most KV tiles start first and the short ones fill the
   // tail (longest job first).
   // The tile's 128 rows are 128 / pack queries of `pack` heads that share a KV head: a prompt of 777 queries and four
   // heads a KV head is 25 tiles, not 4 x 7, and fewer pairs lie behind the diagonal (32 / 8 heads, causal, us before and
   // after: 2190 x 2190 head dim 128 45.2 / 40.5, 64 39.6 / 35.5; 1960 of 2045, four sequences, 159.5 / 146.6 and
   // 133.2 / 118.3; 4096 x 4096 128.3 / 125.5 and 107.2 / 103.7).
-  const int mt = (int)(gridDim.z - 1 - blockIdx.z), h0 = blockIdx.x * p.pack, b = blockIdx.y;
+  const int h0 = blockIdx.x * p.pack, b = blockIdx.y;
   const int kvh = h0 / (p.H / p.Hkv);
   const int tile_m = kBM >> p.pack_log2;
-  const int m0 = mt * tile_m;
-  // tokens this query tile can see: all N, or (causal) up to the diagonal of its last row
-  const int n_vis = p.causal ? min(p.N, p.N - p.M + m0 + tile_m) : p.N;
-  const int n_tiles = n_vis > 0 ? (n_vis + kBN - 1) / kBN : 0;
-  // The S accumulators of 64 columns come first (P, as bf16 pairs, overwrites the first 32 columns of the accumulator
-  // it was computed from), O behind them.
-  constexpr uint32_t kOCol = SB * kBN, kCols = SB == 1 ? 128 : 256;
-  static_assert(kOCol + D <= kCols, "accumulators must fit the allocation");
+  auto first_row = [&](int i) { return (p.row_tiles - 1 - ((int)blockIdx.z * T + i)) * tile_m; };   // negative: no such tile
+  // KV tiles that a query tile can see: of all N tokens, or (causal) up to the diagonal of its last row
+  auto kv_tiles = [&](int i) {
+    const int m0 = first_row(i);
+    if (m0 < 0) return 0;
+    const int n_vis = p.causal ? min(p.N, p.N - p.M + m0 + tile_m) : p.N;
+    return n_vis > 0 ? (n_vis + kBN - 1) / kBN : 0;
+  };
+  int n_tiles[T];
+#pragma unroll
+  for (int i = 0; i < T; ++i) n_tiles[i] = kv_tiles(i);
+  const int n_most = n_tiles[0];
 
   if (threadIdx.x == 0) {
-    mk::mbar_init(mk::smem_u32(&sh->q_full), 1);
-    for (int s = 0; s < 2; ++s) {
+#pragma unroll
+    for (int i = 0; i < T; ++i) {
+      mk::mbar_init(mk::smem_u32(&sh->q_full[i]), 1);
+      mk::mbar_init(mk::smem_u32(&sh->s_free[i]), 4);
+      for (int k = 2 * i; k < 2 * i + 2; ++k) {
+        mk::mbar_init(mk::smem_u32(&sh->s_full[k]), 1);
+        mk::mbar_init(mk::smem_u32(&sh->p_ready[k]), 4);
+        mk::mbar_init(mk::smem_u32(&sh->pv_done[k]), 1);
+      }
+    }
+    for (int s = 0; s < F::KS; ++s) {
       mk::mbar_init(mk::smem_u32(&sh->k_full[s]), 1);
-      mk::mbar_init(mk::smem_u32(&sh->k_empty[s]), 1);
+      mk::mbar_init(mk::smem_u32(&sh->k_empty[s]), T);
+    }
+    for (int s = 0; s < F::VS; ++s) {
       mk::mbar_init(mk::smem_u32(&sh->v_full[s]), 1);
-      mk::mbar_init(mk::smem_u32(&sh->v_empty[s]), 1);
-      mk::mbar_init(mk::smem_u32(&sh->s_ready[s]), 1);
-      mk::mbar_init(mk::smem_u32(&sh->p_ready[s]), 128);
-      mk::mbar_init(mk::smem_u32(&sh->pv_done[s]), 1);
+      mk::mbar_init(mk::smem_u32(&sh->v_empty[s]), T);
     }
     sh->abort_flag = 0;
     mk::fence_mbar_init();
   }
-  constexpr int kMmaWarp = SB == 1 ? 0 : 1;
   __syncwarp();
-  if (warp == kMmaWarp) tmem_alloc(mk::smem_u32(&sh->tmem_base), kCols);
+  if (warp == kLoadWarp) tmem_alloc(mk::smem_u32(&sh->tmem_base), F::kCols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&sh->tmem_base);
+  constexpr int SB = F::SB;
+  constexpr uint32_t kSCol = D, kPCol = D + (SB == 2 ? 0 : kBN);
+  int32_t* flag = &sh->abort_flag;
   mk::prior_work_done();
   if (p.next_early) mk::next_may_start();
 
-  // Tile j uses slot j & 1 of every double-buffered resource; its barrier phase is (j >> 1) & 1.
-  if (SB == 1 && warp == 0) {
-    // Loads and products from one warp: S(0), then for every tile P V(j) and S(j + 1) once P(j) is there.  When it is,
-    // S(j) and P V(j - 1) are finished (the row threads read S(j), which was issued behind P V(j - 1)), so K(j + 2) and
-    // V(j + 1) may follow into their slots with no barrier of their own.
-    const uint32_t id_s = idesc_bf16(kBN, false), id_o = idesc_bf16(D, true);
-    const bool one = elect_one();
-    const uint32_t elected = one ? 1u : 0u;
-    auto load_kv = [&](int j, bool is_v) {
-      if (j >= n_tiles) return;
-      const uint32_t fb = mk::smem_u32(is_v ? &sh->v_full[j & 1] : &sh->k_full[j & 1]);
-      const uint32_t dst = (is_v ? v_s : k_s) + (uint32_t)(j & 1) * kKVTile;
-      if (one) {
-        mk::mbar_arrive_expect_tx(fb, kKVTile);
-        for (int x = 0; x < NB; ++x) tma_load_4d(dst + x * kKVBox, is_v ? &map_v : &map_k, x * 64, j * kBN, kvh, b, fb);
-      }
-    };
-    if (one) {
-      const uint32_t qb = mk::smem_u32(&sh->q_full);
-      mk::mbar_arrive_expect_tx(qb, kTile);
-      for (int x = 0; x < NB; ++x) tma_load_4d(q_s + x * kBox, &map_q, x * 64, h0, m0, b, qb);
-    }
-    load_kv(0, false);
-    load_kv(0, true);
-    load_kv(1, false);
-    bool ok = wait_bar_warp(p, sh, mk::smem_u32(&sh->q_full), 0, PF_ST_TIMEOUT_FULL, -1);
-    auto issue_s = [&](int j) -> bool {
-      const int s = j & 1;
-      if (!wait_bar_warp(p, sh, mk::smem_u32(&sh->k_full[s]), (uint32_t)(j >> 1) & 1u, PF_ST_TIMEOUT_FULL, j)) return false;
-      tc_fence_after();
-#pragma unroll
-      for (int k = 0; k < D / 16; ++k) {
-        const uint32_t in_box = (uint32_t)(k & 3) * 32u;
-        tc_mma(tmem, desc_kmajor(q_s + (uint32_t)(k >> 2) * kBox + in_box),
-               desc_kmajor(k_s + s * kKVTile + (uint32_t)(k >> 2) * kKVBox + in_box), id_s, k > 0 ? 1u : 0u, elected);
-      }
-      tc_commit(mk::smem_u32(&sh->s_ready[0]), elected);
-      return true;
-    };
-    if (ok && n_tiles > 0) ok = issue_s(0);
-    for (int j = 0; j < n_tiles && ok; ++j) {
-      const int s = j & 1;
-      ok = wait_bar_warp(p, sh, mk::smem_u32(&sh->p_ready[0]), (uint32_t)j & 1u, PF_ST_TIMEOUT_P, j);
-      if (!ok) break;
-      load_kv(j + 2, false);
-      load_kv(j + 1, true);
-      if (j + 2 >= n_tiles) mk::next_may_start();
-      ok = wait_bar_warp(p, sh, mk::smem_u32(&sh->v_full[s]), (uint32_t)(j >> 1) & 1u, PF_ST_TIMEOUT_FULL, j);
-      if (!ok) break;
-      tc_fence_after();
-#pragma unroll
-      for (int k = 0; k < kBN / 16; ++k) {
-        // P: 16 tokens = 8 tensor-memory columns of bf16 pairs; V: MN-major, 16 tokens = 16 rows of 128 bytes
-        const uint64_t dv = desc_mnmajor(v_s + (uint32_t)s * kKVTile + (uint32_t)k * 2048u, kKVBox);
-        tc_mma_ts(tmem + kOCol, tmem + (uint32_t)k * 8u, dv, id_o, (j > 0 || k > 0) ? 1u : 0u, elected);
-      }
-      // (the tensor cores run the products in this order: S(j + 1) overwrites P(j) behind P V(j))
-      if (j + 1 < n_tiles) ok = issue_s(j + 1);
-      else tc_commit(mk::smem_u32(&sh->pv_done[0]), elected);
-    }
-    mk::next_may_start();
-    if (*reinterpret_cast<volatile int32_t*>(&sh->abort_flag)) {
-      // shared memory must outlive the copies in flight: a bounded wait for whatever was issued last
-      const uint64_t t0 = mk::globaltimer_ns();
-      while (mk::globaltimer_ns() - t0 < 20000ull) {
-      }
-    }
-  } else if (SB == 2 && warp == 0) {
+  if (warp == kLoadWarp) {
     if (lane == 0) {
-      const uint32_t qb = mk::smem_u32(&sh->q_full);
-      mk::mbar_arrive_expect_tx(qb, kTile);
-      for (int x = 0; x < NB; ++x) tma_load_4d(q_s + x * kBox, &map_q, x * 64, h0, m0, b, qb);
+      auto load_q = [&](int i) {
+        if (n_tiles[i] == 0) return;
+        const uint32_t qb = mk::smem_u32(&sh->q_full[i]);
+        mk::mbar_arrive_expect_tx(qb, F::kQTile);
+        for (int x = 0; x < F::NB; ++x) tma_load_4d(q_s + i * F::kQTile + x * kBox, &map_q, x * 64, h0, first_row(i), b, qb);
+      };
       auto load_kv = [&](int j, bool is_v) -> bool {
-        const int s = j & 1;
-        const uint32_t ph = (uint32_t)(j >> 1) & 1u;
+        const int n = is_v ? F::VS : F::KS, s = j % n;
+        const uint32_t ph = (uint32_t)(j / n) & 1u;
         uint64_t* empty = is_v ? &sh->v_empty[s] : &sh->k_empty[s];
         uint64_t* full = is_v ? &sh->v_full[s] : &sh->k_full[s];
-        if (!wait_bar(p, sh, mk::smem_u32(empty), ph ^ 1u, PF_ST_TIMEOUT_EMPTY, j)) return false;
+        if (!wait_bar(p, flag, mk::smem_u32(empty), ph ^ 1u, PF_ST_TIMEOUT_EMPTY, j)) return false;
         const uint32_t fb = mk::smem_u32(full);
-        mk::mbar_arrive_expect_tx(fb, kKVTile);
-        const uint32_t dst = (is_v ? v_s : k_s) + (uint32_t)s * kKVTile;
-        for (int x = 0; x < NB; ++x) tma_load_4d(dst + x * kKVBox, is_v ? &map_v : &map_k, x * 64, j * kBN, kvh, b, fb);
+        mk::mbar_arrive_expect_tx(fb, F::kKVTile);
+        const uint32_t dst = (is_v ? v_s : k_s) + (uint32_t)s * F::kKVTile;
+        for (int x = 0; x < F::NB; ++x) tma_load_4d(dst + x * F::kKVBox, is_v ? &map_v : &map_k, x * 64, j * kBN, kvh, b, fb);
         return true;
       };
       // K runs one tile ahead of V: S(j + 1) is issued before P(j) V(j)
-      bool pok = n_tiles > 0 ? load_kv(0, false) : true;
-      for (int j = 0; j < n_tiles && pok; ++j) {
-        if (j + 1 < n_tiles && !load_kv(j + 1, false)) break;
+      load_q(0);
+      bool pok = n_most > 0 ? load_kv(0, false) : true;
+#pragma unroll
+      for (int i = 1; i < T; ++i) load_q(i);
+      for (int j = 0; j < n_most && pok; ++j) {
+        if (j + 1 < n_most && !load_kv(j + 1, false)) break;
         if (!load_kv(j, true)) break;
       }
       mk::next_may_start();
-      if (*reinterpret_cast<volatile int32_t*>(&sh->abort_flag)) {
+      if (*reinterpret_cast<volatile int32_t*>(flag)) {
         // shared memory must outlive the copies in flight: a bounded wait for whatever was issued last
         const uint64_t t0 = mk::globaltimer_ns();
         while (mk::globaltimer_ns() - t0 < 20000ull) {
         }
       }
     }
-  } else if (SB == 2 && warp == 1) {
-    // Head dim 64 issues as a whole warp (see tc_mma).  At 128 one lane that waits and issues is the lighter neighbour
-    // where prompts fill the device (causal, 32 / 8 heads, 2190 x 2190 42.2 us against 45.2, 4096 x 4096 145.7 against
-    // 150.3).  A tile that has its SM to itself would be quicker by the warp (512 x 512 10.4 us, 9.9 so; 300 behind 1700
-    // tokens 28.1, 26.7).
-    constexpr bool kOneLane = D == 128;
-    if (!kOneLane || lane == 0) {
-      auto wait_mma = [&](uint32_t bar, uint32_t parity, int code, int aux) -> bool {
-        if constexpr (kOneLane) return wait_bar(p, sh, bar, parity, code, aux);
-        else return wait_bar_warp(p, sh, bar, parity, code, aux);
-      };
-      const uint32_t id_s = idesc_bf16(kBN, false), id_o = idesc_bf16(D, true);
-      const uint32_t elected = kOneLane || elect_one() ? 1u : 0u;
-      bool ok = wait_mma(mk::smem_u32(&sh->q_full), 0, PF_ST_TIMEOUT_FULL, -1);
-      auto issue_s = [&](int j) -> bool {
-        const int s = j & 1;
-        if (!wait_mma(mk::smem_u32(&sh->k_full[s]), (uint32_t)(j >> 1) & 1u, PF_ST_TIMEOUT_FULL, j)) return false;
-        tc_fence_after();
+  } else if (warp >= 4 * T) {
+    // products of tile i, in the order S(0), S(1), P V(0), S(2), P V(1), ...
+    // (the tile, and with it every descriptor, is known to be uniform: see tc_mma)
+    const int i = T == 1 ? 0 : __shfl_sync(0xffffffffu, warp - 4 * T, 0), nt = kv_tiles(i);
+    const uint32_t id_s = idesc_bf16(kBN, false), id_o = idesc_bf16(D, true), elected = elect_one() ? 1u : 0u;
+    const uint32_t o = tmem + i * F::kTileCols, q = q_s + i * F::kQTile;
+    const uint32_t s_full = mk::smem_u32(&sh->s_full[2 * i]), s_free = mk::smem_u32(&sh->s_free[i]);
+    const uint32_t p_ready = mk::smem_u32(&sh->p_ready[2 * i]), pv_done = mk::smem_u32(&sh->pv_done[2 * i]);
+    auto issue_s = [&](int j) -> bool {
+      const int s = j % F::KS;
+      if (!wait_hot(p, flag, mk::smem_u32(&sh->k_full[s]), (uint32_t)(j / F::KS) & 1u, PF_ST_TIMEOUT_FULL, j)) return false;
+      if (SB == 1 && j > 0 && !wait_hot(p, flag, s_free, (uint32_t)(j - 1) & 1u, PF_ST_TIMEOUT_S, j)) return false;
+      tc_fence_after();
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t in_box = (uint32_t)(k & 3) * 32u;
-          tc_mma(tmem + (uint32_t)s * kBN, desc_kmajor(q_s + (uint32_t)(k >> 2) * kBox + in_box),
-                 desc_kmajor(k_s + s * kKVTile + (uint32_t)(k >> 2) * kKVBox + in_box), id_s, k > 0 ? 1u : 0u, elected);
-        }
-        tc_commit(mk::smem_u32(&sh->s_ready[s]), elected);
-        tc_commit(mk::smem_u32(&sh->k_empty[s]), elected);
-        return true;
-      };
-      // Issue order S(0), S(1), P V(0), S(2), P V(1), S(3), ...  The tensor cores run the products in this
-      // order, so S(j + 2) overwrites accumulator j & 1 only after P V(j) has read P(j) from it, and the
-      // row threads find S(j + 1) finished while P V(j) is still running.
-      if (ok && n_tiles > 0) ok = issue_s(0);
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        if (j + 1 < n_tiles) ok = issue_s(j + 1);
-        if (!ok) break;
-        const int s = j & 1;
-        const uint32_t ph = (uint32_t)(j >> 1) & 1u;
-        // O += P V once the row threads have written P (and rescaled O)
-        ok = wait_mma(mk::smem_u32(&sh->p_ready[s]), ph, PF_ST_TIMEOUT_P, j) &&
-             wait_mma(mk::smem_u32(&sh->v_full[s]), ph, PF_ST_TIMEOUT_FULL, j);
-        if (!ok) break;
-        tc_fence_after();
-#pragma unroll
-        for (int k = 0; k < kBN / 16; ++k) {
-          // P: 16 tokens = 8 tensor-memory columns of bf16 pairs; V: MN-major, 16 tokens = 16 rows of 128 bytes
-          const uint64_t dv = desc_mnmajor(v_s + (uint32_t)s * kKVTile + (uint32_t)k * 2048u, kKVBox);
-          tc_mma_ts(tmem + kOCol, tmem + (uint32_t)s * kBN + (uint32_t)k * 8u, dv, id_o, (j > 0 || k > 0) ? 1u : 0u, elected);
-        }
-        tc_commit(mk::smem_u32(&sh->pv_done[s]), elected);
-        tc_commit(mk::smem_u32(&sh->v_empty[s]), elected);
+      for (int k = 0; k < D / 16; ++k) {
+        const uint32_t in_box = (uint32_t)(k & 3) * 32u;
+        tc_mma(o + kSCol + (uint32_t)(j % SB) * kBN, desc_kmajor(q + (uint32_t)(k >> 2) * kBox + in_box),
+               desc_kmajor(k_s + s * F::kKVTile + (uint32_t)(k >> 2) * F::kKVBox + in_box), id_s, k > 0 ? 1u : 0u, elected);
       }
+      tc_commit(s_full + (uint32_t)(j % SB) * 8u, elected);
+      tc_commit(mk::smem_u32(&sh->k_empty[s]), elected);
+      return true;
+    };
+    bool ok = nt == 0 || (wait_hot(p, flag, mk::smem_u32(&sh->q_full[i]), 0, PF_ST_TIMEOUT_FULL, -1) && issue_s(0));
+#pragma unroll 1
+    for (int j = 0; j < nt && ok; ++j) {
+      if (__builtin_expect(j + 1 < nt, 1)) ok = issue_s(j + 1);
+      if (!ok) break;
+      const int s = j % F::VS;
+      // O += P V once the row threads have written P (and rescaled O)
+      ok = wait_hot(p, flag, p_ready + (uint32_t)(j % SB) * 8u, (uint32_t)(j / SB) & 1u, PF_ST_TIMEOUT_P, j) &&
+           wait_hot(p, flag, mk::smem_u32(&sh->v_full[s]), (uint32_t)(j / F::VS) & 1u, PF_ST_TIMEOUT_FULL, j);
+      if (!ok) break;
+      tc_fence_after();
+#pragma unroll
+      for (int k = 0; k < kBN / 16; ++k) {
+        // P: 16 tokens = 8 tensor-memory columns of bf16 pairs; V: MN-major, 16 tokens = 16 rows of 128 bytes
+        const uint64_t dv = desc_mnmajor(v_s + (uint32_t)s * F::kKVTile + (uint32_t)k * 2048u, F::kKVBox);
+        tc_mma_ts(o, o + kPCol + (uint32_t)(j % SB) * kBN + (uint32_t)k * 8u, dv, id_o, (j > 0 || k > 0) ? 1u : 0u, elected);
+      }
+      tc_commit(pv_done + (uint32_t)(j % SB) * 8u, elected);
+      tc_commit(mk::smem_u32(&sh->v_empty[s]), elected);
     }
-  } else {
+    // of the KV tiles that only the longer tiles have, this one is done with each slot as soon as it is filled
+    for (int j = nt; j < n_most && ok; ++j) {
+      ok = wait_hot(p, flag, mk::smem_u32(&sh->k_full[j % F::KS]), (uint32_t)(j / F::KS) & 1u, PF_ST_TIMEOUT_FULL, j);
+      if (ok && elected) mk::mbar_arrive(mk::smem_u32(&sh->k_empty[j % F::KS]));
+      ok = ok && wait_hot(p, flag, mk::smem_u32(&sh->v_full[j % F::VS]), (uint32_t)(j / F::VS) & 1u, PF_ST_TIMEOUT_FULL, j);
+      if (ok && elected) mk::mbar_arrive(mk::smem_u32(&sh->v_empty[j % F::VS]));
+    }
+  } else if (first_row(warp >> 2) >= 0) {
     // row threads: warp w may touch tensor-memory lanes 32 * (w % 4) ..
-    const int qd = warp & 3;
+    const int ti = warp >> 2, qd = warp & 3;
+    const int nt = kv_tiles(ti);
     const int row = qd * 32 + lane;                 // query row inside the tile = TMEM lane
-    const int m = m0 + (row >> p.pack_log2), h = h0 + (row & (p.pack - 1));
+    const int m = first_row(ti) + (row >> p.pack_log2), h = h0 + (row & (p.pack - 1));
     const int lim = p.causal ? (p.N - p.M + m) : (p.N - 1);   // last visible token of this row
     // Only the tiles on the causal diagonal and the last one of a ragged cache need the per-score mask; the first n_open
     // do not.  They take another mix of exponentials (see p_pass), so which they are is a matter of results: it goes by
     // blocks of 32 queries, whatever the heads in a tile.  (Every row of a warp is in one block.)
     const int n_open = min(p.causal ? p.N - p.M + (m & ~31) + 1 : p.N, p.N) / kBN;
-    const uint32_t lane_addr = tmem + ((uint32_t)(qd * 32) << 16);
+    const uint32_t lane_addr = tmem + (uint32_t)ti * F::kTileCols + ((uint32_t)(qd * 32) << 16);
+    const uint32_t s_full = mk::smem_u32(&sh->s_full[2 * ti]), s_free = mk::smem_u32(&sh->s_free[ti]);
+    const uint32_t p_ready = mk::smem_u32(&sh->p_ready[2 * ti]), pv_done = mk::smem_u32(&sh->pv_done[2 * ti]);
     const uint64_t scale2 = pack2(p.scale_log2, p.scale_log2);
     float mx = -INFINITY, sum = 0.f;
     bool ok = true;
-    for (int j = 0; j < n_tiles; ++j) {
-      ok = wait_bar(p, sh, mk::smem_u32(&sh->s_ready[j & (SB - 1)]), (uint32_t)(j / SB) & 1u, PF_ST_TIMEOUT_S, j);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
+    // One KV tile, in straight code (see wait_hot); masked tiles have a copy of their own.
+    const int n_plain = min(nt, __shfl_sync(0xffffffffu, n_open, 0));   // (known to be uniform)
+    auto kv_tile = [&](int j, auto is_open) -> bool {
+      constexpr bool kOpen = decltype(is_open)::value;
+      if (!wait_hot(p, flag, s_full + (uint32_t)(j % SB) * 8u, (uint32_t)(j / SB) & 1u, PF_ST_TIMEOUT_S, j)) return false;
       tc_fence_after();
-      const bool open = __all_sync(0xffffffffu, j < n_open);   // (the vote makes it known to be uniform)
-      const uint32_t s_addr = lane_addr + (uint32_t)(j & (SB - 1)) * kBN;
+      const uint32_t s_addr = lane_addr + kSCol + (uint32_t)(j % SB) * kBN;
       uint32_t r[kBN];                               // this row of S, then of P (bf16 pairs in r[0 .. 32))
       tmem_ld64(s_addr, r);
-      if (!open) {
+      if constexpr (SB == 1) {
+        // S(j + 1) may follow
+        tc_fence_before();
+        arrive_if(s_free, lane == 0);
+      }
+      if constexpr (!kOpen) {
 #pragma unroll
         for (int i = 0; i < kBN; ++i) {
           const int tok = j * kBN + i;
@@ -525,74 +523,59 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       const float tmax = max3(fmaxf(t4[0], t4[1]), t4[2], t4[3]) * p.scale_log2;   // the scale is positive
       // mx is the exponent reference in use, not the running maximum: it moves only when a maximum has grown
       // by more than 2^8 since it was set, so O is rescaled rarely (and no P exceeds 2^8).
-      float alpha = 1.f;
-      if (tmax > mx + 8.f) {                         // also the first visible tile (mx = -inf)
-        alpha = exp2f(mx - tmax);                    // 0 when mx = -inf
-        mx = tmax;
+      if (__builtin_expect(__any_sync(0xffffffffu, tmax > mx + 8.f), 0)) {     // also the first visible tile (mx = -inf)
+        const bool grown = tmax > mx + 8.f;
+        const float alpha = grown ? exp2f(mx - tmax) : 1.f;                    // 0 when mx = -inf
+        mx = grown ? tmax : mx;
+        sum *= alpha;
+        // (With two accumulators S(j) was issued after P V(j - 2), so the parity of that barrier is unambiguous.)
+        if (j > 0 && !rescale<D>(p, flag, lane_addr, alpha, pv_done + (uint32_t)((j - 1) % SB) * 8u, (uint32_t)((j - 1) / SB) & 1u, j)) return false;
       }
-      if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-        // O is free only after the previous P V has finished with it.  S(j) was issued after P V(j - 2), so
-        // that phase of this barrier is behind us and the parity is unambiguous.  (With one accumulator S(j) was
-        // issued after P V(j - 1), and its commit covers both.)
-        if (SB == 2) {
-          ok = wait_bar(p, sh, mk::smem_u32(&sh->pv_done[(j - 1) & 1]), (uint32_t)((j - 1) >> 1) & 1u, PF_ST_TIMEOUT_O, j);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          tc_fence_after();
-        }
-#pragma unroll 1
-        for (int c = 0; c < D; c += 32) {
-          uint32_t o[32];
-          tmem_ld32(lane_addr + kOCol + (uint32_t)c, o);
-#pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-          tmem_st32(lane_addr + kOCol + (uint32_t)c, o);
-        }
-      }
-      sum *= alpha;
       const float muse = mx == -INFINITY ? 0.f : mx;
       const uint64_t ref2 = pack2(-muse, -muse);
       // P = exp2(s * scale - reference), two scores per multiply-add, add and conversion
-      uint64_t tsum2 = pack2(0.f, 0.f);
-      auto p_pass = [&](auto mixed) {
+      uint64_t ts[4] = {0, 0, 0, 0};
 #pragma unroll
-        for (int i = 0; i < kBN; i += 2) {
-          const uint64_t x2 = fma2(pack2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), scale2, ref2);
-          float e0, e1;
-          if (decltype(mixed)::value && ((i >> 1) % (MK_PF_POLY > 0 ? MK_PF_POLY : 1)) == 0) {   // compile-time pattern
-            exp2_poly2(x2, e0, e1);
-          } else {
-            float x0, x1;
-            unpack2(x2, x0, x1);
-            e0 = exp2f(x0);
-            e1 = exp2f(x1);
-          }
-          const __nv_bfloat162 pk = __floats2bfloat162_rn(e0, e1);
-          // the row sum is taken before the rounding to bf16 (an unbiased 2^-9 relative error per term)
-          tsum2 = add2(tsum2, pack2(e0, e1));
-          r[i >> 1] = *reinterpret_cast<const uint32_t*>(&pk);
+      for (int i = 0; i < kBN; i += 2) {
+        const uint64_t x2 = fma2(pack2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), scale2, ref2);
+        float e0, e1;
+        // masked tiles keep the exp2 unit for every score: exp2(-inf) is exactly 0 there
+        if (MK_PF_POLY > 0 && D == 64 && kOpen && (i >> 1) % (MK_PF_POLY > 0 ? MK_PF_POLY : 1) == 0) {   // compile-time pattern
+          exp2_poly2(x2, e0, e1);
+        } else {
+          float x0, x1;
+          unpack2(x2, x0, x1);
+          e0 = exp2f(x0);
+          e1 = exp2f(x1);
         }
-      };
-      // masked tiles keep the exp2 unit for every score: exp2(-inf) is exactly 0 there
-      if (MK_PF_POLY > 0 && D == 64 && open)
-        p_pass(std::true_type{});
-      else
-        p_pass(std::false_type{});
+        const __nv_bfloat162 pk = __floats2bfloat162_rn(e0, e1);
+        // the row sum is taken before the rounding to bf16 (an unbiased 2^-9 relative error per term)
+        ts[(i >> 1) & 3] = add2(ts[(i >> 1) & 3], pack2(e0, e1));
+        r[i >> 1] = *reinterpret_cast<const uint32_t*>(&pk);
+      }
       float t0, t1;
-      unpack2(tsum2, t0, t1);
+      unpack2(add2(add2(ts[0], ts[1]), add2(ts[2], ts[3])), t0, t1);
       sum += t0 + t1;
-      // P goes where its S came from: 64 bf16 = the first 32 columns of the accumulator
-      tmem_st32(s_addr, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
+      if constexpr (SB == 1) {
+        // P(j - 1) has been read
+        if (!wait_hot(p, flag, pv_done, (uint32_t)(j - 1) & 1u, PF_ST_TIMEOUT_O, j)) return false;
+        tc_fence_after();
+      }
+      tmem_st32(SB == 1 ? lane_addr + kPCol : s_addr, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
       tmem_wait_st();
       tc_fence_before();
-      mk::mbar_arrive(mk::smem_u32(&sh->p_ready[j & (SB - 1)]));
-    }
+      __syncwarp();
+      // (a warp may be a tile ahead of the others: S(j + 1) does not wait for all of P(j) with two accumulators, so each has its barrier)
+      arrive_if(p_ready + (uint32_t)(j % SB) * 8u, lane == 0);
+      return true;
+    };
+    int j = 0;
+#pragma unroll 1
+    for (; j < n_plain && ok; ++j) ok = kv_tile(j, std::true_type{});
+#pragma unroll 1
+    for (; j < nt && ok; ++j) ok = kv_tile(j, std::false_type{});
     // epilogue: O / sum -> bf16
-    if (ok && n_tiles > 0) {
-      ok = wait_bar(p, sh, mk::smem_u32(&sh->pv_done[(n_tiles - 1) & (SB - 1)]),
-                    SB == 1 ? 0u : (uint32_t)((n_tiles - 1) >> 1) & 1u, PF_ST_TIMEOUT_O, n_tiles);
-      ok = __all_sync(0xffffffffu, ok);
-    }
+    if (ok && nt > 0) ok = wait_hot(p, flag, pv_done + (uint32_t)((nt - 1) % SB) * 8u, (uint32_t)((nt - 1) / SB) & 1u, PF_ST_TIMEOUT_O, nt);
     tc_fence_after();
     if (ok) {
       const float inv = sum > 0.f ? 1.f / sum : 0.f;
@@ -600,8 +583,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #pragma unroll 1
       for (int c = 0; c < D; c += 32) {
         uint32_t o[32];
-        if (n_tiles > 0) {
-          tmem_ld32(lane_addr + kOCol + (uint32_t)c, o);
+        if (nt > 0) {
+          tmem_ld32(lane_addr + (uint32_t)c, o);
         } else {
 #pragma unroll
           for (int i = 0; i < 32; ++i) o[i] = 0u;
@@ -627,7 +610,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   }
   __syncthreads();
   tc_fence_after();
-  if (warp == kMmaWarp) tmem_dealloc(tmem, kCols);
+  if (warp == kLoadWarp) tmem_dealloc(tmem, F::kCols);
 }
 
 static std::string g_err;
@@ -700,6 +683,9 @@ static int encode_rows_map(CUtensorMap* out, const void* base, int D, int rows, 
 struct Device {
   int sms = 0, smem_optin = 0, cc = 0;
 };
+static const void* kernel_of(int D, int T) {
+  return reinterpret_cast<const void*>(D == 128 ? &prefill_kernel<128, 1> : (T == 3 ? &prefill_kernel<64, 3> : &prefill_kernel<64, 1>));
+}
 static const Device* device_facts(int dev) {
   constexpr int kMax = 64;
   static Device facts[kMax];
@@ -714,11 +700,9 @@ static const Device* device_facts(int dev) {
           cudaDeviceGetAttribute(&d.smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
           cudaDeviceGetAttribute(&d.cc, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess)
         return nullptr;
-      if (d.cc == 10 &&
-          (cudaFuncSetAttribute(prefill_kernel<64, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem_optin) != cudaSuccess ||
-           cudaFuncSetAttribute(prefill_kernel<64, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem_optin) != cudaSuccess ||
-           cudaFuncSetAttribute(prefill_kernel<128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem_optin) != cudaSuccess))
-        return nullptr;
+      if (d.cc == 10)
+        for (const void* f : {kernel_of(64, 1), kernel_of(64, 3), kernel_of(128, 1)})
+          if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem_optin) != cudaSuccess) return nullptr;
       facts[dev] = d;
       known[dev].store(true, std::memory_order_release);
     }
@@ -735,7 +719,7 @@ struct Plan {
   int pack;         // query heads of a KV head in one tile
   int row_tiles;
   int64_t tiles;    // of all heads and batch entries
-  bool three;       // the form with one S accumulator, three CTAs to an SM
+  bool three;       // the form with three tiles a CTA
 };
 
 static Plan plan(int B, int H, int Hkv, int M, int N, int D, bool causal, int sms) {
@@ -747,23 +731,36 @@ static Plan plan(int B, int H, int Hkv, int M, int N, int D, bool causal, int sm
   const int64_t per_row = (int64_t)(H / r.pack) * B;
   r.row_tiles = (M + tile_m - 1) / tile_m;
   r.tiles = per_row * r.row_tiles;
-  // Three CTAs an SM do no more per time than two, and a tile then takes a quarter longer (every one: 1.2 us a KV tile,
-  // with two 0.9 beside another CTA and less alone).  Where all tiles fit the device at once so and two an SM need a
-  // second round, that round is the two shortest of a slot's tiles, one behind the other: it must be the longer way by
-  // more than the longest tile's loss.  Under a causal mask from the first token it never is.
-  // us with two / three, 32 / 8 heads, in brackets KV tiles of the slot against 1.4 times those of the longest tile:
-  //   causal 1185 x 1185 18.9 / 23.3 (2, 27), 1408 21.5 / 27.0 (8, 31), 1760 25.5 / 33.7 (19, 39), two sequences of 864
-  //   16.2 / 19.0 (10, 20); 1400 behind 600 tokens 30.9 / 38.9 (27, 45), behind 1600 54.8 / 57.2 (58, 66), behind 2600
-  //   81.5 / 77.0 (90, 88); two sequences of 777 behind 1223 46.6 / 41.5 (46, 45), behind 2223 71.3 / 59.8 (78, 66);
-  //   no mask, 1300 x 1300 35.9 / 32.5 (42, 29), 1760 x 4096 95.4 / 88.2 (128, 90).
+  // Which form.  One KV tile of a CTA takes 0.8 us where two tiles share the SM and 1.05 us where three do.  Where all tiles fit
+  // the device at once as threes and two an SM need a second round, that round is the two shortest of a slot's tiles, one behind the other: it
+  // must be the longer way by more than the longest tile's loss and what the threes lose by beginning later (us with one / three tiles a CTA,
+  // 32 / 8 heads, causal, 1408 x 1408 20.7 / 26.4, 1600 behind 700 tokens 38.1 / 41.2, behind 2496 81.8 / 68.3; no mask, 1300 x 1300
+  // 33.8 / 27.4, 1760 x 4096 89.2 / 85.2).  Above, by the KV tiles of the busiest of a few slots when CTAs are dealt out there and
+  // back, the longest first (no mask, 1900 x 1900 54.8 / 67.1, 3000 x 3000 117.9 / 100.6; causal, 2048 x 2048 31.9 / 37.1,
+  // 2600 x 2600 46.9 / 45.5, 4096 x 4096 102.1 / 92.5): of 63 such sizes the choice was 1.1 % over the better form on average.
   r.three = false;
   const int64_t slots = 2 * (int64_t)sms;
-  if (D == 64 && r.tiles > slots && r.tiles <= 3 * (int64_t)sms) {
-    auto kv_tiles = [&](int64_t rank) {   // of the rank-th tile, the longest first
-      const int64_t rows_end = (r.row_tiles - rank / per_row) * tile_m;
+  if (D == 64 && r.tiles > slots) {
+    auto kv_tiles = [&](int64_t rank, int group) {   // of the rank-th CTA, the longest first
+      const int64_t rows_end = (r.row_tiles - rank / per_row * group) * tile_m;
       return ((causal ? std::min<int64_t>(N, N - M + rows_end) : N) + kBN - 1) / kBN;
     };
-    r.three = 5 * (kv_tiles(slots - 1) + kv_tiles(slots)) > 7 * kv_tiles(0);
+    auto busiest = [&](int group, int64_t n_slots) {
+      const int64_t n = per_row * ((r.row_tiles + group - 1) / group);
+      int64_t most = 0;
+      for (int64_t q = 0; q < 5; ++q) {
+        const int64_t slot = q * (n_slots - 1) / 4;
+        int64_t sum = 0;
+        for (int64_t round = 0; round * n_slots < n && round < 64; ++round) {
+          const int64_t rank = round * n_slots + (round & 1 ? n_slots - 1 - slot : slot);
+          if (rank < n) sum += kv_tiles(rank, group);
+        }
+        most = std::max(most, sum);
+      }
+      return most;
+    };
+    if (r.tiles <= 3 * (int64_t)sms) r.three = 5 * (kv_tiles(slots - 1, 1) + kv_tiles(slots, 1)) > 7 * kv_tiles(0, 1);
+    else r.three = 5 * busiest(3, sms) < 4 * busiest(1, slots);
   }
   return r;
 }
@@ -795,18 +792,17 @@ int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, 
   if (!d) return fail(-1001, "mk_flash_prefill_bf16: cannot read the attributes of device %d", dev);
   if (d->cc != 10) return fail(-6, "mk_flash_prefill_bf16 needs an sm_100 device (compute capability %d.x found)", d->cc);
   const int smem_optin = d->smem_optin;
-  const int bn = kBN;                              // tokens per KV tile
   CUtensorMap mq, mkk, mv;
   const Plan pl = plan(B, H, Hkv, M, N, D, causal != 0, d->sms);
   const int pack = pl.pack;
   int rc = encode_query_map(&mq, q, D, M, H, B, q_strides[2], q_strides[1], q_strides[0], pack);
   if (rc) return rc;
-  rc = encode_rows_map(&mkk, k, D, N, Hkv, B, k_strides[2], k_strides[1], k_strides[0], bn, "k");
+  rc = encode_rows_map(&mkk, k, D, N, Hkv, B, k_strides[2], k_strides[1], k_strides[0], kBN, "k");
   if (rc) return rc;
-  rc = encode_rows_map(&mv, v, D, N, Hkv, B, v_strides[2], v_strides[1], v_strides[0], bn, "v");
+  rc = encode_rows_map(&mv, v, D, N, Hkv, B, v_strides[2], v_strides[1], v_strides[0], kBN, "v");
   if (rc) return rc;
-  const size_t tile = (size_t)(D / 64) * kBox, kv_tile = (size_t)(D / 64) * bn * 128;
-  const size_t smem = 1024 + tile + 4 * kv_tile + sizeof(Shared);
+  const int T = pl.three ? 3 : 1;
+  const size_t smem = D == 128 ? Form<128, 1>::kSmem : (T == 3 ? Form<64, 3>::kSmem : Form<64, 1>::kSmem);
   if ((int)smem > smem_optin) return fail(-4, "mk_flash_prefill_bf16: %zu bytes of shared memory needed, %d available", smem, smem_optin);
   Params p;
   p.o = reinterpret_cast<__nv_bfloat16*>(o);
@@ -815,23 +811,24 @@ int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, 
   p.o_sb = o_strides[0], p.o_sh = o_strides[1], p.o_sm = o_strides[2];
   p.B = B, p.H = H, p.Hkv = Hkv, p.M = M, p.N = N, p.D = D;
   p.causal = causal ? 1 : 0;
+  p.row_tiles = pl.row_tiles;
   p.pack = pack;
   p.pack_log2 = 0;
   while ((1 << p.pack_log2) < pack) ++p.pack_log2;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.timeout_ns = (uint64_t)(timeout_ms > 0 ? timeout_ms : 1000) * 1000000ull;
-  const dim3 grid(H / pack, B, pl.row_tiles);
+  const dim3 grid(H / pack, B, (pl.row_tiles + T - 1) / T);
   // Where this grid leaves slots empty (two CTAs an SM), the next one is let in late: its CTAs would pile up on the
   // SMs that are free now (causal, 32 / 8 heads, head dim 64, early / late: 777 x 777, 200 tiles 12.1 us / 11.2, 1024 x 1024,
   // 256 tiles 16.3 / 13.5).  With the slots taken several times over it makes no difference up to 62 us a pass (2048 x 2048
   // to two sequences of 2045), then early is 0.7 % faster (4096 x 4096 109.7 / 110.4); just above one round late would
-  // still be the better one (1185 x 1185, 304 tiles 18.5 / 16.0, 1500 x 1500, 376 tiles 22.2 / 20.4).  At 128 late is
-  // never behind by more than a run's noise.
-  p.next_early = D == 64 && !pl.three && pl.tiles >= 2 * (int64_t)d->sms ? 1 : 0;
+  // still be the better one (1185 x 1185, 304 tiles 18.5 / 16.0, 1500 x 1500, 376 tiles 22.2 / 20.4).  At 128 early is 1 to 3 %
+  // faster from two rounds on (2048 x 2048 36.9 / 37.3, 2190 x 2190 41.0 / 42.4).
+  p.next_early = !pl.three && pl.tiles >= 2 * (int64_t)d->sms ? 1 : 0;
   // the kernel may be placed while the one before it in the stream drains (it waits before it touches memory)
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
-  cfg.blockDim = dim3(pl.three ? kThreads<1> : kThreads<2>);
+  cfg.blockDim = dim3((5 * T + 1) * 32);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = reinterpret_cast<cudaStream_t>(cuda_stream);
   cudaLaunchAttribute attr[1];
@@ -839,9 +836,8 @@ int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = pl.three ? cudaLaunchKernelEx(&cfg, prefill_kernel<64, 1>, mq, mkk, mv, p)
-                  : D == 64 ? cudaLaunchKernelEx(&cfg, prefill_kernel<64, 2>, mq, mkk, mv, p)
-                            : cudaLaunchKernelEx(&cfg, prefill_kernel<128, 2>, mq, mkk, mv, p);
+  void* args[4] = {&mq, &mkk, &mv, &p};
+  cudaError_t e = cudaLaunchKernelExC(&cfg, kernel_of(D, T), args);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return fail(-(int)e - 1000, "mk_flash_prefill_bf16 launch: %s", cudaGetErrorString(e));
   return 0;
@@ -852,7 +848,7 @@ int mk_flash_prefill_plan(int B, int H, int Hkv, int M, int N, int D, int causal
   if (!out || B < 1 || H < 1 || Hkv < 1 || M < 1 || N < 1 || H % Hkv || (D != 64 && D != 128) || (causal && M > N) || sms < 1)
     return fail(-2, "mk_flash_prefill_plan: bad sizes");
   const Plan pl = plan(B, H, Hkv, M, N, D, causal != 0, sms);
-  out[0] = pl.three ? kCtasPerSm<1> : kCtasPerSm<2>, out[1] = pl.pack, out[2] = pl.row_tiles;
+  out[0] = pl.three ? 3 : 2, out[1] = pl.pack, out[2] = pl.row_tiles;
   out[3] = (int32_t)std::min<int64_t>(pl.tiles, INT32_MAX);
   return 0;
 }
