@@ -531,6 +531,14 @@ int mk_gemm_bf16(const void* a, const void* b, void* c, int M, int N, int K, int
 int mk_gemm_bf16_packed(const void* a, const void* b_packed, void* c, int M, int N, int K, int64_t lda, int64_t ldc,
                         void* workspace, uint64_t workspace_bytes, int split_k, int activation, int timeout_ms,
                         void* cuda_stream);
+/* mk_gemm_bf16 (or, with `packed`, mk_gemm_bf16_packed) from one record: the fields are the arguments. */
+typedef struct {
+  uint64_t a, b, c;                        /* device pointers */
+  uint64_t workspace, workspace_bytes, cuda_stream;
+  int64_t lda, ldb, ldc, split_k, timeout_ms;
+  int32_t M, N, K, activation, packed, reserved;
+} mk_gemm_call_t;
+int mk_gemm_bf16_call(const void* call /* mk_gemm_call_t, of any alignment */);
 int mk_gemm_bf16_status(const void* workspace, int32_t out[4]);
 /* How mk_gemm_bf16 cuts a product of these sizes on the current device (ldb: the
  * weight's row stride, 0 for a packed weight): out[0] 1 = CTA pairs on 256 weight
@@ -559,6 +567,17 @@ int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, 
                           int N, int D, const int64_t q_strides[3], const int64_t k_strides[3],
                           const int64_t v_strides[3], const int64_t o_strides[3], float scale, int causal,
                           void* workspace, uint64_t workspace_bytes, int timeout_ms, void* cuda_stream);
+/* The same from one record, for callers to whom an argument costs time (a foreign-function interface converts each of the 22
+ * above by itself): the fields are the arguments. */
+typedef struct {
+  uint64_t q, k, v, o, lse;                /* device pointers */
+  uint64_t workspace, workspace_bytes, cuda_stream;
+  int64_t q_strides[3], k_strides[3], v_strides[3], o_strides[3];
+  int64_t timeout_ms;
+  double scale;
+  int32_t B, H, Hkv, M, N, D, causal, reserved;
+} mk_flash_prefill_call_t;
+int mk_flash_prefill_call(const void* call /* mk_flash_prefill_call_t, of any alignment */);
 int mk_flash_prefill_status(const void* workspace, int32_t out[4]);
 /* How mk_flash_prefill_bf16 cuts a call of these sizes on a device of `sms` multiprocessors: out[0] tiles that share an SM (2,
  * a CTA each, or 3 in one CTA); [1] query heads of a KV head in one tile of 128 rows; [2] row tiles;

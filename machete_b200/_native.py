@@ -8,6 +8,7 @@ structures below mirror the C header field by field.
 from __future__ import annotations
 
 import ctypes as C
+import struct
 import threading
 from pathlib import Path
 
@@ -119,6 +120,10 @@ class Launch(C.Structure):
 
 LAUNCH_ROWWISE, LAUNCH_MATVEC, LAUNCH_ATTENTION = 0, 1, 2
 
+# mk_gemm_call_t and mk_flash_prefill_call_t as bytes: ctypes takes 0.1 us for each argument
+GEMM_CALL = struct.Struct("<6Q5q6i")
+PREFILL_CALL = struct.Struct("<8Q13qd8i")
+
 EXPORTS = [
     "mk_abi_version", "mk_last_error", "mk_device_info", "mk_workspace_bytes", "mk_create", "mk_run", "mk_launches_per_run",
     "mk_launch_plan", "mk_plan_launches",
@@ -126,9 +131,9 @@ EXPORTS = [
     "mk_update_op", "mk_read_counters", "mk_destroy",
     "mk_standalone_workspace_bytes", "mk_matvec_bf16", "mk_matvec_nvfp4", "mk_flash_decode",
     "mk_flash_decode_noalloc", "mk_flash_decode_noalloc_status",
-    "mk_gemm_bf16_workspace_bytes", "mk_gemm_bf16", "mk_gemm_bf16_packed", "mk_gemm_bf16_status", "mk_gemm_bf16_plan",
+    "mk_gemm_bf16_workspace_bytes", "mk_gemm_bf16", "mk_gemm_bf16_packed", "mk_gemm_bf16_call", "mk_gemm_bf16_status", "mk_gemm_bf16_plan",
     "mk_gemm_last_error",
-    "mk_flash_prefill_bf16", "mk_flash_prefill_plan", "mk_flash_prefill_status", "mk_flash_prefill_last_error",
+    "mk_flash_prefill_bf16", "mk_flash_prefill_call", "mk_flash_prefill_plan", "mk_flash_prefill_status", "mk_flash_prefill_last_error",
 ]
 
 _lib = None
@@ -211,6 +216,8 @@ def _declare(h: C.CDLL) -> None:
     h.mk_gemm_bf16.restype = C.c_int
     h.mk_gemm_bf16_packed.argtypes = [vp, vp, vp, i32, i32, i32, i64, i64, vp, u64, i32, i32, i32, vp]
     h.mk_gemm_bf16_packed.restype = C.c_int
+    h.mk_gemm_bf16_call.argtypes = [C.c_char_p]       # GEMM_CALL.pack(...): the bytes are the record
+    h.mk_gemm_bf16_call.restype = C.c_int
     h.mk_gemm_bf16_status.argtypes = [vp, C.POINTER(i32)]
     h.mk_gemm_bf16_status.restype = C.c_int
     h.mk_gemm_bf16_plan.argtypes = [i32, i32, i32, i64, C.POINTER(i32)]
@@ -220,6 +227,8 @@ def _declare(h: C.CDLL) -> None:
     h.mk_flash_prefill_bf16.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp, vp, vp, f32, i32,
                                         vp, u64, i32, vp]
     h.mk_flash_prefill_bf16.restype = C.c_int
+    h.mk_flash_prefill_call.argtypes = [C.c_char_p]   # PREFILL_CALL.pack(...)
+    h.mk_flash_prefill_call.restype = C.c_int
     h.mk_flash_prefill_plan.argtypes = [i32] * 8 + [C.POINTER(i32)]
     h.mk_flash_prefill_plan.restype = C.c_int
     h.mk_flash_prefill_status.argtypes = [vp, C.POINTER(i32)]

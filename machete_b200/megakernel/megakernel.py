@@ -298,12 +298,15 @@ class Megakernel:
             self._validate_tensors()
         self.compile()
         if stream is None:
-            handle = torch.cuda.current_stream(self._dev).cuda_stream
+            # (without building a Stream object, which takes longer than the validation: 16 x 1024 -> 1024 5.0 us a run, 4.0 so, which is the device's time)
+            handle = torch._C._cuda_getCurrentRawStream(self._dev)
         elif hasattr(stream, "cuda_stream"):
             handle = stream.cuda_stream
         else:
             handle = int(stream)
-        N.check(N.lib().mk_run(self._handle, C.c_void_p(handle)), "mk_run")
+        rc = N.lib().mk_run(self._handle, handle)
+        if rc:
+            N.check(rc, "mk_run")
         if sync:
             self.wait()
 
@@ -318,7 +321,7 @@ class Megakernel:
             self._validate_tensors()
         self.compile()
         if stream is None:
-            handle = torch.cuda.current_stream(self._dev).cuda_stream
+            handle = torch._C._cuda_getCurrentRawStream(self._dev)
         elif hasattr(stream, "cuda_stream"):
             handle = stream.cuda_stream
         else:
@@ -569,8 +572,9 @@ class Megakernel:
 
     def _validate_tensors(self) -> None:
         for op in self.ops:
+            refs = op.tensor_refs
             for name, ptr in op.tensor_ptrs.items():
-                ref = op.tensor_refs.get(name)
+                ref = refs.get(name)
                 if ref is not None and ref.data_ptr() != ptr:
                     raise RuntimeError(
                         f"{op.op_cls.__name__}: tensor '{name}' was reallocated after schedule(); "
