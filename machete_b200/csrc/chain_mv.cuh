@@ -3,7 +3,8 @@
 //
 // What a launch is bound by is HBM for a long product and, for the short ones of a decode step, the way from the end
 // of the kernel before to the first product and from the last product to the end of this one.  So:
-//   * weights do not depend on the kernel before: the ring of pages is filled before the wait for that kernel;
+//   * weights do not depend on the kernel before: the ring of pages is filled before the wait for that kernel, as far as the
+//     rows' way is not blocked by it (see MvLaunch::ahead);
 //   * what a launch needs to know is read before it waits for the kernel before (records are written by copies only, which
 //     no launch overtakes); in the parameters they would cost the host 0.6 us a KB of them at every launch;
 //   * a page is shared by AS warps.  The persistent kernel's warp rotates its products over independent accumulators
@@ -48,8 +49,9 @@ struct MvLaunch {
   int32_t stages, page_bytes, sets_log2;        // ring slots, and sets of slots for partial sums
   int32_t slot_off, act_off, page_off;          // shared memory, bytes
   // n / d as (n * magic) >> 22 for the small numbers here: rows by tokens a sequence, threads by 16-byte chunks of a row
-  int32_t s_magic, chunk_magic[kChainOps];
-  int32_t pad[12];
+  int32_t s_magic, stage_magic, chunk_magic[kChainOps];   // (stage: pages by ring slots)
+  int32_t ahead;                                          // pages that are requested before the rows are staged
+  int32_t pad[10];
 };
 // What a launch costs the host goes by where its parameters end: 24 or 32 bytes behind a multiple of 64 2.0 us, elsewhere 2.4 (NVIDIA
 // driver 580, 488 to 768 bytes, the stream idle; 16 x 1024 -> 1024 through Megakernel.run 5.3 us a pass with 600 bytes, 5.7 with 616).  Hence the pad:
@@ -706,15 +708,18 @@ __device__ __forceinline__ void chain_finish(Ctx& c, const mk_op_t* ops, const C
 }
 
 // Waits until the ring's slot holds its k-th page: when all `handed_back` shares of the earlier ones are in, and only then,
-// the barrier's parity says which page is there.  One vote for both.
+// the barrier's parity says which page is there.  One vote for both, and one straight way through where the page is there.
+__device__ __forceinline__ bool chain_page_there(Ctx& c, uint32_t slot, uint32_t k, uint32_t handed_back) {
+  const uint32_t released = *reinterpret_cast<volatile uint32_t*>(&c.ctrl->released[slot]);   // (looked at before the barrier)
+  const bool there = mbar_try_wait(full_bar(c, slot), k & 1u);
+  return __all_sync(0xffffffffu, there & (released >= handed_back));
+}
 __device__ __forceinline__ bool chain_acquire(Ctx& c, uint32_t slot, uint32_t k, uint32_t handed_back) {
-  volatile uint32_t* released = &c.ctrl->released[slot];
-  const uint32_t bar = full_bar(c, slot);
   uint64_t t0 = 0;
   for (;;) {
 #pragma unroll 1
     for (int i = 0; i < 64; ++i)
-      if (__all_sync(0xffffffffu, *released >= handed_back && mbar_try_wait(bar, k & 1u))) return true;
+      if (__builtin_expect(chain_page_there(c, slot, k, handed_back), 1)) return true;
     if (give_up_check(c, t0, MK_ST_TIMEOUT_PAGE_FULL, (int)slot, (int)k)) {
       c.dead = true;
       return false;
@@ -759,8 +764,8 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
   }
   const int units = local < total ? (total - local + count - 1) / count : 0;
   const int P = L.pages[op0], parts = L.parts[op0];
-  // pages of a unit go to AS warps each, or all of them to the same AS
-  const int step = L.spread ? AS : 0, arrivals = L.spread ? parts * AS : AS, last_pages = L.spread ? parts : 1;
+  // shares of a unit that its sum waits for, and pages that are the last of a partial sum
+  const int arrivals = L.spread ? parts * AS : AS, last_pages = L.spread ? parts : 1;
 
   const bool early = (L.flags & kChainEarlyLoads) != 0;
   if (c.warp == W) {
@@ -770,6 +775,7 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
       mbar_init(smem_u32(&c.ctrl->empty[c.lane]), AS);
       c.ctrl->released[c.lane] = 0;
     }
+    if (c.lane == 0) mbar_init(smem_u32(&c.ctrl->staged), 1);
     if (c.lane < 4) c.ctrl->mv_arrive[c.lane] = c.ctrl->mv_done[c.lane] = 0;
     if (c.lane == 0) c.ctrl->abort_flag = c.ctrl->pos_bad = 0;
     fence_mbar_init();
@@ -798,7 +804,8 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
         if (u == 0 && !early) prior_work_done();
 #pragma unroll 1
         for (int p = 0; p < P; ++p) {
-          if (k > 0 && !wait_mbar_one(c, empty_bar(c, slot), (k & 1u) ^ 1u, MK_ST_TIMEOUT_PAGE_EMPTY, (int)issued)) {
+          if ((issued == (uint32_t)L.ahead && !wait_mbar_one(c, smem_u32(&c.ctrl->staged), 0u, MK_ST_TIMEOUT_PAGE_EMPTY, (int)issued)) ||
+              (k > 0 && !wait_mbar_one(c, empty_bar(c, slot), (k & 1u) ^ 1u, MK_ST_TIMEOUT_PAGE_EMPTY, (int)issued))) {
             dead = true;
             break;
           }
@@ -888,6 +895,7 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
   // The next launch starts, and begins to fetch its weights, only now: its copies would stand in the way of this launch's
   // activations.  (No launch behind the first starts before all CTAs of this one have come here, behind the wait: what ran
   // before the program is visible to every load of the later launches, early or not.)
+  if (threadIdx.x == 0) mbar_arrive(smem_u32(&c.ctrl->staged));
   next_may_start();
 
   const int g = c.lane >> 2;
@@ -896,20 +904,38 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
   const bool f16s = WF == 2 && sop->i[MK_MV_WFMT] == MK_W_NVFP4_F16S32;
   constexpr int NA = Cut::NA, AN = Cut::AN, NN = Cut::NN;
   float4* slots = reinterpret_cast<float4*>(smem + L.slot_off);
-  uint32_t slot = 0, k = 0;          // the page's place in the ring, and pages in its slot before it
-  int turn = c.warp;                 // this warp less the warp whose turn the unit's first page is, mod W
-  for (int u = 0; u < units && !c.dead; ++u) {
+  // Groups of AS warps take the CTA's partial sums in turn (dealt out), or its units, and walk straight from one of their pages
+  // to the next.  Looking at all pages for those that are its own cost a warp some 1500 clocks between two pages of 4000
+  // clocks of products (NVFP4 1 x 4096 -> 14336), since taken branches wait for instructions: 8B NVFP4 step us batch 1 2255 ->
+  // 2194, batch 8 3516 -> 3410, 1B shape batch 16 1185 -> 1165.  (Aligned groups: with one warp more from unit to unit, so
+  // that the one that adds a unit up sits the next one out, 2233, 3487 and 1190.)
+  constexpr int G = W / AS;
+  const int h = c.warp & (AS - 1), grp = c.warp / AS;
+  const int a0 = (h & (Cut::AH - 1)) * AN, n0 = (h / Cut::AH) * NN;   // this warp's accumulators and n-tiles
+  // (rows past M read row 0: their columns of the accumulators are never stored.  The row's parity, which places
+  // its chunks, is the lane's: an odd lane of a missing row finds other values of row 0, as good as any.)
+  uint32_t xrow[NN];
+#pragma unroll
+  for (int n = 0; n < NN; ++n) {
+    const int m = (n0 + n) * 8 + g;
+    xrow[n] = c.act_u32 + (uint32_t)(m < M ? m : 0) * xs;
+  }
+  const int spread = L.spread;
+  const int u_step = spread ? 1 : G, q_step = spread ? G : 1;
+  int q0 = spread ? grp : 0;         // this group's first partial sum of unit u
+#pragma unroll 1
+  for (int u = spread ? 0 : grp; u < units && !c.dead; u += u_step) {
     const uint32_t set = (uint32_t)u & ((1u << L.sets_log2) - 1u), gen = (uint32_t)u >> L.sets_log2;
     float4* mine = slots + (size_t)set * (uint32_t)(parts * NA * NT) * 32u + c.lane;
     bool entered = false;
-    int part = 0;
 #pragma unroll 1
-    for (int p = 0; p < P; ++p) {
-      const int h = (turn - part * step) & (W - 1);
-      if (h < AS) {
+    for (int lap = 0; lap < P; lap += parts) {      // (pages of a unit beyond its partial sums go round again, in the ring's order)
+#pragma unroll 1
+      for (int part = q0; part < parts && lap + part < P; part += q_step) {
+        const int p = lap + part;
+        const uint32_t page_no = (uint32_t)(u * P + p), k = (uint32_t)small_div((int)page_no, L.stage_magic), slot = page_no - k * (uint32_t)L.stages;
         const uint32_t page = c.pages_u32 + slot * page_bytes;
-        // (only when all earlier pages of the slot are handed back does the barrier's parity say which page is there)
-        if (!chain_acquire(c, slot, k, k * AS)) break;
+        if (!chain_acquire(c, slot, k, k * AS)) goto out;
         const ChainUnit& cu = tab.unit[u & (kChainUnits - 1)];
         if (p == 0 && h == 0 && (cu.flags & (kEpiRope | kEpiResidual)) && c.lane < M) {
           // what the unit's epilogue reads: into L1 now
@@ -922,27 +948,20 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
             asm volatile("prefetch.global.L1 [%0];" ::"l"(op->p[MK_MV_P_EPI_RES] + (uint64_t)(row.er + cu.rowA0) * 2u));
           }
         }
-        const int a0 = (h & (Cut::AH - 1)) * AN, n0 = (h / Cut::AH) * NN;   // this warp's accumulators and n-tiles
         auto rec = [&](int a, int n) -> float4& { return mine[((part * NA + a0 + a) * NT + n0 + n) * 32]; };
         float acc[AN][NN][4];
 #pragma unroll
         for (int a = 0; a < AN; ++a)
 #pragma unroll
-          for (int n = 0; n < NN; ++n) {
-            if (p >= parts) {   // a further page of the same partial sum: this warp left it here
+          for (int n = 0; n < NN; ++n) acc[a][n][0] = acc[a][n][1] = acc[a][n][2] = acc[a][n][3] = 0.f;
+        if (__builtin_expect(lap > 0, 0)) {   // a further page of the same partial sum: this warp left it here
+#pragma unroll
+          for (int a = 0; a < AN; ++a)
+#pragma unroll
+            for (int n = 0; n < NN; ++n) {
               const float4 v = rec(a, n);
               acc[a][n][0] = v.x, acc[a][n][1] = v.y, acc[a][n][2] = v.z, acc[a][n][3] = v.w;
-            } else {
-              acc[a][n][0] = acc[a][n][1] = acc[a][n][2] = acc[a][n][3] = 0.f;
             }
-          }
-        // (rows past M read row 0: their columns of the accumulators are never stored.  The row's parity, which places
-        // its chunks, is the lane's: an odd lane of a missing row finds other values of row 0, as good as any.)
-        uint32_t xrow[NN];
-#pragma unroll
-        for (int n = 0; n < NN; ++n) {
-          const int m = (n0 + n) * 8 + g;
-          xrow[n] = c.act_u32 + (uint32_t)(m < M ? m : 0) * xs;
         }
         const int k0 = p * Kc, kc = min(Kc, K - k0);
         if constexpr (WF == 2)
@@ -954,7 +973,7 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
           mbar_arrive(empty_bar(c, slot));
           atomicAdd(&c.ctrl->released[slot], 1u);
         }
-        if (!entered && gen > 0 && !wait_smem_ge(c, &c.ctrl->mv_done[set], gen, u)) break;   // the set's previous user must have been summed
+        if (!entered && gen > 0 && !wait_smem_ge(c, &c.ctrl->mv_done[set], gen, u)) goto out;   // the set's previous user must have been summed
         entered = true;
 #pragma unroll
         for (int a = 0; a < AN; ++a)
@@ -973,15 +992,13 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
           if (last) chain_finish<ROWS, WF, NA, KS>(c, ops, rows, cu, local + u * count, mine, parts, set, gen);
         }
       }
-      if (++part == parts) part = 0;
-      if (++slot == (uint32_t)L.stages) {
-        slot = 0;
-        ++k;
-      }
     }
-    // (dealt out: one more, as the warps of a unit's last page arrive last and one of them adds the unit up)
-    turn = (turn - (L.spread ? arrivals + 1 : AS)) & (W - 1);
+    if (spread) {
+      q0 -= parts;
+      while (q0 < 0) q0 += G;
+    }
   }
+out:;
 }
 
 }  // namespace mk
