@@ -51,7 +51,8 @@ struct MvLaunch {
   // n / d as (n * magic) >> 22 for the small numbers here: rows by tokens a sequence, threads by 16-byte chunks of a row
   int32_t s_magic, stage_magic, chunk_magic[kChainOps];   // (stage: pages by ring slots)
   int32_t ahead;                                          // pages that are requested before the rows are staged
-  int32_t pad[10];
+  int32_t norm_off, res_off;                              // the norm's weights' and residual rows' place in the ring behind those pages, or -1
+  int32_t pad[8];
 };
 // What a launch costs the host goes by where its parameters end: 24 or 32 bytes behind a multiple of 64 2.0 us, elsewhere 2.4 (NVIDIA
 // driver 580, 488 to 768 bytes, the stream idle; 16 x 1024 -> 1024 through Megakernel.run 5.3 us a pass with 600 bytes, 5.7 with 616).  Hence the pad:
@@ -256,6 +257,184 @@ __device__ __forceinline__ void chain_stage_plain(Ctx& c, const mk_op_t* op, int
         unpack8(v[j], MK_T_BF16, f);
         sts128(at[j], pack8(f, MK_T_FP16));
       }
+    }
+  }
+}
+
+// Whether a kernel's rows come by bulk copies: nine rows and more of dense weights, and NVFP4 rows of sixteen warps.  (us a step, rows
+// through registers and by copies: 8B NVFP4 batch 8 3391 / 3206, batch 6 - / 2421; 1B shape batch 16 1136 / 1113, batch 8 787 / 789,
+// batch 4 732 / 753, batch 2 694 / 711; one row, and NVFP4 4 x 4096 -> 14336 by eight warps, 13.7 / 14.8, are slower so too.)
+__host__ __device__ constexpr bool chain_fetches(int rows, int wf, int warps) { return warps == 16 && (rows == 16 || wf == 2); }
+// The rows come by bulk copies, a lane's row each, to where they are staged; residual rows
+// and the norm's weights to ring slots that the loader leaves empty until then.  They are there after some 2000 clocks, and
+// what is left is arithmetic: every warp's jobs side by side, a norm weight unpacked once for all rows.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+template <int WF>
+__device__ __forceinline__ void chain_fetch_rows(Ctx& c, const MvLaunch& L, const mk_op_t* op, int M, const ChainIn* in) {
+  const int K = op->i[MK_MV_K];
+  const uint32_t bytes = (uint32_t)K * 2u, bar = smem_u32(&c.ctrl->rows_in);
+  const uint16_t* x = reinterpret_cast<const uint16_t*>(op->p[MK_MV_P_X]);
+  const uint16_t* ri = reinterpret_cast<const uint16_t*>(op->p[MK_MV_P_RES_IN]);
+  const bool norm = op->i[MK_MV_PRO] != MK_PRO_NONE && L.norm_off >= 0;
+  const bool add = op->i[MK_MV_PRO] == MK_PRO_ADD_RMS && ri != nullptr && L.res_off >= 0;
+  if (c.warp == 0) {
+    if (c.lane == 0) {
+      mbar_arrive_expect_tx(bar, ((uint32_t)M * (add ? 2u : 1u) + (norm ? 1u : 0u)) * bytes);
+      if (norm) bulk_load(c.pages_u32 + (uint32_t)L.norm_off, reinterpret_cast<const void*>(op->p[MK_MV_P_NORM_W]), bytes, bar);
+    }
+    __syncwarp();
+    if (c.lane < M) {
+      bulk_load(c.act_u32 + (uint32_t)c.lane * chain_row_stride<WF>(K), x + in[c.lane].x, bytes, bar);
+      if (add) bulk_load(c.pages_u32 + (uint32_t)L.res_off + (uint32_t)c.lane * bytes, ri + in[c.lane].ri, bytes, bar);
+    }
+    __syncwarp();
+  }
+  uint64_t t0 = 0;
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 64; ++i)
+      if (__builtin_expect(__all_sync(0xffffffffu, mbar_try_wait(bar, 0u)), 1)) return;
+    if (give_up_check(c, t0, MK_ST_TIMEOUT_PAGE_FULL, -1, 0)) {
+      c.dead = true;
+      return;
+    }
+  }
+}
+
+// chain_stage_rms for rows that lie in shared memory, with the same jobs and sums.  Rows are changed where they lie: a warp reads
+// 32 chunks and writes them back, NVFP4 rows to other places among the same eight (see chain_chunk).
+template <int WF, int R, int W>
+__device__ __forceinline__ void chain_norm_rows(Ctx& c, const MvLaunch& L, const mk_op_t* op, const ChainIn* in, const mk_op_t* res_op) {
+  constexpr int T = kConsumerWarps * 32;
+  const int K = op->i[MK_MV_K], M = op->i[MK_MV_M];
+  const uint32_t xs = chain_row_stride<WF>(K);
+  const int chunks = K >> 3;
+  const uint16_t* ri = reinterpret_cast<const uint16_t*>(op->p[MK_MV_P_RES_IN]);
+  const uint16_t* nw = reinterpret_cast<const uint16_t*>(op->p[MK_MV_P_NORM_W]);
+  const bool add = op->i[MK_MV_PRO] == MK_PRO_ADD_RMS && ri != nullptr;
+  uint16_t* ro = add && res_op ? reinterpret_cast<uint16_t*>(res_op->p[MK_MV_P_RES_OUT]) : nullptr;
+  const uint4 z = make_uint4(0, 0, 0, 0);
+  auto norm_w = [&](int ch) { return L.norm_off >= 0 ? lds128(c.pages_u32 + (uint32_t)L.norm_off + (uint32_t)ch * 16u) : *reinterpret_cast<const uint4*>(nw + ch * 8); };
+  const int jobs = kConsumerWarps * M;
+#pragma unroll 1
+  for (int j0 = c.warp; j0 < jobs; j0 += R * W) {
+    int row[R], part[R];
+    float sum[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int job = j0 + j * W;
+      row[j] = job / kConsumerWarps;
+      part[j] = job < jobs ? (job - row[j] * kConsumerWarps) * 32 : chunks;   // (a missing job has no chunks)
+      sum[j] = 0.f;
+    }
+#pragma unroll 1
+    for (int base = 0; base < chunks; base += T) {
+      bool any = false;
+#pragma unroll
+      for (int j = 0; j < R; ++j) any |= base + part[j] < chunks;
+      if (!any) break;
+      uint4 v[R], r[R], wv[R];
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        const int ch = base + part[j] + c.lane;
+        const bool ok = ch < chunks;
+        v[j] = ok ? lds128(c.act_u32 + (uint32_t)row[j] * xs + (uint32_t)ch * 16u) : z;
+        r[j] = wv[j] = z;
+        if (ok && add) r[j] = L.res_off >= 0 ? lds128(c.pages_u32 + (uint32_t)L.res_off + (uint32_t)(row[j] * chunks + ch) * 16u) : ldcg128(ri + in[row[j]].ri + ch * 8);
+        if (WF == 0 && ok) wv[j] = norm_w(ch);
+      }
+      if (WF == 2) __syncwarp();
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        const int ch = base + part[j] + c.lane;
+        if (ch >= chunks) continue;
+        uint4 o = v[j];
+        if (add) {
+          o = add8(o, r[j], MK_T_BF16);
+          if (ro) *reinterpret_cast<uint4*>(ro + in[row[j]].ro + ch * 8) = o;
+        }
+        float f[8];
+        unpack8(o, MK_T_BF16, f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sum[j] += f[i] * f[i];
+        if (WF == 0) o = mul8_bf16(o, wv[j]);
+        sts128(c.act_u32 + (uint32_t)row[j] * xs + chain_chunk<WF>(row[j], ch), o);
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int j = 0; j < R; ++j) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], o);
+#pragma unroll
+    for (int j = 0; j < R; ++j)
+      if (c.lane == 0 && j0 + j * W < jobs) c.ctrl->red[j0 + j * W] = sum[j];   // = row * 7 + the job's warp
+  }
+  if constexpr (WF == 2) {
+    // second pass: normalise and convert to the products' type, a thread the same chunk of every row
+    named_bar_sync(kChainBarrier, W * 32);
+    float rstd = 0.f;                      // of row `lane`
+    if (c.lane < M) {
+      float tot = 0.f;
+#pragma unroll
+      for (int w = 0; w < kConsumerWarps; ++w) tot += c.ctrl->red[c.lane * kConsumerWarps + w];
+      rstd = rsqrtf(tot / (float)K + op->f[MK_MV_F_EPS]);
+    }
+#pragma unroll 1
+    for (int ch0 = c.warp * 32; ch0 < chunks; ch0 += W * 32) {
+      const int ch = ch0 + c.lane;
+      const bool ok = ch < chunks;
+      float w[8];
+      unpack8(ok ? norm_w(ch) : z, MK_T_BF16, w);
+#pragma unroll 4
+      for (int m = 0; m < M; ++m) {
+        const float rs = __shfl_sync(0xffffffffu, rstd, m);
+        const uint32_t at = c.act_u32 + (uint32_t)m * xs + chain_chunk<WF>(m, ok ? ch : 0);
+        float f[8];
+        unpack8(ok ? lds128(at) : z, MK_T_BF16, f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] = f[i] * rs * w[i];
+        if (ok) sts128(at, pack8(f, MK_T_FP16));
+      }
+    }
+  }
+}
+
+// Fetched rows without a prologue are staged as they come, but for NVFP4 weights, whose products take f16: a thread's chunks as in
+// chain_stage_plain, four a turn.  (Eight chunks that change places are one warp's, in one turn: all are read before one is written.)
+template <int W>
+__device__ __forceinline__ void chain_to_f16(Ctx& c, const mk_op_t* op, int M, const ChainWalk& w) {
+  const int K = op->i[MK_MV_K];
+  const uint32_t xs = chain_row_stride<2>(K);
+  const int chunks = K >> 3;
+  int m = w.m0, ch = w.ch0;
+#pragma unroll 1
+  for (int done = 0; done < M * chunks; done += 4 * W * 32) {
+    uint4 v[4];
+    uint32_t at[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      at[j] = 0u;
+      if (m < M) {
+        v[j] = lds128(c.act_u32 + (uint32_t)m * xs + (uint32_t)ch * 16u);
+        at[j] = c.act_u32 + (uint32_t)m * xs + chain_chunk<2>(m, ch);
+      }
+      m += w.dm;
+      ch += w.dch;
+      if (ch >= chunks) {
+        ch -= chunks;
+        ++m;
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (at[j] == 0u) break;
+      float f[8];
+      unpack8(v[j], MK_T_BF16, f);
+      sts128(at[j], pack8(f, MK_T_FP16));
     }
   }
 }
@@ -775,7 +954,10 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
       mbar_init(smem_u32(&c.ctrl->empty[c.lane]), AS);
       c.ctrl->released[c.lane] = 0;
     }
-    if (c.lane == 0) mbar_init(smem_u32(&c.ctrl->staged), 1);
+    if (c.lane == 0) {
+      mbar_init(smem_u32(&c.ctrl->staged), 1);
+      mbar_init(smem_u32(&c.ctrl->rows_in), 1);
+    }
     if (c.lane < 4) c.ctrl->mv_arrive[c.lane] = c.ctrl->mv_done[c.lane] = 0;
     if (c.lane == 0) c.ctrl->abort_flag = c.ctrl->pos_bad = 0;
     fence_mbar_init();
@@ -883,7 +1065,14 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
   }
   if (units > 0) {
     const mk_op_t* res_op = L.res_op >= 0 && blockIdx.x == 0 ? ops + L.res_op : nullptr;
-    if (pro == MK_PRO_NONE) {
+    if constexpr (chain_fetches(ROWS, WF, W)) {
+      chain_fetch_rows<WF>(c, L, sop, M, tab.in);
+      if (pro == MK_PRO_NONE) {
+        if constexpr (WF == 2) chain_to_f16<W>(c, sop, M, walk);
+      } else if constexpr (WF != 1) {
+        chain_norm_rows<WF, 4, W>(c, L, sop, tab.in, res_op);
+      }
+    } else if (pro == MK_PRO_NONE) {
       chain_stage_plain<WF>(c, sop, M, tab.in, walk);
     } else if constexpr (WF != 1) {
       // rows' parts, and chunks of each, requested together

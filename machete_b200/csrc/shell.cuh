@@ -128,7 +128,7 @@ enum {
 struct Ctrl {
   uint64_t full[kMaxPages];
   uint64_t empty[kMaxPages];
-  uint64_t staged;     // (chains) the launch's rows are there, and its loader may go on
+  uint64_t rows_in, staged;   // (chains) the launch's rows have arrived; they are staged, and its loader may go on
   int32_t abort_flag;
   int32_t is_last;
   // Split-K slot sets: arrivals of the current user, and how many users of
