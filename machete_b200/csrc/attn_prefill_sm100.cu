@@ -824,8 +824,10 @@ int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, 
   // 256 tiles 16.3 / 13.5).  With the slots taken several times over it makes no difference up to 62 us a pass (2048 x 2048
   // to two sequences of 2045), then early is 0.7 % faster (4096 x 4096 109.7 / 110.4); just above one round late would
   // still be the better one (1185 x 1185, 304 tiles 18.5 / 16.0, 1500 x 1500, 376 tiles 22.2 / 20.4).  At 128 early is 1 to 3 %
-  // faster from two rounds on (2048 x 2048 36.9 / 37.3, 2190 x 2190 41.0 / 42.4).
-  p.next_early = !pl.three && pl.tiles >= 2 * (int64_t)d->sms ? 1 : 0;
+  // faster between one and a half rounds and three (2048 x 2048 36.9 / 37.3, 2190 x 2190 41.0 / 42.4), late below (1600 x 1600 28.1 / 26.8)
+  // and, by the power it takes, above (4096 x 4096 148.4 / 146.0 back to back).
+  const int64_t sms = d->sms;
+  p.next_early = !pl.three && (D == 64 ? pl.tiles >= 2 * sms : pl.tiles > 3 * sms && pl.tiles < 6 * sms) ? 1 : 0;
   // the kernel may be placed while the one before it in the stream drains (it waits before it touches memory)
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
