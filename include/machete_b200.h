@@ -390,6 +390,9 @@ typedef struct mk_launch {
  * `smem_optin` bytes of shared memory a CTA; pointers in the program are not followed but for its tables. */
 int mk_launch_plan(mk_handle_t h, mk_launch_t* out, int32_t max);
 int mk_plan_launches(const mk_program_t* prog, int32_t num_sms, int32_t smem_optin, mk_launch_t* out, int32_t max);
+/* Where a matvec launch with a ring of `stages` slots puts a CTA's page, counted from 0: out[0] the slot, out[1] the pages in
+ * that slot before it. */
+int mk_ring_place(int32_t stages, int64_t page, int32_t out[2]);
 /* Copy the 16-word device status block to `out` (synchronises the device).
  * out[0] == 0 means no device-side error. */
 int mk_status(mk_handle_t h, int32_t out[16]);

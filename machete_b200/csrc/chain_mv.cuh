@@ -49,7 +49,7 @@ struct MvLaunch {
   int32_t stages, page_bytes, sets_log2;        // ring slots, and sets of slots for partial sums
   int32_t slot_off, act_off, page_off;          // shared memory, bytes
   // n / d as (n * magic) >> 22 for the small numbers here: rows by tokens a sequence, threads by 16-byte chunks of a row
-  int32_t s_magic, stage_magic, chunk_magic[kChainOps];   // (stage: pages by ring slots)
+  int32_t s_magic, stage_magic, chunk_magic[kChainOps];   // (stage: pages by ring slots, see ring_lap)
   int32_t ahead;                                          // pages that are requested before the rows are staged
   int32_t norm_off, res_off;                              // the norm's weights' and residual rows' place in the ring behind those pages, or -1
   int32_t pad[8];
@@ -76,6 +76,13 @@ struct ChainUnit {
 enum { kEpiNormed = 1, kEpiScaled = 2, kEpiPair = 4, kEpiRope = 8, kEpiSiluMul = 16, kEpiRelu = 32, kEpiSilu = 64, kEpiResidual = 128,
        kEpiTop1 = 256, kEpiFp32 = 512, kEpiFp16 = 1024, kEpiKsum = 2048 };
 __device__ __forceinline__ int small_div(int n, int magic) { return (int)(((uint32_t)n * (uint32_t)magic) >> 22); }
+// How often the ring has gone round before a CTA's page: page / stages.  The product has 64 bits, as a CTA's pages are as many as its
+// share of the weights has (in 32 bits it wraps at 1024 pages a slot); exact below 2^30 / kChainMaxStages pages, of which a chain
+// has fewer (kChainMaxPages).
+__host__ __device__ constexpr uint32_t ring_magic(int stages) { return ((1u << 30) + (uint32_t)stages - 1u) / (uint32_t)stages; }
+__host__ __device__ constexpr uint32_t ring_lap(uint32_t page, uint32_t magic) { return (uint32_t)(((uint64_t)page * magic) >> 30); }
+constexpr int64_t kChainMaxPages = 1 << 26;      // of a launch
+static_assert(kChainMaxPages * kChainMaxStages <= 1 << 30, "ring_lap must be exact");
 constexpr int kChainUnits = 32;   // units between the loader's and the last finisher's: at most 12 pages + 4 slot sets
 struct ChainTab {
   ChainIn in[32];
@@ -1122,7 +1129,7 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
 #pragma unroll 1
       for (int part = q0; part < parts && lap + part < P; part += q_step) {
         const int p = lap + part;
-        const uint32_t page_no = (uint32_t)(u * P + p), k = (uint32_t)small_div((int)page_no, L.stage_magic), slot = page_no - k * (uint32_t)L.stages;
+        const uint32_t page_no = (uint32_t)(u * P + p), k = ring_lap(page_no, (uint32_t)L.stage_magic), slot = page_no - k * (uint32_t)L.stages;
         const uint32_t page = c.pages_u32 + slot * page_bytes;
         if (!chain_acquire(c, slot, k, k * AS)) goto out;
         const ChainUnit& cu = tab.unit[u & (kChainUnits - 1)];

@@ -1023,6 +1023,15 @@ int mk_plan_launches(const mk_program_t* prog, int32_t num_sms, int32_t smem_opt
   return guarded([&] { return plan_launches(prog, num_sms, smem_optin, out, max); });
 }
 
+int mk_ring_place(int32_t stages, int64_t page, int32_t out[2]) {
+  using namespace mk;
+  if (!out || stages < 1 || stages > kChainMaxStages || page < 0 || page >= kChainMaxPages) return fail(-1, "mk_ring_place: bad argument");
+  const uint32_t lap = ring_lap((uint32_t)page, ring_magic(stages));
+  out[0] = (int32_t)((uint32_t)page - lap * (uint32_t)stages);
+  out[1] = (int32_t)lap;
+  return 0;
+}
+
 int mk_launches_per_run(mk_handle_t h) {
   if (!h) return 0;
   return guarded([&] { return h->pv.trace != nullptr ? 1 : std::max(1, (int)current_plan(h)->steps.size()); });
