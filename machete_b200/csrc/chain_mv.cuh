@@ -279,6 +279,22 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
                : "memory");
 }
+// A warp has given up its wait for them, or something has gone wrong elsewhere.  The copies must have landed before the CTA exits, so it
+// waits on, with a limit.  Where they do not come the CTA stores nothing of them: its copies of the records lose their residual
+// outputs, which a warp reads behind this, and its units get an arrival count that no sum waits for.
+static __device__ __noinline__ void rows_late(const MvLaunch* L, Ctrl* ctrl, uint32_t bar) {
+  const uint64_t t0 = globaltimer_ns();
+  for (;;) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, 0u))) return;
+    if (__any_sync(0xffffffffu, globaltimer_ns() - t0 > L->pv.timeout_ns)) break;
+  }
+  if ((threadIdx.x & 31) == 0) {
+    for (int set = 0; set < 4; ++set) atomicOr(&ctrl->mv_arrive[set], 0x80000000u);
+    mk_op_t* ops = reinterpret_cast<ChainTab*>(reinterpret_cast<uint8_t*>(ctrl) + kCtrlStructBytes)->op;
+    for (int i = 0; i < L->n_ops; ++i) *reinterpret_cast<volatile uint64_t*>(&ops[i].p[MK_MV_P_RES_OUT]) = 0;
+  }
+  __syncwarp();
+}
 template <int WF>
 __device__ __forceinline__ void chain_fetch_rows(Ctx& c, const MvLaunch& L, const mk_op_t* op, int M, const ChainIn* in) {
   const int K = op->i[MK_MV_K];
@@ -305,6 +321,7 @@ __device__ __forceinline__ void chain_fetch_rows(Ctx& c, const MvLaunch& L, cons
     for (int i = 0; i < 64; ++i)
       if (__builtin_expect(__all_sync(0xffffffffu, mbar_try_wait(bar, 0u)), 1)) return;
     if (give_up_check(c, t0, MK_ST_TIMEOUT_PAGE_FULL, -1, 0)) {
+      rows_late(&L, c.ctrl, bar);
       c.dead = true;
       return;
     }
