@@ -563,7 +563,7 @@ const char* mk_gemm_last_error(void);
  *   (B,N,Hkv,D) cache views fit), D = 64 or 128 contiguous, every stride a
  *   multiple of 8 elements, bases 16-byte aligned.  lse: [B][H][M] fp32 or NULL.
  *   workspace: 256 bytes of device memory, 256-byte aligned, ZERO before first
- *   use (the device status block; it stays zero unless a wait ran out).
+ *   use (the device status block; it stays zero unless a wait ran out).  scale: any finite value.
  * Returns 0 or a negative code (mk_flash_prefill_last_error); a device-side
  * time-out shows in mk_flash_prefill_status (out[0] != 0), which synchronises. */
 int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, float* lse, int B, int H, int Hkv, int M,

@@ -39,6 +39,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <float.h>
 #include <math.h>
 #include <stdarg.h>
 #include <stdint.h>
@@ -47,6 +48,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <mutex>
 #include <string>
 #include <type_traits>
@@ -65,12 +67,13 @@ struct Params {
   float* lse;            // [B, H, M] or null
   int32_t* status;
   int64_t o_sb, o_sh, o_sm;
-  int B, H, Hkv, M, N, D;
+  int B, H, Hkv, M, N;
+  uint32_t negate_q;     // the product descriptor's bit that takes -Q (a negative scale)
   int causal;
   int row_tiles;
   int pack, pack_log2;   // query heads of a KV head in one tile: row r is query r >> pack_log2 of head r & (pack - 1)
   int next_early;        // the kernel behind this one may be placed from the start (else: with the last load)
-  float scale_log2;      // scale * log2(e)
+  float scale_log2;      // |scale| * log2(e), > 0
   uint64_t timeout_ns;
 };
 
@@ -431,7 +434,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     // products of tile i, in the order S(0), S(1), P V(0), S(2), P V(1), ...
     // (the tile, and with it every descriptor, is known to be uniform: see tc_mma)
     const int i = T == 1 ? 0 : __shfl_sync(0xffffffffu, warp - 4 * T, 0), nt = kv_tiles(i);
-    const uint32_t id_s = idesc_bf16(kBN, false), id_o = idesc_bf16(D, true), elected = elect_one() ? 1u : 0u;
+    const uint32_t id_s = idesc_bf16(kBN, false) | p.negate_q, id_o = idesc_bf16(D, true), elected = elect_one() ? 1u : 0u;
     const uint32_t o = tmem + i * F::kTileCols, q = q_s + i * F::kQTile;
     const uint32_t s_full = mk::smem_u32(&sh->s_full[2 * i]), s_free = mk::smem_u32(&sh->s_free[i]);
     const uint32_t p_ready = mk::smem_u32(&sh->p_ready[2 * i]), pv_done = mk::smem_u32(&sh->pv_done[2 * i]);
@@ -521,7 +524,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #pragma unroll
         for (int u = 0; u < 4; ++u) t4[u] = max3(t4[u], __uint_as_float(r[i + 2 * u]), __uint_as_float(r[i + 2 * u + 1]));
       }
-      const float tmax = max3(fmaxf(t4[0], t4[1]), t4[2], t4[3]) * p.scale_log2;   // the scale is positive
+      const float tmax = max3(fmaxf(t4[0], t4[1]), t4[2], t4[3]) * p.scale_log2;   // positive: see mk_flash_prefill_bf16
       // mx is the exponent reference in use, not the running maximum: it moves only when a maximum has grown
       // by more than 2^8 since it was set, so O is rescaled rarely (and no P exceeds 2^8).
       if (__builtin_expect(__any_sync(0xffffffffu, tmax > mx + 8.f), 0)) {     // also the first visible tile (mx = -inf)
@@ -783,6 +786,8 @@ int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, 
     return fail(-2, "mk_flash_prefill_bf16: B, H, Hkv, M, N must be positive and H a multiple of Hkv");
   if (D != 64 && D != 128) return fail(-2, "mk_flash_prefill_bf16: head dim must be 64 or 128, got %d", D);
   if (B > 65535 || (M + 127) / 128 > 65535) return fail(-2, "mk_flash_prefill_bf16: at most 65535 batch entries and 65535 query tiles of 128 rows");
+  const float scale_log2 = scale * 1.4426950408889634f;
+  if (!std::isfinite(scale_log2)) return fail(-2, "mk_flash_prefill_bf16: the scale must be finite");
   if (causal && M > N) return fail(-2, "mk_flash_prefill_bf16: causal attention needs M <= N (the queries are the last M tokens)");
   if (workspace_bytes < 256 || ((uint64_t)workspace & 255)) return fail(-2, "mk_flash_prefill_bf16: workspace of 256 aligned bytes");
   if (((uint64_t)o & 15) || o_strides[2] % 8 || o_strides[1] % 8 || o_strides[0] % 8)
@@ -810,13 +815,16 @@ int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, 
   p.lse = lse;
   p.status = reinterpret_cast<int32_t*>(workspace);
   p.o_sb = o_strides[0], p.o_sh = o_strides[1], p.o_sm = o_strides[2];
-  p.B = B, p.H = H, p.Hkv = Hkv, p.M = M, p.N = N, p.D = D;
+  p.B = B, p.H = H, p.Hkv = Hkv, p.M = M, p.N = N;
   p.causal = causal ? 1 : 0;
   p.row_tiles = pl.row_tiles;
   p.pack = pack;
   p.pack_log2 = 0;
   while ((1 << p.pack_log2) < pack) ++p.pack_log2;
-  p.scale_log2 = scale * 1.4426950408889634f;
+  // The row threads take the maximum of the scores before they scale it, and mask with -inf: the factor there is positive.  The sign of the
+  // scale goes to the products, and zero becomes the smallest normal number, times which no score differs from another.
+  p.scale_log2 = std::max(std::fabs(scale_log2), FLT_MIN);
+  p.negate_q = scale < 0.f ? 1u << 13 : 0u;
   p.timeout_ns = (uint64_t)(timeout_ms > 0 ? timeout_ms : 1000) * 1000000ull;
   const dim3 grid(H / pack, B, (pl.row_tiles + T - 1) / T);
   // Where this grid leaves slots empty (two CTAs an SM), the next one is let in late: its CTAs would pile up on the

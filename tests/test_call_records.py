@@ -1,6 +1,7 @@
 """The records that carry the arguments of a prompt attention and of a GEMM to the library (CPU): sizes, order and refusals."""
 
 import ctypes as C
+import math
 
 import pytest
 
@@ -32,9 +33,9 @@ def test_a_packed_record_is_the_c_structure(fmt, cls):
     assert flat == values
 
 
-def _prefill(q=1 << 20, B=1, H=8, Hkv=2, M=4, Nk=4, D=64, causal=1, ws=1 << 20, ws_bytes=256):
+def _prefill(q=1 << 20, B=1, H=8, Hkv=2, M=4, Nk=4, D=64, causal=1, ws=1 << 20, ws_bytes=256, scale=0.125):
     strides = (H * M * D, M * D, D, Hkv * Nk * D, Nk * D, D, Hkv * Nk * D, Nk * D, D, H * M * D, M * D, D)
-    return N.lib().mk_flash_prefill_call(N.PREFILL_CALL.pack(q, q, q, q, 0, ws, ws_bytes, 0, *strides, 1000, 0.125, B, H, Hkv, M, Nk, D, causal, 0))
+    return N.lib().mk_flash_prefill_call(N.PREFILL_CALL.pack(q, q, q, q, 0, ws, ws_bytes, 0, *strides, 1000, scale, B, H, Hkv, M, Nk, D, causal, 0))
 
 
 def test_refusals_are_those_of_the_argument_form():
@@ -43,6 +44,9 @@ def test_refusals_are_those_of_the_argument_form():
     assert _prefill(q=0) == -1
     for bad in (dict(D=96), dict(Hkv=3), dict(M=5), dict(M=0), dict(ws_bytes=255), dict(ws=(1 << 20) + 128)):
         assert _prefill(**bad) == -2, bad
+    for scale in (math.nan, math.inf, -math.inf, 1e39, 3e38):        # (3e38 * log2(e) is beyond fp32)
+        assert _prefill(scale=scale) == -2, scale
+        assert b"scale" in lib.mk_flash_prefill_last_error()
     one = 1 << 20
 
     def gemm(a=one, K=64, lda=64, packed=0, act=0):

@@ -55,3 +55,19 @@ def test_the_form_leaves_the_bits():
         for b in range(2):
             flash_prefill(q[b:b + 1], k[b:b + 1], v[b:b + 1], each[b:b + 1], causal=True, check_status=True)
         assert torch.equal(both, each)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,M,Nk,causal", [(1, 200, 333, True), (1, 130, 77, False), (2, 777, 2000, True)])
+@pytest.mark.parametrize("scale", [-0.125, 0.0, -0.0, 1e-40, -3.0])
+def test_scales_of_either_sign_and_none(D, B, M, Nk, causal, scale):
+    # masked scores leave the softmax whatever the sign; no scale is the mean over the visible tokens
+    g = torch.Generator(device="cuda").manual_seed(M + D)
+    q = torch.randn(B, 32, M, D, generator=g, device="cuda").to(BF)
+    k, v = (torch.randn(B, 8, Nk, D, generator=g, device="cuda").to(BF) for _ in range(2))
+    o, lse = torch.full_like(q, 7.0), torch.zeros(B, 32, M, device="cuda")
+    flash_prefill(q, k, v, o, causal=causal, scale=scale, lse=lse, check_status=True)
+    want, want_lse = _reference(q.double() * (scale * D ** 0.5), k, v, causal)
+    assert_parity(o, want, f"scale {scale}")
+    # (fp32 products of D terms of size 1, scaled: a few 2^-24 of the largest score, some 40 * 3)
+    assert float((lse.double() - want_lse).abs().max()) < 2e-3
