@@ -35,6 +35,36 @@ def test_edges_of_the_window():
     assert plan(1, 1300, 1300, causal=False, H=8, Hkv=8)[1:] == [1, 11, 88]
 
 
+@pytest.mark.parametrize("B,M,Nk,causal,form", [(1, 2048, 2048, True, 2), (1, 2600, 2600, True, 2), (1, 4096, 4096, True, 3), (1, 1900, 1900, False, 2),
+                                                (1, 3000, 3000, False, 3), (2, 4096, 4096, True, 3)])
+def test_several_rounds(B, M, Nk, causal, form):
+    assert plan(B, M, Nk, causal=causal)[0] == form and plan(B, M, Nk, causal=causal)[3] > 444
+
+
+def _busiest(B, M, Nk, causal, group, slots):
+    """KV tiles of the busiest of five slots, every CTA dealt out there and back, the longest first."""
+    rows, per_row = -(-M // 32), 8 * B
+    n = per_row * -(-rows // group)
+
+    def kv(rank):
+        end = (rows - rank // per_row * group) * 32
+        return -(-(min(Nk, Nk - M + end) if causal else Nk) // 64)
+
+    def slot_sum(slot):
+        ranks = (r * slots + (slots - 1 - slot if r & 1 else slot) for r in range(-(-n // slots)))
+        return sum(kv(x) for x in ranks if x < n)
+    return max(slot_sum(q * (slots - 1) // 4) for q in range(5))
+
+
+# 60 to 4000 rounds; short prompts of which each has one CTA of three tiles or two, filled or not
+@pytest.mark.parametrize("B,M,Nk,causal", [(b, m, n, c) for c in (True, False) for b, m, n in (
+    (17, 4096, 4096), (19, 4096, 4096), (24, 4096, 4096), (32, 4096, 4096), (100, 4096, 4096), (1, 131072, 131072), (5000, 32, 900),
+    (60000, 64, 100), (9000, 96, 96), (9000, 128, 128), (30000, 170, 400), (3000, 333, 1000))])
+def test_many_rounds_are_looked_at_in_full(B, M, Nk, causal):
+    one, three = _busiest(B, M, Nk, causal, 1, 296), _busiest(B, M, Nk, causal, 3, 148)
+    assert plan(B, M, Nk, causal=causal)[0] == (3 if 5 * three < 4 * one else 2), (one, three)
+
+
 def test_bad_sizes_are_refused():
     out = (C.c_int32 * 4)()
     for args in ((1, 32, 8, 10, 9, 64, 1, 148), (1, 32, 7, 9, 9, 64, 1, 148), (1, 32, 8, 9, 9, 96, 1, 148), (1, 32, 8, 9, 9, 64, 1, 0)):
