@@ -274,9 +274,9 @@ __device__ __forceinline__ void arrive_if(uint32_t bar, bool yes) {
   asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %1, 0;\n\t@q mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar), "r"((uint32_t)yes)
                : "memory");
 }
-// The row threads' loop is longer than what a scheduler keeps of its instructions, so every taken branch in it waits for
-// an instruction fetch, some forty clocks: waits that find their phase complete, which most do, run straight on, and
-// what is rare stands out of line.  (A tile that has its SM to itself, 128 queries behind 3968 tokens, us with the slow paths in
+// Waits that find their phase complete, which most do, run straight on, and what is rare stands out of line: by device clocks a taken
+// branch in the row threads' loop costs some forty of them.  (The loop is longer than what a scheduler keeps of its instructions, so
+// an instruction fetch is the likely reason; no counter was taken of it.)  (A tile that has its SM to itself, 128 queries behind 3968 tokens, us with the slow paths in
 // the loop and so: head dim 64 42.2 / 38.4, 128 50.8 / 44.8; 777 queries behind 2223 tokens, two sequences, head dim 128 78.6 / 70.1.)
 __device__ __noinline__ bool wait_cold(const Params& p, int32_t* abort_flag, uint32_t bar, uint32_t parity, int code, int aux) {
   return __all_sync(0xffffffffu, wait_bar(p, abort_flag, bar, parity, code, aux));
@@ -340,9 +340,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   // down, so that under a causal mask the tiles with the most KV tiles start first and the short ones fill the
   // tail (longest job first).
   // The tile's 128 rows are 128 / pack queries of `pack` heads that share a KV head: a prompt of 777 queries and four
-  // heads a KV head is 25 tiles, not 4 x 7, and fewer pairs lie behind the diagonal (32 / 8 heads, causal, us before and
-  // after: 2190 x 2190 head dim 128 45.2 / 40.5, 64 39.6 / 35.5; 1960 of 2045, four sequences, 159.5 / 146.6 and
-  // 133.2 / 118.3; 4096 x 4096 128.3 / 125.5 and 107.2 / 103.7).
+  // heads a KV head is 25 tiles, not 4 x 7, and fewer pairs lie behind the diagonal (32 / 8 heads, causal, us with one head a
+  // tile and four: 2190 x 2190 head dim 128 50.6 / 46.3, 64 39.4 / 35.5; 1960 of 2045, four sequences, 170.4 / 156.2 and 120.5 / 106.5;
+  // 4096 x 4096 137.8 / 135.7 and 95.9 / 94.4).
   const int h0 = blockIdx.x * p.pack, b = blockIdx.y;
   const int kvh = h0 / (p.H / p.Hkv);
   const int tile_m = kBM >> p.pack_log2;
@@ -432,6 +432,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     }
   } else if (warp >= 4 * T) {
     // products of tile i, in the order S(0), S(1), P V(0), S(2), P V(1), ...
+    // (By the whole warp at head dim 128 as well.  us, one lane that waits and issues / the warp, causal: 512 x 512 11.7 / 10.7, 300 behind 1700
+    // tokens 30.3 / 26.0, 2190 x 2190 50.7 / 49.9, 4096 x 4096 153.2 / 149.7, no mask 311 / 271.)
     // (the tile, and with it every descriptor, is known to be uniform: see tc_mma)
     const int i = T == 1 ? 0 : __shfl_sync(0xffffffffu, warp - 4 * T, 0), nt = kv_tiles(i);
     const uint32_t id_s = idesc_bf16(kBN, false) | p.negate_q, id_o = idesc_bf16(D, true), elected = elect_one() ? 1u : 0u;
@@ -488,7 +490,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     const int m = first_row(ti) + (row >> p.pack_log2), h = h0 + (row & (p.pack - 1));
     const int lim = p.causal ? (p.N - p.M + m) : (p.N - 1);   // last visible token of this row
     // Only the tiles on the causal diagonal and the last one of a ragged cache need the per-score mask; the first n_open
-    // do not.  They take another mix of exponentials (see p_pass), so which they are is a matter of results: it goes by
+    // do not.  They take another mix of exponentials (exp2_poly2), so which they are is a matter of results: it goes by
     // blocks of 32 queries, whatever the heads in a tile.  (Every row of a warp is in one block.)
     const int n_open = min(p.causal ? p.N - p.M + (m & ~31) + 1 : p.N, p.N) / kBN;
     const uint32_t lane_addr = tmem + (uint32_t)ti * F::kTileCols + ((uint32_t)(qd * 32) << 16);
@@ -830,15 +832,14 @@ int mk_flash_prefill_bf16(const void* q, const void* k, const void* v, void* o, 
   p.negate_q = scale < 0.f ? 1u << 13 : 0u;
   p.timeout_ns = (uint64_t)(timeout_ms > 0 ? timeout_ms : 1000) * 1000000ull;
   const dim3 grid(H / pack, B, (pl.row_tiles + T - 1) / T);
-  // Where this grid leaves slots empty (two CTAs an SM), the next one is let in late: its CTAs would pile up on the
-  // SMs that are free now (causal, 32 / 8 heads, head dim 64, early / late: 777 x 777, 200 tiles 12.1 us / 11.2, 1024 x 1024,
-  // 256 tiles 16.3 / 13.5).  With the slots taken several times over it makes no difference up to 62 us a pass (2048 x 2048
-  // to two sequences of 2045), then early is 0.7 % faster (4096 x 4096 109.7 / 110.4); just above one round late would
-  // still be the better one (1185 x 1185, 304 tiles 18.5 / 16.0, 1500 x 1500, 376 tiles 22.2 / 20.4).  At 128 early is 1 to 3 %
-  // faster between one and a half rounds and three (2048 x 2048 36.9 / 37.3, 2190 x 2190 41.0 / 42.4), late below (1600 x 1600 28.1 / 26.8)
-  // and, by the power it takes, above (4096 x 4096 148.4 / 146.0 back to back).
+  // Where this grid leaves slots empty (two CTAs an SM), the next one is let in late: its CTAs would pile up on the SMs that are
+  // free now (us back to back, causal, 32 / 8 heads, early / late: head dim 64 777 x 777, 200 tiles 12.6 / 10.9, 1024 x 1024, 256 tiles 16.7 /
+  // 13.6; 128 1024 x 1024 20.4 / 16.7).  Just above one round late is still the better one, at head dim 64 by more than the rule takes (1185 x
+  // 1185, 304 tiles 19.1 / 16.8, 1500 x 1500, 376 tiles 22.7 / 20.4; 128 1600 x 1600, 400 tiles 29.3 / 28.0).  From one and a half rounds on
+  // early is up to 1.5 % faster (64 2048 x 2048 31.7 / 31.9, 2400 x 2400 41.2 / 41.7; 128 2048 x 2048 41.4 / 41.8, 2190 x 2190 46.9 / 47.6), from
+  // three on neither by more than the runs differ (128 3000 x 3000 78.7 / 79.7, 4096 x 4096 137.0 / 137.2, four sequences of 2048 154.5 / 153.1).
   const int64_t sms = d->sms;
-  p.next_early = !pl.three && (D == 64 ? pl.tiles >= 2 * sms : pl.tiles > 3 * sms && pl.tiles < 6 * sms) ? 1 : 0;
+  p.next_early = !pl.three && (D == 64 ? pl.tiles >= 2 * sms : pl.tiles > 3 * sms) ? 1 : 0;
   // the kernel may be placed while the one before it in the stream drains (it waits before it touches memory)
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
