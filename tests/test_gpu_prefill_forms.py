@@ -10,6 +10,7 @@ import torch
 
 from machete_b200 import _native as N
 from machete_b200.kernels.attention import flash_prefill
+from tests import test_gpu_launch_overlap as overlap
 from tests.test_gpu_prefill_attention import _reference
 from tests.util import assert_parity
 
@@ -71,3 +72,31 @@ def test_scales_of_either_sign_and_none(D, B, M, Nk, causal, scale):
     assert_parity(o, want, f"scale {scale}")
     # (fp32 products of D terms of size 1, scaled: a few 2^-24 of the largest score, some 40 * 3)
     assert float((lse.double() - want_lse).abs().max()) < 2e-3
+
+
+@pytest.mark.parametrize("B,M,Nk", [(2, 777, 2000), (5, 1100, 3100)])
+@pytest.mark.parametrize("falling", [False, True])
+def test_row_maxima_that_keep_growing_in_three_tiles(B, M, Nk, falling):
+    # every KV tile raises the exponent reference of every row (or of every other query's, beside rows that keep theirs): O is
+    # rescaled while the other tiles' products run.  Tolerance: as for the same values in the form of one tile
+    H, Hkv = (32, 8) if B == 2 else (8, 8)
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert _form(B, H, Hkv, M, Nk, True)[0] == 3
+    g = torch.Generator(device="cuda").manual_seed(M + falling)
+    q = torch.ones(B, H, M, 64, device="cuda").to(BF)
+    if falling:
+        q[:, :, 1::2] = -1
+    k = (torch.arange(Nk, device="cuda")[None, None, :, None] / 16 + torch.rand(B, Hkv, Nk, 64, generator=g, device="cuda")).to(BF)
+    v = torch.randn(B, Hkv, Nk, 64, generator=g, device="cuda").to(BF)
+    o = torch.full_like(q, 7.0)
+    for _ in range(3):
+        flash_prefill(q, k, v, o, causal=True, check_status=True)
+        for b in range(B):
+            assert_parity(o[b:b + 1], _reference(q[b:b + 1], k[b:b + 1], v[b:b + 1], True)[0], f"growing maxima, sequence {b}")
+
+
+def test_three_tiles_a_cta_between_other_kernels():
+    # all of an SM's tensor memory is taken and given back between kernels that start early
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert _form(1, overlap.HEADS, overlap.KV_HEADS, 8100, 8100, True)[0] == 3
+    overlap.test_a_chain_of_kernels_sees_what_the_one_before_it_wrote(8100, 64)

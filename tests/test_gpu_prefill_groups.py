@@ -29,7 +29,7 @@ def test_packed_heads(D, layout, H, Hkv, M, N):
     assert float((lse.double() - want_lse).abs().max()) < 2e-3
 
 
-# 148 SMs: two CTAs each up to 296 tiles of 32 queries x 4 heads, three up to 444, two again above
+# 148 SMs: 296 tiles of 32 queries x 4 heads are two each, 444 three; which form a count takes goes by its KV tiles
 @pytest.mark.parametrize("batch,M,N", [(1, 1184, 1184), (1, 1185, 1200), (2, 700, 1000), (2, 864, 900), (2, 897, 900)])
 def test_tile_counts_at_the_edges_of_the_two_forms(batch, M, N):
     g = torch.Generator(device="cuda").manual_seed(M)

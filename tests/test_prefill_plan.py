@@ -1,4 +1,4 @@
-"""How prompt attention is cut (CPU): three CTAs an SM only where the second round of two an SM would be the longer way."""
+"""How prompt attention is cut (CPU): three tiles a CTA only where the busiest SM then has less to do."""
 
 import ctypes as C
 
@@ -39,6 +39,11 @@ def test_edges_of_the_window():
                                                 (1, 3000, 3000, False, 3), (2, 4096, 4096, True, 3)])
 def test_several_rounds(B, M, Nk, causal, form):
     assert plan(B, M, Nk, causal=causal)[0] == form and plan(B, M, Nk, causal=causal)[3] > 444
+
+
+def test_sequences_together_and_by_themselves():
+    # what tests/test_gpu_prefill_forms.py compares bit for bit
+    assert plan(2, 777, 3000)[0] == 3 and plan(1, 777, 3000)[0] == 2
 
 
 def _busiest(B, M, Nk, causal, group, slots):
