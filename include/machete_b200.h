@@ -390,6 +390,10 @@ typedef struct mk_launch {
  * `smem_optin` bytes of shared memory a CTA; pointers in the program are not followed but for its tables. */
 int mk_launch_plan(mk_handle_t h, mk_launch_t* out, int32_t max);
 int mk_plan_launches(const mk_program_t* prog, int32_t num_sms, int32_t smem_optin, mk_launch_t* out, int32_t max);
+/* Where launch number `launch` of mk_plan_launches, a matvec launch, keeps what in a CTA's shared memory: out[0] partial sums,
+ * [1] rows, [2] ring; [3] bytes of a ring slot, [4] slots, [5] pages requested before the rows are staged; [6] the norm's weights and
+ * [7] the residual rows until then, counted from the ring, or -1 where they are read from global memory. */
+int mk_plan_staging(const mk_program_t* prog, int32_t num_sms, int32_t smem_optin, int32_t launch, int32_t out[8]);
 /* Where a matvec launch with a ring of `stages` slots puts a CTA's page, counted from 0: out[0] the slot, out[1] the pages in
  * that slot before it. */
 int mk_ring_place(int32_t stages, int64_t page, int32_t out[2]);

@@ -126,7 +126,7 @@ PREFILL_CALL = struct.Struct("<8Q13qd8i")
 
 EXPORTS = [
     "mk_abi_version", "mk_last_error", "mk_device_info", "mk_workspace_bytes", "mk_create", "mk_run", "mk_launches_per_run",
-    "mk_launch_plan", "mk_plan_launches", "mk_ring_place",
+    "mk_launch_plan", "mk_plan_launches", "mk_plan_staging", "mk_ring_place",
     "mk_status", "mk_workspace_status", "mk_set_trace", "mk_reset", "mk_launch_count", "mk_state_placement", "mk_set_launch_count",
     "mk_update_op", "mk_read_counters", "mk_destroy",
     "mk_standalone_workspace_bytes", "mk_matvec_bf16", "mk_matvec_nvfp4", "mk_flash_decode",
@@ -189,6 +189,7 @@ def _declare(h: C.CDLL) -> None:
     h.mk_launches_per_run.argtypes = [vp]
     h.mk_launch_plan.argtypes = [vp, C.POINTER(Launch), i32]
     h.mk_plan_launches.argtypes = [C.POINTER(Program), i32, i32, C.POINTER(Launch), i32]
+    h.mk_plan_staging.argtypes = [C.POINTER(Program), i32, i32, i32, C.POINTER(i32)]
     h.mk_ring_place.argtypes = [i32, C.c_int64, C.POINTER(i32)]
     h.mk_status.argtypes = [vp, C.POINTER(i32)]
     h.mk_workspace_status.argtypes = [vp, C.POINTER(i32)]

@@ -997,13 +997,14 @@ int mk_launch_plan(mk_handle_t h, mk_launch_t* out, int32_t max) {
   return guarded([&] { return tell_launches(current_plan(h)->steps, h->ops, out, max); });
 }
 
-static int plan_launches(const mk_program_t* prog, int32_t num_sms, int32_t smem_optin, mk_launch_t* out, int32_t max) {
+static int plan_steps(const mk_program_t* prog, int32_t num_sms, int32_t smem_optin, std::vector<mk_op_t>* at, std::vector<mk::ChainStep>* steps) {
   using namespace mk;
-  if (num_sms < 1 || smem_optin < 1 || (max > 0 && !out)) return fail(-1, "bad argument");
+  if (num_sms < 1 || smem_optin < 1) return fail(-1, "bad argument");
   int smem_bytes = 0;
   const int rc = validate_program(prog, smem_optin, num_sms, &smem_bytes);
   if (rc) return rc;
-  std::vector<mk_op_t> ops(prog->ops, prog->ops + prog->n_ops);
+  std::vector<mk_op_t>& ops = *at;
+  ops.assign(prog->ops, prog->ops + prog->n_ops);
   for (mk_op_t& op : ops) fill_derived(op);
   ProgramView pv;
   memset(&pv, 0, sizeof(pv));
@@ -1014,13 +1015,35 @@ static int plan_launches(const mk_program_t* prog, int32_t num_sms, int32_t smem
   pv.pos_count = prog->position_count > 0 ? prog->position_count : 1;
   const ChainTables tables = read_chain_tables(prog);
   set_windows(ops, tables, prog->position_limit);
-  std::vector<ChainStep> steps;
-  if (!(prog->flags & MK_PROG_SINGLE_LAUNCH)) build_chain(ops, tables, pv, nullptr, num_sms, smem_optin, &steps);
-  return tell_launches(steps, ops, out, max);
+  if (!(prog->flags & MK_PROG_SINGLE_LAUNCH)) build_chain(ops, tables, pv, nullptr, num_sms, smem_optin, steps);
+  return 0;
 }
 
 int mk_plan_launches(const mk_program_t* prog, int32_t num_sms, int32_t smem_optin, mk_launch_t* out, int32_t max) {
-  return guarded([&] { return plan_launches(prog, num_sms, smem_optin, out, max); });
+  using namespace mk;
+  return guarded([&] {
+    std::vector<mk_op_t> ops;
+    std::vector<ChainStep> steps;
+    if (max > 0 && !out) return fail(-1, "bad argument");
+    const int rc = plan_steps(prog, num_sms, smem_optin, &ops, &steps);
+    return rc ? rc : tell_launches(steps, ops, out, max);
+  });
+}
+
+int mk_plan_staging(const mk_program_t* prog, int32_t num_sms, int32_t smem_optin, int32_t launch, int32_t out[8]) {
+  using namespace mk;
+  return guarded([&] {
+    std::vector<mk_op_t> ops;
+    std::vector<ChainStep> steps;
+    if (!out) return fail(-1, "bad argument");
+    const int rc = plan_steps(prog, num_sms, smem_optin, &ops, &steps);
+    if (rc) return rc;
+    if (launch < 0 || launch >= (int)steps.size() || steps[launch].what.kind != MK_LAUNCH_MATVEC) return fail(-1, "mk_plan_staging: no such matvec launch");
+    const MvLaunch& l = *static_cast<const MvLaunch*>(steps[launch].params.get());
+    const int32_t v[8] = {l.slot_off, l.act_off, l.page_off, l.page_bytes, l.stages, l.ahead, l.norm_off, l.res_off};
+    memcpy(out, v, sizeof(v));
+    return 0;
+  });
 }
 
 int mk_ring_place(int32_t stages, int64_t page, int32_t out[2]) {
