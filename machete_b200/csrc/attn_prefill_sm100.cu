@@ -276,8 +276,9 @@ __device__ __forceinline__ void arrive_if(uint32_t bar, bool yes) {
 }
 // Waits that find their phase complete, which most do, run straight on, and what is rare stands out of line: by device clocks a taken
 // branch in the row threads' loop costs some forty of them.  (The loop is longer than what a scheduler keeps of its instructions, so
-// an instruction fetch is the likely reason; no counter was taken of it.)  (A tile that has its SM to itself, 128 queries behind 3968 tokens, us with the slow paths in
-// the loop and so: head dim 64 42.2 / 38.4, 128 50.8 / 44.8; 777 queries behind 2223 tokens, two sequences, head dim 128 78.6 / 70.1.)
+// an instruction fetch is the likely reason; no counter was taken of it.  us with the slow paths in the loop and so: a tile that
+// has its SM to itself, 128 queries behind 3968 tokens, head dim 64 42.2 / 38.4, 128 50.8 / 44.8; 777 queries behind 2223 tokens, two
+// sequences, head dim 128 78.6 / 70.1.)
 __device__ __noinline__ bool wait_cold(const Params& p, int32_t* abort_flag, uint32_t bar, uint32_t parity, int code, int aux) {
   return __all_sync(0xffffffffu, wait_bar(p, abort_flag, bar, parity, code, aux));
 }
