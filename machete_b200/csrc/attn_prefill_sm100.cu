@@ -275,10 +275,10 @@ __device__ __forceinline__ void arrive_if(uint32_t bar, bool yes) {
                : "memory");
 }
 // Waits that find their phase complete, which most do, run straight on, and what is rare stands out of line: by device clocks a taken
-// branch in the row threads' loop costs some forty of them.  (The loop is longer than what a scheduler keeps of its instructions, so
-// an instruction fetch is the likely reason; no counter was taken of it.  us with the slow paths in the loop and so: a tile that
-// has its SM to itself, 128 queries behind 3968 tokens, head dim 64 42.2 / 38.4, 128 50.8 / 44.8; 777 queries behind 2223 tokens, two
-// sequences, head dim 128 78.6 / 70.1.)
+// branch in the row threads' loop costs some forty of them.  (With the slow paths in the loop and so, us: a tile that has its SM to
+// itself, 128 queries behind 3968 tokens, head dim 64 42.2 / 38.4, 128 50.8 / 44.8; 777 queries behind 2223 tokens, two sequences, head
+// dim 128 78.6 / 70.1.  Of the lone tile at 128, ncu, stalled warps an issue: fixed latencies 2.47 / 1.96, long scoreboard 1.19 / 1.03, branches
+// being resolved 0.56 / 0.46, no instruction 0.30 / 0.27: it is the branches' own latency more than the fetch behind them.)
 __device__ __noinline__ bool wait_cold(const Params& p, int32_t* abort_flag, uint32_t bar, uint32_t parity, int code, int aux) {
   return __all_sync(0xffffffffu, wait_bar(p, abort_flag, bar, parity, code, aux));
 }

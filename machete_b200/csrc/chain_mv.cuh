@@ -1119,7 +1119,7 @@ __global__ void __launch_bounds__(kChainThreads<W>, ROWS <= 8 && W == 8 ? 2 : 1)
   float4* slots = reinterpret_cast<float4*>(smem + L.slot_off);
   // Groups of AS warps take the CTA's partial sums in turn (dealt out), or its units, and walk straight from one of their pages
   // to the next.  Looking at all pages for those that are its own cost a warp some 1500 clocks between two pages of 4000
-  // clocks of products (NVFP4 1 x 4096 -> 14336), by device clocks, likely as taken branches wait for instructions: 8B NVFP4 step us batch 1 2255 ->
+  // clocks of products (NVFP4 1 x 4096 -> 14336), by device clocks: 8B NVFP4 step us batch 1 2255 ->
   // 2194, batch 8 3516 -> 3410, 1B shape batch 16 1185 -> 1165.  (Aligned groups: with one warp more from unit to unit, so
   // that the one that adds a unit up sits the next one out, 2233, 3487 and 1190.)
   constexpr int G = W / AS;
